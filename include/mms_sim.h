@@ -53,9 +53,11 @@ extern "C" {
                                      pass the same flags to the workspace query  */
 #define MMS_FLAG_CROWDED 8u       /* a hint, results do not depend on it: another
                                      launch is expected to fill most of the GPU
-                                     while this one repairs its chunks, so its
-                                     repairs stay packed 32 to a warp unless only
-                                     a handful are left                          */
+                                     while this one repairs its chunks               */
+#define MMS_FLAG_NO_TWINS 16u     /* a hint, results do not depend on it: do not look for
+                                     interchangeable groups.  For lists whose placements
+                                     have none (saves the bookkeeping); pass the same
+                                     flags to the workspace query                    */
 
 /* The request trace: what controller.py:323-339 caches per Workload
  * (model_ids, slos) plus Workload.arrivals (simulator/workload.py:272). */
@@ -104,24 +106,18 @@ typedef struct {
  *  With MMS_FLAG_LEGACY_CLOCK: S == 2 and latency[m][c] = {sum, max} of
  *  controller.py:440-441, every group has 1 stage.
  *
- * Mirrors (optional, a speed-up only; nothing in the reference corresponds).
- * Groups with the same parallel config and the same models are
+ * Mirrors.  Groups with the same parallel config and the same models are
  * interchangeable, and a chunk simulated speculatively (see mms_sim_options)
- * often comes out with their roles permuted, which the exact chain pass
- * then has to re-simulate.  The caller may append, behind the num_scored
- * candidates it wants results for, MIRROR candidates: a copy of a scored
- * candidate's tables whose speculative chunks start with the clock vectors
- * of some groups exchanged.  The chain pass takes each chunk from the
- * candidate's own run or from one of its mirrors', whichever started from a
- * state equivalent to the true one, so results stay exact.
+ * often comes out with their roles exchanged.  The library finds such groups
+ * itself and takes such a run over under other labels; MIRROR candidates
+ * (copies of a candidate's tables behind the num_scored ones the caller
+ * wants results for) are accepted, checked and not used.
  *   num_scored   candidates [0, num_scored) get outputs (every output array
  *                has num_scored rows); 0 means all
  *   partner      i32[B] or NULL: for a scored candidate its first mirror (or
- *                -1), for a mirror the candidate it mirrors; the mirrors of
- *                one candidate are consecutive
+ *                -1), for a mirror the candidate it mirrors
  *   mirror_swap  u32[B][2] or NULL: for a mirror, up to four exchanges of two
- *                groups, applied in order; each is two bytes (group ids a, b),
- *                0xFF = unused
+ *                groups
  */
 typedef struct {
     int32_t num_candidates;        /* B */
@@ -151,9 +147,9 @@ typedef struct {
 typedef struct {
     int32_t chunk_requests;
     int32_t warmup_requests;
-    int32_t repair_rounds;         /* validate+repair rounds before the chain pass (0 = default) */
-    int32_t repair_segments;       /* segments (of 1024 requests) one repair may run per round;
-                                      it goes on in the next round (0 = default, <0 = no cap) */
+    int32_t repair_rounds;         /* rounds of parallel repairs before the last, serial pass (0 = default) */
+    int32_t repair_segments;       /* accepted, without effect: a repair runs until a stored run
+                                      can take over                                        */
 } mms_sim_options;
 
 /* How numpy sums N doubles (pairwise, blocks of <= 128, eight interleaved

@@ -32,6 +32,7 @@ FLAG_PER_REQUEST = 1
 FLAG_LEGACY_CLOCK = 2
 FLAG_NO_GROUP_GOOD = 4
 FLAG_CROWDED = 8
+FLAG_NO_TWINS = 16
 
 STATIC_SCRATCH_BYTES = 32 << 20
 
@@ -142,7 +143,7 @@ def host_lib():
             H.mms_host_configs.restype = ctypes.c_int64
             H.mms_host_configs.argtypes = [_vp, ctypes.c_int64, _vp, ctypes.c_int64, _vp]
             H.mms_host_encode.restype = ctypes.c_int
-            H.mms_host_encode.argtypes = [ctypes.c_int64] * 4 + [_vp] * 14 + [ctypes.c_int64]
+            H.mms_host_encode.argtypes = [ctypes.c_int64] * 4 + [_vp] * 15 + [ctypes.c_int64]
             _host = H
     return _host
 

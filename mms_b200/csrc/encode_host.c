@@ -271,7 +271,8 @@ static uint64_t mix64(uint64_t x)
  * groups ascending; *n_twin_items = n.  A placement whose classes can be
  * permuted in more than max_perms ways (the product of the factorials of
  * their sizes) is left out: it gets no mirror candidates anyway, and early in
- * a search nearly every placement is one.  counts is scratch of M + 1 entries,
+ * a search nearly every placement is one.  has_twins[b] tells of every placement whether it
+ * has such groups at all.  counts is scratch of M + 1 entries,
  * mark of M.  Unused cells of the tables must come zeroed.
  * Returns 0, or 1 when a model id is outside [0, M). */
 struct encode_ctx {
@@ -282,6 +283,7 @@ struct encode_ctx {
     uint32_t *model_rep, *group_info;
     int64_t *slots;
     int32_t *twin_items;
+    uint8_t *has_twins;
     int64_t max_perms;
 };
 
@@ -341,6 +343,7 @@ static int encode_range(const struct encode_ctx *c, int64_t b0, int64_t b1, int6
             slot += pp;
         }
         c->slots[b] = slot;
+        c->has_twins[b] = 0;
         /* interchangeable groups: same column, same set of models (non-empty) */
         if (ng <= 256) {
             int64_t first_of[256];                     /* start of each group's models */
@@ -375,6 +378,7 @@ static int encode_range(const struct encode_ctx *c, int64_t b0, int64_t b1, int6
                     done[h2] = 1;
                 }
                 if (found) {
+                    c->has_twins[b] = 1;
                     int64_t size = 0;
                     for (int64_t k = n_items - 1; k >= first_item && twin_items[3 * k + 1] == cls; --k)
                         ++size;
@@ -413,11 +417,11 @@ int mms_host_encode(int64_t B, int64_t M, int64_t G, int64_t P,
                     const int64_t *n_groups, const int64_t *cfg, const int32_t *cfg_index,
                     const int64_t *column_of, const int64_t *n_in_group, const int64_t *placed_model,
                     uint16_t *model_off, uint32_t *model_rep, uint32_t *group_info,
-                    int64_t *slots, int32_t *twin_items, int64_t *n_twin_items,
+                    int64_t *slots, int32_t *twin_items, int64_t *n_twin_items, uint8_t *has_twins,
                     int64_t *counts, int64_t *mark, int64_t max_perms)
 {
     struct encode_ctx ctx = {M, G, P, n_groups, cfg, column_of, n_in_group, placed_model, cfg_index,
-                             model_off, model_rep, group_info, slots, twin_items, max_perms};
+                             model_off, model_rep, group_info, slots, twin_items, has_twins, max_perms};
     /* placements are independent: a long list is cut into ranges, one thread each (the
      * caller holds the GIL; these threads touch no Python object) */
     int threads = mms_host_threads > 0 ? mms_host_threads : 4;

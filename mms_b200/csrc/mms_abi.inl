@@ -39,17 +39,35 @@ static int32_t plan_leaves(int64_t n)
 }
 
 struct Geometry {
-    int32_t K, NS, seg_len, seg_per_chunk, warmup, lat_smem_elems, rounds, repair_cap,
-        block_warps, narrow_limit, lat_f64;
-    size_t smem_stream, smem_repair;
+    int32_t K, NS, seg_len, seg_per_chunk, warmup, lat_smem_elems, rounds,
+        block_warps, lat_f64, window_blocks, win_table_elems;
+    bool window;
+    size_t smem_stream, smem_window;
     size_t off_leaf, off_seg_end, off_chunk_start, off_decisions, off_work_count, off_work_items,
-        off_repair_from, off_rows, off_seg_src, off_compat, off_seg_leaf, off_group_info,
-        off_own_rewritten;
+        off_rows, off_seg_leaf, off_group_info, off_columns, off_stamp, off_link, off_flags, off_rel,
+        off_tie, off_swaps, off_perm, off_twin_class, off_group_column, off_group_models;
+    int32_t group_words;
     size_t smem_count;        // shared memory of count_kernel
     size_t total;
 };
 
 static size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
+
+// Is the speculative pass of this batch faster with one candidate per warp than with 32?  A
+// warp of the former takes 0.15 to 0.2 us a request when it is alone on its scheduler and 0.4
+// us beside two others; a warp of the latter 0.5 us alone and 0.9 us beside eleven on its SM, but
+// for 32 candidates: one candidate per warp pays while the GPU is short of candidates.
+// Estimated microseconds of both.
+static bool window_pays(int64_t N, int64_t B, int64_t K_wide, int64_t K_win, int64_t warm, int sm_count)
+{
+    const double n_win = (double)N / K_win + (K_win > 1 ? warm : 0);
+    const double n_wide = (double)N / K_wide + (K_wide > 1 ? warm : 0);
+    const double warps_win = (double)B * K_win / (4.0 * sm_count);
+    const double t_win = n_win * (warps_win <= 1.0 ? 0.18 : 0.18 + 0.11 * (warps_win - 1.0));
+    double share = (double)((B + 31) / 32) * K_wide / (12.0 * sm_count);
+    if (share > 1.0) share = 1.0;
+    return t_win < n_wide * (0.5 + 0.4 * share);
+}
 
 // Chunking, shared-memory and scratch geometry of one call.
 static int plan_call(int64_t N, const mms_placements *c, const mms_sim_options *opts,
@@ -70,13 +88,13 @@ static int plan_call(int64_t N, const mms_placements *c, const mms_sim_options *
     if (mirrors && ((flags & MMS_FLAG_PER_REQUEST) || !c->partner || !c->mirror_swap))
         return MMS_ERR_ARG;
 
-    const int64_t B = c->num_candidates;
+    // mirrors are accepted and not needed any more
+    const int64_t B = c->num_scored ? c->num_scored : c->num_candidates;
     // blocks that fit an SM at once, from the kernel's shared-memory use
     const size_t lat_elems0 = (size_t)c->num_models * c->num_columns * c->max_stages + 8;
     const int lat_on_chip0 = (c->latency_stride == 0 && lat_elems0 * sizeof(float) <= (size_t)kLatSmemBytes)
                                  ? (int)lat_elems0 : 0;
-    const SmemLayout L0 = smem_layout(c->num_models, c->max_groups, c->max_placed, c->max_slots,
-                                      c->max_stages, group_good, lat_on_chip0);
+    const SmemLayout L0 = smem_layout(c->max_slots, c->max_stages, lat_on_chip0);
     int sm_count = 148, dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess ||
         cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
@@ -104,42 +122,70 @@ static int plan_call(int64_t N, const mms_placements *c, const mms_sim_options *
     // no resident warp.
     g->lat_f64 = 0;
     if (lat_on_chip0) {
-        const SmemLayout L64 = smem_layout(c->num_models, c->max_groups, c->max_placed,
-                                           c->max_slots, c->max_stages, group_good, lat_on_chip0,
-                                           true);
+        const SmemLayout L64 = smem_layout(c->max_slots, c->max_stages, lat_on_chip0, true);
         int64_t per_sm64;
         int block_warps64;
         fit(L64, per_sm64, block_warps64);
         if (per_sm64 >= per_sm) { g->lat_f64 = 1; block_warps = block_warps64; }
     }
     const int64_t resident_slots = (int64_t)sm_count * per_sm;
-    int64_t chunk = opts ? opts->chunk_requests : 0;
+    // the window kernels: blocks resident on an SM, from their shared memory (the table as
+    // doubles) and their register budget
+    size_t table = window_table_elems(c->num_models, c->num_columns, c->max_stages,
+                                      (flags & MMS_FLAG_LEGACY_CLOCK) != 0);
+    if (c->latency_stride != 0 || table * sizeof(double) > 2 * (size_t)kLatSmemBytes) table = 0;
+    g->win_table_elems = (int32_t)table;
+    g->smem_window = window_layout(c->max_slots, c->max_groups, c->max_stages, c->max_placed, table).total;
+    if (g->smem_window > 227 * 1024) return MMS_ERR_UNSUPPORTED;
+    int64_t window_per_sm = 233472 / (int64_t)(g->smem_window + 1024);
+    if (window_per_sm > kWindowBlocksPerSm) window_per_sm = kWindowBlocksPerSm;
+    g->window_blocks = (int32_t)(window_per_sm * sm_count);
+    const int64_t chunk = opts ? opts->chunk_requests : 0;
     int64_t warm = opts ? opts->warmup_requests : 0;
-    // segments: the unit of state snapshots and repairs
-    const int64_t seg = 1024;
-    const int64_t NS = N / seg > 0 ? N / seg : 1;
-    int64_t spc;                                   // segments per chunk
-    if (chunk < 0 || N < 8192 || B == 0) {
-        spc = NS;
-    } else if (chunk > 0) {
-        spc = (chunk + seg / 2) / seg;
-    } else {
-        // Chunks are the units of parallel work: as many as fill nine tenths
-        // of ONE wave of the resident warps (SMs x warps per SM at this
-        // kernel's shared-memory use; a second wave would pay the run-in
-        // twice), but never chunks shorter than 3 segments.  More chunks mean
-        // more boundaries to validate and repair.  The chunk length is that
-        // ideal rounded to the nearest number of segments, or the next longer
-        // one when the chunks would not fit the wave any more.
-        const int64_t lanes = resident_slots * kLanes;
-        spc = B > 0 ? (20 * NS * B + 9 * lanes) / (18 * lanes) : NS;      // round(NS / K_ideal)
-        if (spc < 3) spc = 3;
-        if (spc > NS) spc = NS;
-        if (B > 0 && ((NS + spc - 1) / spc) * B > lanes) spc += 1;
+    // Run-in: enough requests for every group to have had an idle moment and every replicated
+    // model a request.  Both grow with the cluster: of the boundaries of random placements at
+    // 0.8 to 2 requests a second and device, with 16 clock slots none fails behind 256
+    // requests, with 64 slots 5 % fail behind 1024 and 1.7 % behind 2048.
+    if (warm <= 0) {
+        warm = 32 * (int64_t)c->max_slots;
+        if (warm < 128) warm = 128;
+        if (warm > 2048) warm = 2048;
     }
-    if (spc < 1) spc = 1;
-    if (spc > NS) spc = NS;
-    const int64_t K = (NS + spc - 1) / spc;
+    // Segments are the unit of state snapshots and repairs, chunks (runs of segments) the unit
+    // of parallel work.  The 32-candidate kernel takes as many chunks as fill nine tenths of
+    // ONE wave of the resident warps (SMs x warps per SM at its shared-memory use; a second
+    // wave would pay the run-in twice), but none shorter than min_chunk.
+    struct Cut { int64_t seg, NS, spc, K; };
+    auto cut_trace = [&](int64_t seg, int64_t lanes, int64_t min_chunk) {
+        Cut x;
+        x.seg = seg;
+        x.NS = N / seg > 0 ? N / seg : 1;
+        if (chunk < 0 || N < 4 * seg || B == 0) {
+            x.spc = x.NS;
+        } else if (chunk > 0) {
+            x.spc = (chunk + seg / 2) / seg;
+        } else {
+            // the ideal length rounded to the nearest number of segments, or the next longer
+            // one when the chunks would not fit the wave any more
+            x.spc = (20 * x.NS * B + 9 * lanes) / (18 * lanes);
+            if (x.spc * seg < min_chunk) x.spc = (min_chunk + seg - 1) / seg;
+            if (x.spc < 1) x.spc = 1;
+            if (x.spc < x.NS && ((x.NS + x.spc - 1) / x.spc) * B > lanes) x.spc += 1;
+        }
+        if (x.spc < 1) x.spc = 1;
+        if (x.spc > x.NS) x.spc = x.NS;
+        x.K = (x.NS + x.spc - 1) / x.spc;
+        return x;
+    };
+    // segments of 128 requests where the snapshots are few (they are 8 bytes per clock slot,
+    // candidate and segment), of 1024 in the large batches
+    const int64_t seg = (double)N * (double)c->max_slots * (double)B * 8.0 / 128.0 <= 256e6 ? 128 : 1024;
+    const Cut wide = cut_trace(seg, resident_slots * kLanes, seg == 1024 ? 3 * seg : warm / 2);
+    const Cut win = cut_trace(seg, (int64_t)g->window_blocks * kWindowWarps, seg);
+    // Which speculative pass: see window_pays.
+    g->window = window_pays(N, B, wide.K, win.K, warm, sm_count);
+    const Cut &x = g->window ? win : wide;
+    const int64_t NS = x.NS, spc = x.spc, K = x.K;
     if (K * (B > 0 ? B : 1) >= 0x7FFFFFFFLL) return MMS_ERR_UNSUPPORTED;   // work-list encoding
     // A launch that fills less than half of the GPU goes out in smaller
     // blocks, one per SM: a warp that shares its SM with two others runs
@@ -152,55 +198,54 @@ static int plan_call(int64_t N, const mms_placements *c, const mms_sim_options *
         if (block_warps < 1) block_warps = 1;
     }
     g->block_warps = block_warps;
-    if (warm <= 0) warm = 2048;
     int rounds = opts ? opts->repair_rounds : 0;
     if (rounds <= 0) rounds = kDefaultRepairRounds;
     if (rounds > kMaxRepairRounds) rounds = kMaxRepairRounds;
-    int cap = opts ? opts->repair_segments : 0;
-    if (cap == 0) cap = kDefaultRepairSegments;
-    if (cap < 0) cap = 0;
-    g->rounds = rounds; g->repair_cap = cap;
-    g->K = (int32_t)K; g->NS = (int32_t)NS; g->seg_len = (int32_t)seg;
+    g->rounds = rounds;
+    g->K = (int32_t)K; g->NS = (int32_t)NS; g->seg_len = (int32_t)x.seg;
     g->seg_per_chunk = (int32_t)spc; g->warmup = (int32_t)warm;
 
     // the shared table goes on chip (f32), with 8 readable entries of padding
     const size_t lat_elems = (size_t)c->num_models * c->num_columns * c->max_stages + 8;
     g->lat_smem_elems = (c->latency_stride == 0 && lat_elems * sizeof(float) <= (size_t)kLatSmemBytes)
                             ? (int32_t)lat_elems : 0;
-    const SmemLayout L = smem_layout(c->num_models, c->max_groups, c->max_placed, c->max_slots,
-                                     c->max_stages, group_good, g->lat_smem_elems,
+    const SmemLayout L = smem_layout(c->max_slots, c->max_stages, g->lat_smem_elems,
                                      g->lat_smem_elems != 0 && g->lat_f64 != 0);
     g->smem_stream = L.warp0 + (size_t)g->block_warps * L.warp_bytes;
-    // ... the repair scratch, then the decoded-request records of the step that decodes ahead
-    g->smem_repair = staging_offset(L.total, c->max_slots, c->max_groups) + kStagedBytes;
-    if (g->smem_repair > 227 * 1024) return MMS_ERR_UNSUPPORTED;
     // the tally's per-lane histograms (count_kernel)
     g->smem_count = sizeof(uint32_t) * (size_t)(c->max_groups + (c->num_models + 1) / 2) * kLanes;
     if (g->smem_count > 227 * 1024) return MMS_ERR_UNSUPPORTED;
-    // one-chunk-per-warp repairs: as many as are resident at once (12 warps of
-    // this register use per SM, or what shared memory admits)
-    int64_t narrow_per_sm = 233472 / (int64_t)(g->smem_repair + 1024);
-    if (narrow_per_sm > 12) narrow_per_sm = 12;
-    g->narrow_limit = (int32_t)(narrow_per_sm * sm_count);
-    // beside a launch that holds most SMs for itself, what is left over takes few blocks
-    if ((flags & MMS_FLAG_CROWDED) && g->narrow_limit > 48) g->narrow_limit = 48;
-
     size_t off = 0;
     g->off_rows = off;        off += align256(2 * sizeof(uint32_t) * kRowWords * (size_t)((B + kLanes - 1) / kLanes * kLanes) *
                                                (c->num_models + 1) + 256);
     g->off_leaf = off;        off += align256(sizeof(double) * (size_t)plan_leaves(N) * B);
     g->off_decisions = off;   off += align256((c->max_groups > 126 ? 2 : 1) * (size_t)((N + 3) / 4 * 4 + 4) *
                                                (size_t)((B + 31) / 32 * 32));
-    g->off_work_count = off;  off += align256(sizeof(uint32_t) * (kMaxRepairRounds + 1));
-    g->off_repair_from = off; off += align256(sizeof(int32_t) * (size_t)K * B);
+    g->off_work_count = off;  off += align256(2 * sizeof(uint32_t) * kMaxRepairRounds);
     g->off_work_items = off;  off += align256(sizeof(uint32_t) * (size_t)K * B);
-    g->off_seg_src = off;     off += align256(sizeof(int32_t) * (size_t)NS * B);
-    g->off_compat = off;      off += align256(sizeof(uint16_t) * (size_t)K * B);
     g->off_seg_leaf = off;    off += align256(sizeof(int32_t) * (size_t)(NS + 1));
     g->off_group_info = off;  off += align256(sizeof(uint32_t) * (size_t)B * c->max_groups + 4);
-    g->off_own_rewritten = off; off += align256((size_t)K * B + 4);
-    g->off_seg_end = off;     off += K > 1 ? align256(sizeof(double) * (size_t)NS * c->max_slots * B) : 0;
-    g->off_chunk_start = off; off += K > 1 ? align256(sizeof(double) * (size_t)K * c->max_slots * B) : 0;
+    g->off_group_column = off; off += align256(sizeof(uint32_t) * (size_t)B * c->max_groups + 4);
+    g->off_columns = off;     off += align256(sizeof(uint32_t) * ((size_t)c->num_columns + 1));
+    g->off_flags = off;       off += align256(3 * (size_t)B + 4);      // relabelled, open, twins
+    g->group_words = 0;
+    if (K > 1) {
+        const size_t G = (size_t)c->max_groups;
+        g->off_stamp = off;        off += align256((size_t)K * B);
+        g->off_link = off;         off += align256((size_t)K * B);
+        g->off_rel = off;          off += align256((size_t)NS * B);
+        g->off_tie = off;          off += align256(sizeof(uint64_t) * (size_t)NS * B);
+        g->off_perm = off;         off += align256((size_t)NS * B * G + 4);
+        g->off_twin_class = off;   off += align256(sizeof(uint16_t) * (size_t)B * G + 4);
+        if (c->num_models <= kTwinModels && !(flags & MMS_FLAG_NO_TWINS))
+            g->group_words = (c->num_models + 63) / 64;
+        g->off_swaps = off;
+        if (g->group_words) off += align256(sizeof(uint32_t) * (size_t)((N + 3) / 4 * 4 + 4) * (size_t)((B + 31) / 32 * 32));
+        g->off_group_models = off;
+        off += align256(sizeof(uint64_t) * (size_t)B * G * (size_t)g->group_words + 8);
+        g->off_seg_end = off;     off += align256(sizeof(double) * (size_t)NS * c->max_slots * B);
+        g->off_chunk_start = off; off += align256(sizeof(double) * (size_t)K * c->max_slots * B);
+    }
     g->total = off;
     return MMS_OK;
 }
@@ -262,7 +307,7 @@ static int allow_smem(const void *func, size_t bytes)
         if (rc_ != MMS_OK) return rc_; \
     } while (0)
 
-template <bool kFull, bool kGroupGood, bool kLegacy>
+template <bool kFull, bool kLegacy>
 static int launch_sim(KernelArgs &ka, const ClearArgs &ca, const Geometry &g, cudaStream_t st)
 {
     // everything a call clears, then the tables its kernels read: two launches
@@ -277,45 +322,53 @@ static int launch_sim(KernelArgs &ka, const ClearArgs &ca, const Geometry &g, cu
         build_tables_kernel<<<(unsigned)blocks, 256, 0, st>>>(ka, ca);
         MMS_CUDA(cudaGetLastError());
     }
-    auto stream_k = sim_stream_kernel<kFull, kGroupGood, kLegacy>;
-    MMS_TRY(allow_smem((const void *)stream_k, g.smem_stream));
-    const int64_t per_block = (int64_t)kLanes * g.block_warps;
-    const int64_t streams = (int64_t)ka.B * ka.K;
+    if (ka.K > 1 && ca.group_words && ka.G > 0) {
+        const int64_t groups = (int64_t)ka.B * ka.G;
+        twins_kernel<<<(unsigned)((groups + 127) / 128), 128, 0, st>>>(ka, ca);
+        MMS_CUDA(cudaGetLastError());
+    }
     ProfileSpan stream_span(MMS_PROFILE_STREAM, st);
-    stream_k<<<(unsigned)((streams + per_block - 1) / per_block), (unsigned)per_block,
-               g.smem_stream, st>>>(ka);
+    const int64_t streams = (int64_t)ka.B * ka.K;
+    const auto window_blocks = [&](int64_t warps) {
+        const int64_t blocks = (warps + kWindowWarps - 1) / kWindowWarps;
+        return (unsigned)(blocks < g.window_blocks ? blocks : g.window_blocks);
+    };
+    if (g.window) {
+        auto stream_k = ka.swaps ? window_stream_kernel<kLegacy, true> : window_stream_kernel<kLegacy, false>;
+        MMS_TRY(allow_smem((const void *)stream_k, g.smem_window));
+        stream_k<<<window_blocks(streams), kWindowWarps * kLanes, g.smem_window, st>>>(ka);
+    } else {
+        auto stream_k = ka.swaps ? sim_stream_kernel<kFull, kLegacy, true> : sim_stream_kernel<kFull, kLegacy, false>;
+        MMS_TRY(allow_smem((const void *)stream_k, g.smem_stream));
+        const int64_t per_block = (int64_t)kLanes * g.block_warps;
+        stream_k<<<(unsigned)((streams + per_block - 1) / per_block), (unsigned)per_block,
+                   g.smem_stream, st>>>(ka);
+    }
     MMS_CUDA(cudaGetLastError());
     stream_span.stop();
     if (ka.K > 1) {
-        auto repair_k = sim_repair_kernel<kFull, kGroupGood, kLegacy, false>;
-        auto chain_k = sim_chain_kernel<kFull, kGroupGood, kLegacy, false>;
-        auto repair_narrow_k = sim_repair_kernel<kFull, kGroupGood, kLegacy, true>;
-        auto chain_narrow_k = sim_chain_kernel<kFull, kGroupGood, kLegacy, true>;
-        MMS_TRY(allow_smem((const void *)repair_k, g.smem_repair));
-        MMS_TRY(allow_smem((const void *)chain_k, g.smem_repair));
-        MMS_TRY(allow_smem((const void *)repair_narrow_k, g.smem_repair));
-        MMS_TRY(allow_smem((const void *)chain_narrow_k, g.smem_repair));
+        auto walk_k = ka.swaps ? walk_kernel<kLegacy, true> : walk_kernel<kLegacy, false>;
+        auto finish_k = ka.swaps ? finish_kernel<kLegacy, true> : finish_kernel<kLegacy, false>;
+        MMS_TRY(allow_smem((const void *)walk_k, g.smem_window));
+        MMS_TRY(allow_smem((const void *)finish_k, g.smem_window));
         const int64_t bounds = (int64_t)ka.B * (ka.K - 1);
-        for (int r = 0; r < g.rounds; ++r) {
+        const size_t link_smem = kLinkWarps * link_warp_bytes(ka.T, ka.G);
+        // round g.rounds only judges the boundaries, for finish_kernel
+        for (int r = 0; r <= g.rounds; ++r) {
             ka.round = r;
-            validate_kernel<<<(unsigned)((bounds + 127) / 128), 128, 0, st>>>(ka);
+            link_kernel<<<(unsigned)((bounds + kLinkWarps * kLanes - 1) / (kLinkWarps * kLanes)),
+                          kLinkWarps * kLanes, link_smem, st>>>(ka);
             MMS_CUDA(cudaGetLastError());
-            resolve_kernel<<<(unsigned)((ka.Bs + 3) / 4), 4 * kLanes, 0, st>>>(ka);
+            if (r == g.rounds) break;
+            resolve_kernel<<<(unsigned)((ka.B + 3) / 4), 4 * kLanes, 0, st>>>(ka);
             MMS_CUDA(cudaGetLastError());
             // sized for the worst case; blocks past the work list return at once
-            repair_k<<<(unsigned)((bounds + kLanes - 1) / kLanes), kLanes, g.smem_repair, st>>>(ka);
+            walk_k<<<window_blocks(bounds), kWindowWarps * kLanes, g.smem_window, st>>>(ka);
             MMS_CUDA(cudaGetLastError());
-            // the same list one chunk to a warp, when it is short (see sim_repair_kernel)
-            const int64_t narrow = bounds < ka.narrow_limit ? bounds : ka.narrow_limit;
-            if (narrow > 0) {
-                repair_narrow_k<<<(unsigned)narrow, kLanes, g.smem_repair, st>>>(ka);
-                MMS_CUDA(cudaGetLastError());
-            }
         }
         ProfileSpan chain_span(MMS_PROFILE_CHAIN, st);
-        chain_k<<<(unsigned)((ka.Bs + kLanes - 1) / kLanes), kLanes, g.smem_repair, st>>>(ka);
-        MMS_CUDA(cudaGetLastError());
-        chain_narrow_k<<<(unsigned)ka.Bs, kLanes, g.smem_repair, st>>>(ka);
+        finish_k<<<(unsigned)((ka.B + kWindowWarps - 1) / kWindowWarps), kWindowWarps * kLanes,
+                   g.smem_window, st>>>(ka);
         MMS_CUDA(cudaGetLastError());
         chain_span.stop();
     }
@@ -428,7 +481,7 @@ int mms_sim_mixed(const mms_trace *trace, const mms_placements *cands, const mms
     using namespace mms;
     if (!trace || !cands || !plan || !ws || !out) return MMS_ERR_ARG;
     if (flags & ~(MMS_FLAG_PER_REQUEST | MMS_FLAG_LEGACY_CLOCK | MMS_FLAG_NO_GROUP_GOOD |
-                  MMS_FLAG_CROWDED))
+                  MMS_FLAG_CROWDED | MMS_FLAG_NO_TWINS))
         return MMS_ERR_ARG;
     const int64_t N = trace->num_requests;
     const bool gg = !(flags & MMS_FLAG_NO_GROUP_GOOD);
@@ -436,15 +489,14 @@ int mms_sim_mixed(const mms_trace *trace, const mms_placements *cands, const mms
     Geometry g;
     int rc = plan_call(N, cands, opts, flags, gg, &g);
     if (rc) return rc;
-    const int32_t B = cands->num_candidates;
+    const int32_t B = cands->num_scored ? cands->num_scored : cands->num_candidates;
     if (B == 0) return MMS_OK;
     if (!out->model_num_requests || !out->model_num_good || !out->group_num_requests ||
         !out->good_total || !out->latency_sum || !out->status || !model_hist)
         return MMS_ERR_ARG;
     if (N > 0 && (!trace->arrivals || !trace->model_ids || !trace->slos)) return MMS_ERR_ARG;
     if (trace->num_traces < 0 || trace->num_traces > 0x7FFFFFFF) return MMS_ERR_ARG;
-    if (trace->num_traces > 1 &&
-        (cands->num_scored ? cands->num_scored : cands->num_candidates) > trace->num_traces)
+    if (trace->num_traces > 1 && B > trace->num_traces)
         return MMS_ERR_ARG;                 // every scored candidate needs a trace of its own
     if (!cands->model_off || !cands->group_info || !cands->model_rep || !cands->latency)
         return MMS_ERR_ARG;
@@ -464,8 +516,7 @@ int mms_sim_mixed(const mms_trace *trace, const mms_placements *cands, const mms
     ka.unsorted = trace->num_traces > 1
                       ? model_hist + (size_t)trace->num_traces * (cands->num_models + 1)
                       : model_hist + cands->num_models;
-    ka.B = B; ka.Bs = cands->num_scored ? cands->num_scored : B;
-    ka.partner = cands->partner; ka.mirror_swap = cands->mirror_swap;
+    ka.B = B;
     ka.M = cands->num_models; ka.G = cands->max_groups; ka.P = cands->max_placed;
     ka.T = cands->max_slots; ka.S = cands->max_stages; ka.C = cands->num_columns;
     ka.model_off = cands->model_off; ka.model_rep = cands->model_rep;
@@ -482,18 +533,18 @@ int mms_sim_mixed(const mms_trace *trace, const mms_placements *cands, const mms
     ka.dec_wide = cands->max_groups > 126;
     ka.dec_pitch = ((int64_t)B + 31) / 32 * 32;
     ka.work_count = (uint32_t *)(scratch + g.off_work_count);
+    ka.work_next = ka.work_count + kMaxRepairRounds;
     ka.work_items = (uint32_t *)(scratch + g.off_work_items);
-    ka.repair_from = (int32_t *)(scratch + g.off_repair_from);
-    ka.seg_src = (int32_t *)(scratch + g.off_seg_src);
-    ka.compat = (uint16_t *)(scratch + g.off_compat);
-    ka.own_rewritten = (uint8_t *)(scratch + g.off_own_rewritten);
+    ka.stamp = scratch + g.off_stamp; ka.link = scratch + g.off_link;
+    ka.relabelled = scratch + g.off_flags; ka.open = ka.relabelled + B;
+    ka.rel = scratch + g.off_rel; ka.tie = (uint64_t *)(scratch + g.off_tie); ka.perm = scratch + g.off_perm;
+    ka.swaps = g.group_words ? (uint32_t *)(scratch + g.off_swaps) : nullptr;
     ka.seg_first_leaf = (int32_t *)(scratch + g.off_seg_leaf);
-    ka.repair_cap = g.repair_cap;
-    ka.narrow_limit = g.narrow_limit;
+    ka.window = g.window;
     ka.seg_end = (double *)(scratch + g.off_seg_end);
     ka.chunk_start = (double *)(scratch + g.off_chunk_start);
     ka.status = out->status;
-    ka.finish = out->finish; ka.good = out->good;
+    ka.finish = full ? out->finish : nullptr; ka.good = full ? out->good : nullptr;
     ka.resimulated = out->resimulated;
 
     ClearArgs ca;
@@ -503,38 +554,39 @@ int mms_sim_mixed(const mms_trace *trace, const mms_placements *cands, const mms
     ca.group_num_requests = out->group_num_requests;
     ca.group_num_good = gg ? out->group_num_good : nullptr;
     ca.good_total = out->good_total;
+    ca.column_stages = (uint32_t *)(scratch + g.off_columns);
+    ca.irregular = ca.column_stages + cands->num_columns;
+    ca.group_words = g.group_words;
+    ca.group_models = (uint64_t *)(scratch + g.off_group_models);
+    ca.group_column = (uint32_t *)(scratch + g.off_group_column);
+    ca.twin_class = (uint16_t *)(scratch + g.off_twin_class); ca.twins = ka.open + B;
+    ka.group_column = ca.group_column;
+    ka.twin_class = ca.twin_class; ka.twins = ca.twins;
+    ka.column_stages = ca.column_stages; ka.irregular = ca.irregular;
+    ka.win_table_elems = g.win_table_elems;
     ka.group_info = ca.group_info;       // the checked copy, contested bits derived on the device
     ProfileSpan call_span(MMS_PROFILE_CALL, st);
     const bool legacy = (flags & MMS_FLAG_LEGACY_CLOCK) != 0;
-    const int variant = (full ? 4 : 0) | (gg ? 2 : 0) | (legacy ? 1 : 0);
-    switch (variant) {
-        case 0: rc = launch_sim<false, false, false>(ka, ca, g, st); break;
-        case 1: rc = launch_sim<false, false, true>(ka, ca, g, st); break;
-        case 2: rc = launch_sim<false, true, false>(ka, ca, g, st); break;
-        case 3: rc = launch_sim<false, true, true>(ka, ca, g, st); break;
-        case 4: rc = launch_sim<true, false, false>(ka, ca, g, st); break;
-        case 5: rc = launch_sim<true, false, true>(ka, ca, g, st); break;
-        case 6: rc = launch_sim<true, true, false>(ka, ca, g, st); break;
-        default: rc = launch_sim<true, true, true>(ka, ca, g, st); break;
-    }
+    if (full) rc = legacy ? launch_sim<true, true>(ka, ca, g, st) : launch_sim<true, false>(ka, ca, g, st);
+    else rc = legacy ? launch_sim<false, true>(ka, ca, g, st) : launch_sim<false, false>(ka, ca, g, st);
     if (rc) return rc;
 
-    // tally the recorded decisions of the selected runs (outputs were cleared up front)
+    // tally the recorded decisions (outputs were cleared up front)
     const size_t hist_bytes = g.smem_count;
     auto count_k = ka.dec_wide ? count_kernel<uint16_t> : count_kernel<uint8_t>;
     MMS_TRY(allow_smem((const void *)count_k, hist_bytes));
     int32_t seg_per_block = ka.NS / 96 > 0 ? ka.NS / 96 : 1;   // 16-bit counts: at most 32 segments
     if (seg_per_block > 32) seg_per_block = 32;
-    // one more row of blocks (the first) forms the latency sums
-    const dim3 count_grid((unsigned)((ka.Bs + kLanes - 1) / kLanes),
-                          (unsigned)((ka.NS + seg_per_block - 1) / seg_per_block) + 1);
+    // 32 more rows of blocks (the first) form the latency sums
+    const dim3 count_grid((unsigned)((ka.B + kLanes - 1) / kLanes),
+                          (unsigned)((ka.NS + seg_per_block - 1) / seg_per_block) + kLanes);
     count_k<<<count_grid, kLanes, hist_bytes, st>>>(ka, seg_per_block, gg, out->model_num_good,
                                                     out->group_num_requests, out->group_num_good,
                                                     out->good_total, plan->leaf_merges,
                                                     out->latency_sum);
     MMS_CUDA(cudaGetLastError());
     if (ka.M > 0) {
-        const int64_t cells = (int64_t)ka.Bs * ka.M;
+        const int64_t cells = (int64_t)ka.B * ka.M;
         model_requests_kernel<<<(unsigned)((cells + 127) / 128), 128, 0, st>>>(ka, out->model_num_requests);
         MMS_CUDA(cudaGetLastError());
     }
@@ -879,9 +931,10 @@ int mms_sim_batching(const mms_trace *trace, const mms_placements *cands,
     }
     KernelArgs fa;                         // what finalize_kernel reads; one run per candidate
     memset(&fa, 0, sizeof(fa));
-    fa.B = fa.Bs = B; fa.M = a.M; fa.num_leaves = plan->num_leaves;
+    fa.B = B; fa.M = a.M; fa.num_leaves = plan->num_leaves; fa.N = N;
+    fa.leaf_start = plan->leaf_start;
     fa.leaf_sums = leaf_sums; fa.status = out->status;
-    finalize_kernel<<<(B + 31) / 32, 32, 0, st>>>(
+    finalize_kernel<<<(B + 3) / 4, 4 * kLanes, 0, st>>>(
         fa, plan->leaf_merges, out->model_num_good, out->good_total, out->latency_sum);
     MMS_CUDA(cudaGetLastError());
     return MMS_OK;

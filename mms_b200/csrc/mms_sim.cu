@@ -10,39 +10,27 @@
 // comes from (a) the candidates of the batch and (b) cutting each candidate's
 // trace into chunks that are simulated SPECULATIVELY at the same time:
 //
-//   stream kernel   one thread per (candidate, chunk).  A chunk starts from
-//                   idle clocks a few thousand requests before its first
-//                   request (run-in, nothing recorded), stores the clock
-//                   vector it has when the chunk proper begins and after
-//                   every segment, and records its decisions and latency sums.
-//                   A MIRROR candidate (a copy of a candidate with
-//                   interchangeable groups) exchanges those groups' clocks
-//                   after the run-in: a second guess at the state.
-//   validate kernel one thread per stored run and chunk boundary: which
-//                   stored runs of the next chunk start from a state
-//                   EQUIVALENT to the one this run ended in
-//                   (states_equivalent: equal futures, provably)?
-//   resolve kernel  one warp per candidate follows the chain of chunks
-//                   through those answers; where no stored run continues
-//                   the chain, the true state is copied in and the chunk
-//                   goes on a work list.
-//   repair kernel   one thread per listed chunk re-simulates it from the true
-//                   state, segment by segment, until its state is equivalent
-//                   to what a stored run had at that point; the rest of the
-//                   chunk is taken from that run.  32 chunks to a warp, or,
-//                   for a short list, one (with a step that branches).
-//                   validate + resolve + repair run a few rounds (a repaired
-//                   chunk can end differently and invalidate its successor).
-//   chain kernel    one thread per candidate that is still unsettled walks
-//                   all boundaries in order and repairs in place whatever the
-//                   rounds left — it makes the result exact whatever the
-//                   chunking and the rounds.
-//   count kernel    tallies the recorded decisions of the selected runs into
-//                   the counters and combines the per-leaf latency sums in
-//                   numpy's pairwise order.
-//
-// The 32 lanes of a warp are 32 candidates on the same chunk (one broadcast
-// load per trace element) whenever the batch has 32 or more candidates.
+//   stream kernel   the speculative pass.  A chunk starts from idle clocks some
+//                   requests before its first one (run-in, nothing recorded), stores the
+//                   clock vector it has when the chunk proper begins and after
+//                   every segment, and records its decisions and latency sums.  Large
+//                   batches: one thread per (candidate, chunk), 32 candidates to a
+//                   warp (sim_stream_kernel); small ones: one warp (sim_window.cuh).
+//   link kernel     one thread per chunk boundary: does the chunk's run start from a state
+//                   EQUIVALENT to the one the run before it ended in (states_equivalent:
+//                   equal futures, provably), as it is or under other labels of
+//                   interchangeable groups (warp_relabel)?
+//   resolve kernel  one warp per candidate lists the chunks behind failed boundaries.
+//   walk kernel     one warp per listed chunk re-simulates it, and what follows, from the state
+//                   the chunk before it ended in until the stored run can take over.
+//                   link + resolve + walk run a few rounds (a walk that started from a
+//                   wrong state has to be done again).
+//   finish kernel   one warp per candidate that is still open, or has relabelled segments,
+//                   goes through them in order, re-simulates whatever the rounds
+//                   left and translates labels into group numbers — it makes the result exact
+//                   whatever the chunking and the rounds.
+//   count kernel    tallies the recorded decisions into the counters and combines the
+//                   per-leaf latency sums in numpy's pairwise order.
 #include <cuda_runtime.h>
 
 #include <cstdint>
@@ -53,17 +41,18 @@
 #include "mms_sim.h"
 #include "sim_batching.cuh"
 #include "sim_chunk.cuh"
+#include "sim_window.cuh"
 
 namespace mms {
 
 constexpr int kMaxSumDepth = 48;        // pair-sum stack of the numpy order
 constexpr int kLatSmemBytes = 32 * 1024;
 constexpr int kMaxRepairRounds = 16;
+constexpr int kTwinModels = 256;        // models a launch with interchangeable groups may have
 constexpr int kDefaultRepairRounds = 4;
-constexpr int kDefaultRepairSegments = -1;   // no cap: measured best on the benchmark shape
 
 // What a call clears before its kernels run, in one launch (grid-stride): the
-// work lists and run selections of the time-parallel machinery, the outputs
+// work lists and marks of the time-parallel machinery, the outputs
 // the tally adds into, the status words — and the kernels' own copy of
 // group_info, bounds-checked (a bad entry becomes an empty group) and with the
 // "contested" bit (bit 16) cleared: build_tables_kernel derives that bit from
@@ -71,10 +60,20 @@ constexpr int kDefaultRepairSegments = -1;   // no cap: measured best on the ben
 struct ClearArgs {
     const uint32_t *group_info_in;    // the caller's [B][G]
     uint32_t *group_info;             // scratch copy the kernels read
-    int32_t *model_num_good;          // [Bs][M]
-    int32_t *group_num_requests;      // [Bs][G]
-    int32_t *group_num_good;          // [Bs][G] or null
-    int64_t *good_total;              // [Bs]
+    int32_t *model_num_good;          // [B][M]
+    int32_t *group_num_requests;      // [B][G]
+    int32_t *group_num_good;          // [B][G] or null
+    int64_t *good_total;              // [B]
+    // for twins_kernel
+    int32_t group_words;              // 64-bit words of a group's model set; 0: too many models
+    uint64_t *group_models;           // [B][G][group_words]
+    uint32_t *group_column;           // [B][G] latency column of the group; 0xFFFFFFFF: no model
+    uint16_t *twin_class;             // see KernelArgs
+    uint8_t *twins;
+    uint32_t *column_stages;          // [C] stages of the groups that use the column
+    uint32_t *irregular;              // != 0: a column is used with different numbers of stages, a
+                                      //   replica's slots are not its group's, a group has several
+                                      //   columns, or a replica list is not in ascending group order
 };
 
 __device__ inline bool group_info_valid(const KernelArgs &a, uint32_t info)
@@ -87,26 +86,37 @@ __global__ void clear_kernel(const KernelArgs a, const ClearArgs c)
 {
     const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const int64_t nth = (int64_t)gridDim.x * blockDim.x;
-    for (int64_t i = tid; i < (int64_t)a.NS * a.B; i += nth) a.seg_src[i] = -1;
-    for (int64_t i = tid; i < (int64_t)a.K * a.B; i += nth) {
-        a.repair_from[i] = -1;
-        a.own_rewritten[i] = 0;
+    if (a.K > 1) {
+        for (int64_t i = tid; i < (int64_t)a.NS * a.B; i += nth) a.rel[i] = 0;
+        for (int64_t i = tid; i < (int64_t)a.K * a.B; i += nth) a.stamp[i] = 0;
+        for (int64_t i = tid; i < (int64_t)a.B * a.G; i += nth) {
+            for (int k = 0; k < c.group_words; ++k) c.group_models[i * c.group_words + k] = 0;
+        }
+        for (int64_t i = tid; i < a.B; i += nth) { c.twins[i] = 0; a.open[i] = 0; a.relabelled[i] = 0; }
+    }
+    if (a.swaps && !a.window) {          // the windows write every word of a candidate with twins
+        const int64_t quads = (a.N + 3) / 4 * a.dec_pitch;
+        for (int64_t i = tid; i < quads; i += nth)
+            reinterpret_cast<uint4 *>(a.swaps)[i] = make_uint4(0, 0, 0, 0);
     }
     for (int64_t i = tid; i < (int64_t)a.B * a.G; i += nth) {
+        c.group_column[i] = 0xFFFFFFFFu;
         const uint32_t info = c.group_info_in[i];
         c.group_info[i] = group_info_valid(a, info) ? (info & ~0x10000u) : 0u;
     }
-    for (int64_t i = tid; i < (int64_t)a.Bs * a.M; i += nth) c.model_num_good[i] = 0;
-    for (int64_t i = tid; i < (int64_t)a.Bs * a.G; i += nth) {
+    for (int64_t i = tid; i < (int64_t)a.B * a.M; i += nth) c.model_num_good[i] = 0;
+    for (int64_t i = tid; i < (int64_t)a.B * a.G; i += nth) {
         c.group_num_requests[i] = 0;
         if (c.group_num_good) c.group_num_good[i] = 0;
     }
-    for (int64_t i = tid; i < a.Bs; i += nth) {
+    for (int64_t i = tid; i < a.B; i += nth) {
         c.good_total[i] = 0;
         a.status[i] = 0;
         if (a.resimulated) a.resimulated[i] = 0;
     }
-    for (int64_t i = tid; i <= kMaxRepairRounds; i += nth) a.work_count[i] = 0;
+    for (int64_t i = tid; i < a.C; i += nth) c.column_stages[i] = 0;
+    if (tid == 0) *c.irregular = 0;
+    for (int64_t i = tid; i < kMaxRepairRounds; i += nth) { a.work_count[i] = 0; a.work_next[i] = 0; }
 }
 
 // Builds, in one launch behind clear_kernel, the tables the simulation kernels
@@ -125,7 +135,7 @@ __global__ void build_tables_kernel(const KernelArgs a, const ClearArgs c)
             : leaf_lower_bound(a.leaf_start, a.num_leaves, q * a.seg_len);
     for (int64_t i = tid; i < (int64_t)a.B * a.G; i += nth)
         if (!group_info_valid(a, c.group_info_in[i]))
-            atomicOr(&a.status[status_row(a, i / a.G)], MMS_STATUS_BAD_INDEX);
+            atomicOr(&a.status[i / a.G], MMS_STATUS_BAD_INDEX);
     for (int64_t t = tid; t < (int64_t)a.B * (a.M + 1); t += nth) {
         const int64_t b = t / (a.M + 1);
         const int m = (int)(t % (a.M + 1));
@@ -140,15 +150,29 @@ __global__ void build_tables_kernel(const KernelArgs a, const ClearArgs c)
                     const uint32_t ent = a.model_rep[(size_t)b * a.P + r];
                     const uint32_t ns = (ent >> 16) & 0xFFu, first = (ent >> 8) & 0xFFu;
                     if ((ent & 0xFFu) >= (uint32_t)a.G || ns == 0 || first + ns > (uint32_t)a.T ||
-                        ns > (uint32_t)a.S || (ent >> 24) >= (uint32_t)a.C)
+                        ns > (uint32_t)a.S || (ent >> 24) >= (uint32_t)a.C) {
                         bad = true;
-                    else if (r - lo < 8)
+                        continue;
+                    }
+                    // the window kernels lay pipelines out by group and by column
+                    const uint32_t was = atomicCAS(&c.column_stages[ent >> 24], 0u, ns);
+                    if ((was != 0 && was != ns) ||
+                        ((c.group_info_in[(size_t)b * a.G + (ent & 0xFFu)] & 0xFFFFu) != (first | (ns << 8))))
+                        *c.irregular = 1;
+                    const size_t gg = (size_t)b * a.G + (ent & 0xFFu);
+                    const uint32_t col = atomicCAS(&c.group_column[gg], 0xFFFFFFFFu, ent >> 24);
+                    if (col != 0xFFFFFFFFu && col != ent >> 24) *c.irregular = 1;
+                    // ... and take the first of the smallest clocks for the lowest group number
+                    if (r > lo && (a.model_rep[(size_t)b * a.P + r - 1] & 0xFFu) >= (ent & 0xFFu)) *c.irregular = 1;
+                    if (a.K > 1 && c.group_words)
+                        atomicOr((unsigned long long *)&c.group_models[gg * c.group_words + (m >> 6)], 1ull << (m & 63));
+                    if (r - lo < 8)
                         e[r - lo] = rep_to_last(ent);
                 }
                 if (hi - lo > 8) e[7] = kMoreReplicas;
             }
             if (bad) {
-                atomicOr(&a.status[status_row(a, b)], MMS_STATUS_BAD_INDEX);
+                atomicOr(&a.status[b], MMS_STATUS_BAD_INDEX);
                 for (int k = 0; k < 8; ++k) e[k] = kNoReplica;
             } else if (hi - lo > 1) {
                 // dispatch compares the last-stage clocks of these groups with '<'
@@ -165,10 +189,9 @@ __global__ void build_tables_kernel(const KernelArgs a, const ClearArgs c)
 
 // This lane's view of candidate b: offsets of its shared-memory state (clocks
 // zeroed) and pointers to its tables in global memory.
-template <bool kGroupGood>
 __device__ inline Lane setup_lane(const KernelArgs &a, int64_t b, int lane, int warp = 0)
 {
-    const SmemLayout L = smem_layout(a.M, a.G, a.P, a.T, a.S, kGroupGood, a.lat_smem_elems, a.lat_f64 != 0);
+    const SmemLayout L = smem_layout(a.T, a.S, a.lat_smem_elems, a.lat_f64 != 0);
     const size_t base = L.warp0 + (size_t)warp * L.warp_bytes;
     Lane ln;
     ln.clk = (uint32_t)((base + L.clocks) / sizeof(double)) + lane;
@@ -188,7 +211,9 @@ __device__ inline Lane setup_lane(const KernelArgs &a, int64_t b, int lane, int 
     ln.lat_f64 = a.lat_f64 != 0;
     ln.M = a.M; ln.C = a.C; ln.S = a.S;
     ln.status = 0;
-    ln.staging = 0;
+    ln.tie = 0;
+    ln.swaps = a.swaps ? a.swaps + 4 * b : nullptr;
+    ln.twin_class = a.swaps && a.twins[b] ? a.twin_class + (size_t)b * a.G : nullptr;
     for (int t = 0; t < a.T + kClockPad; ++t) SM_F64(ln.clk + t * kLanes) = 0.0;
     return ln;
 }
@@ -221,62 +246,21 @@ __device__ inline void init_pipe(const KernelArgs &a, Pipe &p, int64_t b)
     p.last = (int32_t)(a.N - 1);
 }
 
-// What the slim form of the narrow step (sim_step, kSlim) takes for granted.
-__device__ inline bool slim_shape(const KernelArgs &a)
-{
-    return a.lat_smem_elems != 0 && a.lat_f64 != 0 && !a.dec_wide;
-}
-
-// Byte offset of the decoded-request records behind the repair scratch.
-__host__ __device__ inline size_t staging_offset(size_t layout_total, int T, int G)
-{
-    return (layout_total + (sizeof(double) * (size_t)T + (size_t)G) * kLanes + 15) & ~(size_t)15;
-}
-
-// What the step that decodes ahead (staged_step) takes for granted, beyond the slim step:
-// every shared-memory index fits 16 bits, and no model of candidate b has more than eight
-// replicas.  Called by all 32 lanes of a warp; the answer is the same in all of them.
-__device__ inline bool staged_shape(const KernelArgs &a, const SmemLayout &L, int64_t b)
-{
-    if (!slim_shape(a) || a.trace_pitch < 1) return false;
-    if ((staging_offset(L.total, a.T, a.G) + kStagedBytes) / sizeof(double) >= 65536) return false;
-    const uint16_t *off = a.model_off + (size_t)b * (a.M + 1);
-    bool many = false;
-    for (int m = threadIdx.x & (kLanes - 1); m < a.M; m += kLanes) many |= off[m + 1] - off[m] > 8;
-    return !__any_sync(0xFFFFFFFFu, many);
-}
-
-// Extra shared memory of the kernels that repair: the state the previous run
-// stored (f64 [T]) and the scratch list of states_equivalent (u8 [G]).
-__device__ inline void repair_scratch(const KernelArgs &a, const SmemLayout &L, int lane,
-                                      uint32_t &old_state, uint32_t &stale_buf)
-{
-    old_state = (uint32_t)(L.total / sizeof(double)) + lane;
-    stale_buf = (uint32_t)(L.total + sizeof(double) * (size_t)a.T * kLanes) + lane;
-}
-
 // Blocks of block_warps warps (they share the latency table and nothing else).
-template <bool kFull, bool kGroupGood, bool kLegacy>
+template <bool kFull, bool kLegacy, bool kTwins>
 __global__ void __launch_bounds__(kLanes * kMaxBlockWarps, 1)
-sim_stream_kernel(const KernelArgs a)
+sim_stream_kernel(const __grid_constant__ KernelArgs a)
 {
     const int lane = threadIdx.x & (kLanes - 1);
     const int warp = threadIdx.x / kLanes;
-    stage_latency_table(a, smem_layout(a.M, a.G, a.P, a.T, a.S, kGroupGood, a.lat_smem_elems, a.lat_f64 != 0));
+    stage_latency_table(a, smem_layout(a.T, a.S, a.lat_smem_elems, a.lat_f64 != 0));
     const bool chunked = can_chunk(a);
     const int64_t stream = ((int64_t)blockIdx.x * a.block_warps + warp) * kLanes + lane;
     if (stream >= (int64_t)a.B * a.K) return;   // lanes never wait for each other below
     const int32_t j = (int32_t)(stream / a.B);
     const int64_t b = stream % a.B;
     if (a.N == 0 || (!chunked && j > 0)) return;
-    // a mirror only runs the speculative chunks
-    const bool mirror = b >= a.Bs;
-    if (mirror && (j == 0 || !chunked)) return;
-    const uint64_t swap = (mirror && a.mirror_swap)
-                              ? ((uint64_t)a.mirror_swap[2 * b + 1] << 32) | a.mirror_swap[2 * b]
-                              : ~0ull;
-
-    Lane ln = setup_lane<kGroupGood>(a, b, lane, warp);
+    Lane ln = setup_lane(a, b, lane, warp);
     Pipe p;
     init_pipe(a, p, b);
     // not chunked: one chunk holding every segment, plain sequential simulation
@@ -288,382 +272,475 @@ sim_stream_kernel(const KernelArgs a)
         const int32_t first = a.leaf_start[seg_leaf(a, j * a.seg_per_chunk)];
         begin = first - a.warmup > 0 ? first - a.warmup : 0;
     }
-    run_chunk<kFull, kGroupGood, kLegacy>(ka, ln, p, b, j, begin, false,
-                                          chunked, 0, 0, -1, 0, swap);
-    if (ln.status) atomicOr(&a.status[status_row(a, b)], ln.status);
+    run_chunk<kFull, kLegacy, kTwins>(ka, ln, p, b, j, begin, chunked);
+    if (ln.status) atomicOr(&a.status[b], ln.status);
 }
 
-// One thread per (array u, chunk j >= 1), u a scored candidate or a mirror:
-// which stored runs of chunk j start from a state that continues the state
-// array u holds at the end of chunk j-1 (states_equivalent: equal futures,
-// provably)?  Bit 0: the array of the candidate itself, bit 1 + i: its i-th
-// mirror.
-__global__ void validate_kernel(const KernelArgs a)
+// Classes of interchangeable groups (warp_relabel): same stages, same latency column, same
+// set of models.  One thread per (candidate, group); behind build_tables_kernel, which
+// collects every group's models as a bit set (a launch with more than kTwinModels models has
+// no classes).
+__global__ void twins_kernel(const KernelArgs a, const ClearArgs c)
 {
     const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (!can_chunk(a) || t >= (int64_t)a.B * (a.K - 1)) return;
-    // a round that repaired nothing left every state, and so every mask, as it was
-    if (a.round > 0 && a.work_count[a.round - 1] == 0) return;
-    if (t == 0) a.work_count[kMaxRepairRounds] = 0;   // resolve_kernel counts the unsettled there
-    const int32_t j = (int32_t)(t / a.B) + 1;
-    const int64_t u = t % a.B;
-    const int64_t b = status_row(a, u);                // the scored candidate u belongs to
-    if (u >= a.Bs && (j == 1 || a.partner[u] != b)) return;   // a mirror has no chunk 0
-    int64_t m_end;
-    const int64_t m_first = mirrors_of(a, b, m_end);
+    if (t >= (int64_t)a.B * a.G || *a.irregular) return;
+    const int64_t b = t / a.G;
+    const int g = (int)(t % a.G);
+    const int W = c.group_words;
+    const uint64_t *mine = c.group_models + (size_t)t * W;
+    uint64_t some = 0;
+    for (int k = 0; k < W; ++k) some |= mine[k];
+    const uint32_t ns = (a.group_info[t] >> 8) & 0xFFu, column = c.group_column[t];
+    int cls = g, rank = 0;
+    if (some && ns && column < (uint32_t)a.C) {
+        for (int h = 0; h < g; ++h) {
+            const size_t u = (size_t)b * a.G + h;
+            if (((a.group_info[u] >> 8) & 0xFFu) != ns || c.group_column[u] != column) continue;
+            const uint64_t *other = c.group_models + u * W;
+            bool same = true;
+            for (int k = 0; k < W && same; ++k) same = mine[k] == other[k];
+            if (same) { if (cls == g) cls = h; ++rank; }
+        }
+    }
+    c.twin_class[t] = (uint16_t)(cls | (rank << 8));
+    if (cls != g) c.twins[b] = 1;
+}
+
+// Does the run of chunk j of candidate b continue the run of the chunk before it, in the
+// same labels (states_equivalent: equal futures, provably)?
+__device__ inline bool continues(const KernelArgs &a, int32_t j, int64_t b)
+{
     const int32_t q_prev = j * a.seg_per_chunk - 1;
     const double tau = arrival_at(a, b, a.leaf_start[seg_leaf(a, q_prev + 1)]);
     const size_t B = (size_t)a.B;
-    const double *X = a.seg_end + (size_t)q_prev * a.T * B + u;
+    const double *X = a.seg_end + (size_t)q_prev * a.T * B + b;
+    const double *Y = a.chunk_start + (size_t)j * a.T * B + b;
     uint8_t stale[MMS_MAX_GROUPS];
-    uint32_t mask = 0;
-    for (int64_t r = 0; r <= m_end - m_first && r < 16; ++r) {
-        const double *Y = a.chunk_start + (size_t)j * a.T * B + (r == 0 ? b : m_first + r - 1);
-        if (states_equivalent(a, b, [&](uint32_t s) { return X[s * B]; },
-                              [&](uint32_t s) { return Y[s * B]; }, tau,
-                              [&](int w) -> uint8_t & { return stale[w]; }))
-            mask |= 1u << r;
+    return states_equivalent(a, b, [&](uint32_t s) { return X[s * B]; },
+                             [&](uint32_t s) { return Y[s * B]; }, tau,
+                             [&](int w) -> uint8_t & { return stale[w]; });
+}
+
+// A round that walked nothing left every state as it was.
+__device__ inline bool nothing_changed(const KernelArgs &a)
+{
+    return a.round > 0 && a.work_count[a.round - 1] == 0;
+}
+
+constexpr int kLinkWarps = 4;
+
+// Shared memory of a link_kernel warp: two states, last-stage clocks, permutation, ranks.
+__host__ __device__ inline size_t link_warp_bytes(int T, int G)
+{
+    return (sizeof(double) * (2 * (size_t)T + (size_t)G) + 3 * (size_t)G + 15) & ~(size_t)15;
+}
+
+// Judges the chunk boundaries whose sides the round before changed (all of them in round 0): one
+// thread per boundary compares the states as they are; those that differ and belong to a
+// candidate with interchangeable groups are then compared under other labels, by the whole
+// warp.
+__global__ void __launch_bounds__(kLinkWarps * kLanes)
+link_kernel(const __grid_constant__ KernelArgs a)
+{
+    if (!can_chunk(a) || nothing_changed(a)) return;
+    const int lane = threadIdx.x & (kLanes - 1), warp = threadIdx.x / kLanes;
+    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const size_t B = (size_t)a.B;
+    const int64_t b = t % a.B;
+    const int32_t j = (int32_t)(t / a.B) + 1;
+    bool again = false;
+    if (t < (int64_t)a.B * (a.K - 1)) {
+        const size_t cell = (size_t)j * B + b;
+        if (a.round == 0 || a.stamp[cell - B] == (uint8_t)a.round || a.stamp[cell] == (uint8_t)a.round) {
+            const bool ok = continues(a, j, b);
+            a.link[cell] = ok;
+            a.rel[(size_t)(j * a.seg_per_chunk) * B + b] = 0;
+            again = !ok && a.twins[b];
+        }
     }
-    a.compat[(size_t)j * B + u] = (uint16_t)mask;
+    uint32_t todo = __ballot_sync(0xFFFFFFFFu, again);
+    if (!todo) return;
+    const size_t base = (size_t)warp * link_warp_bytes(a.T, a.G);
+    const uint32_t x = (uint32_t)(base / sizeof(double));
+    RelabelScratch s;
+    s.z = x + a.T;
+    s.last = s.z + a.T;
+    s.perm = (uint32_t)(base + sizeof(double) * (2 * (size_t)a.T + (size_t)a.G));
+    s.rank = s.perm + a.G;
+    for (; todo; todo &= todo - 1) {
+        const int k = __ffs((int)todo) - 1;
+        const int64_t bb = __shfl_sync(0xFFFFFFFFu, b, k);
+        const int32_t jj = __shfl_sync(0xFFFFFFFFu, j, k);
+        const int32_t q0 = jj * a.seg_per_chunk;
+        const double tau = arrival_at(a, bb, a.leaf_start[seg_leaf(a, q0)]);
+        __syncwarp();
+        for (int t = lane; t < a.T; t += kLanes)
+            SM_F64(x + t) = a.seg_end[((size_t)(q0 - 1) * a.T + t) * B + bb];
+        __syncwarp();
+        const auto info = [&](int g) { return a.group_info[(size_t)bb * a.G + g]; };
+        const auto X = [&](uint32_t t) { return SM_F64(x + t); };
+        if (!warp_relabel(a.G, a.T, a.twin_class + (size_t)bb * a.G, info, X,
+                          a.chunk_start + (size_t)jj * a.T * B + bb, B, s) ||
+            !warp_equivalent(a.G, info, X, [&](uint32_t t) { return SM_F64(s.z + t); }, tau))
+            continue;
+        const size_t cell = (size_t)q0 * B + bb;
+        for (int g = lane; g < a.G; g += kLanes) a.perm[cell * a.G + g] = smem[s.perm + g];
+        if (lane == 0) {
+            a.rel[cell] = 1;
+            a.relabelled[bb] = 1;
+            a.link[(size_t)jj * B + bb] = 1;
+        }
+    }
 }
 
-// Chunk j of candidate b is about to be re-simulated from a NEW start state
-// while an earlier, capped repair of it (from an older start state) is still
-// unfinished: that repair left its own end-of-segment states in the segments it
-// got through, and behind them the records are still those of the speculative
-// run, which it never matched.  The new repair must not settle against those
-// left-over states (it would then keep the unmatched rest), so they are made
-// unequal to everything: a NaN in clock slot 0 fails both "equal" and "in the
-// past".  The segments behind them hold states of runs that go on to the end
-// of the chunk, which a repair may settle against as usual.
-__device__ inline void forget_capped_repair(const KernelArgs &a, int64_t b, int32_t j)
+// One warp per candidate: lists the chunks to be walked in this round — those behind a failed
+// boundary that itself has a good one before it — and copies the state they start from.
+// The walk from there goes through the failed boundaries behind it.  Where a third of the
+// boundaries fail (a placement under sustained overload: states hardly ever settle) most walks
+// would start from states that are not the true ones either and have to be done again; such a
+// candidate is left to finish_kernel, which walks once.
+__global__ void resolve_kernel(const __grid_constant__ KernelArgs a)
 {
-    const int32_t pending = a.repair_from[(size_t)j * a.B + b];
-    const double nan = __longlong_as_double(0x7FF8000000000000LL);
-    for (int32_t q = j * a.seg_per_chunk; q < pending; ++q)
-        a.seg_end[(size_t)q * a.T * a.B + b] = nan;
-    a.repair_from[(size_t)j * a.B + b] = -1;
-}
-
-// One warp per scored candidate: follows the chain of chunks through the
-// masks of validate_kernel.  A chunk keeps the run selected for it when that
-// one continues the chunk before it; else it is taken from the first mirror
-// that does; else the true state is copied into the candidate's own array and
-// the chunk goes on the work list.  Behind a listed chunk the walk goes on
-// with the old data; the next round (or the chain kernel) sees the new one.
-// A candidate whose walk lists nothing is settled: every chunk continues the
-// one before it.  That is noted in row 0 of the masks (no boundary uses it)
-// and lets the chain kernel skip the candidate.
-__global__ void resolve_kernel(const KernelArgs a)
-{
-    // a warp per candidate: lane 0 walks, all lanes copy a state when one is to be copied
     const int lane = threadIdx.x & (kLanes - 1);
     const int64_t b = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / kLanes;
-    if (!can_chunk(a) || b >= a.Bs) return;
-    if (a.round > 0 && a.work_count[a.round - 1] == 0) return;    // same masks, same answer
-    bool settled = true;
-    int64_t m_end;
-    const int64_t m_first = mirrors_of(a, b, m_end);
+    if (!can_chunk(a) || b >= a.B || nothing_changed(a)) return;
     const size_t B = (size_t)a.B;
-    int32_t redone = 0;
-    // A candidate nearly all of whose boundaries fail (a placement under sustained overload:
-    // no state ever settles, a repaired chunk only moves the failure to the next boundary)
-    // gains nothing from the rounds: every chunk would be re-simulated in each of them and
-    // once more by the chain kernel.  It is left to the chain kernel as it is.
-    {
-        int32_t fails = 0;
-        for (int32_t j = 1 + lane; j < a.K; j += kLanes) {
-            const int32_t q0 = j * a.seg_per_chunk;
-            const int32_t e = a.seg_src[(size_t)(q0 - 1) * B + b];
-            const int32_t s0 = a.seg_src[(size_t)q0 * B + b];
-            const uint32_t mask = a.compat[(size_t)j * B + (e < 0 ? b : e)];
-            const uint32_t bit = s0 < 0 ? 0u : (uint32_t)(s0 - m_first + 1);
-            fails += !((bit < 16 && ((mask >> bit) & 1u)) || mask != 0);
+    int32_t fails = 0;
+    for (int32_t j = 1 + lane; j < a.K; j += kLanes) fails += !a.link[(size_t)j * B + b];
+    fails = __reduce_add_sync(0xFFFFFFFFu, fails);
+    if (lane == 0) a.open[b] = fails != 0;
+    if (fails == 0 || (a.K > 8 && (int64_t)fails * 3 >= (int64_t)(a.K - 1))) return;
+    int32_t listed = 0;
+    for (int32_t j0 = 1; j0 < a.K; j0 += kLanes) {
+        const int32_t j = j0 + lane;
+        const bool head = j < a.K && !a.link[(size_t)j * B + b] && (j == 1 || a.link[(size_t)(j - 1) * B + b]);
+        if (head) {
+            a.work_items[atomicAdd(&a.work_count[a.round], 1u)] = (uint32_t)((int64_t)j * a.B + b);
+            a.stamp[(size_t)j * B + b] = (uint8_t)(a.round + 1);
         }
-        fails = __reduce_add_sync(0xFFFFFFFFu, fails);
-        if (a.K > 8 && (int64_t)fails * 8 >= (int64_t)(a.K - 1) * 7) {
-            if (lane == 0) {
-                a.compat[b] = 0;
-                atomicAdd(&a.work_count[kMaxRepairRounds], 1u);
-            }
-            return;
-        }
-    }
-    for (int32_t j = 1; j < a.K; ++j) {
-        const int32_t q0 = j * a.seg_per_chunk;
-        const int32_t q1 = q0 + a.seg_per_chunk < a.NS ? q0 + a.seg_per_chunk : a.NS;
-        int64_t copy_from = -1;          // candidate whose end state becomes chunk j's start
-        if (lane == 0) {
-            const int32_t e = a.seg_src[(size_t)(q0 - 1) * B + b];     // whose end of chunk j-1 counts
-            const int32_t s0 = a.seg_src[(size_t)q0 * B + b];          // whose start of chunk j
-            const uint32_t mask = a.compat[(size_t)j * B + (e < 0 ? b : e)];
-            const uint32_t bit = s0 < 0 ? 0u : (uint32_t)(s0 - m_first + 1);
-            if (bit < 16 && ((mask >> bit) & 1u)) {
-                if (s0 < 0 && a.repair_from[(size_t)j * B + b] >= 0) {   // a capped repair goes on
-                    const uint32_t slot = atomicAdd(&a.work_count[a.round], 1u);
-                    a.work_items[slot] = (uint32_t)((int64_t)j * a.B + b) | 0x80000000u;
-                    settled = false;
-                }
-            } else if (s0 >= 0 && (mask & 1u) && !a.own_rewritten[(size_t)j * B + b]) {
-                // a mirror's run was selected, but it is the candidate's own speculative
-                // run — untouched so far — that continues the chunk before
-                for (int32_t q = q0; q < q1; ++q) a.seg_src[(size_t)q * B + b] = -1;
-                a.repair_from[(size_t)j * B + b] = -1;
-            } else if (mask >> 1) {
-                const int32_t v = (int32_t)m_first + (__ffs((int)(mask >> 1)) - 1);
-                for (int32_t q = q0; q < q1; ++q) a.seg_src[(size_t)q * B + b] = v;
-                a.repair_from[(size_t)j * B + b] = -1;
-            } else {
-                copy_from = e < 0 ? b : e;
-                // The whole chunk is redone.  Its run selection stays as it is until the
-                // repair has compared its state with the selected run's, segment by
-                // segment (run_chunk then makes each segment it ran the candidate's own):
-                // the selected runs of consecutive segments continue one another, which a
-                // selection changed here by hand would not.
-                forget_capped_repair(a, b, j);
-                const uint32_t slot = atomicAdd(&a.work_count[a.round], 1u);
-                a.work_items[slot] = (uint32_t)((int64_t)j * a.B + b);
-                ++redone;
-                settled = false;
-            }
-        }
-        copy_from = __shfl_sync(0xFFFFFFFFu, copy_from, 0);
-        if (copy_from >= 0) {
-            const double *X = a.seg_end + (size_t)(q0 - 1) * a.T * B + copy_from;
-            double *Y = a.chunk_start + (size_t)j * a.T * B + b;
+        for (uint32_t todo = __ballot_sync(0xFFFFFFFFu, head); todo; todo &= todo - 1, ++listed) {
+            const int32_t k = j0 + __ffs((int)todo) - 1;
+            const double *X = a.seg_end + (size_t)(k * a.seg_per_chunk - 1) * a.T * B + b;
+            double *Y = a.chunk_start + (size_t)k * a.T * B + b;
             for (int s = lane; s < a.T; s += kLanes) Y[s * B] = X[s * B];
         }
     }
-    if (lane != 0) return;
-    a.compat[b] = settled ? 1 : 0;
-    if (!settled) atomicAdd(&a.work_count[kMaxRepairRounds], 1u);
-    if (a.resimulated && redone) atomicAdd(&a.resimulated[b], redone);
+    if (a.resimulated && lane == 0 && listed) atomicAdd(&a.resimulated[b], listed);
 }
 
-// One thread per chunk on the work list of this round.  A long list is
-// worked 32 chunks to a warp (kNarrow false).  A short one — the late rounds,
-// where what is left is a few long dependent repairs and the GPU is otherwise
-// idle — one chunk to a warp, with the step that branches (kNarrow): the
-// duration of a round is that of its longest repair, and a lone lane gets
-// through a request in a quarter fewer instructions.  Both kernels are
-// launched every round; the one whose turn it is not returns at once.
-template <bool kFull, bool kGroupGood, bool kLegacy, bool kNarrow>
-__global__ void __launch_bounds__(kLanes, 1)
-sim_repair_kernel(const KernelArgs a)
+// The speculative pass of a small batch: one warp per (chunk, candidate), by windows.
+template <bool kLegacy, bool kTwins>
+__global__ void __launch_bounds__(kWindowWarps * kLanes, kWindowBlocksPerSm)
+window_stream_kernel(const __grid_constant__ KernelArgs a)
 {
-    const int lane = kNarrow ? 0 : threadIdx.x;
-    const uint32_t count = a.work_count[a.round];
-    if ((count <= (uint32_t)a.narrow_limit) != kNarrow) return;
-    if ((uint64_t)blockIdx.x * (kNarrow ? 1 : kLanes) >= count) return;
-    const SmemLayout L = smem_layout(a.M, a.G, a.P, a.T, a.S, kGroupGood, a.lat_smem_elems, a.lat_f64 != 0);
-    stage_latency_table(a, L);
-    const uint32_t w = kNarrow ? blockIdx.x : blockIdx.x * kLanes + lane;
-    if (w >= count) return;
-    const uint32_t item = a.work_items[w] & 0x7FFFFFFFu;
-    const bool resume = (a.work_items[w] >> 31) != 0;
-    const int32_t j = (int32_t)(item / (uint32_t)a.B);
-    const int64_t b = item % (uint32_t)a.B;
-    // one chunk to a warp: the lone lane, or — where the step that decodes ahead applies —
-    // all 32 lanes as copies of it
-    constexpr bool kCanSlim = kNarrow && !kFull && !kLegacy;
-    bool staged = false;
-    if constexpr (kCanSlim) staged = staged_shape(a, L, b);
-    if (kNarrow && !staged && threadIdx.x != 0) return;
-
-    Lane ln = setup_lane<kGroupGood>(a, b, lane);
-    ln.staging = staged ? (uint32_t)staging_offset(L.total, a.T, a.G) : 0u;
-    uint32_t old_state, stale_buf;
-    repair_scratch(a, L, lane, old_state, stale_buf);
-    // start of the chunk from the copied-in true state, or where a capped
-    // repair stopped, from the state it left after the segment before
-    const int32_t q_begin = resume ? a.repair_from[(size_t)j * a.B + b] : j * a.seg_per_chunk;
-    const double *src = resume ? a.seg_end + (size_t)(q_begin - 1) * a.T * a.B
-                               : a.chunk_start + (size_t)j * a.T * a.B;
-    for (int t = 0; t < a.T; ++t) SM_F64(ln.clk + t * kLanes) = src[(size_t)t * a.B + b];
-    Pipe p;
-    init_pipe(a, p, b);
-    const int32_t first = a.leaf_start[seg_leaf(a, q_begin)];
-    int64_t m_end;
-    const int64_t m_first = mirrors_of(a, b, m_end);
-    const bool own_pure = !a.own_rewritten[(size_t)j * a.B + b];
-    if (staged) __syncwarp();            // every copy has read the flag before one sets it
-    a.own_rewritten[(size_t)j * a.B + b] = 1;
-    if (kCanSlim && staged)
-        a.repair_from[(size_t)j * a.B + b] =
-            run_chunk<kFull, kGroupGood, kLegacy, kNarrow, kCanSlim, kCanSlim>(
-                a, ln, p, b, j, first, true, true, old_state, stale_buf, q_begin,
-                a.repair_cap, ~0ull, m_first, m_end, own_pure);
-    else if (kCanSlim && slim_shape(a))
-        a.repair_from[(size_t)j * a.B + b] =
-            run_chunk<kFull, kGroupGood, kLegacy, kNarrow, kCanSlim>(
-                a, ln, p, b, j, first, true, true, old_state, stale_buf, q_begin,
-                a.repair_cap, ~0ull, m_first, m_end, own_pure);
-    else
-        a.repair_from[(size_t)j * a.B + b] = run_chunk<kFull, kGroupGood, kLegacy, kNarrow>(
-            a, ln, p, b, j, first, true, true, old_state, stale_buf, q_begin,
-            a.repair_cap, ~0ull, m_first, m_end, own_pure);
-    if (ln.status) atomicOr(&a.status[b], ln.status);
-}
-
-// One thread per scored candidate: walks the chunk boundaries in order.  A
-// chunk keeps the run selected for it when that one continues the chunk
-// before it, else takes the first mirror's run that does, else is repaired in
-// place in the candidate's own array.  After it, every segment that counts
-// was simulated from a state equivalent to the true one.  Like the repairs, it
-// comes in two forms, 32 candidates to a warp or (kNarrow, when few are left
-// unsettled) one.
-template <bool kFull, bool kGroupGood, bool kLegacy, bool kNarrow>
-__global__ void __launch_bounds__(kLanes, 1)
-sim_chain_kernel(const KernelArgs a)
-{
-    const int lane = kNarrow ? 0 : threadIdx.x;
-    if (!can_chunk(a) || a.N == 0) return;
-    if ((a.work_count[kMaxRepairRounds] <= (uint32_t)a.narrow_limit) != kNarrow) return;
-    if (kNarrow && a.compat[blockIdx.x]) return;          // whole block: nothing to stage for
-    const SmemLayout L = smem_layout(a.M, a.G, a.P, a.T, a.S, kGroupGood, a.lat_smem_elems, a.lat_f64 != 0);
-    stage_latency_table(a, L);
-    const int64_t b = kNarrow ? (int64_t)blockIdx.x : (int64_t)blockIdx.x * kLanes + lane;
-    if (b >= a.Bs) return;
-    if (a.compat[b]) return;             // settled by the last walk of resolve_kernel
-    // one candidate to a warp: the lone lane, or all 32 lanes as copies of it (see
-    // sim_repair_kernel)
-    constexpr bool kCanSlim = kNarrow && !kFull && !kLegacy;
-    bool staged = false;
-    if constexpr (kCanSlim) staged = staged_shape(a, L, b);
-    if (kNarrow && !staged && threadIdx.x != 0) return;
-    int64_t m_end;
-    const int64_t m_first = mirrors_of(a, b, m_end);
-
-    Lane ln = setup_lane<kGroupGood>(a, b, lane);
-    ln.staging = staged ? (uint32_t)staging_offset(L.total, a.T, a.G) : 0u;
-    uint32_t old_state, stale_buf;
-    repair_scratch(a, L, lane, old_state, stale_buf);
-    Pipe p;
-    init_pipe(a, p, b);
-    int32_t redone = 0;
-    for (int32_t j = 1; j < a.K; ++j) {
-        const int32_t q0 = j * a.seg_per_chunk;
-        const int32_t q1 = q0 + a.seg_per_chunk < a.NS ? q0 + a.seg_per_chunk : a.NS;
-        const int64_t first = a.leaf_start[seg_leaf(a, q0)];
-        const double tau = arrival_at(a, b, first);
-        const int32_t e = a.seg_src[(size_t)(q0 - 1) * a.B + b];
-        const int32_t s0 = a.seg_src[(size_t)q0 * a.B + b];
-        for (int t = 0; t < a.T; ++t)
-            SM_F64(ln.clk + t * kLanes) =
-                a.seg_end[((size_t)(q0 - 1) * a.T + t) * a.B + (e < 0 ? b : e)];
-        auto continues = [&](int64_t v) {
-            for (int t = 0; t < a.T; ++t)
-                SM_F64(old_state + t * kLanes) = a.chunk_start[((size_t)j * a.T + t) * a.B + v];
-            return states_equivalent(
-                a, b, [&](uint32_t s) { return SM_F64(ln.clk + s * kLanes); },
-                [&](uint32_t s) { return SM_F64(old_state + s * kLanes); }, tau,
-                [&](int u) -> uint8_t & { return smem[stale_buf + u * kLanes]; });
-        };
-        int32_t q_begin = q0;
-        int32_t begin = (int32_t)first;
-        if (continues(s0 < 0 ? b : s0)) {
-            // the chunk continues its predecessor; finish a repair a round left capped
-            q_begin = s0 < 0 ? a.repair_from[(size_t)j * a.B + b] : -1;
-            if (q_begin < 0) continue;
-            begin = a.leaf_start[seg_leaf(a, q_begin)];
-            for (int t = 0; t < a.T; ++t)
-                SM_F64(ln.clk + t * kLanes) = a.seg_end[((size_t)(q_begin - 1) * a.T + t) * a.B + b];
-        } else {
-            const bool own_pure = !a.own_rewritten[(size_t)j * a.B + b];
-            if (s0 >= 0 && own_pure && continues(b)) {     // back to the own speculative run
-                for (int32_t q = q0; q < q1; ++q) a.seg_src[(size_t)q * a.B + b] = -1;
-                continue;
-            }
-            int64_t found = -1;
-            for (int64_t m = m_first; m < m_end && found < 0; ++m)
-                if (m != s0 && continues(m)) found = m;
-            if (found >= 0) {
-                for (int32_t q = q0; q < q1; ++q) a.seg_src[(size_t)q * a.B + b] = (int32_t)found;
-                continue;
-            }
-            if (staged) __syncwarp();    // the comparisons above read what is written now
-            for (int t = 0; t < a.T; ++t)
-                a.chunk_start[((size_t)j * a.T + t) * a.B + b] = SM_F64(ln.clk + t * kLanes);
-            forget_capped_repair(a, b, j);
+    window_stage_table<kLegacy>(a);
+    if (a.N == 0) return;
+    const bool chunked = can_chunk(a);
+    // not chunked: one chunk holding every segment, plain sequential simulation
+    KernelArgs ka = a;
+    if (!chunked) ka.seg_per_chunk = a.NS;
+    const int64_t items = (int64_t)a.B * (chunked ? a.K : 1);
+    const int64_t step = (int64_t)gridDim.x * kWindowWarps;
+    for (int64_t it = (int64_t)blockIdx.x * kWindowWarps + threadIdx.x / kLanes; it < items; it += step) {
+        const int32_t j = (int32_t)(it / a.B);
+        const int64_t b = it % a.B;
+        Window w;
+        window_setup<kLegacy, kTwins>(a, w, b);
+        int32_t begin = 0;
+        if (j > 0) {
+            const int32_t first = a.leaf_start[seg_leaf(a, j * a.seg_per_chunk)];
+            begin = first - a.warmup > 0 ? first - a.warmup : 0;
         }
-        ++redone;
-        const bool own_pure = !a.own_rewritten[(size_t)j * a.B + b];
-        if (staged) __syncwarp();        // every copy has read the flag before one sets it
-        a.own_rewritten[(size_t)j * a.B + b] = 1;
-        if (kCanSlim && staged)
-            run_chunk<kFull, kGroupGood, kLegacy, kNarrow, kCanSlim, kCanSlim>(
-                a, ln, p, b, j, begin, true, true, old_state, stale_buf, q_begin, 0, ~0ull,
-                m_first, m_end, own_pure);
-        else if (kCanSlim && slim_shape(a))
-            run_chunk<kFull, kGroupGood, kLegacy, kNarrow, kCanSlim>(
-                a, ln, p, b, j, begin, true, true, old_state, stale_buf, q_begin, 0, ~0ull,
-                m_first, m_end, own_pure);
-        else
-            run_chunk<kFull, kGroupGood, kLegacy, kNarrow>(a, ln, p, b, j, begin, true, true,
-                                                           old_state, stale_buf, q_begin, 0, ~0ull,
-                                                           m_first, m_end, own_pure);
-        a.repair_from[(size_t)j * a.B + b] = -1;
+        window_run<kLegacy, kTwins>(ka, w, kNoWalk, j, begin, chunked, j * a.seg_per_chunk);
+        if (w.status) atomicOr(&a.status[b], w.status);
     }
-    if (a.resimulated && redone && (!kNarrow || threadIdx.x == 0))
-        atomicAdd(&a.resimulated[b], redone);
-    if (ln.status) atomicOr(&a.status[b], ln.status);
 }
 
-// Combines the leaf sums of candidate b in numpy's pairing order
-// (controller.py:402 consumes the mean).  Leaf sums are fetched eight at a
-// time so that the loads overlap.  With seg_src == nullptr every leaf sum is
-// the candidate's own.
-__device__ inline void sum_leaves(const KernelArgs &a, int64_t b, const uint8_t *leaf_merges,
-                                  double *latency_sum)
+// The chunks on the work list of this round, one to a warp, taken from the
+// list as warps become free: each is re-simulated from the state the chunk before it ended in,
+// and the chunks behind it as well, until the stored run can take over or the next listed
+// chunk comes.  A round lasts as long as its longest walk, so what counts is how fast ONE
+// candidate gets through its requests: a lane of the 32-candidate step takes 0.5 to 0.9 us a
+// request, windows 0.1 to 0.4 us.
+template <bool kLegacy, bool kTwins>
+__global__ void __launch_bounds__(kWindowWarps * kLanes, kWindowBlocksPerSm)
+walk_kernel(const __grid_constant__ KernelArgs a)
 {
-    const int32_t num_leaves = a.num_leaves;
+    const uint32_t count = a.work_count[a.round];
+    if ((uint64_t)blockIdx.x * kWindowWarps >= count) return;
+    window_stage_table<kLegacy>(a);
+    const int lane = threadIdx.x & (kLanes - 1);
+    for (;;) {
+        uint32_t at = 0;
+        if (lane == 0) at = atomicAdd(&a.work_next[a.round], 1u);
+        at = __shfl_sync(0xFFFFFFFFu, at, 0);
+        if (at >= count) return;
+        const uint32_t item = a.work_items[at];
+        const int32_t j = (int32_t)(item / (uint32_t)a.B);
+        const int64_t b = item % (uint32_t)a.B;
+        Window w;
+        window_setup<kLegacy, kTwins>(a, w, b);
+        const double *src = a.chunk_start + (size_t)j * a.T * a.B + b;
+        for (int t = lane; t < a.T; t += kLanes) WIN_CLOCK(w, t) = src[(size_t)t * a.B];
+        __syncwarp();
+        const int32_t q0 = j * a.seg_per_chunk;
+        window_run<kLegacy, kTwins>(a, w, kWalkRound, j, a.leaf_start[seg_leaf(a, q0)], true, q0);
+        if (w.status) atomicOr(&a.status[b], w.status);
+    }
+}
+
+// The labels of a candidate's segments, followed from one to the next by a warp: `pi` (u8[G] in
+// shared memory) translates the labels of the segment at hand into group numbers.
+struct Labels {
+    uint32_t pi, tmp;                        // u8 indices; tmp: scratch of the same size
+    const uint16_t *cls;                     // the candidate's classes of twins
+    uint64_t moved;                          // classes in which pi is not the identity
+};
+
+__device__ inline void labels_reset(Labels &l, int G)
+{
+    __syncwarp();
+    for (int g = threadIdx.x & (kLanes - 1); g < G; g += kLanes) smem[l.pi + g] = (uint8_t)g;
+    l.moved = 0;
+    __syncwarp();
+}
+
+// Into tmp: the translation behind `perm` (label -> label of the segment before).  Returns
+// the classes in which it is not the identity.
+__device__ inline uint64_t labels_through(const Labels &l, int G, const uint8_t *perm)
+{
+    __syncwarp();
+    for (int g = threadIdx.x & (kLanes - 1); g < G; g += kLanes) smem[l.tmp + g] = smem[l.pi + perm[g]];
+    __syncwarp();
+    return moved_classes(l.cls, G, [&](int g) { return smem[l.tmp + g]; });
+}
+
+__device__ inline void labels_take(Labels &l, int G, uint64_t moved)
+{
+    __syncwarp();
+    for (int g = threadIdx.x & (kLanes - 1); g < G; g += kLanes) smem[l.pi + g] = smem[l.tmp + g];
+    l.moved = moved;
+    __syncwarp();
+}
+
+// The first segment from q on that changes labels or starts a chunk behind a failed boundary
+// (NS: none).
+__device__ inline int32_t next_event(const KernelArgs &a, int64_t b, int32_t q)
+{
+    const int lane = threadIdx.x & (kLanes - 1);
+    const size_t B = (size_t)a.B;
+    for (; q < a.NS; q += kLanes) {
+        const int32_t s = q + lane;
+        const bool event = s < a.NS &&
+                           (a.rel[(size_t)s * B + b] ||
+                            (s % a.seg_per_chunk == 0 && !a.link[(size_t)(s / a.seg_per_chunk) * B + b]));
+        const uint32_t todo = __ballot_sync(0xFFFFFFFFu, event);
+        if (todo) return q + __ffs((int)todo) - 1;
+    }
+    return a.NS;
+}
+
+// Translates the decision records of segment q into group numbers, 32 requests at a time, and
+// follows the labels through the choices between twins in the same state (see warp_relabel).
+__device__ inline void name_segment(const KernelArgs &a, int64_t b, Labels &l, int32_t q)
+{
+    const int lane = threadIdx.x & (kLanes - 1);
+    const int32_t i0 = a.leaf_start[seg_leaf(a, q)];
+    const int32_t i1 = seg_leaf(a, q + 1) < a.num_leaves ? a.leaf_start[seg_leaf(a, q + 1)] : (int32_t)a.N;
+    const uint32_t flag = a.dec_wide ? 0x8000u : 0x80u;
+    for (int32_t base = i0; base < i1 && l.moved; base += kLanes) {
+        const int32_t i = base + lane;
+        const size_t at = (((size_t)(i >> 2) * a.dec_pitch) + b) * 4 + (size_t)(i & 3);
+        uint32_t rec = 0, swap = 0;
+        if (i < i1) {
+            rec = a.dec_wide ? static_cast<uint16_t *>(a.decisions)[at] : static_cast<uint8_t *>(a.decisions)[at];
+            swap = rec ? a.swaps[at] : 0u;
+        }
+        const uint32_t label = rec ? (rec & (flag - 1)) - 1 : 0u;
+        const bool concerns = swap && (class_bit(l.cls[label]) & l.moved);
+        uint32_t group = label;
+        int from = 0;
+        for (uint32_t todo = __ballot_sync(0xFFFFFFFFu, concerns);; todo &= todo - 1) {
+            const int k = todo ? __ffs((int)todo) - 1 : kLanes;
+            if (lane >= from && lane < k && rec) group = smem[l.pi + label];
+            if (!todo) break;
+            from = k;
+            // the true choice is the smallest group number among the replicas in the picked one's
+            // state; the label that has it changes places with the picked one
+            const uint32_t mask = __shfl_sync(0xFFFFFFFFu, swap, k), mine = __shfl_sync(0xFFFFFFFFu, label, k);
+            uint32_t key = 0xFFFFFFFFu;              // group << 8 | label
+            for (int g = lane; g < a.G; g += kLanes)
+                if ((l.cls[g] & 0xFFu) == (l.cls[mine] & 0xFFu) && (l.cls[g] >> 8) < 32 &&
+                    ((mask >> (l.cls[g] >> 8)) & 1u)) {
+                    const uint32_t mapped = ((uint32_t)smem[l.pi + g] << 8) | (uint32_t)g;
+                    key = mapped < key ? mapped : key;
+                }
+            key = __reduce_min_sync(0xFFFFFFFFu, key);
+            const uint32_t other = key & 0xFFu;
+            if (other != mine) {
+                __syncwarp();
+                if (lane == 0) {
+                    const uint8_t g = smem[l.pi + mine];
+                    smem[l.pi + mine] = (uint8_t)(key >> 8);
+                    smem[l.pi + other] = g;
+                }
+                __syncwarp();
+            }
+        }
+        if (rec && group != label) {
+            rec = (rec & flag) | (group + 1);
+            if (a.dec_wide) static_cast<uint16_t *>(a.decisions)[at] = (uint16_t)rec;
+            else static_cast<uint8_t *>(a.decisions)[at] = (uint8_t)rec;
+        }
+        __syncwarp();
+        l.moved = moved_classes(l.cls, a.G, [&](int g) { return smem[l.pi + g]; });
+    }
+}
+
+// One warp per candidate that has an open boundary or relabelled segments: goes through the
+// segments in order with the translation of their labels into group numbers, and translates
+// their records.  At a failed boundary, and at a segment in other labels in which a group number
+// decided between different states, it walks from the true state (under the true labels)
+// until what is stored can take over.  After it, every segment was simulated from a state
+// equivalent to the true one under a translation that is exact for it: the result does
+// not depend on the chunking or the rounds.
+template <bool kLegacy, bool kTwins>
+__global__ void __launch_bounds__(kWindowWarps * kLanes, kWindowBlocksPerSm)
+finish_kernel(const __grid_constant__ KernelArgs a)
+{
+    if (!can_chunk(a) || a.N == 0) return;
+    const int lane = threadIdx.x & (kLanes - 1);
+    const int64_t b = (int64_t)blockIdx.x * kWindowWarps + threadIdx.x / kLanes;
+    const bool mine = b < a.B && (a.open[b] || a.relabelled[b]);
+    if (!__syncthreads_or(mine)) return;
+    window_stage_table<kLegacy>(a);
+    if (!mine) return;
+    const size_t B = (size_t)a.B;
+    Window w;
+    window_setup<kLegacy, kTwins>(a, w, b);
+    Labels l;
+    l.pi = w.labels;
+    l.tmp = w.re.perm;
+    l.cls = a.twin_class + (size_t)b * a.G;
+    labels_reset(l, a.G);
+    int32_t q = a.seg_per_chunk;             // chunk 0 is the true run
+    for (;;) {
+        if (!l.moved) q = next_event(a, b, q);
+        if (q >= a.NS) break;
+        const size_t cell = (size_t)q * B + b;
+        const int32_t j = q / a.seg_per_chunk;
+        const bool first = q % a.seg_per_chunk == 0;
+        if (!first || a.link[(size_t)j * B + b]) {
+            uint64_t moved = l.moved;
+            const bool other = a.rel[cell] != 0;
+            if (other) moved = labels_through(l, a.G, a.perm + cell * a.G);
+            if (!(moved && (a.tie[cell] & moved))) {
+                if (other) labels_take(l, a.G, moved);
+                if (l.moved) name_segment(a, b, l, q);
+                ++q;
+                continue;
+            }
+        }
+        // from the true state, under the true labels (l.pi is still that of segment q - 1)
+        for (int g = lane; g < a.G; g += kLanes) {
+            const uint32_t from = SM_U32(w.info + g), to = SM_U32(w.info + smem[l.pi + g]);
+            for (uint32_t k = 0; k < ((from >> 8) & 0xFFu); ++k)
+                WIN_CLOCK(w, (to & 0xFFu) + k) =
+                    a.seg_end[((size_t)(q - 1) * a.T + (from & 0xFFu) + k) * B + b];
+        }
+        __syncwarp();
+        if (first)
+            for (int t = lane; t < a.T; t += kLanes)
+                a.chunk_start[((size_t)j * a.T + t) * B + b] = WIN_CLOCK(w, t);
+        if (lane == 0) {
+            a.rel[cell] = 0;
+            if (a.resimulated) atomicAdd(&a.resimulated[b], 1);
+        }
+        __syncwarp();
+        const int32_t e = window_run<kLegacy, kTwins>(a, w, kWalkChain, j, a.leaf_start[seg_leaf(a, q)], true, q);
+        labels_reset(l, a.G);
+        q = e;
+    }
+    if (w.status) atomicOr(&a.status[b], w.status);
+}
+
+// Stack machine over leaves [l0, l1) of candidate b: their sums combined in numpy's
+// pairing order as far as the merges stay inside the range (a subtree).
+__device__ inline double sum_subtree(const KernelArgs &a, int64_t b, const uint8_t *leaf_merges,
+                                     int32_t l0, int32_t l1, bool &bad)
+{
     double stack[kMaxSumDepth];
     int sp = 0;
-    int32_t q = -1, seg_stop = 0;        // leaves [.., seg_stop) belong to segment q
-    int64_t from = b;
-    for (int32_t base = 0; base < num_leaves; base += 8) {
+    for (int32_t base = l0; base < l1; base += 8) {
         double v[8];
         uint8_t mg[8];
 #pragma unroll
-        for (int u = 0; u < 8; ++u) {
-            const int32_t leaf = base + u < num_leaves ? base + u : num_leaves - 1;
-            while (leaf >= seg_stop) {
-                if (!a.seg_src) { seg_stop = num_leaves; break; }
-                ++q;
-                const int32_t src = a.seg_src[(size_t)q * a.B + b];
-                from = src >= 0 ? src : b;
-                seg_stop = seg_leaf(a, q + 1);
-            }
-            v[u] = a.leaf_sums[(size_t)leaf * a.B + from];
+        for (int u = 0; u < 8; ++u) {            // fetched together, so that the loads overlap
+            const int32_t leaf = base + u < l1 ? base + u : l1 - 1;
+            v[u] = a.leaf_sums[(size_t)leaf * a.B + b];
             mg[u] = leaf_merges[leaf];
         }
 #pragma unroll
         for (int u = 0; u < 8; ++u) {
-            if (base + u >= num_leaves) break;
+            if (base + u >= l1) break;
             if (sp < kMaxSumDepth) stack[sp] = v[u];
             ++sp;
+            // the merges behind a subtree's last leaf that reach beyond it are its parents'
             for (int k = mg[u]; k > 0 && sp >= 2; --k) {
                 --sp;
                 if (sp < kMaxSumDepth) stack[sp - 1] = stack[sp - 1] + stack[sp];
             }
         }
     }
-    if (sp > kMaxSumDepth) atomicOr(&a.status[b], MMS_STATUS_BAD_INDEX);
-    latency_sum[b] = (num_leaves > 0) ? stack[0] : 0.0;
+    bad |= sp > kMaxSumDepth;
+    return sp > 0 ? stack[0] : 0.0;
 }
 
-// One thread per scored candidate: the latency sum, and the total of the good
+// The latency sum of candidate b in numpy's pairing order (controller.py:402 consumes the
+// mean), by the lanes of a warp: numpy splits n elements at n / 2 rounded down to a multiple
+// of eight while there are more than 128, so the first levels of the tree are known from N
+// alone and lane k sums the k-th of up to 32 subtrees; the levels above are left + right.
+// (One thread alone took 125 us for 256 leaves: a dependent chain of loads.)
+__device__ inline void sum_leaves(const KernelArgs &a, int64_t b, const uint8_t *leaf_merges,
+                                  double *latency_sum)
+{
+    const int lane = threadIdx.x & (kLanes - 1);
+    int depth = 0;                                   // every node above this level is split
+    while (depth < 5 && (a.N >> (depth + 1)) > 160) ++depth;
+    int64_t base = 0, n = a.N;
+    for (int d = depth - 1; d >= 0; --d) {
+        int64_t half = n / 2;
+        half -= half % 8;
+        if ((lane >> d) & 1) { base += half; n -= half; } else n = half;
+    }
+    bool bad = false;
+    double v = 0.0;
+    if (lane < (1 << depth)) {
+        const int32_t l0 = leaf_lower_bound(a.leaf_start, a.num_leaves, base);
+        const int32_t l1 = leaf_lower_bound(a.leaf_start, a.num_leaves, base + n);
+        v = sum_subtree(a, b, leaf_merges, l0, l1, bad);
+    }
+    for (int d = 0; d < depth; ++d) {
+        const double right = __shfl_down_sync(0xFFFFFFFFu, v, 1 << d);
+        if ((lane & ((2 << d) - 1)) == 0) v = v + right;
+    }
+    if (bad) atomicOr(&a.status[b], MMS_STATUS_BAD_INDEX);
+    if (lane == 0) latency_sum[b] = v;
+}
+
+// One warp per candidate: the latency sum, and the total of the good
 // requests (controller.py:401) from the per-model counts.
 __global__ void finalize_kernel(const KernelArgs a, const uint8_t *leaf_merges,
                                 const int32_t *model_num_good, int64_t *good_total,
                                 double *latency_sum)
 {
-    const int64_t b = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (b >= a.Bs) return;
+    const int64_t b = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / kLanes;
+    if (b >= a.B) return;
     sum_leaves(a, b, leaf_merges, latency_sum);
-    int64_t total = 0;
-    for (int m = 0; m < a.M; ++m) total += model_num_good[(size_t)b * a.M + m];
-    good_total[b] = total;
+    int32_t total = 0;
+    for (int m = threadIdx.x & (kLanes - 1); m < a.M; m += kLanes) total += model_num_good[(size_t)b * a.M + m];
+    total = __reduce_add_sync(0xFFFFFFFFu, total);
+    if ((threadIdx.x & (kLanes - 1)) == 0) good_total[b] = total;
 }
 
 // Tallies the recorded decisions of the runs that count (controller.py:587,
@@ -671,19 +748,17 @@ __global__ void finalize_kernel(const KernelArgs a, const uint8_t *leaf_merges,
 // lane, so their decisions of one request are one 64-byte access) over a
 // range of at most 32 segments (fewer than 65 536 requests); each lane counts
 // in its own 16-bit shared-memory histograms and adds them to the
-// outputs (good_total among them), which must be zero on entry.  One more row
-// of blocks (blockIdx.y == 0, so that it starts first) forms the candidates'
-// latency sums beside the tally: that walk is one dependent chain per
-// candidate and hides under it.
+// outputs (good_total among them), which must be zero on entry.  32 more rows
+// of blocks (the first ones) form the candidates' latency sums beside the tally, a warp each.
 template <typename Dec>
 __global__ void __launch_bounds__(kLanes)
 count_kernel(const KernelArgs a, int32_t seg_per_block, bool group_good, int32_t *model_num_good,
              int32_t *group_num_requests, int32_t *group_num_good, int64_t *good_total,
              const uint8_t *leaf_merges, double *latency_sum)
 {
-    if (blockIdx.y == 0) {
-        const int64_t c = (int64_t)blockIdx.x * kLanes + threadIdx.x;
-        if (c < a.Bs) sum_leaves(a, c, leaf_merges, latency_sum);
+    if (blockIdx.y < kLanes) {
+        const int64_t c = (int64_t)blockIdx.x * kLanes + blockIdx.y;
+        if (c < a.B) sum_leaves(a, c, leaf_merges, latency_sum);
         return;
     }
     constexpr int kAcceptedBit = 8 * sizeof(Dec) - 1;
@@ -701,15 +776,14 @@ count_kernel(const KernelArgs a, int32_t seg_per_block, bool group_good, int32_t
     for (int g = 0; g < a.G; ++g) grp[g * kLanes + lane] = 0;
     for (int h = 0; h < (a.M + 1) / 2; ++h)
         reinterpret_cast<uint32_t *>(mod)[h * kLanes + lane] = 0;
-    if (b >= a.Bs || a.num_leaves == 0) return;
+    if (b >= a.B || a.num_leaves == 0) return;
     const size_t tb = trace_base(a, b);
-    const int32_t q0 = (blockIdx.y - 1) * seg_per_block;
+    const int32_t q0 = (blockIdx.y - kLanes) * seg_per_block;
     const int32_t q1 = q0 + seg_per_block < a.NS ? q0 + seg_per_block : a.NS;
     for (int32_t q = q0; q < q1; ++q) {
-        const int32_t src = a.seg_src[(size_t)q * a.B + b];
         // four consecutive requests of a candidate are one aligned group of records
         struct alignas(4 * sizeof(Dec)) Quad { Dec r[4]; };
-        const Quad *col = static_cast<const Quad *>(a.decisions) + (src >= 0 ? src : b);
+        const Quad *col = static_cast<const Quad *>(a.decisions) + b;
         const int32_t i_begin = a.leaf_start[seg_leaf(a, q)];
         const int32_t i1 = seg_leaf(a, q + 1) < a.num_leaves ? a.leaf_start[seg_leaf(a, q + 1)]
                                                              : (int32_t)a.N;
@@ -767,7 +841,7 @@ count_kernel(const KernelArgs a, int32_t seg_per_block, bool group_good, int32_t
 __global__ void model_requests_kernel(const KernelArgs a, int32_t *model_num_requests)
 {
     const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= (int64_t)a.Bs * a.M) return;
+    if (t >= (int64_t)a.B * a.M) return;
     const int64_t b = t / a.M;
     const int m = (int)(t % a.M);
     model_num_requests[t] = a.model_hist[(a.trace_pitch > 1 ? (size_t)b * (a.M + 1) : 0) + m];

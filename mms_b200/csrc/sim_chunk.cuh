@@ -24,9 +24,6 @@ struct KernelArgs {
     const int32_t *unsorted;      // number of unsorted / non-finite positions in the trace(s)
     // placements
     int32_t B, M, G, P, T, S, C;
-    int32_t Bs;                   // candidates with outputs; [Bs, B) are mirrors
-    const int32_t *partner;       // [B] or null
-    const uint32_t *mirror_swap;  // [B][2] or null
     const uint16_t *model_off;
     const uint32_t *model_rep;
     const uint32_t *group_info;
@@ -57,25 +54,32 @@ struct KernelArgs {
                                   //   dispatched, else (group + 1) | accepted << 7 (or << 15),
                                   //   see count_kernel
     bool dec_wide;
-    uint32_t *work_count;         // [rounds]
-    uint32_t *work_items;         // [B * K]: chunk * B + candidate; bit 31 = continue a repair
-    int32_t *repair_from;         // [K][B]: segment a capped repair of chunk j stopped at, or -1
-    int32_t *seg_src;             // [NS][B]: whose run of segment q counts for candidate b (its
-                                  //          own or one of its mirrors'); -1 = its own
-    uint8_t *own_rewritten;       // [K][B]: a repair has written into candidate b's own arrays of
-                                  //         chunk j (they are no longer its speculative run from
-                                  //         the chunk's first segment to its last)
-    uint16_t *compat;             // [K][B]: for run u of chunk j-1, the runs of chunk j whose
-                                  //         start continues u's end (bit 0: the candidate's own
-                                  //         array, bit 1 + i: its i-th mirror)
+    uint32_t *work_count;         // [kMaxRepairRounds] entries per round
+    uint32_t *work_next;          // [kMaxRepairRounds] next list entry to be taken, per round
+    uint32_t *work_items;         // [B * K]: chunk * B + candidate
+    uint8_t *stamp;               // [K][B]: 1 + the last round in which the chunk was walked
+    uint8_t *link;                // [K][B]: the run of chunk j continues the run of chunk j-1
+    uint8_t *open;                // [B]: some boundary of the candidate does not
+    // relabelling, see warp_relabel
+    const uint16_t *twin_class;   // [B][G]: smallest group interchangeable with the group | the
+                                  //   group's rank among those << 8
+    const uint8_t *twins;         // [B]: some group has an interchangeable one
+    uint8_t *rel;                 // [NS][B]: segment q is written in other labels than segment q-1
+    uint8_t *perm;                // [NS][B][G]: label in segment q -> label in segment q-1
+    uint64_t *tie;                // [NS][B]: classes of twins (class_bit) for which a group number
+                                  //   decided a choice in segment q between different states
+    uint32_t *swaps;              // laid out as byte decisions: twins between which a group number
+                                  //   decided, all in the same state (bit k: rank k of the class);
+                                  //   0: none.  Null: no candidate has twins
+    uint8_t *relabelled;          // [B]: some segment has one
     int32_t *seg_first_leaf;      // [NS + 1]: first leaf of each segment
-    int32_t narrow_limit;         // repairs of at most this many chunks (or candidates) run one
-                                  //   per warp, see sim_repair_kernel
-    int32_t repair_cap;           // segments a repair may run per round
+    int32_t win_table_elems;      // entries of the window kernels' on-chip latency table; 0: off chip
+    const uint32_t *column_stages, *irregular, *group_column;    // see ClearArgs
+    bool window;                  // the speculative pass is window_stream_kernel's
     int32_t round;
     // outputs
     uint32_t *status;             // [B]
-    double *finish;               // [B][N] or null
+    double *finish;               // [B][N], or null: no per-request outputs wanted
     uint8_t *good;                // [B][N] or null
     int32_t *resimulated;         // [B] or null
 };
@@ -113,40 +117,16 @@ __device__ inline size_t row_plane(const KernelArgs &a)
     return (size_t)((a.B + kLanes - 1) / kLanes) * (a.M + 1) * kLanes;
 }
 
-// The mirrors of scored candidate b are candidates [first, end): returns
-// first and sets end (first == end: none).
-__device__ inline int64_t mirrors_of(const KernelArgs &a, int64_t b, int64_t &end)
-{
-    end = 0;
-    if (!a.partner || a.Bs == a.B) return 0;
-    const int64_t first = a.partner[b];
-    if (first < a.Bs || first >= a.B) return 0;
-    int64_t m = first;
-    while (m < a.B && a.partner[m] == b) ++m;
-    end = m;
-    return first;
-}
-
-// Row of the status output candidate b reports to: its own, or for a mirror
-// the row of the candidate it mirrors (outputs have Bs rows).
-__device__ inline int64_t status_row(const KernelArgs &a, int64_t b)
-{
-    if (b < a.Bs) return b;
-    const int32_t p = a.partner ? a.partner[b] : 0;
-    return (p >= 0 && p < a.Bs) ? p : 0;
-}
-
 // True when the trace can be cut (sorted, finite arrival times).
 __device__ inline bool can_chunk(const KernelArgs &a)
 {
     return a.K > 1 && *a.unsorted == 0;
 }
 
-// Offset of request 0 of the trace candidate b simulates (a mirror: the trace
-// of the candidate it mirrors).
+// Offset of request 0 of the trace candidate b simulates.
 __device__ inline size_t trace_base(const KernelArgs &a, int64_t b)
 {
-    return a.trace_pitch > 1 ? (size_t)status_row(a, b) : 0;
+    return a.trace_pitch > 1 ? (size_t)b : 0;
 }
 
 // Arrival time of request i in candidate b's trace.
@@ -202,57 +182,157 @@ __device__ inline bool states_equivalent(const KernelArgs &a, int64_t b, LoadX X
     return true;
 }
 
-// Runs chunk j of candidate b on this lane: requests [begin, first) as run-in
-// (nothing recorded; `first` is the chunk's first request), then the chunk's
-// segments, recording decisions, per-request outputs (kFull) and one latency
-// sum per leaf.  Within a leaf the latency of request k goes to partial sum
-// k mod 8, as numpy's pairwise sum does: the eight partial sums rotate
-// through p0 so that the loop holds ONE copy of the step.
+// The same with the lanes of a warp over the groups: X(slot) and Z(slot) give the two
+// states, info(g) the group table.  The answer is the same in all lanes.
+template <typename Info, typename LoadX, typename LoadZ>
+__device__ inline bool warp_equivalent(int G, Info info, LoadX X, LoadZ Z, double tau)
+{
+    const int lane = threadIdx.x & (kLanes - 1);
+    uint32_t any_stale = 0;
+    for (int g0 = 0; g0 < G; g0 += kLanes) {
+        const int g = g0 + lane;
+        const uint32_t in = g < G ? info(g) : 0u;
+        const uint32_t slot = in & 0xFFu, ns = (in >> 8) & 0xFFu;
+        bool bad = false, stale = false;
+        for (uint32_t k = 0; k < ns; ++k) {
+            const double x = X(slot + k), z = Z(slot + k);
+            const bool past = x < tau && z < tau;
+            bad |= !(x == z || past);
+            if (k == ns - 1) stale = past && x != z && ((in >> 16) & 1u);
+        }
+        if (__any_sync(0xFFFFFFFFu, bad)) return false;
+        any_stale |= __ballot_sync(0xFFFFFFFFu, stale);
+    }
+    if (!any_stale) return true;
+    for (int u = 0; u < G; ++u) {
+        const uint32_t iu = info(u);
+        const uint32_t nu = (iu >> 8) & 0xFFu;
+        if (nu == 0 || !((iu >> 16) & 1u)) continue;
+        const uint32_t su = (iu & 0xFFu) + nu - 1;
+        const double xu = X(su), zu = Z(su);
+        if (xu == zu || !(xu < tau && zu < tau)) continue;
+        bool bad = false;
+        for (int g = lane; g < G; g += kLanes) {
+            const uint32_t in = info(g);
+            const uint32_t ns = (in >> 8) & 0xFFu;
+            if (ns == 0 || !((in >> 16) & 1u)) continue;
+            const uint32_t sv = (in & 0xFFu) + ns - 1;
+            const double xv = X(sv), zv = Z(sv);
+            bad |= (xu < xv) != (zu < zv) || (xu > xv) != (zu > zv);
+        }
+        if (__any_sync(0xFFFFFFFFu, bad)) return false;
+    }
+    return true;
+}
+
+// RELABELLING.  Groups with the same parallel config and the same models (twins, found
+// on the device: twins_kernel) are interchangeable, and which of them is ahead depends on
+// history long past: a speculative run often comes out with their roles exchanged.
+// Such a run is the true one under other labels.  Let Z be the state it starts
+// from, X the true state, and p a permutation within the classes of twins with X ~ p(Z) (equivalent
+// in the sense above after p has moved every group's clocks).  Then the run makes, request by
+// request, the choice p would translate into the true one — the replicas of a model are
+// closed under p, their latencies are the same, the smallest last-stage clock is the
+// same — EXCEPT where the smallest clock belongs to several replicas and the group number
+// decides (bursts of requests with one arrival time do that all the time).  Mostly those are
+// twins in the same state, all clocks alike: then any of them can stand for any other, and p
+// is replaced, from that request on, by the permutation with two of them exchanged that
+// translates the run's choice into the true one.  The simulation notes these requests (`swaps`).
+// Where the replicas are not in the same state it notes their classes for the segment
+// (`tie`), and a segment is only taken over under labels that leave those classes alone.
+// finish_kernel translates the decision records into group numbers; nothing else has labels.
 //
-//   speculative (repair == false): the clock vector after the run-in is
-//       stored as the chunk's start state, and every segment's end state.
-//   repair: the lane's clocks already hold the true state at `first`.  After
-//       each segment the new state is compared with the states stored runs
-//       had at that point (the run selected for the segment so far, the
-//       mirrors [m_first, m_end) of the candidate and, with own_pure, the
-//       candidate's own speculative run where another run is selected); once
-//       it is equivalent to one, the rest of the chunk is taken from that run
-//       (seg_src) and the lane stops.  own_pure: no repair has written into
-//       the candidate's own arrays of this chunk before this one, so behind
-//       the segment being compared they still hold the speculative run.
-//       The segments a repair runs become the candidate's own.  A repair
-//       may start at a later segment q_begin of the chunk (its clocks then
-//       hold the state after segment q_begin - 1) and may be capped at `cap`
-//       segments (0 = no cap).
-// Returns -1 when the chunk is finished (ran to its end, or settled), else
-// the segment at which the capped repair has to be continued.
+// p has to keep the order of the last-stage clocks within a class (every group of a class serves
+// a replicated model), so it is the one that sorts them, equal ones by group number.
 //
-// kStaged (with kSlim): the step that lets the warp decode ahead (staged_step);
-// every lane of the warp must be here, set up as lane 0 (see sim_core.cuh).
-template <bool kFull, bool kGroupGood, bool kLegacy, bool kNarrow = false, bool kSlim = false,
-          bool kStaged = false>
-__device__ inline int32_t run_chunk(const KernelArgs &a, Lane &ln, Pipe &p,
-                                    int64_t b, int32_t j, int32_t begin,
-                                    bool repair, bool snapshots, uint32_t old_state,
-                                    uint32_t stale_buf, int32_t q_begin = -1, int32_t cap = 0,
-                                    uint64_t swap_pairs = ~0ull, int64_t m_first = 0,
-                                    int64_t m_end = 0, bool own_pure = false)
+// Writes p (label of Z -> label of X; u8[G], and the identity for groups without twins) and
+// p(Z) to shared memory; `last` (f64[G]) and `rank` (u8[2G]) are scratch there.  Y is the saved
+// state, entries `pitch` apart.  Returns whether p is not the identity.
+struct RelabelScratch { uint32_t z, last, perm, rank; };       // f64, f64, u8, u8 indices
+
+template <typename Info, typename LoadX>
+__device__ inline bool warp_relabel(int G, int T, const uint16_t *cls, Info info, LoadX X,
+                                    const double *Y, size_t pitch, const RelabelScratch &s)
+{
+    const int lane = threadIdx.x & (kLanes - 1);
+    __syncwarp();
+    for (int g = lane; g < G; g += kLanes) {
+        const uint32_t in = info(g);
+        const uint32_t ns = (in >> 8) & 0xFFu;
+        SM_F64(s.last + g) = ns ? Y[(size_t)((in & 0xFFu) + ns - 1) * pitch] : 0.0;
+    }
+    __syncwarp();
+    for (int g = lane; g < G; g += kLanes) {
+        const uint32_t in = info(g);
+        const uint32_t ns = (in >> 8) & 0xFFu;
+        const uint32_t c = cls[g] & 0xFFu;
+        const double x = ns ? X((in & 0xFFu) + ns - 1) : 0.0, y = SM_F64(s.last + g);
+        uint32_t rx = 0, ry = 0;
+        for (int h = (int)c; h < G; ++h) {                // members of the class: c is its smallest
+            if ((cls[h] & 0xFFu) != c || h == g) continue;
+            const uint32_t ih = info(h);
+            const double xh = X((ih & 0xFFu) + ((ih >> 8) & 0xFFu) - 1), yh = SM_F64(s.last + h);
+            rx += xh < x || (xh == x && h < g);
+            ry += yh < y || (yh == y && h < g);
+        }
+        smem[s.rank + g] = (uint8_t)rx;
+        smem[s.rank + G + g] = (uint8_t)ry;
+    }
+    __syncwarp();
+    bool moved = false;
+    for (int g = lane; g < G; g += kLanes) {
+        const uint32_t c = cls[g] & 0xFFu, r = smem[s.rank + G + g];
+        int to = g;
+        for (int h = (int)c; h < G; ++h)
+            if ((cls[h] & 0xFFu) == c && smem[s.rank + h] == r) { to = h; break; }
+        smem[s.perm + g] = (uint8_t)to;
+        moved |= to != g;
+        const uint32_t ig = info(g), it = info(to);
+        for (uint32_t k = 0; k < ((ig >> 8) & 0xFFu); ++k)
+            SM_F64(s.z + (it & 0xFFu) + k) = Y[(size_t)((ig & 0xFFu) + k) * pitch];
+    }
+    (void)T;
+    __syncwarp();
+    return __any_sync(0xFFFFFFFFu, moved);
+}
+
+// Bit of a class of twins in a tie mask (more than 64 classes share bits, which only costs
+// re-simulations).
+__device__ __forceinline__ uint64_t class_bit(uint16_t twin_class) { return 1ull << (twin_class & 63u); }
+
+// Classes that a permutation moves, by a warp: perm(g) is the image of group g.
+template <typename Perm>
+__device__ inline uint64_t moved_classes(const uint16_t *twin_class, int G, Perm perm)
+{
+    uint64_t moved = 0;
+    for (int g = threadIdx.x & (kLanes - 1); g < G; g += kLanes)
+        if (perm(g) != (uint8_t)g) moved |= class_bit(twin_class[g]);
+    const uint32_t lo = __reduce_or_sync(0xFFFFFFFFu, (uint32_t)moved);
+    const uint32_t hi = __reduce_or_sync(0xFFFFFFFFu, (uint32_t)(moved >> 32));
+    return ((uint64_t)hi << 32) | lo;
+}
+
+// Runs chunk j of candidate b on this lane, speculatively: requests [begin, first)
+// as run-in (nothing recorded; `first` is the chunk's first request), then the
+// chunk's segments, recording decisions, per-request outputs (kFull) and one latency
+// sum per leaf.  With `snapshots` the clock vector after the run-in is stored as the
+// chunk's start state, and every segment's end state.  Within a leaf the latency
+// of request k goes to partial sum k mod 8, as numpy's pairwise sum does.
+template <bool kFull, bool kLegacy, bool kTwins>
+__device__ inline void run_chunk(const KernelArgs &a, Lane &ln, Pipe &p, int64_t b, int32_t j,
+                                 int32_t begin, bool snapshots)
 {
     double *fin_out = kFull ? a.finish + (size_t)b * a.N : nullptr;
     uint8_t *good_out = kFull ? a.good + (size_t)b * a.N : nullptr;
-    const int32_t q0 = q_begin >= 0 ? q_begin : j * a.seg_per_chunk;
+    int32_t q = j * a.seg_per_chunk;
     const int32_t q1 = (j + 1) * a.seg_per_chunk < a.NS ? (j + 1) * a.seg_per_chunk : a.NS;
-    int32_t q = q0;
-    int32_t leaf = seg_leaf(a, q0);
-    int32_t seg_stop = seg_leaf(a, q0 + 1);
+    int32_t leaf = seg_leaf(a, q);
+    int32_t seg_stop = seg_leaf(a, q + 1);
     const int32_t first = leaf < a.num_leaves ? a.leaf_start[leaf] : (int32_t)a.N;
     leaf -= 1;                      // the run-in counts as a leaf that is not recorded
     int32_t i = begin, span_end = first;
     bool record = false;
-    int32_t done = 0;
-    static_assert(!kStaged || kSlim, "the staged step is a form of the slim step");
-    Staged st;
-    if constexpr (kStaged) st = staged_init(ln); else pipe_prime(ln, p, begin);
+    pipe_prime(ln, p, begin);
     for (;;) {
         // Within a leaf the latency of request k goes to partial sum k mod 8
         // (leaves start at multiples of 8).  The latencies of eight requests
@@ -264,12 +344,7 @@ __device__ inline int32_t run_chunk(const KernelArgs &a, Lane &ln, Pipe &p,
         double p0 = 0.0, p1 = 0.0, p2 = 0.0, p3 = 0.0, p4 = 0.0, p5 = 0.0, p6 = 0.0, p7 = 0.0;
         double r = 0.0;
         auto one = [&](int32_t ii) {
-            double d;
-            if constexpr (kStaged)
-                d = staged_step(ln, p, st, ii, record);
-            else
-                d = sim_step<kFull, kGroupGood, kLegacy, kNarrow, kSlim>(ln, p, ii, record,
-                                                                         fin_out, good_out);
+            const double d = sim_step<kFull, kLegacy, kTwins>(ln, p, ii, record, fin_out, good_out);
             if (ii < body_end) {
                 SM_F64(ring + (uint32_t)(ii & 7) * kLanes) = d;
                 if ((ii & 7) == 7) {
@@ -284,93 +359,34 @@ __device__ inline int32_t run_chunk(const KernelArgs &a, Lane &ln, Pipe &p,
                 r += d;
             }
         };
-#ifndef MMS_SLIM_UNROLL
-#define MMS_SLIM_UNROLL 1
-#endif
-#ifndef MMS_WIDE_UNROLL
-#define MMS_WIDE_UNROLL 1
-#endif
-        if constexpr ((kSlim && !kStaged && MMS_SLIM_UNROLL) || (!kNarrow && MMS_WIDE_UNROLL)) {
-            // three requests per turn: the values fetched ahead rotate through three sets of
-            // registers, and after three steps every set is back where it was — no moves (two
-            // dozen per request otherwise; in the 32-candidate kernels as well: stream kernel
-            // 17.0 -> 16.1 ms)
-            for (; i + 3 <= span_end; i += 3) { one(i); one(i + 1); one(i + 2); }
-        }
+        // three requests per turn: the values fetched ahead rotate through three sets of
+        // registers, and after three steps every set is back where it was — no moves (two
+        // dozen per request otherwise: stream kernel 17.0 -> 16.1 ms)
+        for (; i + 3 <= span_end; i += 3) { one(i); one(i + 1); one(i + 2); }
 #pragma unroll 1
         for (; i < span_end; ++i) one(i);
         if (!record) {
-            // a mirror starts its chunk with interchangeable groups exchanged
-            for (int k = 0; k < 4 && swap_pairs != ~0ull; ++k) {
-                const uint32_t ga = (uint32_t)(swap_pairs >> (16 * k)) & 0xFFu;
-                const uint32_t gb = (uint32_t)(swap_pairs >> (16 * k + 8)) & 0xFFu;
-                if (ga >= (uint32_t)a.G || gb >= (uint32_t)a.G) continue;
-                const uint32_t ia = a.group_info[(size_t)b * a.G + ga];
-                const uint32_t ib = a.group_info[(size_t)b * a.G + gb];
-                const uint32_t ns = (ia >> 8) & 0xFFu;
-                if (ns != ((ib >> 8) & 0xFFu)) continue;
-                for (uint32_t t = 0; t < ns; ++t) {
-                    const uint32_t sa = ln.clk + ((ia & 0xFFu) + t) * kLanes;
-                    const uint32_t sb = ln.clk + ((ib & 0xFFu) + t) * kLanes;
-                    const double va = SM_F64(sa);
-                    SM_F64(sa) = SM_F64(sb);
-                    SM_F64(sb) = va;
-                }
-            }
-            if (!repair && snapshots)   // the state this speculative chunk starts from
+            ln.tie = 0;
+            if (snapshots)   // the state this speculative chunk starts from
                 for (int t = 0; t < a.T; ++t)
                     a.chunk_start[((size_t)j * a.T + t) * a.B + b] = SM_F64(ln.clk + t * kLanes);
         } else {
             a.leaf_sums[(size_t)leaf * a.B + b] = r;
             if (leaf + 1 == seg_stop) {             // segment q is complete
-                ++done;
-                // A repair stops when its state is equivalent to the state some
-                // stored run had at this point: the run currently selected for
-                // this segment, or a mirror's.  The rest of the chunk is then
-                // taken from that run.
-                bool settled = false, reselect = false;
-                int32_t settle_src = -1;
-                if (repair && snapshots && span_end < a.N) {
-                    const double tau = arrival_at(a, b, span_end);
-                    const int32_t cur = a.seg_src[(size_t)q * a.B + b];
-                    // r == 0: the selected run; r == 1: the own speculative run, where
-                    // another is selected; r >= 2: the mirrors
-                    for (int64_t r = 0; r <= m_end - m_first + 1 && !settled; ++r) {
-                        int64_t v;
-                        if (r == 0) v = cur < 0 ? b : cur;
-                        else if (r == 1) { if (cur < 0 || !own_pure) continue; v = b; }
-                        else { v = m_first + r - 2; if (v == cur) continue; }
-                        for (int t = 0; t < a.T; ++t)
-                            SM_F64(old_state + t * kLanes) =
-                                a.seg_end[((size_t)q * a.T + t) * a.B + v];
-                        settled = states_equivalent(
-                            a, b, [&](uint32_t s) { return SM_F64(ln.clk + s * kLanes); },
-                            [&](uint32_t s) { return SM_F64(old_state + s * kLanes); }, tau,
-                            [&](int u) -> uint8_t & { return smem[stale_buf + u * kLanes]; });
-                        if (settled && r > 0) { reselect = true; settle_src = v == b ? -1 : (int32_t)v; }
-                    }
-                }
-                // (all lanes of a staged warp run this code as copies of one another: none
-                // may overwrite what another has yet to compare)
-                if constexpr (kStaged) __syncwarp();
                 if (snapshots) {
+                    if constexpr (kTwins) {
+                        a.tie[(size_t)q * a.B + b] = ln.tie;
+                        ln.tie = 0;
+                    }
                     for (int t = 0; t < a.T; ++t)
                         a.seg_end[((size_t)q * a.T + t) * a.B + b] = SM_F64(ln.clk + t * kLanes);
-                    if (repair) a.seg_src[(size_t)q * a.B + b] = -1;
                 }
-                if (settled) {
-                    if (reselect)
-                        for (int32_t r = q + 1; r < q1; ++r)
-                            a.seg_src[(size_t)r * a.B + b] = settle_src;
-                    return -1;
-                }
-                if (++q >= q1) return -1;
-                if (cap > 0 && done >= cap) return q;
+                if (++q >= q1) return;
                 seg_stop = seg_leaf(a, q + 1);
             }
         }
         ++leaf;
-        if (leaf >= a.num_leaves) return -1;        // only an empty trace gets here
+        if (leaf >= a.num_leaves) return;        // only an empty trace gets here
         record = true;
         span_end = a.leaf_start[leaf + 1];
     }

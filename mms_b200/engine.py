@@ -390,7 +390,7 @@ class EncodedBatch:
     """Host arrays of a placement batch in the layout of mms_placements."""
 
     def __init__(self, B, M, G, P, T, S, C, model_off, model_rep, group_info, num_groups,
-                 num_replicas, twins=None):
+                 num_replicas, twins=None, has_twins=None):
         self.B, self.M, self.G, self.P, self.T, self.S, self.C = B, M, G, P, T, S, C
         self.model_off = model_off        # u16[B][M+1]
         self.model_rep = model_rep        # u32[B][P]
@@ -400,7 +400,12 @@ class EncodedBatch:
         # (candidate index, [[group ids of one class of interchangeable groups], ...])
         # for every placement that has such groups, see twin_groups()
         self.twins = twins
+        # bool[B]: the placement has interchangeable groups at all (None: not known)
+        self.has_twins = has_twins
         self._mirror_table = None         # see mirror_table()
+
+    def may_have_twins(self):
+        return self.has_twins is None or bool(np.any(self.has_twins))
 
     def mirror_table(self):
         """(counts i64[len(twins)], words u64[sum(counts)]): the exchange lists of
@@ -419,7 +424,8 @@ class EncodedBatch:
         twins = [(int(new_id[self.twins[k][0]]), self.twins[k][1]) for k in keep]
         sub = EncodedBatch(len(index), self.M, self.G, self.P, self.T, self.S, self.C,
                            self.model_off[index], self.model_rep[index], self.group_info[index],
-                           self.num_groups[index], self.num_replicas[index], twins)
+                           self.num_groups[index], self.num_replicas[index], twins,
+                           None if self.has_twins is None else self.has_twins[index])
         if self._mirror_table is not None:
             counts, words = self._mirror_table
             keep = np.asarray(keep, np.int64)
@@ -439,7 +445,8 @@ class EncodedBatch:
         return EncodedBatch(B * count, self.M, self.G, self.P, self.T, self.S, self.C,
                             np.tile(self.model_off, (count, 1)), np.tile(self.model_rep, (count, 1)),
                             np.tile(self.group_info, (count, 1)), np.tile(self.num_groups, count),
-                            np.tile(self.num_replicas, count), twins)
+                            np.tile(self.num_replicas, count), twins,
+                            None if self.has_twins is None else np.tile(self.has_twins, count))
 
     def with_mirrors(self):
         """The tables with mirror candidates appended for every placement
@@ -715,6 +722,7 @@ def _encode_native(H, B, M, table, n_groups, cfg, n_in_group, placed_model) -> E
     slots = np.zeros(max(B, 1), np.int64)
     items = np.empty((max(tot_groups, 1), 3), np.int32)
     n_items = np.zeros(1, np.int64)
+    has_twins = np.zeros(max(B, 1), np.uint8)
     counts = np.zeros(M + 1, np.int64)
     mark = np.zeros(max(M, 1), np.int64)
     n_groups = np.ascontiguousarray(n_groups, np.int64)
@@ -722,7 +730,7 @@ def _encode_native(H, B, M, table, n_groups, cfg, n_in_group, placed_model) -> E
                            cfg_index.ctypes.data, column_of.ctypes.data, n_in_group.ctypes.data,
                            placed_model.ctypes.data, model_off.ctypes.data, model_rep.ctypes.data,
                            group_info.ctypes.data, slots.ctypes.data, items.ctypes.data,
-                           n_items.ctypes.data, counts.ctypes.data, mark.ctypes.data,
+                           n_items.ctypes.data, has_twins.ctypes.data, counts.ctypes.data, mark.ctypes.data,
                            MAX_MIRRORS + 1)
     if rc == 1:
         raise IndexError("model id in group_models is out of range")
@@ -739,7 +747,7 @@ def _encode_native(H, B, M, table, n_groups, cfg, n_in_group, placed_model) -> E
         twins[-1][1][-1].append(g)
         prev_b, prev_c = b, c
     return EncodedBatch(B, M, Gc, Pc, max(T, 1), S, C, model_off, model_rep, group_info,
-                        n_groups, placed_per_b.astype(np.int64), twins)
+                        n_groups, placed_per_b.astype(np.int64), twins, has_twins[:B].astype(bool))
 
 
 def encode_placements(placements: Sequence, table: LatencyTable, num_models: int,
@@ -1050,15 +1058,9 @@ def _launch(*args, rows_on_device=False, **kwargs):
     return _collect(_submit(*args, **kwargs), rows_on_device)
 
 
-SPLIT_MIN_EASY = 512      # placements without mirrors a batch must have to be split
-SPLIT_MIN_HARD = 32       # ... and placements with mirrors
-# Run-in of the launch that holds the placements with mirrors, when a batch is split (the
-# library's default is 2048): the few chunks of these placements that no stored run continues
-# are re-simulated one after the other by single lanes, and the longest such chain decides when
-# the launch ends.  A longer run-in makes its speculative pass longer (which delays the other
-# launch's) and those chains shorter.  Measured over four candidate lists, slowest / mean step:
-# 24.7 / 22.6 ms with 2048, 22.6 / 22.0 ms with 2560, 22.9 / 22.3 ms with 3072.
-HARD_RUN_IN = 2560
+# A batch is split when it has at least so many placements without interchangeable groups
+SPLIT_MIN_EASY = 512
+SPLIT_MIN_HARD = 32       # ... and so many with such groups
 _SIDE_STREAMS = {}
 
 
@@ -1076,37 +1078,34 @@ class ResidentBatch:
     """An encoded batch with its tables, scratch and outputs on the GPU, ready
     to be launched (any number of times).
 
-    A batch whose placements partly have mirrors is launched as TWO calls of
-    mms_sim_mixed on two side streams: the placements with mirrors first, cut
-    into many short chunks, and the rest beside them.  The first finish their
-    speculative pass early, and their repair rounds — a few long, serial
-    re-simulations that leave the GPU almost idle — run while the rest are
-    still in theirs.  Results are the same as from one call."""
+    A batch whose placements partly have interchangeable groups is launched as
+    TWO calls of mms_sim_mixed on two side streams: those placements first, and
+    the rest, for which the library then needs no bookkeeping of such groups
+    (FLAG_NO_TWINS), beside them.  The first are few and finish their
+    speculative pass early; their repairs — serial re-simulations that leave
+    the GPU almost idle — run while the rest are still in theirs.  Results
+    are the same as from one call."""
 
     def __init__(self, trace, enc: EncodedBatch, table: LatencyTable, group_good=False,
                  pinned=False, options=None, mirrors=True, split=True, crowded=False,
                  hard_options=None, launch_now=False):
-        """crowded: other launches will be filling the GPU while this batch
+        """mirrors: False = the library does not look for interchangeable groups
+        (slower on placements that have them).
+        crowded: other launches will be filling the GPU while this batch
         repairs its chunks (a pipelined part that is not the last).
         hard_options: sim_options for the launch that holds the placements with
-        mirrors, when the batch is split (default: `options`).
+        interchangeable groups, when the batch is split (default: `options`).
         launch_now: every call is enqueued as soon as its tables are uploaded
         (as launch() would afterwards), so that the GPU starts on the first
         while the host prepares the second."""
         self.trace, self.enc = trace, enc
         dev = trace.device
-        ext_owner = []
-        if mirrors and enc.twins:
-            counts, _ = enc.mirror_table()
-            ext_owner = [b for (b, _), c in zip(enc.twins, counts.tolist()) if c]
         parts = [(None, enc)]
-        if (split and len(ext_owner) >= SPLIT_MIN_HARD
-                and enc.B - len(ext_owner) >= SPLIT_MIN_EASY):
-            hard = np.asarray(ext_owner, np.int64)
-            rest = np.ones(enc.B, bool)
-            rest[hard] = False
-            easy = np.flatnonzero(rest)
-            parts = [(hard, enc.take(hard)), (easy, enc.take(easy))]
+        if split and mirrors and enc.has_twins is not None:
+            hard = np.flatnonzero(enc.has_twins)
+            if len(hard) >= SPLIT_MIN_HARD and enc.B - len(hard) >= SPLIT_MIN_EASY:
+                easy = np.flatnonzero(~enc.has_twins)
+                parts = [(hard, enc.take(hard)), (easy, enc.take(easy))]
         self.index = [p[0] for p in parts]
         self.jobs = []
         self.h2d_bytes = 0
@@ -1119,23 +1118,11 @@ class ResidentBatch:
         for k, (_, e) in enumerate(parts):
             # the first of two calls repairs while the second one fills the GPU
             flags = nat.FLAG_CROWDED if (crowded or k + 1 < len(parts)) else 0
-            # (the second of two parts holds the placements without mirrors)
-            ext = e.with_mirrors() if mirrors and not (len(parts) > 1 and k == 1) else None
-            opts_k = options
-            if len(parts) > 1 and k == 0:
-                if hard_options is not None:
-                    opts_k = hard_options
-                elif options is None or options.warmup_requests == 0:
-                    o = options if options is not None else sim_options()
-                    opts_k = sim_options(o.chunk_requests, HARD_RUN_IN, o.repair_rounds,
-                                         o.repair_segments)
-            if ext is not None:
-                off, rep, info, partner, swap = ext
-                job = _prepare(trace, len(partner), e.M, e.G, e.P, e.T, e.S, e.C, off, rep, info,
-                               lat, 0, flags, group_good, pinned, opts_k, e.B, partner, swap)
-            else:
-                job = _prepare(trace, e.B, e.M, e.G, e.P, e.T, e.S, e.C, e.model_off, e.model_rep,
-                               e.group_info, lat, 0, flags, group_good, pinned, opts_k)
+            if not mirrors or not e.may_have_twins():
+                flags |= nat.FLAG_NO_TWINS
+            opts_k = hard_options if len(parts) > 1 and k == 0 and hard_options is not None else options
+            job = _prepare(trace, e.B, e.M, e.G, e.P, e.T, e.S, e.C, e.model_off, e.model_rep,
+                           e.group_info, lat, 0, flags, group_good, pinned, opts_k)
             self.jobs.append(job)
             self.h2d_bytes += job.h2d
             if launch_now:              # the GPU starts on this call while the next is prepared
@@ -1216,9 +1203,10 @@ def run_batch(trace: DeviceTrace, enc: EncodedBatch, table: LatencyTable,
               per_request=False, group_good=False, pinned=False, options=None, mirrors=True,
               split=True, crowded=False, rows_on_device=False):
     """Simulates every placement of `enc` against `trace`
-    (simulate_requests_mixed, controller.py:561-628).  `mirrors`: placements
-    with interchangeable groups get a mirror candidate (a speed-up of the
-    time-parallel execution; results are the same with and without).
+    (simulate_requests_mixed, controller.py:561-628).  `mirrors`: the library
+    may take over speculative runs in which interchangeable groups have changed
+    places (a speed-up of the time-parallel execution; results are the same
+    with and without).
     `crowded`: the MMS_FLAG_CROWDED hint (results are the same).
     `rows_on_device` (with per_request): finish and good stay on the GPU, as
     BatchResult.finish_device / .good_device."""
@@ -1228,7 +1216,8 @@ def run_batch(trace: DeviceTrace, enc: EncodedBatch, table: LatencyTable,
     return _launch(trace, enc.B, enc.M, enc.G, enc.P, enc.T, enc.S, enc.C,
                    enc.model_off, enc.model_rep, enc.group_info,
                    table.device(trace.device), 0,
-                   nat.FLAG_PER_REQUEST | (nat.FLAG_CROWDED if crowded else 0), group_good,
+                   nat.FLAG_PER_REQUEST | (nat.FLAG_CROWDED if crowded else 0)
+                   | (0 if mirrors and enc.may_have_twins() else nat.FLAG_NO_TWINS), group_good,
                    pinned, options, rows_on_device=rows_on_device)
 
 

@@ -127,14 +127,16 @@ class PlacementEvaluator:
                                         len(self.model_names), device=device)
         self.table = engine.LatencyTable(self.prof_ress)
         self.options = options          # engine.sim_options(...) or None
-        # A long list is encoded and launched in parts.  The first part only has
+        # A list of some length is encoded and launched in parts.  The first part only has
         # to cover the host's work on the second, so it is the smaller one; more
         # and smaller parts cost more on the GPU (shorter chunks, more run-in)
-        # than the encoding they hide.
+        # than the encoding they hide.  A long list (pipeline_max_list) goes out as one: what
+        # parts cost grows with it (4096 placements: 29.8 ms as one, 32.8 ms in two parts).
         self.pipeline_parts = 2
         self.pipeline_min_part = 768    # placements per part, at least
+        self.pipeline_max_list = 2048
         self.pipeline_shares = (3, 5)   # relative sizes of the parts (None: equal)
-        # placements with mirror candidates as a launch of their own inside a
+        # placements with interchangeable groups as a launch of their own inside a
         # part: one flag, or one per part.  Only the last part needs it: the
         # serial repairs of an earlier part run beside the parts behind it anyway.
         self.pipeline_split = (False, True)
@@ -153,6 +155,8 @@ class PlacementEvaluator:
         encodes the next part while the GPU simulates the previous ones."""
         n = len(sols)
         parts = max(1, min(self.pipeline_parts, n // self.pipeline_min_part))
+        if n >= self.pipeline_max_list:
+            parts = 1
         if parts == 1:
             enc = engine.encode_placements(sols, self.table, len(self.model_names))
             res, h2d, d2h = engine.run_batch(self.trace, enc, self.table, pinned=pinned,

@@ -1,0 +1,157 @@
+"""The one-candidate-per-warp engine, the walks and the relabelling of runs in which
+interchangeable groups have changed places: every output against the checker, at the
+sizes where the code branches."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _profiles(num_models, degrees, seed):
+    from mms_b200.profiling import LatencyMemData, ParallelConfig, ProfilingResult
+    rng = np.random.RandomState(seed)
+    out = []
+    for m in range(num_models):
+        base = float(rng.choice([0.02, 0.05, 0.05, 0.11]))
+        out.append(ProfilingResult(f"m{m}", {
+            ParallelConfig(1, 1, p): LatencyMemData({1: [base / p * 1.1] * p}, {1: [0.0] * p}, [1.0] * p)
+            for p in degrees}))
+    return out
+
+
+def _trace(n, num_models, rate, seed, grid=0.0):
+    """Bursty arrivals; grid > 0 rounds them, so that many requests arrive together."""
+    rng = np.random.RandomState(seed)
+    ts = np.cumsum(rng.gamma(0.15, 1 / 0.15 / rate, size=n))
+    if grid:
+        ts = np.floor(ts / grid) * grid
+    ids = np.minimum(rng.geometric(0.35, size=n) - 1, num_models).astype(np.int32)
+    ids[ids == num_models] = -1                       # requests of an unknown model
+    return ts, ids, np.full(n, 0.4, np.float32)
+
+
+def _check(placements, profs, ts, ids, slos, chunk, run_in, rounds=0, per_request=True, mirrors=True):
+    from mms_b200 import engine
+    from oracle import tables
+    M = len(profs)
+    trace = engine.DeviceTrace(ts, ids, slos, M)
+    table = engine.LatencyTable(profs)
+    enc = engine.encode_placements(placements, table, M)
+    res, _, _ = engine.run_batch(trace, enc, table, per_request=per_request, group_good=True,
+                                 options=engine.sim_options(chunk, run_in, rounds), mirrors=mirrors)
+    for b, p in enumerate(placements):
+        fin, good, mreq, mgood, greq, ggood = tables.one_placement(p, profs, ids, slos, ts)
+        if per_request:
+            assert res.finish[b].tobytes() == fin.tobytes(), b
+            assert np.array_equal(res.good[b], good), b
+        assert res.good_total[b] == np.count_nonzero(good), b
+        assert res.latency_sum[b] == float(np.add.reduce(fin - ts)), b
+        assert np.array_equal(res.model_num_requests[b], mreq), b
+        assert np.array_equal(res.model_num_good[b], mgood), b
+        assert np.array_equal(res.group_num_requests[b, :len(greq)], greq), b
+        assert np.array_equal(res.group_num_good[b, :len(ggood)], ggood), b
+    return res
+
+
+def _placement(degrees, models):
+    from mms_b200.placement import ModelPlacement
+    from mms_b200.profiling import ParallelConfig
+    return ModelPlacement([ParallelConfig(1, 1, p) for p in degrees], models)
+
+
+@pytest.mark.parametrize("groups", [1, 31, 32, 33, 63, 64, 65])
+@pytest.mark.parametrize("depth", [1, 2, 3])
+def test_group_counts_and_depths(groups, depth):
+    """A group per lane up to 32 (or two up to 64, in shallow pipelines), windows beyond;
+    depths that are powers of two and not."""
+    rng = np.random.RandomState(groups * 10 + depth)
+    M = 9
+    profs = _profiles(M, (1, depth), 1)
+    ts, ids, slos = _trace(1500, M, 6.0 * groups, 2)
+    degrees = [depth if g % 3 else 1 for g in range(groups)]
+    models = [sorted(rng.choice(M, size=rng.randint(1, 4), replace=False).tolist()) for _ in range(groups)]
+    _check([_placement(degrees, models)], profs, ts, ids, slos, 256, 64)
+
+
+@pytest.mark.parametrize("depth", [4, 8, 9])
+@pytest.mark.parametrize("groups", [3, 20, 28])
+def test_deep_pipelines(groups, depth):
+    M = 6
+    profs = _profiles(M, (1, depth), 3)
+    ts, ids, slos = _trace(1200, M, 5.0 * groups, 4)
+    degrees = [depth if g % 2 else 1 for g in range(groups)]
+    _check([_placement(degrees, [[g % M, (g + 1) % M] for g in range(groups)])], profs, ts, ids, slos,
+           384, 128)
+
+
+@pytest.mark.parametrize("replicas", [1, 4, 5, 8, 9, 32, 33, 40])
+@pytest.mark.parametrize("count", [1, 40])
+def test_numbers_of_replicas(replicas, count):
+    """Replica lists at the edges of a row, of two rows, of a warp; one placement and enough of
+    them to fill warps with candidates."""
+    M = 3
+    profs = _profiles(M, (1,), 5)
+    ts, ids, slos = _trace(1300, M, 20.0 * replicas, 6)
+    sols = [_placement([1] * (replicas + 1), [[0] + ([1] if (g + k) % 2 else []) for g in range(replicas)] + [[2]])
+            for k in range(count)]
+    _check(sols, profs, ts, ids, slos, 256, 32)
+
+
+@pytest.mark.parametrize("grid", [0.0, 0.01, 0.25])
+@pytest.mark.parametrize("chunk,run_in,rounds", [(0, 0, 0), (128, 128, 1), (512, 16, 4), (1024, 2048, 16)])
+def test_interchangeable_groups_and_equal_arrival_times(grid, chunk, run_in, rounds):
+    """Twins of one and of several stages, in classes of 2 to 33, beside groups that share some
+    of their models; with arrival times on a grid the group number decides all the time, between
+    twins in one state and between groups that are no twins."""
+    M = 5
+    profs = _profiles(M, (1, 2, 4), 7)
+    ts, ids, slos = _trace(6000, M, 120.0, 8, grid)
+    sols = [
+        _placement([1] * 8, [[0, 1]] * 4 + [[0, 2]] * 2 + [[0], [3, 4]]),
+        _placement([2] * 6 + [1] * 4, [[0, 1]] * 3 + [[1, 2]] * 3 + [[0]] * 2 + [[3, 4]] * 2),
+        _placement([4] * 5 + [1], [[0, 1, 2]] * 4 + [[3, 4], [0]]),
+        _placement([1] * 36, [[0, 1]] * 33 + [[0], [2], [3, 4]]),
+        _placement([4, 4, 2, 2, 1, 1, 1], [[0, 1]] * 2 + [[0, 1]] * 2 + [[0, 1]] * 2 + [[2, 3, 4]]),
+    ]
+    _check(sols, profs, ts, ids, slos, chunk, run_in, rounds)
+    _check(sols * 8, profs, ts, ids, slos, chunk, run_in, rounds, per_request=False)
+    _check(sols, profs, ts, ids, slos, chunk, run_in, rounds, mirrors=False)
+
+
+def test_relabelling_spares_repairs():
+    """Interchangeable groups alone do not make chunks fail: with relabelling hardly any is
+    simulated again, without it most are."""
+    M = 4
+    profs = _profiles(M, (1,), 9)
+    rng = np.random.RandomState(10)
+    ts = np.cumsum(rng.exponential(1 / 80.0, size=30000))
+    ids = rng.randint(0, M, size=30000).astype(np.int32)
+    slos = np.full(30000, 0.5, np.float32)
+    sols = [_placement([1] * 12, [[0, 1]] * 6 + [[2, 3]] * 6)]
+    with_ = _check(sols, profs, ts, ids, slos, 256, 256).resimulated.sum()
+    without = _check(sols, profs, ts, ids, slos, 256, 256, mirrors=False).resimulated.sum()
+    assert with_ * 4 < without
+
+
+def test_replica_lists_in_any_order_and_negative_times():
+    """The drop-in takes rows of m_id2g_id as they are: ties go to the first of the row, not to
+    the lowest group; arrival times may be negative."""
+    from mms_b200 import simulator
+    from oracle import cpu
+    rng = np.random.RandomState(11)
+    n, M, G, S = 3000, 4, 5, 2
+    ts = np.cumsum(rng.gamma(0.2, 0.05, size=n)) - 20.0
+    ids = rng.randint(-1, M, size=n).astype(np.int32)
+    slo = np.full(n, 0.3, np.float32)
+    ns = np.array([2, 1, 2, 1, 2], np.int32)
+    lat = rng.uniform(0.01, 0.08, size=(M, G, S)).astype(np.float32)
+    for m2g in ([[0, 1, 2, -1], [1, 3, -1, -1], [2, 4, -1, -1], [0, 1, 3, 4]],
+                [[2, 0, 1, -1], [3, 1, -1, -1], [4, 2, -1, -1], [4, 3, 1, 0]]):
+        m2g = np.array(m2g, np.int32)
+        fin = np.empty(n); good = np.empty(n, bool)
+        efin = np.empty(n); egood = np.empty(n, bool)
+        got = simulator.simulate_requests_mixed(fin, good, ts, ids, slo, m2g, ns, lat, n)
+        exp = cpu.simulate_requests_mixed(efin, egood, ts, ids, slo, m2g, ns, lat, n)
+        assert fin.tobytes() == efin.tobytes() and np.array_equal(good, egood)
+        for x, y in zip(got, exp):
+            assert np.array_equal(x, y)
