@@ -8,7 +8,9 @@ include/mms_sim.h describes.  PyTorch is used for device memory and streams
 only; all compute goes through the C ABI in libmms_sim.so.
 """
 import ctypes
+import functools
 import operator
+from contextlib import nullcontext
 from itertools import chain, permutations, product
 from math import factorial
 from typing import List, Sequence
@@ -36,6 +38,15 @@ def _stream_ptr():
     return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
 
 
+_NO_CONTEXT = nullcontext()
+
+
+def _on(dev):
+    """`dev` as the current device (entering torch.cuda.device for the device that is current
+    anyway costs as much as a kernel launch)."""
+    return _NO_CONTEXT if dev.index == torch.cuda.current_device() else torch.cuda.device(dev)
+
+
 def _to_device(arr: np.ndarray, device, pinned=False):
     t = torch.from_numpy(np.ascontiguousarray(arr))
     if pinned:
@@ -43,15 +54,23 @@ def _to_device(arr: np.ndarray, device, pinned=False):
     return t.to(device, non_blocking=pinned)
 
 
-_UPLOAD_STAGE = {}       # device -> page-locked staging buffer of _to_device_many
-_UPLOAD_STAGE_MAX = 128 << 20
+# Uploads up to this size go straight from pageable memory: the driver takes such a copy into
+# a buffer of its own before the call returns, and nothing waits for the GPU.
+_SMALL_UPLOAD = 64 << 10
+_TORCH_TYPE = {np.dtype(k): v for k, v in (
+    (np.uint8, torch.uint8), (np.uint16, torch.uint16), (np.int32, torch.int32),
+    (np.uint32, torch.uint32), (np.int64, torch.int64), (np.float32, torch.float32),
+    (np.float64, torch.float64))}
+_STAGED_UPLOAD = 128 << 20       # larger ones are not worth holding that much page-locked memory
 
 
 def _to_device_many(arrays, device):
-    """Several host arrays to the device as ONE transfer from a page-locked staging
-    buffer (kept per device): a launch uploads half a dozen small tables, and each
-    transfer from pageable memory costs tens of microseconds whatever its size.
-    Returns device tensors that are views of one buffer, each 16-byte aligned."""
+    """Several host arrays to the device as ONE transfer: a launch uploads half a
+    dozen small tables, and each transfer costs tens of microseconds whatever its
+    size.  Small ones are packed in pageable memory, larger ones in page-locked
+    memory from torch's host allocator (which keeps a block until the copies
+    from it are done).  Returns device tensors that are views of one buffer, each
+    16-byte aligned."""
     device = torch.device(device)
     arrays = [np.ascontiguousarray(a) for a in arrays]
     offsets, total = [], 0
@@ -59,24 +78,35 @@ def _to_device_many(arrays, device):
         offsets.append(total)
         total += (a.nbytes + 15) & ~15
     total = max(total, 16)
-    if total > _UPLOAD_STAGE_MAX:         # not worth holding that much page-locked memory
+    if total > _STAGED_UPLOAD:
         return [_to_device(a, device) for a in arrays]
-    stage = _UPLOAD_STAGE.get(device)
-    if stage is None or stage.numel() < total:
-        stage = torch.empty(min(max(2 * total, 1 << 20), _UPLOAD_STAGE_MAX),
-                            dtype=torch.uint8).pin_memory()
-        _UPLOAD_STAGE[device] = stage
+    small = total <= _SMALL_UPLOAD
+    stage = torch.empty(total, dtype=torch.uint8, pin_memory=not small)
     host = stage.numpy()
     for a, o in zip(arrays, offsets):
         if a.nbytes:
             host[o:o + a.nbytes] = a.reshape(-1).view(np.uint8)
     buf = torch.empty(total, dtype=torch.uint8, device=device)
-    buf.copy_(stage[:total])              # returns when the copy is done: the stage is free again
-    out = []
-    for a, o in zip(arrays, offsets):
-        dtype = torch.from_numpy(np.empty(0, a.dtype)).dtype
-        out.append(buf[o:o + a.nbytes].view(dtype).reshape(a.shape))
-    return out
+    buf.copy_(stage, non_blocking=True)
+    return [buf[o:o + a.nbytes].view(_TORCH_TYPE[a.dtype]).reshape(a.shape)
+            for a, o in zip(arrays, offsets)]
+
+
+@functools.lru_cache(maxsize=64)
+def _sum_plan(n):
+    """(leaf starts i32[leaves + 1], merges u8[max(leaves, 1)]) of numpy's pairwise sum of n
+    elements (mms_sum_plan)."""
+    L = nat.lib()
+    n_leaves = L.mms_sum_plan_leaves(n)
+    if n_leaves < 0:
+        nat.check(n_leaves, "mms_sum_plan_leaves")
+    leaf_start = np.zeros(n_leaves + 1, np.int32)
+    leaf_merges = np.zeros(max(n_leaves, 1), np.uint8)
+    nat.check(L.mms_sum_plan_fill(n, leaf_start.ctypes.data, leaf_merges.ctypes.data),
+              "mms_sum_plan_fill")
+    leaf_start.setflags(write=False)
+    leaf_merges.setflags(write=False)
+    return leaf_start, leaf_merges
 
 
 class DeviceTrace:
@@ -99,19 +129,13 @@ class DeviceTrace:
         self.host_arrivals = arrivals
         self.h2d_bytes = arrivals.nbytes + model_ids.nbytes + slos.nbytes
         L = nat.lib()
-        with torch.cuda.device(self.device):
-            n_leaves = L.mms_sum_plan_leaves(self.num_requests)
-            if n_leaves < 0:
-                nat.check(n_leaves, "mms_sum_plan_leaves")
-            leaf_start = np.zeros(n_leaves + 1, np.int32)
-            leaf_merges = np.zeros(max(n_leaves, 1), np.uint8)
-            nat.check(L.mms_sum_plan_fill(self.num_requests, leaf_start.ctypes.data,
-                                          leaf_merges.ctypes.data), "mms_sum_plan_fill")
-            self.num_leaves = n_leaves
+        leaf_start, leaf_merges = _sum_plan(self.num_requests)
+        self.num_leaves = len(leaf_start) - 1
+        with _on(self.device):
             (self.arrivals, self.model_ids, self.slos, self.leaf_start,
              self.leaf_merges) = _to_device_many(
                 (arrivals, model_ids, slos, leaf_start, leaf_merges), self.device)
-            self.model_hist = torch.zeros(self.num_models + 1, dtype=torch.int32,
+            self.model_hist = torch.empty(self.num_models + 1, dtype=torch.int32,
                                           device=self.device)
             tr = self.c_trace()
             nat.check(L.mms_trace_model_histogram(ctypes.byref(tr), self.num_models,
@@ -122,7 +146,7 @@ class DeviceTrace:
         """i32[N] on the device: index of the next request with the same model
         (the per-model FIFO queues of the batching simulator run along it)."""
         if getattr(self, "_next_same", None) is None:
-            with torch.cuda.device(self.device):
+            with _on(self.device):
                 buf = torch.empty(max(self.num_requests, 1), dtype=torch.int32,
                                   device=self.device)
                 tr = self.c_trace()
@@ -295,16 +319,9 @@ class DeviceTraceBatch:
             nat.check(L.mms_trace_pack(_ptr(cat_arr), _ptr(cat_mid), _ptr(cat_slo), _ptr(d_off),
                                        T, N, _ptr(self.arrivals), _ptr(self.model_ids),
                                        _ptr(self.slos), _stream_ptr()), "mms_trace_pack")
-            n_leaves = L.mms_sum_plan_leaves(N)
-            if n_leaves < 0:
-                nat.check(n_leaves, "mms_sum_plan_leaves")
-            leaf_start = np.zeros(n_leaves + 1, np.int32)
-            leaf_merges = np.zeros(max(n_leaves, 1), np.uint8)
-            nat.check(L.mms_sum_plan_fill(N, leaf_start.ctypes.data, leaf_merges.ctypes.data),
-                      "mms_sum_plan_fill")
-            self.num_leaves = n_leaves
-            self.leaf_start = _to_device(leaf_start, dev)
-            self.leaf_merges = _to_device(leaf_merges, dev)
+            leaf_start, leaf_merges = _sum_plan(N)
+            self.num_leaves = len(leaf_start) - 1
+            self.leaf_start, self.leaf_merges = _to_device_many((leaf_start, leaf_merges), dev)
             # [T][M + 1] counts, then the total of unsorted positions (T == 1: plain [M + 1])
             cells = T * (self.num_models + 1) + (1 if T > 1 else 0)
             self.model_hist = torch.zeros(cells, dtype=torch.int32, device=dev)
@@ -870,8 +887,14 @@ def sim_options(chunk_requests=0, warmup_requests=0, repair_rounds=0, repair_seg
 
 class _Pending:
     """A submitted launch: device tensors and what collect() needs."""
-    __slots__ = ("keep", "out", "B", "Bs", "M", "N", "full", "want_group_good", "h2d", "stream",
+    __slots__ = ("keep", "buf", "fields", "rows", "B", "M", "N", "full", "h2d", "stream",
                  "scratch", "call", "trace")
+
+    def field(self, name):
+        """One output as a device tensor (a view of the launch's output buffer)."""
+        at, dtype, shape = self.fields[name]
+        size = int(np.prod(shape)) * np.dtype(dtype).itemsize
+        return self.buf[at:at + size].view(_TORCH_TYPE[np.dtype(dtype)]).reshape(shape)
 
 
 # Scratch buffers of finished launches, per device, kept for the next ones: a
@@ -898,15 +921,12 @@ def _return_scratch(dev, t):
 
 
 def _submit(trace: DeviceTrace, B, M, G, P, T, S, C, model_off, model_rep, group_info,
-            latency, latency_stride, flags, want_group_good, pinned=False, options=None,
-            num_scored=None, partner=None, mirror_swap=None) -> _Pending:
+            latency, latency_stride, flags, want_group_good, pinned=False,
+            options=None) -> _Pending:
     """Uploads the tables and enqueues mms_sim_mixed on the current stream;
-    nothing waits for the GPU.  With num_scored < B the candidates behind the
-    first num_scored are mirrors (partner, mirror_swap as in mms_placements)
-    and get no results."""
+    nothing waits for the GPU."""
     job = _prepare(trace, B, M, G, P, T, S, C, model_off, model_rep, group_info, latency,
-                   latency_stride, flags, want_group_good, pinned, options, num_scored, partner,
-                   mirror_swap)
+                   latency_stride, flags, want_group_good, pinned, options)
     _enqueue(job)
     return job
 
@@ -916,7 +936,7 @@ def _enqueue(job: _Pending):
     again, if the caller wishes: everything it reads stays on the device)."""
     trace = job.trace
     cands, opts, ws, out, flags = job.call
-    with torch.cuda.device(trace.device):
+    with _on(trace.device):
         tr, plan = trace.c_trace(), trace.c_plan()
         rc = nat.lib().mms_sim_mixed(ctypes.byref(tr), ctypes.byref(cands), ctypes.byref(plan),
                                      _ptr(trace.model_hist), ctypes.byref(opts), ctypes.byref(ws),
@@ -926,8 +946,8 @@ def _enqueue(job: _Pending):
 
 
 def _prepare(trace: DeviceTrace, B, M, G, P, T, S, C, model_off, model_rep, group_info,
-             latency, latency_stride, flags, want_group_good, pinned=False, options=None,
-             num_scored=None, partner=None, mirror_swap=None) -> _Pending:
+             latency, latency_stride, flags, want_group_good, pinned=False,
+             options=None) -> _Pending:
     """Uploads the tables and allocates scratch and outputs of one launch."""
     _require_cuda()
     L = nat.lib()
@@ -937,82 +957,91 @@ def _prepare(trace: DeviceTrace, B, M, G, P, T, S, C, model_off, model_rep, grou
     if not want_group_good:
         flags |= nat.FLAG_NO_GROUP_GOOD
     job = _Pending()
-    with torch.cuda.device(dev):
+    with _on(dev):
         h2d = model_off.nbytes + model_rep.nbytes + group_info.nbytes
-        Bs = B if num_scored is None else int(num_scored)
-        d_partner = d_swap = None
         if pinned:
             d_off = _to_device(model_off, dev, pinned)
             d_rep = _to_device(model_rep, dev, pinned)
             d_info = _to_device(group_info, dev, pinned)
-            if Bs != B:
-                d_partner = _to_device(partner, dev, pinned)
-                d_swap = _to_device(mirror_swap, dev, pinned)
-        elif Bs != B:
-            d_off, d_rep, d_info, d_partner, d_swap = _to_device_many(
-                (model_off, model_rep, group_info, partner, mirror_swap), dev)
         else:
             d_off, d_rep, d_info = _to_device_many((model_off, model_rep, group_info), dev)
-        if Bs != B:
-            h2d += partner.nbytes + mirror_swap.nbytes
         d_lat = latency if isinstance(latency, torch.Tensor) else _to_device(latency, dev, pinned)
-        cands = nat.Placements(B, M, G, P, T, S, C, Bs if Bs != B else 0, _ptr(d_off), _ptr(d_rep),
-                               _ptr(d_info), _ptr(d_lat), int(latency_stride), _ptr(d_partner),
-                               _ptr(d_swap))
+        cands = nat.Placements(B, M, G, P, T, S, C, 0, _ptr(d_off), _ptr(d_rep), _ptr(d_info),
+                               _ptr(d_lat), int(latency_stride), None, None)
         need = L.mms_sim_workspace_bytes(N, ctypes.byref(cands), ctypes.byref(opts), flags)
         if need == 0 and B > 0:
             raise NotImplementedError("placement batch outside the kernel limits "
                                       "(see MMS_MAX_* in include/mms_sim.h)")
         ws_t = _take_scratch(dev, max(need, 256))
         ws = nat.Workspace(_ptr(ws_t), need)
-        i32 = dict(dtype=torch.int32, device=dev)
-        rows = max(Bs, 1)
-        o_mreq = torch.empty((rows, max(M, 1)), **i32)
-        o_mgood = torch.empty((rows, max(M, 1)), **i32)
-        o_greq = torch.empty((rows, G), **i32)
-        o_ggood = torch.empty((rows, G), **i32) if want_group_good else None
-        o_total = torch.empty(rows, dtype=torch.int64, device=dev)
-        o_lsum = torch.empty(rows, dtype=torch.float64, device=dev)
-        o_status = torch.zeros(rows, dtype=torch.int32, device=dev)
-        o_redo = torch.zeros(rows, dtype=torch.int32, device=dev)
+        # the outputs in one buffer: one allocation here, one transfer when they are read
+        rows = max(B, 1)
+        fields, total = {}, 0
+        for name, dtype, shape in (
+                ("good_total", np.int64, (rows,)), ("latency_sum", np.float64, (rows,)),
+                ("model_num_requests", np.int32, (rows, max(M, 1))),
+                ("model_num_good", np.int32, (rows, max(M, 1))),
+                ("group_num_requests", np.int32, (rows, G)),
+                ("group_num_good", np.int32, (rows, G) if want_group_good else None),
+                ("status", np.uint32, (rows,)), ("resimulated", np.int32, (rows,))):
+            if shape is not None:
+                fields[name] = (total, dtype, shape)
+                total += (int(np.prod(shape)) * np.dtype(dtype).itemsize + 15) & ~15
+        buf = torch.empty(max(total, 16), dtype=torch.uint8, device=dev)
         full = bool(flags & nat.FLAG_PER_REQUEST)
         o_fin = torch.empty((rows, max(N, 1)), dtype=torch.float64, device=dev) if full else None
         o_good = torch.empty((rows, max(N, 1)), dtype=torch.uint8, device=dev) if full else None
-        out = nat.Results(_ptr(o_mreq), _ptr(o_mgood), _ptr(o_greq), _ptr(o_ggood),
-                          _ptr(o_total), _ptr(o_lsum), _ptr(o_status), _ptr(o_fin), _ptr(o_good),
-                          _ptr(o_redo))
+        base = buf.data_ptr()
+
+        def at(name):
+            return ctypes.c_void_p(base + fields[name][0] if name in fields else 0)
+        out = nat.Results(at("model_num_requests"), at("model_num_good"), at("group_num_requests"),
+                          at("group_num_good"), at("good_total"), at("latency_sum"), at("status"),
+                          _ptr(o_fin), _ptr(o_good), at("resimulated"))
         job.stream = torch.cuda.current_stream()
     job.call = (cands, opts, ws, out, flags)
     job.trace = trace
-    job.keep = (d_off, d_rep, d_info, d_lat, d_partner, d_swap)
+    job.keep = (d_off, d_rep, d_info, d_lat)
     job.scratch = ws_t
-    job.out = (o_mreq, o_mgood, o_greq, o_ggood, o_total, o_lsum, o_status, o_redo, o_fin, o_good)
-    job.B, job.Bs, job.M, job.N, job.full = B, Bs, M, N, full
-    job.want_group_good, job.h2d = want_group_good, h2d
+    job.buf, job.fields, job.rows = buf, fields, (o_fin, o_good)
+    job.B, job.M, job.N, job.full = B, M, N, full
+    job.h2d = h2d
     return job
+
+
+def _to_host(t):
+    """A device tensor as a numpy array of its own.  Larger ones pass through page-locked
+    memory (torch's host allocator keeps such blocks): the transfer runs at several
+    times the rate of one into pageable memory."""
+    if t.numel() * t.element_size() < (256 << 10):
+        return t.cpu().numpy()
+    stage = torch.empty(t.shape, dtype=t.dtype, pin_memory=True)
+    stage.copy_(t, non_blocking=True)
+    torch.cuda.current_stream(t.device).synchronize()
+    return stage.numpy().copy()
 
 
 def _download(job: _Pending, rows_on_device=False):
     """Waits for the launch and copies its results to the host.  Returns
     (BatchResult, d2h_bytes).  rows_on_device: the per-request outputs are not
     downloaded; the result carries the device tensors instead."""
-    (o_mreq, o_mgood, o_greq, o_ggood, o_total, o_lsum, o_status, o_redo, o_fin, o_good) = job.out
-    Bs, M, N, full = job.Bs, job.M, job.N, job.full
+    B, M, N, full = job.B, job.M, job.N, job.full
+    o_fin, o_good = job.rows
     res = BatchResult()
+    host_rows = full and not rows_on_device
     with torch.cuda.stream(job.stream):
-        res.model_num_requests = o_mreq[:Bs].cpu().numpy()[:, :M]
-        res.model_num_good = o_mgood[:Bs].cpu().numpy()[:, :M]
-        res.group_num_requests = o_greq[:Bs].cpu().numpy()
-        res.group_num_good = o_ggood[:Bs].cpu().numpy() if job.want_group_good else None
-        res.good_total = o_total[:Bs].cpu().numpy()
-        res.latency_sum = o_lsum[:Bs].cpu().numpy()
-        res.status = o_status[:Bs].cpu().numpy().astype(np.uint32)
-        res.resimulated = o_redo[:Bs].cpu().numpy()
-        host_rows = full and not rows_on_device
-        res.finish = o_fin[:Bs].cpu().numpy()[:, :N] if host_rows else None
-        res.good = o_good[:Bs].cpu().numpy()[:, :N].astype(bool) if host_rows else None
+        host = _to_host(job.buf)
+        for name, (at, dtype, shape) in job.fields.items():
+            size = int(np.prod(shape)) * np.dtype(dtype).itemsize
+            setattr(res, name, host[at:at + size].view(dtype).reshape(shape)[:B])
+        res.model_num_requests = res.model_num_requests[:, :M]
+        res.model_num_good = res.model_num_good[:, :M]
+        if "group_num_good" not in job.fields:
+            res.group_num_good = None
+        res.finish = _to_host(o_fin[:B, :N]) if host_rows else None
+        res.good = _to_host(o_good[:B, :N]).view(bool) if host_rows else None
         if full and rows_on_device:
-            res.finish_device, res.good_device = o_fin[:Bs, :N], o_good[:Bs, :N]
+            res.finish_device, res.good_device = o_fin[:B, :N], o_good[:B, :N]
     d2h = sum(x.nbytes for x in (res.model_num_requests, res.model_num_good,
                                  res.group_num_requests, res.good_total, res.latency_sum,
                                  res.status))
@@ -1023,7 +1052,7 @@ def _download(job: _Pending, rows_on_device=False):
 
 def _release(job: _Pending):
     """Hands the scratch buffer back; every kernel that used it has finished."""
-    job.keep = job.out = job.call = None
+    job.keep = job.buf = job.rows = job.call = None
     if job.scratch is not None:
         _return_scratch(job.scratch.device, job.scratch)
         job.scratch = None
@@ -1161,7 +1190,7 @@ class ResidentBatch:
     def device_outputs(self):
         """[(candidate indices or None, good_total i64[.], latency_sum f64[.])] per call, on the
         device."""
-        return [(idx, job.out[4][:job.Bs], job.out[5][:job.Bs])
+        return [(idx, job.field("good_total")[:job.B], job.field("latency_sum")[:job.B])
                 for idx, job in zip(self.index, self.jobs)]
 
     def results(self):
@@ -1213,12 +1242,24 @@ def run_batch(trace: DeviceTrace, enc: EncodedBatch, table: LatencyTable,
     if not per_request:
         return _collect(submit_batch(trace, enc, table, group_good, pinned, options, mirrors,
                                      split, crowded))
-    return _launch(trace, enc.B, enc.M, enc.G, enc.P, enc.T, enc.S, enc.C,
-                   enc.model_off, enc.model_rep, enc.group_info,
-                   table.device(trace.device), 0,
-                   nat.FLAG_PER_REQUEST | (nat.FLAG_CROWDED if crowded else 0)
-                   | (0 if mirrors and enc.may_have_twins() else nat.FLAG_NO_TWINS), group_good,
-                   pinned, options, rows_on_device=rows_on_device)
+    return _collect(_submit_rows(trace, enc, table, group_good, pinned, options, mirrors, crowded),
+                    rows_on_device)
+
+
+def _submit_rows(trace, enc, table, group_good, pinned, options, mirrors, crowded):
+    """One launch with per-request outputs."""
+    flags = (nat.FLAG_PER_REQUEST | (nat.FLAG_CROWDED if crowded else 0)
+             | (0 if mirrors and enc.may_have_twins() else nat.FLAG_NO_TWINS))
+    return _submit(trace, enc.B, enc.M, enc.G, enc.P, enc.T, enc.S, enc.C, enc.model_off,
+                   enc.model_rep, enc.group_info, table.device(trace.device), 0, flags, group_good,
+                   pinned, options)
+
+
+def begin_batch_rows(trace: DeviceTrace, enc: EncodedBatch, table: LatencyTable, group_good=False,
+                     options=None, rows_on_device=False):
+    """run_batch(per_request=True) in two steps: enqueues and returns the function that waits."""
+    job = _submit_rows(trace, enc, table, group_good, False, options, True, False)
+    return lambda: _collect(job, rows_on_device)[0]
 
 
 def encode_dense(m_id2g_id, num_stages, num_models):
@@ -1260,23 +1301,25 @@ def group_lists(model_off, model_rep, group_info, G):
     u32[B][G] = first slot | stages << 8 | column << 16)."""
     B, P = model_rep.shape
     M = model_off.shape[1] - 1
-    group_off = np.zeros((B, G + 1), np.int64)
     group_mod = np.zeros((B, P), np.uint16)
-    group_cfg = np.zeros((B, G), np.uint32)
-    for b in range(B):
-        n = int(model_off[b, M])
-        ents = model_rep[b, :n].astype(np.int64)
-        g = ents & 0xFF
-        m = np.repeat(np.arange(M), np.diff(model_off[b].astype(np.int64)))
-        order = np.lexsort((m, g))                  # by group, models ascending
-        group_mod[b, :n] = m[order]
-        group_off[b, 1:] = np.cumsum(np.bincount(g, minlength=G))
-        info = group_info[b].astype(np.int64)
-        cfg = info & 0xFFFF                         # first slot | stages << 8
-        col = np.zeros(G, np.int64)
-        col[g] = ents >> 24
-        group_cfg[b] = (cfg | (col << 16)).astype(np.uint32)
-    return group_off.astype(np.uint16), group_mod, group_cfg
+    counts = np.diff(model_off.astype(np.int64), axis=1)
+    n = model_off[:, M].astype(np.int64)
+    total = int(n.sum())
+    b = np.repeat(np.arange(B), n)                       # candidate of each (model, group) pair
+    first = np.cumsum(n) - n
+    pos = np.arange(total) - first[b]
+    ents = model_rep[b, pos].astype(np.int64)
+    g = ents & 0xFF
+    m = np.repeat(np.tile(np.arange(M), B), counts.reshape(-1))
+    order = np.lexsort((m, g, b))                        # by candidate, group, models ascending
+    group_mod[b, pos] = m[order]                         # (b[order] is b)
+    per_group = np.bincount(b * G + g, minlength=B * G).reshape(B, G)
+    group_off = np.zeros((B, G + 1), np.uint16)
+    group_off[:, 1:] = np.cumsum(per_group, axis=1)
+    col = np.zeros((B, G), np.int64)
+    col[b, g] = ents >> 24
+    group_cfg = ((group_info[:, :G].astype(np.int64) & 0xFFFF) | (col << 16)).astype(np.uint32)
+    return group_off, group_mod, group_cfg
 
 
 class ResidentBatching:
@@ -1293,9 +1336,9 @@ class ResidentBatching:
         self.trace, self.B, self.M, self.G, self.N = trace, B, M, G, N
         goff, gmod, gcfg = group_lists(model_off, model_rep, group_info, G)
         self.h2d_bytes = sum(x.nbytes for x in (model_off, model_rep, goff, gmod, gcfg))
-        with torch.cuda.device(dev):
-            d_off, d_rep = _to_device(model_off, dev), _to_device(model_rep, dev)
-            d_goff, d_gmod, d_gcfg = (_to_device(x, dev) for x in (goff, gmod, gcfg))
+        with _on(dev):
+            d_off, d_rep, d_goff, d_gmod, d_gcfg = _to_device_many(
+                (model_off, model_rep, goff, gmod, gcfg), dev)
             d_lat = latency if isinstance(latency, torch.Tensor) else _to_device(latency, dev)
             self.cands = nat.Placements(B, M, G, P, T, S, C, 0, _ptr(d_off), _ptr(d_rep), None,
                                         _ptr(d_lat), int(latency_stride))
@@ -1305,26 +1348,31 @@ class ResidentBatching:
                                                       ctypes.byref(self.bat))
             ws_t = torch.empty(max(need, 256), dtype=torch.uint8, device=dev)
             self.ws = nat.Workspace(_ptr(ws_t), need)
-            i32 = dict(dtype=torch.int32, device=dev)
-            o_mreq, o_mgood = torch.zeros((B, max(M, 1)), **i32), torch.zeros((B, max(M, 1)), **i32)
-            o_greq, o_ggood = torch.zeros((B, G), **i32), torch.zeros((B, G), **i32)
-            o_total = torch.zeros(B, dtype=torch.int64, device=dev)
-            o_lsum = torch.zeros(B, dtype=torch.float64, device=dev)
-            o_status = torch.zeros(B, **i32)
+            self.fields, total = {}, 0
+            for name, dtype, shape in (
+                    ("good_total", np.int64, (B,)), ("latency_sum", np.float64, (B,)),
+                    ("model_num_requests", np.int32, (B, max(M, 1))),
+                    ("model_num_good", np.int32, (B, max(M, 1))),
+                    ("group_num_requests", np.int32, (B, G)), ("group_num_good", np.int32, (B, G)),
+                    ("status", np.uint32, (B,)), ("resimulated", np.int32, (B,))):
+                self.fields[name] = (total, dtype, shape)
+                total += (int(np.prod(shape)) * np.dtype(dtype).itemsize + 15) & ~15
+            self.buf = torch.zeros(max(total, 16), dtype=torch.uint8, device=dev)
             o_fin = torch.empty((B, max(N, 1)), dtype=torch.float64, device=dev)
             o_good = torch.empty((B, max(N, 1)), dtype=torch.uint8, device=dev)
-            o_redo = torch.zeros(B, **i32)
-            self.res = nat.Results(_ptr(o_mreq), _ptr(o_mgood), _ptr(o_greq), _ptr(o_ggood),
-                                   _ptr(o_total), _ptr(o_lsum), _ptr(o_status), _ptr(o_fin),
-                                   _ptr(o_good), _ptr(o_redo))
+            base = self.buf.data_ptr()
+            at = {name: ctypes.c_void_p(base + f[0]) for name, f in self.fields.items()}
+            self.res = nat.Results(at["model_num_requests"], at["model_num_good"],
+                                   at["group_num_requests"], at["group_num_good"],
+                                   at["good_total"], at["latency_sum"], at["status"], _ptr(o_fin),
+                                   _ptr(o_good), at["resimulated"])
             self.next_same = trace.next_same_model()
         self.keep = (d_off, d_rep, d_goff, d_gmod, d_gcfg, d_lat, ws_t)
-        self.out = (o_mreq, o_mgood, o_greq, o_ggood, o_total, o_lsum, o_status, o_fin, o_good,
-                    o_redo)
+        self.rows = (o_fin, o_good)
 
     def launch(self):
         trace = self.trace
-        with torch.cuda.device(trace.device):
+        with _on(trace.device):
             tr, plan = trace.c_trace(), trace.c_plan()
             rc = nat.lib().mms_sim_batching(ctypes.byref(tr), ctypes.byref(self.cands),
                                             ctypes.byref(self.bat), _ptr(self.next_same),
@@ -1336,20 +1384,17 @@ class ResidentBatching:
     def results(self, per_request=True, rows_on_device=False):
         """Waits and downloads: (BatchResult, d2h bytes).  rows_on_device: the
         result carries the per-request outputs as device tensors."""
-        (o_mreq, o_mgood, o_greq, o_ggood, o_total, o_lsum, o_status, o_fin, o_good,
-         o_redo) = self.out
+        o_fin, o_good = self.rows
         M, N = self.M, self.N
         res = BatchResult()
-        res.model_num_requests = o_mreq.cpu().numpy()[:, :M]
-        res.model_num_good = o_mgood.cpu().numpy()[:, :M]
-        res.group_num_requests = o_greq.cpu().numpy()
-        res.group_num_good = o_ggood.cpu().numpy()
-        res.good_total = o_total.cpu().numpy()
-        res.latency_sum = o_lsum.cpu().numpy()
-        res.status = o_status.cpu().numpy().astype(np.uint32)
-        res.resimulated = o_redo.cpu().numpy()
-        res.finish = o_fin.cpu().numpy()[:, :N] if per_request else None
-        res.good = o_good.cpu().numpy()[:, :N].astype(bool) if per_request else None
+        host = _to_host(self.buf)
+        for name, (at, dtype, shape) in self.fields.items():
+            size = int(np.prod(shape)) * np.dtype(dtype).itemsize
+            setattr(res, name, host[at:at + size].view(dtype).reshape(shape))
+        res.model_num_requests = res.model_num_requests[:, :M]
+        res.model_num_good = res.model_num_good[:, :M]
+        res.finish = _to_host(o_fin[:, :N]) if per_request else None
+        res.good = _to_host(o_good[:, :N]).view(bool) if per_request else None
         if rows_on_device:
             res.finish_device, res.good_device = o_fin[:, :N], o_good[:, :N]
         d2h = sum(x.nbytes for x in (res.model_num_requests, res.model_num_good,
@@ -1366,24 +1411,35 @@ def launch_batching(trace: DeviceTrace, B, M, G, P, T, S, C, model_off, model_re
     """simulate_requests_mixed_batching (controller.py:630-798) for every
     candidate.  The kernel always writes per-request outputs (the latency sums
     are formed from them); per_request=False does not download them."""
-    job = ResidentBatching(trace, B, M, G, P, T, S, C, model_off, model_rep, group_info, latency,
-                           latency_stride, batch_sizes, heap_capacity).launch()
-    res, _ = job.results(per_request, rows_on_device)
-    if heap_capacity == 0 and np.any(res.status & nat.STATUS_HEAP_OVERFLOW):
-        # the default capacity (G + 16 pending events) is what the simulation was seen to
-        # need; nothing bounds it, so a run that overflowed is repeated with room to spare
-        job = ResidentBatching(trace, B, M, G, P, T, S, C, model_off, model_rep, group_info,
-                               latency, latency_stride, batch_sizes, 8 * G + 64).launch()
+    return _begin_batching(trace, B, M, G, P, T, S, C, model_off, model_rep, group_info, latency,
+                           latency_stride, batch_sizes, heap_capacity, per_request,
+                           rows_on_device)()
+
+
+def _begin_batching(trace, B, M, G, P, T, S, C, model_off, model_rep, group_info, latency,
+                    latency_stride, batch_sizes, heap_capacity, per_request, rows_on_device):
+    """launch_batching in two steps: enqueues and returns the function that waits."""
+    def begin(capacity):
+        return ResidentBatching(trace, B, M, G, P, T, S, C, model_off, model_rep, group_info,
+                                latency, latency_stride, batch_sizes, capacity).launch()
+    job = begin(heap_capacity)
+
+    def collect():
         res, _ = job.results(per_request, rows_on_device)
-    if np.any(res.status):
-        bad = int(np.flatnonzero(res.status)[0])
-        what = {nat.STATUS_HEAP_OVERFLOW: "event heap overflow (raise heap_capacity)",
-                nat.STATUS_QUEUE_LEFT: "a request was left queued",
-                nat.STATUS_BAD_INDEX: "bad table index"}
-        raise RuntimeError(f"batching simulator reported status {int(res.status[bad])} for "
-                           f"candidate {bad}: " + ", ".join(v for k, v in what.items()
-                                                            if res.status[bad] & k))
-    return res
+        if heap_capacity == 0 and np.any(res.status & nat.STATUS_HEAP_OVERFLOW):
+            # the default capacity (G + 16 pending events) is what the simulation was seen to
+            # need; nothing bounds it, so a run that overflowed is repeated with room to spare
+            res, _ = begin(8 * G + 64).results(per_request, rows_on_device)
+        if np.any(res.status):
+            bad = int(np.flatnonzero(res.status)[0])
+            what = {nat.STATUS_HEAP_OVERFLOW: "event heap overflow (raise heap_capacity)",
+                    nat.STATUS_QUEUE_LEFT: "a request was left queued",
+                    nat.STATUS_BAD_INDEX: "bad table index"}
+            raise RuntimeError(f"batching simulator reported status {int(res.status[bad])} for "
+                               f"candidate {bad}: " + ", ".join(v for k, v in what.items()
+                                                                if res.status[bad] & k))
+        return res
+    return collect
 
 
 def resident_batching(trace: DeviceTrace, enc: EncodedBatch, table: LatencyTable,
@@ -1401,9 +1457,15 @@ def run_batch_batching(trace: DeviceTrace, enc: EncodedBatch, table: LatencyTabl
     """Batching simulation of every placement of `enc`; `table` must have been
     built with batch sizes.  per_request=False leaves the per-request outputs
     (9 bytes per candidate and request) on the device."""
+    return begin_batch_batching(trace, enc, table, heap_capacity, per_request, rows_on_device)()
+
+
+def begin_batch_batching(trace: DeviceTrace, enc: EncodedBatch, table: LatencyTable,
+                         heap_capacity=0, per_request=True, rows_on_device=False):
+    """run_batch_batching in two steps: enqueues and returns the function that waits."""
     if table.batch_sizes is None:
         raise ValueError("the latency table has no batch-size axis")
-    return launch_batching(trace, enc.B, enc.M, enc.G, enc.P, enc.T, enc.S, enc.C, enc.model_off,
+    return _begin_batching(trace, enc.B, enc.M, enc.G, enc.P, enc.T, enc.S, enc.C, enc.model_off,
                            enc.model_rep, enc.group_info, table.device(trace.device), 0,
                            table.batch_sizes, heap_capacity, per_request, rows_on_device)
 
@@ -1442,21 +1504,24 @@ def device_compute_stats(arrivals, model_ids, num_models: int, finish, good, fir
             raise NotImplementedError("statistics outside the kernel limits")
         ws_t = _take_scratch(dev, max(need, 256))
         ws = nat.Workspace(_ptr(ws_t), need)
-        f64 = dict(dtype=torch.float64, device=dev)
-        o = {"num_requests": torch.zeros(max(M, 1), dtype=torch.int32, device=dev),
-             "num_good": torch.zeros((B, max(M, 1)), dtype=torch.int32, device=dev),
-             "good_total": torch.zeros(B, dtype=torch.int64, device=dev),
-             "latency_sum": torch.zeros(B, **f64)}
-        for name in STATS_FIELDS[1:]:
-            o[name] = torch.zeros((B, max(M, 1)), **f64)
-        out = nat.StatsOut(*[_ptr(o[k]) for k in ("num_requests",) + STATS_FIELDS
-                             + ("good_total", "latency_sum")])
+        fields, total = {}, 0
+        for name, dtype, shape in (
+                [("good_total", np.int64, (B,)), ("latency_sum", np.float64, (B,))]
+                + [(k, np.float64, (B, max(M, 1))) for k in STATS_FIELDS[1:]]
+                + [("num_good", np.int32, (B, max(M, 1))), ("num_requests", np.int32, (max(M, 1),))]):
+            fields[name] = (total, dtype, shape)
+            total += (int(np.prod(shape)) * np.dtype(dtype).itemsize + 15) & ~15
+        buf = torch.zeros(total, dtype=torch.uint8, device=dev)
+        out = nat.StatsOut(*[ctypes.c_void_p(buf.data_ptr() + fields[k][0])
+                             for k in ("num_requests",) + STATS_FIELDS + ("good_total", "latency_sum")])
         rc = L.mms_compute_stats(_ptr(arrivals), _ptr(model_ids), M, _ptr(finish), _ptr(good),
                                  finish.stride(0), B, first, window, ctypes.byref(ws),
                                  ctypes.byref(out), _stream_ptr())
         nat.check(rc, "mms_compute_stats")
-        res = {k: v.cpu().numpy() for k, v in o.items()}      # waits for the kernels
+        host = _to_host(buf)                                  # waits for the kernels
         _return_scratch(dev, ws_t)
+    res = {k: host[at:at + int(np.prod(shape)) * np.dtype(dtype).itemsize].view(dtype).reshape(shape)
+           for k, (at, dtype, shape) in fields.items()}
     res["d2h_bytes"] = sum(v.nbytes for v in res.values())
     res["num_requests"] = res["num_requests"][:M]
     for name in STATS_FIELDS:

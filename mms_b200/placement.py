@@ -13,8 +13,8 @@ import numpy as np
 
 from . import engine
 from .profiling import ParallelConfig, ProfilingResult  # noqa: F401 (re-exported)
-from .simulator import fast_stats, workload_arrays
-from .workload import GammaProcess, Workload, eps
+from .simulator import workload_arrays
+from .workload import GammaProcess, PerModelStatsResult, StatsResult, Workload, eps
 
 inf = 1e100      # alpa_serve/util.py:23
 
@@ -227,14 +227,21 @@ class PlacementEvaluator:
             return []
         enc, res = self.evaluate(sols)
         start = self.trace.host_arrivals
+        n, interval = len(start), start[-1] - start[0]
+        # fast_stats (controller.py:393-403) for the whole list at once
+        goodputs = res.good_total.astype(np.float64) / n
+        latency_means = res.latency_sum / n
+        model_goodputs = res.model_num_good / (res.model_num_requests + eps)
+        throughputs = res.model_num_requests / interval
         out = []
         for b in range(enc.B):
-            g = int(enc.num_groups[b])
-            stats = fast_stats(self.model_names, start, res.latency_sum[b], res.good_total[b],
-                               res.model_num_requests[b], res.model_num_good[b],
-                               res.group_num_requests[b, :g])
-            out.append((stats.goodput, [x.goodput for x in stats.per_model_stats],
-                        stats.group_num_requests, stats))
+            mine = list(model_goodputs[b])
+            per_model = [PerModelStatsResult(name, k, g, t, 0, 0, 0, 0, [], [], [])
+                         for name, k, g, t in zip(self.model_names, res.model_num_requests[b], mine,
+                                                  throughputs[b])]
+            stats = StatsResult(per_model, tuple(res.group_num_requests[b, :int(enc.num_groups[b])]),
+                                goodputs[b], latency_means[b], n, n / interval)
+            out.append((stats.goodput, mine, stats.group_num_requests, stats))
         return out
 
 

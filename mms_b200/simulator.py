@@ -125,63 +125,70 @@ def approximate_one_case_one_placement(placement, model_names, prof_ress, model_
     group_num_requests, group_num_good_requests).  With rows_on_device (no
     counterpart in the reference) finish and good are torch tensors on the GPU
     (f64[N], u8[N]) instead of numpy arrays: nothing per request is downloaded."""
+    return _begin_one(placement, model_names, prof_ress, model_ids, slos, arrivals, mixed,
+                      enable_batching, rows_on_device)()
+
+
+def _one_clock(placement, prof_ress, M, model_ids, slos, arrivals):
+    """controller.py:431-450: the tables of simulate_requests."""
+    G, N = len(placement.group_configs), len(arrivals)
+    finish = np.empty(N, dtype=np.float64)
+    good = np.empty(N, dtype=bool)
+    max_bs = 1
+    gmax = np.empty((M, G), np.float32)
+    gsum = np.empty((M, G), np.float32)
+    with np.errstate(over="ignore"):
+        for m in range(M):
+            for g in range(G):
+                value = prof_ress[m].para_dict.get(placement.group_configs[g], None)
+                if value:                                  # controller.py:438-443
+                    penalty = 0.009 * len(value.latency[max_bs])
+                    gmax[m][g] = max(value.latency[max_bs]) * (1 + penalty)
+                    gsum[m][g] = sum(value.latency[max_bs]) * (1 + penalty)
+                else:
+                    gmax[m][g] = gsum[m][g] = inf
+    m2g = np.full((M, max(G, 1)), -1, np.int32)
+    fill = [0] * M
+    for g, ms in enumerate(placement.group_models):
+        for m in ms:
+            m2g[m][fill[m]] = g
+            fill[m] += 1
+    counters = simulate_requests(finish, good, arrivals, model_ids, slos, m2g, gmax, gsum, N)
+    return (arrivals, finish, good) + tuple(counters)
+
+
+def _begin_one(placement, model_names, prof_ress, model_ids, slos, arrivals, mixed=True,
+               enable_batching=False, rows_on_device=False, table=None):
+    """approximate_one_case_one_placement in two steps: enqueues the simulation and returns the
+    function that waits for it.  `table`: an engine.LatencyTable to use (and to extend) instead
+    of a new one."""
     M = len(model_names)
     G = len(placement.group_configs)
     N = len(arrivals)
     arrivals = np.asarray(arrivals, dtype=np.float64)
-    if rows_on_device and mixed and G > 0:
-        trace = engine.DeviceTrace(arrivals, model_ids, slos, M)
-        table = engine.LatencyTable(prof_ress, list(batchsize_config) if enable_batching else None)
-        enc = engine.encode_placements([placement], table, M)
-        if enable_batching:
-            res = engine.run_batch_batching(trace, enc, table, per_request=False,
-                                            rows_on_device=True)
-        else:
-            res, _, _ = engine.run_batch(trace, enc, table, per_request=True, group_good=True,
-                                         options=_options, rows_on_device=True)
-        return (arrivals, res.finish_device[0], res.good_device[0]) + tuple(_counters(res, M, G))
-    finish = np.empty(N, dtype=np.float64)
-    good = np.empty(N, dtype=bool)
     if not mixed:
-        max_bs = 1
-        gmax = np.empty((M, G), np.float32)
-        gsum = np.empty((M, G), np.float32)
-        with np.errstate(over="ignore"):
-            for m in range(M):
-                for g in range(G):
-                    value = prof_ress[m].para_dict.get(placement.group_configs[g], None)
-                    if value:                                  # controller.py:438-443
-                        penalty = 0.009 * len(value.latency[max_bs])
-                        gmax[m][g] = max(value.latency[max_bs]) * (1 + penalty)
-                        gsum[m][g] = sum(value.latency[max_bs]) * (1 + penalty)
-                    else:
-                        gmax[m][g] = gsum[m][g] = inf
-        m2g = np.full((M, max(G, 1)), -1, np.int32)
-        fill = [0] * M
-        for g, ms in enumerate(placement.group_models):
-            for m in ms:
-                m2g[m][fill[m]] = g
-                fill[m] += 1
-        counters = simulate_requests(finish, good, arrivals, model_ids, slos, m2g, gmax, gsum, N)
-        return (arrivals, finish, good) + tuple(counters)
-
+        return lambda: _one_clock(placement, prof_ress, M, model_ids, slos, arrivals)
     trace = engine.DeviceTrace(arrivals, model_ids, slos, M)
-    table = engine.LatencyTable(prof_ress, list(batchsize_config) if enable_batching else None)
+    if table is None:
+        table = engine.LatencyTable(prof_ress, list(batchsize_config) if enable_batching else None)
     enc = engine.encode_placements([placement], table, M)
-    if enable_batching and G > 0:
-        res = engine.run_batch_batching(trace, enc, table)
-        finish[:] = res.finish[0]
-        good[:] = res.good[0]
-        return (arrivals, finish, good) + tuple(_counters(res, M, G))
     if G == 0:
         z = np.zeros
-        return (arrivals, arrivals.copy(), np.zeros(N, bool), trace.model_hist.cpu().numpy()[:M],
-                z(M, np.int32), z(0, np.int32), z(0, np.int32))
-    res, _, _ = engine.run_batch(trace, enc, table, per_request=True, group_good=True,
-                                 options=_options)
-    finish[:] = res.finish[0]
-    good[:] = res.good[0]
-    return (arrivals, finish, good) + tuple(_counters(res, M, G))
+        return lambda: (arrivals, arrivals.copy(), np.zeros(N, bool), trace.model_hist.cpu().numpy()[:M],
+                        z(M, np.int32), z(0, np.int32), z(0, np.int32))
+    if enable_batching:
+        collect = engine.begin_batch_batching(trace, enc, table, per_request=not rows_on_device,
+                                              rows_on_device=rows_on_device)
+    else:
+        collect = engine.begin_batch_rows(trace, enc, table, group_good=True, options=_options,
+                                          rows_on_device=rows_on_device)
+
+    def finish():
+        res = collect()
+        rows = (res.finish_device[0], res.good_device[0]) if rows_on_device \
+            else (res.finish[0], res.good[0])
+        return (arrivals,) + rows + tuple(_counters(res, M, G))
+    return finish
 
 
 class DummyController:
@@ -241,15 +248,20 @@ def fast_stats(model_names, start, finish_minus_start_sum, good_total, model_num
     np.mean(finish - start) = (numpy-ordered sum) / N."""
     n = len(start)
     interval = start[-1] - start[0]
-    per_model = [PerModelStatsResult(
-        model_names[i], model_num_requests[i],
-        model_num_good[i] / (model_num_requests[i] + eps),
-        model_num_requests[i] / interval, 0, 0, 0, 0, [], [], [])
-        for i in range(len(model_names))]
+    per_model = _per_model(model_names, model_num_requests, model_num_good, interval)
     goodput = np.float64(good_total) / n
     latency_mean = np.float64(finish_minus_start_sum) / n
     return StatsResult(per_model, tuple(group_num_requests), goodput, latency_mean, n,
                        n / interval)
+
+
+def _per_model(model_names, model_num_requests, model_num_good, interval):
+    """The per-model rows of controller.py:393-403 (one division of arrays instead of one of
+    numpy scalars per model: these are a third of a small call)."""
+    goodput = model_num_good / (model_num_requests + eps)
+    throughput = model_num_requests / interval
+    return [PerModelStatsResult(name, k, g, t, 0, 0, 0, 0, [], [], [])
+            for name, k, g, t in zip(model_names, model_num_requests, goodput, throughput)]
 
 
 class DeviceColumn:
@@ -297,15 +309,15 @@ def device_stats(workload, start, finish_dev, good_dev, warmup) -> StatsResult:
             lo, hi = skip, max(n - skip, skip)
     window = hi - lo
     dev = finish_dev.device
-    d_arr = torch.from_numpy(np.ascontiguousarray(start, dtype=np.float64)).to(dev)
-    d_which = torch.from_numpy(which).to(dev)
+    d_arr, d_which = engine._to_device_many((np.asarray(start, np.float64), which), dev)
     K = len(workload.names)
     st = engine.device_compute_stats(d_arr, d_which, K, finish_dev.reshape(1, -1),
                                      good_dev.reshape(1, -1), lo, window)
     start_w, which_w = np.asarray(start)[lo:hi], which[lo:hi]
     # names in order of first appearance, then a stable sort by request count (:321-326)
-    _, first = np.unique(which_w, return_index=True)
-    seen = [int(k) for k in which_w[np.sort(first)]]
+    first = np.full(K, len(which_w), np.int64)
+    first[which_w[::-1]] = np.arange(len(which_w) - 1, -1, -1)      # the last write is the first one
+    seen = [int(k) for k in np.argsort(first, kind="stable") if first[k] < len(which_w)]
     ordered = sorted(seen, key=lambda k: int(st["num_requests"][k]))
     host = {}
 
@@ -370,23 +382,28 @@ def approximate_one_case(case, seed: int = 0, warmup: int = DEFAULT_WARMUP, debu
     on_device = (not fast_stats and hasattr(workload, "name_index") and len(workload) > 1
                  and all(len(p.group_configs) > 0
                          for p in getattr(placement, "placements", [placement])))
-    run = partial(approximate_one_case_one_placement, enable_batching=enable_batching,
-                  rows_on_device=on_device)
+    run = partial(_begin_one, enable_batching=enable_batching, rows_on_device=on_device)
     if hasattr(placement, "placements"):          # ModelPlacementWithReplacement
         arrivals = workload.arrivals
         change_times = list(placement.start_times[1:]) + [inf]
         # controller.py:353-371: a segment ends at the first arrival that is
         # later than the next change time; clocks restart from zero.
         bounds = [0]
-        pt = 0
-        for i in range(len(arrivals)):
-            if arrivals[i] > change_times[pt]:
-                bounds.append(i)
-                pt += 1
+        at = 0                      # one arrival ends at most one segment
+        for change in change_times:
+            later = arrivals[at:] > change
+            if not later.any():
+                break
+            at += int(later.argmax())
+            bounds.append(at)
+            at += 1
         bounds.append(len(arrivals))
+        # all segments are on their way before the first one is waited for
+        table = engine.LatencyTable(prof_ress, list(batchsize_config) if enable_batching else None)
         parts = [run(placement.placements[k], model_names, prof_ress,
                      model_ids[bounds[k]:bounds[k + 1]], slos[bounds[k]:bounds[k + 1]],
-                     arrivals[bounds[k]:bounds[k + 1]]) for k in range(len(bounds) - 1)]
+                     arrivals[bounds[k]:bounds[k + 1]], table=table) for k in range(len(bounds) - 1)]
+        parts = [p() for p in parts]
         start = np.concatenate([p[0] for p in parts])
         if on_device:
             import torch
@@ -401,15 +418,11 @@ def approximate_one_case(case, seed: int = 0, warmup: int = DEFAULT_WARMUP, debu
     else:
         (start, finish, good, model_num_requests, model_num_good,
          group_num_requests, _) = run(placement, model_names, prof_ress, model_ids, slos,
-                                      workload.arrivals)
+                                      workload.arrivals)()
 
     if fast_stats:
         interval = start[-1] - start[0]
-        per_model = [PerModelStatsResult(
-            model_names[i], model_num_requests[i],
-            model_num_good[i] / (model_num_requests[i] + eps),
-            model_num_requests[i] / interval, 0, 0, 0, 0, [], [], [])
-            for i in range(len(model_names))]
+        per_model = _per_model(model_names, model_num_requests, model_num_good, interval)
         stats = StatsResult(per_model, tuple(group_num_requests), np.mean(good),
                             np.mean(finish - start), len(start), len(start) / interval)
     elif on_device:
