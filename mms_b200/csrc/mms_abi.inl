@@ -694,8 +694,8 @@ int mms_trace_next_same_model(const mms_trace *trace, int32_t num_models, int32_
     cudaStream_t st = (cudaStream_t)stream;
     // requests of unknown models (-1) are never queued; give them a defined value
     MMS_CUDA(cudaMemsetAsync(next_same, 0xFF, sizeof(int32_t) * (size_t)trace->num_requests, st));
-    mms::next_same_kernel<<<(num_models + 31) / 32, 32, 0, st>>>(
-        trace->model_ids, trace->num_requests, num_models, next_same);
+    mms::next_same_kernel<<<(unsigned)num_models, mms::kNextWarps * mms::kLanes, 0, st>>>(
+        trace->model_ids, trace->num_requests, next_same);
     MMS_CUDA(cudaGetLastError());
     return MMS_OK;
 }
@@ -736,20 +736,24 @@ static int plan_batching(int64_t N, const mms_placements *c, const mms_batching 
         (void)cudaGetLastError();
         sm_count = 148;
     }
-    // Chunks: as many as fill ONE wave of the blocks that can be resident (shared memory
-    // decides), none shorter than twice the run-in, and no cut at all when that leaves fewer
-    // than two.
-    g->warmup = 2048;
+    // Run-in as in plan_call; chunks: as many as fill ONE wave of the blocks that can be
+    // resident (shared memory decides), none shorter than half the run-in, and no cut at all
+    // when that leaves fewer than two.
+    int64_t warm = 32 * (int64_t)c->max_slots;
+    if (warm < 128) warm = 128;
+    if (warm > 2048) warm = 2048;
+    g->warmup = (int32_t)warm;
+    const int64_t min_chunk = warm / 2 > 256 ? warm / 2 : 256;
     int64_t K = 1;
-    if (B > 0 && N >= 4 * 4096) {
+    if (B > 0 && N >= 4 * min_chunk) {
         const size_t smem = g->simd ? g->smem_simd : g->smem_single;
         int64_t per_sm = (int64_t)(233472 / (smem + 1024));
         if (per_sm > kBatchBlocksPerSm) per_sm = kBatchBlocksPerSm;
         if (per_sm < 1) per_sm = 1;
         const int64_t blocks_per_chunk = g->simd ? g->Bp / kLanes : B;
         K = per_sm * sm_count / blocks_per_chunk;
-        if (K > N / 4096) K = N / 4096;
-        if (K < (g->simd ? 2 : 4)) K = 1;
+        if (K > N / min_chunk) K = N / min_chunk;
+        if (K < 2) K = 1;
     }
     const int64_t len = (N + K - 1) / (K > 0 ? K : 1);
     g->chunk_len = (int32_t)(len > 0 ? len : 1);

@@ -1041,15 +1041,55 @@ __global__ void unsorted_kernel(const double *arrivals, int64_t N, int32_t *coun
     if (bad) atomicAdd(count, bad);
 }
 
-// next_same[i] = next request with request i's model, -1 if none; one thread
-// per model walks the trace backwards.
-__global__ void next_same_kernel(const int32_t *model_ids, int64_t N, int32_t M, int32_t *next_same)
+// next_same[i] = next request with request i's model, -1 if none.  One block per model; its
+// warps take a stretch of the trace each, look for the first request of the model in it (what
+// the stretch before it ends with), then go through the stretch backwards, 32 requests to a
+// vote.  (One thread per model walking the whole trace: 1.2 ms for 27 000 requests.)
+constexpr int kNextWarps = 16;
+
+__global__ void __launch_bounds__(kNextWarps * kLanes)
+next_same_kernel(const int32_t *model_ids, int64_t N, int32_t *next_same)
 {
-    const int m = blockIdx.x * blockDim.x + threadIdx.x;
-    if (m >= M) return;
-    int32_t last = -1;
-    for (int64_t i = N - 1; i >= 0; --i) {
-        if (model_ids[i] == m) { next_same[i] = last; last = (int32_t)i; }
+    __shared__ int32_t first[kNextWarps];
+    constexpr int kAhead = 8;                      // loads in flight
+    const int m = blockIdx.x, lane = threadIdx.x & (kLanes - 1), warp = threadIdx.x / kLanes;
+    const int64_t tiles = (N + kLanes - 1) / kLanes;
+    const int64_t t0 = tiles * warp / kNextWarps, t1 = tiles * (warp + 1) / kNextWarps;
+    int32_t found = 0x7FFFFFFF;
+    for (int64_t t = t0; t < t1; t += kAhead) {
+        int32_t id[kAhead];
+#pragma unroll
+        for (int u = 0; u < kAhead; ++u) {
+            const int64_t i = (t + u) * kLanes + lane;
+            id[u] = t + u < t1 && i < N ? model_ids[i] : -1;
+        }
+#pragma unroll
+        for (int u = 0; u < kAhead; ++u) {
+            const uint32_t has = __ballot_sync(0xFFFFFFFFu, id[u] == m);
+            if (has && found == 0x7FFFFFFF) found = (int32_t)((t + u) * kLanes) + __ffs((int)has) - 1;
+        }
+        if (found != 0x7FFFFFFF) break;
+    }
+    if (lane == 0) first[warp] = found;
+    __syncthreads();
+    int32_t carry = 0x7FFFFFFF;
+    for (int w = warp + 1; w < kNextWarps; ++w) carry = first[w] < carry ? first[w] : carry;
+    if (carry == 0x7FFFFFFF) carry = -1;
+    for (int64_t t = t1; t > t0; t -= kAhead) {    // tiles t - 1, t - 2, ...
+        int32_t id[kAhead];
+#pragma unroll
+        for (int u = 0; u < kAhead; ++u) {
+            const int64_t i = (t - 1 - u) * kLanes + lane;
+            id[u] = t - 1 - u >= t0 && i < N ? model_ids[i] : -1;
+        }
+#pragma unroll
+        for (int u = 0; u < kAhead; ++u) {
+            const uint32_t has = __ballot_sync(0xFFFFFFFFu, id[u] == m);
+            const int32_t base = (int32_t)((t - 1 - u) * kLanes);
+            const uint32_t later = has & ~((2u << lane) - 1u);
+            if (id[u] == m) next_same[base + lane] = later ? base + __ffs((int)later) - 1 : carry;
+            if (has) carry = base + __ffs((int)has) - 1;
+        }
     }
 }
 

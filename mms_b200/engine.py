@@ -376,12 +376,13 @@ class LatencyTable:
                     value = prof.para_dict.get(c, None)
                     if value:
                         penalty = 0.009 * len(value.latency[1])
-                        for k in range(int(c.pp)):
-                            if self.batch_sizes is None:
-                                tab[m, col, k] = value.latency[1][k] * (1 + penalty)
-                            else:
-                                for j, bs in enumerate(self.batch_sizes):
-                                    tab[m, col, k, j] = value.latency[bs][k] * (1 + penalty)
+                        pp = int(c.pp)
+                        if self.batch_sizes is None:
+                            tab[m, col, :pp] = np.asarray(value.latency[1][:pp], np.float64) * (1 + penalty)
+                        else:
+                            for j, bs in enumerate(self.batch_sizes):
+                                tab[m, col, :pp, j] = \
+                                    np.asarray(value.latency[bs][:pp], np.float64) * (1 + penalty)
                     else:
                         tab[m, col] = np.float32(inf)
         self._host = tab
