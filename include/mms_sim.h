@@ -59,6 +59,9 @@ extern "C" {
                                      have none (saves the bookkeeping); pass the same
                                      flags to the workspace query                    */
 
+#define MMS_FLAG_TRACE_ROWS 32u   /* with num_traces > 1: the traces are stored one after
+                                     the other (element i of trace t at t * N + i)   */
+
 /* The request trace: what controller.py:323-339 caches per Workload
  * (model_ids, slos) plus Workload.arrivals (simulator/workload.py:272). */
 typedef struct {
@@ -233,6 +236,15 @@ int mms_trace_model_histogram(const mms_trace *trace, int32_t num_models,
 int mms_trace_pack(const double *arrivals, const int32_t *model_ids, const float *slos,
                    const int64_t *offsets, int64_t num_traces, int64_t padded_requests,
                    double *out_arrivals, int32_t *out_model_ids, float *out_slos, void *stream);
+
+/* The two steps for traces stored one after the other (MMS_FLAG_TRACE_ROWS), each with room for
+ * num_requests requests: mms_trace_pad_rows fills trace t behind its lengths[t] (i64[T], device)
+ * requests as mms_trace describes; mms_trace_rows_histogram counts as
+ * mms_trace_model_histogram does with T > 1 traces. */
+int mms_trace_pad_rows(const int64_t *lengths, int64_t num_traces, int64_t num_requests,
+                       double *arrivals, int32_t *model_ids, float *slos, void *stream);
+int mms_trace_rows_histogram(const double *arrivals, const int32_t *model_ids, int64_t num_traces,
+                             int64_t num_requests, int32_t num_models, int32_t *hist, void *stream);
 
 /* Bytes of scratch mms_sim_mixed needs for this shape and these options. */
 size_t mms_sim_workspace_bytes(int64_t num_requests, const mms_placements *cands,

@@ -33,6 +33,7 @@ FLAG_LEGACY_CLOCK = 2
 FLAG_NO_GROUP_GOOD = 4
 FLAG_CROWDED = 8
 FLAG_NO_TWINS = 16
+FLAG_TRACE_ROWS = 32
 
 STATIC_SCRATCH_BYTES = 32 << 20
 
@@ -63,7 +64,7 @@ EXPORTS = (
     "mms_trace_model_histogram", "mms_sim_workspace_bytes", "mms_sim_mixed",
     "mms_sim_mixed_static", "mms_trace_next_same_model", "mms_sim_batching_workspace_bytes", "mms_sim_batching",
     "mms_profile_begin", "mms_profile_end", "mms_argmax_scores",
-    "mms_trace_pack", "mms_compute_stats_workspace_bytes", "mms_compute_stats",
+    "mms_trace_pack", "mms_trace_pad_rows", "mms_trace_rows_histogram", "mms_compute_stats_workspace_bytes", "mms_compute_stats",
 )
 
 _vp = ctypes.c_void_p
@@ -187,6 +188,11 @@ def lib():
     L.mms_trace_pack.restype = ctypes.c_int
     L.mms_trace_pack.argtypes = [_vp, _vp, _vp, _vp, ctypes.c_int64, ctypes.c_int64, _vp, _vp, _vp,
                                  _vp]
+    L.mms_trace_pad_rows.restype = ctypes.c_int
+    L.mms_trace_pad_rows.argtypes = [_vp, ctypes.c_int64, ctypes.c_int64, _vp, _vp, _vp, _vp]
+    L.mms_trace_rows_histogram.restype = ctypes.c_int
+    L.mms_trace_rows_histogram.argtypes = [_vp, _vp, ctypes.c_int64, ctypes.c_int64, ctypes.c_int32,
+                                           _vp, _vp]
     L.mms_trace_next_same_model.restype = ctypes.c_int
     L.mms_trace_next_same_model.argtypes = [ctypes.POINTER(Trace), ctypes.c_int32, _vp, _vp]
     L.mms_sim_batching_workspace_bytes.restype = ctypes.c_size_t

@@ -481,7 +481,7 @@ int mms_sim_mixed(const mms_trace *trace, const mms_placements *cands, const mms
     using namespace mms;
     if (!trace || !cands || !plan || !ws || !out) return MMS_ERR_ARG;
     if (flags & ~(MMS_FLAG_PER_REQUEST | MMS_FLAG_LEGACY_CLOCK | MMS_FLAG_NO_GROUP_GOOD |
-                  MMS_FLAG_CROWDED | MMS_FLAG_NO_TWINS))
+                  MMS_FLAG_CROWDED | MMS_FLAG_NO_TWINS | MMS_FLAG_TRACE_ROWS))
         return MMS_ERR_ARG;
     const int64_t N = trace->num_requests;
     const bool gg = !(flags & MMS_FLAG_NO_GROUP_GOOD);
@@ -512,7 +512,10 @@ int mms_sim_mixed(const mms_trace *trace, const mms_placements *cands, const mms
     memset(&ka, 0, sizeof(ka));
     ka.arrivals = trace->arrivals; ka.model_ids = trace->model_ids; ka.slos = trace->slos;
     ka.N = N; ka.model_hist = model_hist;
-    ka.trace_pitch = trace->num_traces > 1 ? (int32_t)trace->num_traces : 1;
+    ka.many_traces = trace->num_traces > 1;
+    const bool rows = (flags & MMS_FLAG_TRACE_ROWS) != 0;
+    ka.trace_pitch = ka.many_traces && !rows ? trace->num_traces : 1;
+    ka.trace_stride = ka.many_traces ? (rows ? N : 1) : 0;
     ka.unsorted = trace->num_traces > 1
                       ? model_hist + (size_t)trace->num_traces * (cands->num_models + 1)
                       : model_hist + cands->num_models;
@@ -612,6 +615,38 @@ int mms_trace_pack(const double *arrivals, const int32_t *model_ids, const float
                               (cudaStream_t)stream>>>(arrivals, model_ids, slos, offsets,
                                                       num_traces, padded_requests, out_arrivals,
                                                       out_model_ids, out_slos);
+    MMS_CUDA(cudaGetLastError());
+    return MMS_OK;
+}
+
+int mms_trace_pad_rows(const int64_t *lengths, int64_t num_traces, int64_t num_requests,
+                       double *arrivals, int32_t *model_ids, float *slos, void *stream)
+{
+    if (num_traces < 0 || num_requests < 0) return MMS_ERR_ARG;
+    if (num_traces == 0 || num_requests == 0) return MMS_OK;
+    if (!lengths || !arrivals || !model_ids || !slos) return MMS_ERR_ARG;
+    if (num_traces > 0x7FFFFFFF) return MMS_ERR_UNSUPPORTED;
+    mms::pad_traces_kernel<<<dim3((unsigned)num_traces, 8), 256, 0, (cudaStream_t)stream>>>(
+        lengths, num_requests, arrivals, model_ids, slos);
+    MMS_CUDA(cudaGetLastError());
+    return MMS_OK;
+}
+
+int mms_trace_rows_histogram(const double *arrivals, const int32_t *model_ids, int64_t num_traces,
+                             int64_t num_requests, int32_t num_models, int32_t *hist, void *stream)
+{
+    if (num_traces < 1 || num_requests < 0 || num_models < 0 || !hist) return MMS_ERR_ARG;
+    if (num_traces > 0x7FFFFFFF || ((size_t)num_models + 1) * sizeof(int32_t) > 48 * 1024)
+        return MMS_ERR_UNSUPPORTED;
+    cudaStream_t st = (cudaStream_t)stream;
+    MMS_CUDA(cudaMemsetAsync(hist, 0, sizeof(int32_t) * ((size_t)num_traces * (num_models + 1) + 1), st));
+    if (num_requests == 0) return MMS_OK;
+    if (!arrivals || !model_ids) return MMS_ERR_ARG;
+    int64_t slices = (num_requests + 8191) / 8192;
+    if (slices > 64) slices = 64;
+    mms::histogram_rows_kernel<<<dim3((unsigned)num_traces, (unsigned)slices), 256,
+                                 sizeof(int32_t) * ((size_t)num_models + 1), st>>>(
+        arrivals, model_ids, num_requests, (int32_t)num_traces, num_models, hist);
     MMS_CUDA(cudaGetLastError());
     return MMS_OK;
 }

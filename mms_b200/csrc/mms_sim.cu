@@ -866,7 +866,7 @@ __global__ void model_requests_kernel(const KernelArgs a, int32_t *model_num_req
     if (t >= (int64_t)a.B * a.M) return;
     const int64_t b = t / a.M;
     const int m = (int)(t % a.M);
-    model_num_requests[t] = a.model_hist[(a.trace_pitch > 1 ? (size_t)b * (a.M + 1) : 0) + m];
+    model_num_requests[t] = a.model_hist[(a.many_traces ? (size_t)b * (a.M + 1) : 0) + m];
 }
 
 // Per-model request counts, plus the number of positions where the arrival
@@ -918,6 +918,47 @@ __global__ void histogram_traces_kernel(const double *arrivals, const int32_t *m
             atomicAdd(&hist[tt * (M + 1) + k % (M + 1)], local[k]);
             if (k % (M + 1) == M) atomicAdd(&hist[(size_t)T * (M + 1)], local[k]);
         }
+    }
+}
+
+// The same for T traces stored one after the other ([T][N]): a block covers a slice of
+// one trace.
+__global__ void histogram_rows_kernel(const double *arrivals, const int32_t *model_ids, int64_t N,
+                                      int32_t T, int32_t M, int32_t *hist)
+{
+    extern __shared__ int32_t local[];
+    for (int m = threadIdx.x; m <= M; m += blockDim.x) local[m] = 0;
+    __syncthreads();
+    const int64_t t = blockIdx.x;
+    const double *at = arrivals + t * N;
+    const int32_t *id = model_ids + t * N;
+    const int64_t step = (int64_t)gridDim.y * blockDim.x;
+    for (int64_t i = (int64_t)blockIdx.y * blockDim.x + threadIdx.x; i < N; i += step) {
+        const int32_t m = id[i];
+        if (m >= 0 && m < M) atomicAdd(&local[m], 1);
+        const double x = at[i];
+        if (!(x - x == 0.0) || (i > 0 && !(at[i - 1] <= x))) atomicAdd(&local[M], 1);
+    }
+    __syncthreads();
+    for (int m = threadIdx.x; m <= M; m += blockDim.x)
+        if (local[m]) {
+            atomicAdd(&hist[t * (M + 1) + m], local[m]);
+            if (m == M) atomicAdd(&hist[(size_t)T * (M + 1)], local[m]);
+        }
+}
+
+// Pads trace t of T traces stored one after the other ([T][N]) behind its lengths[t] requests,
+// as pack_traces_kernel does.
+__global__ void pad_traces_kernel(const int64_t *lengths, int64_t N, double *arrivals,
+                                  int32_t *model_ids, float *slos)
+{
+    const int64_t t = blockIdx.x, n = lengths[t];
+    const double last = n > 0 ? arrivals[t * N + n - 1] : 0.0;
+    for (int64_t i = n + (int64_t)blockIdx.y * blockDim.x + threadIdx.x; i < N;
+         i += (int64_t)gridDim.y * blockDim.x) {
+        arrivals[t * N + i] = last;
+        model_ids[t * N + i] = -1;
+        slos[t * N + i] = 0.0f;
     }
 }
 

@@ -18,8 +18,11 @@ struct KernelArgs {
     const int32_t *model_ids;
     const float *slos;
     int64_t N;
-    int32_t trace_pitch;          // 1: one trace for all candidates; T > 1: T traces stored
-                                  //   request-major ([N][T]), candidate b simulates trace b
+    int64_t trace_pitch, trace_stride;    // request i of candidate b's trace is element i *
+                                  //   trace_pitch + b * trace_stride: 1, 0 with one trace for all
+                                  //   candidates; T, 1 with T traces stored request-major ([N][T]);
+                                  //   1, N with T traces stored one after the other ([T][N])
+    bool many_traces;             // candidate b simulates trace b
     const int32_t *model_hist;    // [M + 1] request counts per model ([T][M + 1] with T traces)
     const int32_t *unsorted;      // number of unsorted / non-finite positions in the trace(s)
     // placements
@@ -126,7 +129,7 @@ __device__ inline bool can_chunk(const KernelArgs &a)
 // Offset of request 0 of the trace candidate b simulates.
 __device__ inline size_t trace_base(const KernelArgs &a, int64_t b)
 {
-    return a.trace_pitch > 1 ? (size_t)b : 0;
+    return (size_t)(b * a.trace_stride);
 }
 
 // Arrival time of request i in candidate b's trace.

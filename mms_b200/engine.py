@@ -269,6 +269,8 @@ class DeviceTraceBatch:
     request-major batch is made on the device (mms_trace_pack).
     Duck-type compatible with DeviceTrace where launches are concerned."""
 
+    flags = 0
+
     def __init__(self, arrivals: Sequence, model_ids: Sequence, slos: Sequence, num_models: int,
                  device=None, staged=False):
         """staged: upload through PinnedStager (worth it from about a gigabyte)."""
@@ -283,52 +285,60 @@ class DeviceTraceBatch:
             if not (len(model_ids[t]) == len(slos[t]) == int(self.lengths[t])):
                 raise ValueError(f"trace {t}: arrays differ in length")
         N = int(self.lengths.max())
-        total = int(self.lengths.sum())
         self.num_traces, self.num_requests, self.num_models = T, N, int(num_models)
-        offsets = np.concatenate(([0], np.cumsum(self.lengths))).astype(np.int64)
-        self.h2d_bytes = total * 16 + offsets.nbytes
-        L = nat.lib()
-        dev = self.device
-        with torch.cuda.device(dev):
-            cat_arr = torch.empty(max(total, 1), dtype=torch.float64, device=dev)
-            cat_mid = torch.empty(max(total, 1), dtype=torch.int32, device=dev)
-            cat_slo = torch.empty(max(total, 1), dtype=torch.float32, device=dev)
-            tasks = []
-            for t in range(T):
-                lo, hi = int(offsets[t]), int(offsets[t + 1])
-                if hi > lo:
-                    for dst, src, dtype in ((cat_arr, arrivals[t], np.float64),
-                                            (cat_mid, model_ids[t], np.int32),
-                                            (cat_slo, slos[t], np.float32)):
-                        if isinstance(src, LazyArray):
-                            if src.dtype != dtype:
-                                raise ValueError("lazy trace array of the wrong type")
-                            src = src if staged else src.materialize()
-                        else:
-                            src = np.ascontiguousarray(src, dtype)
-                        tasks.append((dst[lo:hi], src))
-            if staged:
-                PinnedStager.get(dev).upload(tasks)
-            else:
-                for dst, src in tasks:
-                    dst.copy_(torch.from_numpy(src), non_blocking=True)
-            d_off = _to_device(offsets, dev)
-            self.arrivals = torch.empty((max(N, 1), T), dtype=torch.float64, device=dev)
-            self.model_ids = torch.empty((max(N, 1), T), dtype=torch.int32, device=dev)
-            self.slos = torch.empty((max(N, 1), T), dtype=torch.float32, device=dev)
-            nat.check(L.mms_trace_pack(_ptr(cat_arr), _ptr(cat_mid), _ptr(cat_slo), _ptr(d_off),
-                                       T, N, _ptr(self.arrivals), _ptr(self.model_ids),
-                                       _ptr(self.slos), _stream_ptr()), "mms_trace_pack")
+        self.h2d_bytes = int(self.lengths.sum()) * 16 + (T + 1) * 8
+        with torch.cuda.device(self.device):
+            self._store((arrivals, model_ids, slos), staged)
             leaf_start, leaf_merges = _sum_plan(N)
             self.num_leaves = len(leaf_start) - 1
-            self.leaf_start, self.leaf_merges = _to_device_many((leaf_start, leaf_merges), dev)
+            self.leaf_start, self.leaf_merges = _to_device_many((leaf_start, leaf_merges),
+                                                                self.device)
             # [T][M + 1] counts, then the total of unsorted positions (T == 1: plain [M + 1])
             cells = T * (self.num_models + 1) + (1 if T > 1 else 0)
-            self.model_hist = torch.zeros(cells, dtype=torch.int32, device=dev)
-            tr = self.c_trace()
-            nat.check(L.mms_trace_model_histogram(ctypes.byref(tr), self.num_models,
-                                                  _ptr(self.model_hist), _stream_ptr()),
-                      "mms_trace_model_histogram")
+            self.model_hist = torch.zeros(cells, dtype=torch.int32, device=self.device)
+            self._count()
+
+    def _upload(self, sources, staged, place):
+        """Copies array k of trace t to place(k, t), every trace as it is."""
+        tasks = []
+        for t in range(self.num_traces):
+            if not self.lengths[t]:
+                continue
+            for k, dtype in enumerate((np.float64, np.int32, np.float32)):
+                src = sources[k][t]
+                if isinstance(src, LazyArray):
+                    if src.dtype != dtype:
+                        raise ValueError("lazy trace array of the wrong type")
+                    src = src if staged else src.materialize()
+                else:
+                    src = np.ascontiguousarray(src, dtype)
+                tasks.append((place(k, t), src))
+        if staged:
+            PinnedStager.get(self.device).upload(tasks)
+        else:
+            for dst, src in tasks:
+                dst.copy_(torch.from_numpy(src), non_blocking=True)
+
+    def _empty(self, shape):
+        return tuple(torch.empty(shape, dtype=t, device=self.device)
+                     for t in (torch.float64, torch.int32, torch.float32))
+
+    def _store(self, sources, staged):
+        N, T = self.num_requests, self.num_traces
+        offsets = np.concatenate(([0], np.cumsum(self.lengths))).astype(np.int64)
+        cat = self._empty(max(int(offsets[-1]), 1))
+        self._upload(sources, staged, lambda k, t: cat[k][int(offsets[t]):int(offsets[t + 1])])
+        d_off = _to_device(offsets, self.device)
+        self.arrivals, self.model_ids, self.slos = self._empty((max(N, 1), T))
+        nat.check(nat.lib().mms_trace_pack(
+            *(_ptr(x) for x in cat), _ptr(d_off), T, N, _ptr(self.arrivals),
+            _ptr(self.model_ids), _ptr(self.slos), _stream_ptr()), "mms_trace_pack")
+
+    def _count(self):
+        tr = self.c_trace()
+        nat.check(nat.lib().mms_trace_model_histogram(
+            ctypes.byref(tr), self.num_models, _ptr(self.model_hist), _stream_ptr()),
+            "mms_trace_model_histogram")
 
     def c_trace(self):
         return nat.Trace(self.num_requests, _ptr(self.arrivals), _ptr(self.model_ids),
@@ -336,6 +346,32 @@ class DeviceTraceBatch:
 
     def c_plan(self):
         return nat.SumPlan(self.num_leaves, 0, _ptr(self.leaf_start), _ptr(self.leaf_merges))
+
+
+class DeviceTraceRows(DeviceTraceBatch):
+    """The same traces stored one after the other ([T][N]): a warp that
+    simulates one candidate reads 32 consecutive requests of its trace at a
+    time.  Every trace is uploaded straight to its place, so that nothing is
+    copied again on the device."""
+
+    flags = nat.FLAG_TRACE_ROWS
+
+    def _store(self, sources, staged):
+        N, T = self.num_requests, self.num_traces
+        self.arrivals, self.model_ids, self.slos = self._empty((T, max(N, 1)))
+        rows = (self.arrivals, self.model_ids, self.slos)
+        self._upload(sources, staged, lambda k, t: rows[k][t, :int(self.lengths[t])])
+        if np.any(self.lengths < N):
+            d_len = _to_device(self.lengths, self.device)
+            nat.check(nat.lib().mms_trace_pad_rows(_ptr(d_len), T, N, *(_ptr(x) for x in rows),
+                                                   _stream_ptr()), "mms_trace_pad_rows")
+
+    def _count(self):
+        if self.num_traces == 1:                     # one trace: both layouts are the same
+            return super()._count()
+        nat.check(nat.lib().mms_trace_rows_histogram(
+            _ptr(self.arrivals), _ptr(self.model_ids), self.num_traces, self.num_requests,
+            self.num_models, _ptr(self.model_hist), _stream_ptr()), "mms_trace_rows_histogram")
 
 
 class LatencyTable:
@@ -955,6 +991,7 @@ def _prepare(trace: DeviceTrace, B, M, G, P, T, S, C, model_off, model_rep, grou
     dev = trace.device
     N = trace.num_requests
     opts = options if options is not None else sim_options()
+    flags |= getattr(trace, "flags", 0)
     if not want_group_good:
         flags |= nat.FLAG_NO_GROUP_GOOD
     job = _Pending()

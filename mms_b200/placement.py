@@ -291,10 +291,10 @@ class ResidentSweep:
             side = torch.cuda.Stream(device=self.device)
             side.wait_stream(main)
             with torch.cuda.stream(side if eager else main):
-                traces = engine.DeviceTraceBatch([workloads[t].arrivals for t in idx],
-                                                 [arrays[t][0] for t in idx],
-                                                 [arrays[t][1] for t in idx], M,
-                                                 device=self.device, staged=eager)
+                traces = engine.DeviceTraceRows([workloads[t].arrivals for t in idx],
+                                                [arrays[t][0] for t in idx],
+                                                [arrays[t][1] for t in idx], M,
+                                                device=self.device, staged=eager)
                 job = engine.ResidentBatch(traces, sweep.enc.repeat(len(idx)), sweep.table,
                                            options=sweep.options, split=False)
                 if eager:

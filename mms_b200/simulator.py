@@ -241,20 +241,6 @@ def workload_arrays(workload, model_names):
     return ids, slos
 
 
-def fast_stats(model_names, start, finish_minus_start_sum, good_total, model_num_requests,
-               model_num_good, group_num_requests) -> StatsResult:
-    """The no-warm-up statistics of controller.py:393-403, from the reduced
-    quantities the GPU returns: np.mean(good) = good_total / N and
-    np.mean(finish - start) = (numpy-ordered sum) / N."""
-    n = len(start)
-    interval = start[-1] - start[0]
-    per_model = _per_model(model_names, model_num_requests, model_num_good, interval)
-    goodput = np.float64(good_total) / n
-    latency_mean = np.float64(finish_minus_start_sum) / n
-    return StatsResult(per_model, tuple(group_num_requests), goodput, latency_mean, n,
-                       n / interval)
-
-
 def _per_model(model_names, model_num_requests, model_num_good, interval):
     """The per-model rows of controller.py:393-403 (one division of arrays instead of one of
     numpy scalars per model: these are a third of a small call)."""
