@@ -26,6 +26,11 @@ namespace mms {
 constexpr int kWindowWarps = 4;        // warps of a window-kernel block (they share the table)
 constexpr int kWindowBlocksPerSm = 3;
 constexpr size_t kOrderBytes = 32;     // see window_groups
+// Longest pipelines that window_groups serves.  Both ways cost about the same from four stages on
+// (170 ns a request by groups, 145 ns in rounds, 4 groups of 4; 199 and 234 ns, 6 mixed ones); with
+// eight the rounds win (22 mixed groups: 199 and 183 ns; a sweep of 48 overloaded traces: 86 and
+// 62 ms), with one the groups (16 groups under overload: layers of a search 84 and 277 ms).
+constexpr int kGroupDepth = 4;
 constexpr int kWindowList = 1024;      // (group, model) pairs of a candidate kept on chip, at most
 
 // Depth the on-chip tables are laid out for: the batch's deepest pipeline rounded up to a
@@ -177,7 +182,9 @@ __device__ inline void window_setup(const KernelArgs &a, Window &w, int64_t b)
         for (int e = lane; e < a.P; e += kLanes)
             SM_U32(w.list + e) = rep_to_last(a.model_rep[(size_t)b * a.P + e]);
     // lane g's groups, for window_groups
-    w.by_group = w.depth > 0 && (a.G <= kLanes || (a.G <= 2 * kLanes && w.depth <= 2)) && w.lat_on_chip && a.P <= kWindowList && w.arrivals[0] >= 0.0;
+    w.by_group = w.depth > 0 && w.depth <= kGroupDepth &&
+                 (a.G <= kLanes || (a.G <= 2 * kLanes && w.depth <= 2)) && w.lat_on_chip &&
+                 a.P <= kWindowList && w.arrivals[0] >= 0.0;
     w.column = 0;
     for (int h = 0; h < 2; ++h) {
         const int g = lane + h * kLanes;
@@ -316,7 +323,7 @@ __device__ __noinline__ WindowTies window_ties(uint32_t need, uint32_t clk, uint
 // replicas and whoever else is waiting, and nothing of it passes through shared memory: the
 // orders — arrival time, SLO, the model's groups as a mask, its latency row — are laid out there
 // beforehand.  For candidates of up to 32 groups, or 64 in pipelines of one or two stages (two
-// groups to a lane).
+// groups to a lane), and pipelines of up to kGroupDepth stages.
 //
 // Out: fin, rec, tie, swap of the requests in their lanes, as window_rounds leaves them.
 struct __align__(16) WindowOrder {
@@ -730,7 +737,7 @@ __device__ inline int32_t window_run_depth(const KernelArgs &a, Window &w, WalkM
             const uint32_t upto = to - base >= kLanes ? 0xFFFFFFFFu : (1u << (to - base)) - 1u;
             const uint32_t active = upto & ~((1u << (i - base)) - 1u);
             bool rounds = true;
-            if constexpr (kDepth > 0) {
+            if constexpr (kDepth > 0 && kDepth <= kGroupDepth) {
                 if (w.by_group) {
                     rounds = false;
                     const bool in = (active >> lane) & 1u;
