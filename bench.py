@@ -631,7 +631,7 @@ def run_candidates(args, D):
                     "d2h_bytes_per_step": int(d2h)},
             # clear, tables, stream, (link, resolve, walk) per round, link, finish, count,
             # requests per model — per launch — and the argmax
-            "gpu_launches": ((7 + 3 * (args.rounds if args.rounds > 0 else 4) + 1) * args.steps
+            "gpu_launches": ((7 + 3 * (args.rounds if args.rounds > 0 else 1) + 1) * args.steps
                              * len(resident.jobs)),
             "mirror_candidates_per_gpu": int(n_mirrors),
             "launches_per_step": len(resident.jobs),
@@ -1079,7 +1079,7 @@ def run_sweep(args, D, traces=1024, duration=3600.0, steps=None, cpu=True):
                      "algorithmic_bytes_per_launch": dom_units * BYTES_PER_UNIT},
         "e2e": {"value": e2e_value, "unit": UNIT, "h2d_bytes_per_step": int(sweep.last_h2d_bytes),
                 "d2h_bytes_per_step": int(sweep.last_d2h_bytes)},
-        "gpu_launches": (7 + 3 * (args.rounds if args.rounds > 0 else 4)) * n_groups * steps,
+        "gpu_launches": (7 + 3 * (args.rounds if args.rounds > 0 else 1)) * n_groups * steps,
         "chunks_resimulated_per_trace": float(np.mean(res.resimulated)),
         "clocks": clk.summary(),
         "goodput_mean_per_cell": [float(x) for x in (tally_host[:, 0] / np.maximum(tally_host[:, 1], 1))],

@@ -49,7 +49,10 @@ constexpr int kMaxSumDepth = 48;        // pair-sum stack of the numpy order
 constexpr int kLatSmemBytes = 32 * 1024;
 constexpr int kMaxRepairRounds = 16;
 constexpr int kTwinModels = 256;        // models a launch with interchangeable groups may have
-constexpr int kDefaultRepairRounds = 4;
+// One round of parallel walks: what it leaves open is walked once more by finish_kernel in any
+// case, and each further round is three launches (4 rounds and 1: one placement 405 and 386 us,
+// a layer of 2343 86.7 and 79.1 ms, a search 197 and 193 ms, 4096 placements the same).
+constexpr int kDefaultRepairRounds = 1;
 
 // What a call clears before its kernels run, in one launch (grid-stride): the
 // work lists and marks of the time-parallel machinery, the outputs
@@ -679,7 +682,8 @@ finish_kernel(const __grid_constant__ KernelArgs a)
             if (a.resimulated) atomicAdd(&a.resimulated[b], 1);
         }
         __syncwarp();
-        const int32_t e = window_run<kLegacy, kTwins>(a, w, kWalkChain, j, a.leaf_start[seg_leaf(a, q)], true, q);
+        // (nothing is noted about choices between twins: nobody compares with these segments again)
+        const int32_t e = window_run<kLegacy, kTwins, false>(a, w, kWalkChain, j, a.leaf_start[seg_leaf(a, q)], true, q);
         labels_reset(l, a.G);
         q = e;
     }

@@ -657,7 +657,10 @@ __device__ __forceinline__ void window_rounds(const KernelArgs &a, const Window 
 enum WalkMode { kNoWalk = 0, kWalkRound = 1, kWalkChain = 2 };
 constexpr int32_t kMaxPause = 1024;    // requests between two comparisons, at most
 
-template <bool kLegacy, int kDepth, bool kTwins>
+//
+// kTwins: stored runs may be compared under other labels.  kLog: choices that the group number
+// decides are noted (tie, swaps) for those who compare later.
+template <bool kLegacy, int kDepth, bool kTwins, bool kLog>
 __device__ inline int32_t window_run_depth(const KernelArgs &a, Window &w, WalkMode walk, int32_t j,
                                            int32_t begin, bool snapshots, int32_t q_begin)
 {
@@ -745,13 +748,13 @@ __device__ inline int32_t window_run_depth(const KernelArgs &a, Window &w, WalkM
                     __syncwarp();
                     const uint32_t todo = __ballot_sync(0xFFFFFFFFu, in && serves);
                     if (kDepth > 2 || a.G <= kLanes)
-                        window_groups<kDepth, 1, kTwins>(a, w, todo, fin, rec, tie, swap);
+                        window_groups<kDepth, 1, kLog>(a, w, todo, fin, rec, tie, swap);
                     else if constexpr (kDepth <= 2)
-                        window_groups<kDepth, 2, kTwins>(a, w, todo, fin, rec, tie, swap);
+                        window_groups<kDepth, 2, kLog>(a, w, todo, fin, rec, tie, swap);
                 }
             }
             if (rounds)
-                window_rounds<kLegacy, kDepth, kTwins>(a, w, cur, conf, serves, active, fin, rec, tie, swap);
+                window_rounds<kLegacy, kDepth, kLog>(a, w, cur, conf, serves, active, fin, rec, tie, swap);
             if (record) {
                 const bool in = (active >> lane) & 1u;
                 const int32_t at = base + lane;
@@ -767,7 +770,7 @@ __device__ inline int32_t window_run_depth(const KernelArgs &a, Window &w, WalkM
                     if (in && (lane & 3) == 0)
                         static_cast<uint32_t *>(a.decisions)[(size_t)(at >> 2) * a.dec_pitch + b] = word;
                 }
-                if (kTwins && in)            // which choices the group number decided
+                if (kLog && in)              // which choices the group number decided
                     a.swaps[((size_t)(at >> 2) * a.dec_pitch + b) * 4 + (at & 3)] = swap;
                 if (a.finish && in) {
                     a.finish[(size_t)b * a.N + at] = fin;
@@ -817,7 +820,7 @@ __device__ inline int32_t window_run_depth(const KernelArgs &a, Window &w, WalkM
         if (snapshots) {
             const bool compare = walk && pause == 0 && i < a.N;
             if (pause > 0) --pause;
-            if constexpr (kTwins) {
+            if constexpr (kLog) {
                 const uint32_t lo = __reduce_or_sync(0xFFFFFFFFu, (uint32_t)tie);
                 const uint32_t hi = __reduce_or_sync(0xFFFFFFFFu, (uint32_t)(tie >> 32));
                 tie = 0;
@@ -902,11 +905,11 @@ __device__ inline int32_t window_run_depth(const KernelArgs &a, Window &w, WalkM
     }
 }
 
-template <bool kLegacy, bool kTwins>
+template <bool kLegacy, bool kTwins, bool kLog = kTwins>
 __device__ inline int32_t window_run(const KernelArgs &a, Window &w, WalkMode walk, int32_t j,
                                      int32_t begin, bool snapshots, int32_t q_begin)
 {
-#define MMS_WINDOW_DEPTH(D) window_run_depth<kLegacy, D, kTwins>(a, w, walk, j, begin, snapshots, q_begin)
+#define MMS_WINDOW_DEPTH(D) window_run_depth<kLegacy, D, kTwins, kLog>(a, w, walk, j, begin, snapshots, q_begin)
     if constexpr (!kLegacy) {
         switch (w.depth) {
             case 1: return MMS_WINDOW_DEPTH(1);
