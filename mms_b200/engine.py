@@ -451,12 +451,19 @@ class EncodedBatch:
         self.group_info = group_info      # u32[B][G]
         self.num_groups = num_groups      # i64[B]
         self.num_replicas = num_replicas  # i64[B]: sum of len(group_models)
-        # (candidate index, [[group ids of one class of interchangeable groups], ...])
-        # for every placement that has such groups, see twin_groups()
-        self.twins = twins
+        self._twins = twins               # see twins; or a function that makes it
         # bool[B]: the placement has interchangeable groups at all (None: not known)
         self.has_twins = has_twins
         self._mirror_table = None         # see mirror_table()
+
+    @property
+    def twins(self):
+        """[(candidate index, [[group ids of one class of interchangeable groups], ...])]
+        for every placement that has such groups, see twin_groups().  Made when somebody
+        asks: running a batch only needs has_twins."""
+        if callable(self._twins):
+            self._twins = self._twins()
+        return self._twins
 
     def may_have_twins(self):
         return self.has_twins is None or bool(np.any(self.has_twins))
@@ -472,17 +479,20 @@ class EncodedBatch:
     def take(self, index):
         """The sub-batch of the placements `index` (ascending)."""
         index = np.asarray(index, np.int64)
-        new_id = np.full(self.B, -1, np.int64)
-        new_id[index] = np.arange(len(index))
-        keep = [k for k, (b, _) in enumerate(self.twins or []) if new_id[b] >= 0]
-        twins = [(int(new_id[self.twins[k][0]]), self.twins[k][1]) for k in keep]
+
+        def kept():
+            new_id = np.full(self.B, -1, np.int64)
+            new_id[index] = np.arange(len(index))
+            keep = [k for k, (b, _) in enumerate(self.twins or []) if new_id[b] >= 0]
+            return keep, [(int(new_id[self.twins[k][0]]), self.twins[k][1]) for k in keep]
+
         sub = EncodedBatch(len(index), self.M, self.G, self.P, self.T, self.S, self.C,
                            self.model_off[index], self.model_rep[index], self.group_info[index],
-                           self.num_groups[index], self.num_replicas[index], twins,
+                           self.num_groups[index], self.num_replicas[index], lambda: kept()[1],
                            None if self.has_twins is None else self.has_twins[index])
         if self._mirror_table is not None:
             counts, words = self._mirror_table
-            keep = np.asarray(keep, np.int64)
+            keep = np.asarray(kept()[0], np.int64)
             start = np.concatenate(([0], np.cumsum(counts)))[:-1]
             sub_counts = counts[keep]
             # the kept placements' stretches of `words`, one after the other
@@ -495,7 +505,10 @@ class EncodedBatch:
         """This batch `count` times over (placement 0 .. B-1, then again ...):
         the tables of one placement for `count` traces."""
         B = self.B
-        twins = [(b + k * B, classes) for k in range(count) for b, classes in (self.twins or [])]
+
+        def twins():
+            return [(b + k * B, classes) for k in range(count) for b, classes in (self.twins or [])]
+
         return EncodedBatch(B * count, self.M, self.G, self.P, self.T, self.S, self.C,
                             np.tile(self.model_off, (count, 1)), np.tile(self.model_rep, (count, 1)),
                             np.tile(self.group_info, (count, 1)), np.tile(self.num_groups, count),
@@ -790,16 +803,20 @@ def _encode_native(H, B, M, table, n_groups, cfg, n_in_group, placed_model) -> E
         raise IndexError("model id in group_models is out of range")
     T = int(slots[:B].max()) if B else 0
     _too_large(G, T, S, C)
-    twins = []
-    prev_b, prev_c = -1, -1
-    for b, c, g in items[:int(n_items[0])].tolist():
-        if b != prev_b:
-            twins.append((b, []))
-            prev_c = -1
-        if c != prev_c:
-            twins[-1][1].append([])
-        twins[-1][1][-1].append(g)
-        prev_b, prev_c = b, c
+
+    def twins():
+        out = []
+        prev_b, prev_c = -1, -1
+        for b, c, g in items[:int(n_items[0])].tolist():
+            if b != prev_b:
+                out.append((b, []))
+                prev_c = -1
+            if c != prev_c:
+                out[-1][1].append([])
+            out[-1][1][-1].append(g)
+            prev_b, prev_c = b, c
+        return out
+
     return EncodedBatch(B, M, Gc, Pc, max(T, 1), S, C, model_off, model_rep, group_info,
                         n_groups, placed_per_b.astype(np.int64), twins, has_twins[:B].astype(bool))
 
