@@ -806,7 +806,7 @@ static int plan_batching(int64_t N, const mms_placements *c, const mms_batching 
                                           2 * ((size_t)c->num_models + c->max_groups + 2 +
                                                c->max_placed)) + 64);
     g->rounds = kBatchRepairRounds;
-    g->off_work = off;     off += g->K > 1 ? align256(sizeof(uint32_t) * (cells + 64)) : 0;
+    g->off_work = off;     off += g->K > 1 ? align256(sizeof(uint32_t) * (cells + 64) + cells) : 0;
     g->off_start = off;    off += g->K > 1 ? align256(cells * sb) : 0;
     g->off_end = off;      off += g->K > 1 ? align256(cells * sb) : 0;
     g->total = off;
@@ -941,14 +941,17 @@ int mms_sim_batching(const mms_trace *trace, const mms_placements *cands,
         // a few rounds of parallel repairs, one re-simulated chunk per warp, then the chain
         a.work_count = (uint32_t *)(scratch + geo.off_work);
         a.work_items = a.work_count + 64;
+        a.link = (uint8_t *)(a.work_items + (size_t)a.K * B);
         MMS_CUDA(cudaMemsetAsync(a.work_count, 0, sizeof(uint32_t) * 64, st));
         MMS_TRY(allow_smem((const void *)batch_repair_kernel, geo.smem_single));
         const int64_t bounds = (int64_t)B * (a.K - 1);
         ProfileSpan repair_span(MMS_PROFILE_BATCH_REPAIR, st);
-        for (int r = 0; r < geo.rounds; ++r) {
+        a.rounds = geo.rounds;
+        for (int r = 0; r <= geo.rounds; ++r) {
             a.round = r;
             batch_validate_kernel<<<(unsigned)((bounds + 127) / 128), 128, 0, st>>>(a);
             MMS_CUDA(cudaGetLastError());
+            if (r == geo.rounds) break;
             batch_repair_kernel<<<(unsigned)bounds, kLanes, geo.smem_single, st>>>(a);
             MMS_CUDA(cudaGetLastError());
         }
