@@ -450,14 +450,13 @@ def run_candidates(args, D):
     L = nat.lib()
 
     # ---- device-resident arm: tables already in HBM, time the C-ABI call(s) ----
-    # B placements are scored; the ones with interchangeable groups bring mirror candidates
-    # and go into a launch of their own beside the rest (engine.ResidentBatch)
+    # B placements are scored; the ones with interchangeable groups go into a launch of their
+    # own beside the rest (engine.ResidentBatch)
     enc = engine.encode_placements(mine, ev.table, len(ev.model_names))
     hard = engine.sim_options(*[int(x) for x in args.hard.split(",")]) if args.hard else None
     resident = engine.ResidentBatch(ev.trace, enc, ev.table, options=opts,
                                     mirrors=not args.no_mirrors, split=not args.no_split,
                                     hard_options=hard)
-    n_mirrors = sum(job.B - job.Bs for job in resident.jobs)
     flush = torch.empty(256 << 20, dtype=torch.uint8, device=dev)   # > 126 MB of L2
     best = torch.zeros(2, dtype=torch.float64, device=dev)
     gathered = torch.zeros(2 * world, dtype=torch.float64, device=dev)
@@ -506,9 +505,9 @@ def run_candidates(args, D):
     D.barrier()
     span_ms, span_tag = nat.profile_end()
     # the dominant kernel: the stream kernel of the step's largest launch (with a split step,
-    # launch 0 holds the placements with mirror candidates and launch 1 the rest)
+    # launch 0 holds the placements with interchangeable groups and launch 1 the rest)
     per_step = len(resident.jobs)
-    big = int(np.argmax([job.Bs for job in resident.jobs]))
+    big = int(np.argmax([job.B for job in resident.jobs]))
     stream_ms = span_ms[span_tag == nat.PROFILE_STREAM]
     chain_ms = span_ms[span_tag == nat.PROFILE_CHAIN]
     stream_kernel_ms = float(np.mean(stream_ms[big::per_step])) if len(stream_ms) else float("nan")
@@ -518,7 +517,7 @@ def run_candidates(args, D):
     stream_ms_by_launch = [round(float(np.mean(stream_ms[k::per_step])), 3) for k in range(per_step)]
     chain_ms_by_launch = [round(float(np.mean(chain_ms[k::per_step])), 3) for k in range(per_step)] \
         if len(chain_ms) == len(stream_ms) else []
-    kernel_units = resident.jobs[big].Bs * N
+    kernel_units = resident.jobs[big].B * N
     total_ms = D.reduce(sum(times), "max")
     by_rank = [round(float(x), 3) for x in D.gather([float(np.mean(own_times))])[:, 0]]
     final, _ = resident.results()
@@ -599,7 +598,7 @@ def run_candidates(args, D):
         call_achieved = B * N * BYTES_PER_UNIT / (np.mean(times) * 1e-3) / 1e9
         t = STREAM_KERNEL_TRAFFIC
         traffic = t["bytes"] if (t["abi_version"] == L.mms_abi_version() and
-                                 (t["candidates"], t["requests"]) == (resident.jobs[big].Bs, N)) else None
+                                 (t["candidates"], t["requests"]) == (resident.jobs[big].B, N)) else None
         line = {
             "metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world,
             "steps": args.steps, "warmup": max(args.warmup, 3),
@@ -616,7 +615,7 @@ def run_candidates(args, D):
                          "traffic_unit": "bytes per sim_stream_kernel launch (ncu, DRAM read+write)",
                          "dram_gbs": (traffic / (stream_kernel_ms * 1e-3) / 1e9) if traffic else None,
                          "kernel": "sim_stream_kernel", "kernel_ms": stream_kernel_ms,
-                         "kernel_candidates": int(resident.jobs[big].Bs),
+                         "kernel_candidates": int(resident.jobs[big].B),
                          "kernel_launches_timed": int(len(stream_ms)) // per_step,
                          "chain_kernel_ms_max": chain_kernel_ms,
                          # per launch of a step, in launch order (they overlap on the GPU)
@@ -633,7 +632,6 @@ def run_candidates(args, D):
             # requests per model — per launch — and the argmax
             "gpu_launches": ((7 + 3 * (args.rounds if args.rounds > 0 else 1) + 1) * args.steps
                              * len(resident.jobs)),
-            "mirror_candidates_per_gpu": int(n_mirrors),
             "launches_per_step": len(resident.jobs),
             # each rank's simulation per step, before the selection and its exchange
             "kernel_ms_per_step_by_rank": by_rank,
@@ -1047,7 +1045,7 @@ def run_sweep(args, D, traces=1024, duration=3600.0, steps=None, cpu=True):
     peak, which = hbm_peak()
     if chain_by_group and max(chain_by_group) >= max(stream_by_group or [0.0]):
         g = int(np.argmax(chain_by_group))
-        dominant, dom_ms, dom_units = "sim_chain_kernel", chain_by_group[g], group_units[g]
+        dominant, dom_ms, dom_units = "finish_kernel", chain_by_group[g], group_units[g]
     elif stream_by_group:
         g = int(np.argmax(stream_by_group))
         dominant, dom_ms, dom_units = "sim_stream_kernel", stream_by_group[g], group_units[g]

@@ -202,7 +202,7 @@ const char *mms_last_error(void);
  * unsynchronised, so use it from ONE host thread with no other thread inside
  * the library, and on one device. */
 #define MMS_PROFILE_STREAM 0        /* sim_stream_kernel                          */
-#define MMS_PROFILE_CHAIN 1         /* sim_chain_kernel (both forms, one span)    */
+#define MMS_PROFILE_CHAIN 1         /* finish_kernel                              */
 #define MMS_PROFILE_BATCH_STREAM 2  /* batch_stream_kernel                        */
 #define MMS_PROFILE_BATCH_CHAIN 3   /* batch_chain_kernel                         */
 #define MMS_PROFILE_CALL 4          /* a whole mms_sim_mixed call                 */
