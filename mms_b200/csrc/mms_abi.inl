@@ -914,7 +914,7 @@ int mms_sim_batching(const mms_trace *trace, const mms_placements *cands,
     if (out->resimulated)
         MMS_CUDA(cudaMemsetAsync(out->resimulated, 0, sizeof(int32_t) * (size_t)B, st));
     if (N > 0 && a.K > 1) {
-        unsorted_kernel<<<296, 256, 0, st>>>(trace->arrivals, N, (int32_t *)(scratch + geo.off_flag));
+        uncuttable_kernel<<<296, 256, 0, st>>>(a, (int32_t *)(scratch + geo.off_flag));
         MMS_CUDA(cudaGetLastError());
     }
     MMS_TRY(allow_smem((const void *)batch_chain_kernel, geo.smem_single));

@@ -74,9 +74,7 @@ struct ClearArgs {
     uint16_t *twin_class;             // see KernelArgs
     uint8_t *twins;
     uint32_t *column_stages;          // [C] stages of the groups that use the column
-    uint32_t *irregular;              // != 0: a column is used with different numbers of stages, a
-                                      //   replica's slots are not its group's, a group has several
-                                      //   columns, or a replica list is not in ascending group order
+    uint32_t *irregular;              // kIrregularLayout | kIrregularLatency
 };
 
 __device__ inline bool group_info_valid(const KernelArgs &a, uint32_t info)
@@ -128,7 +126,8 @@ __global__ void clear_kernel(const KernelArgs a, const ClearArgs c)
 // the groups of a list with more than one replica as contested; a list with a
 // bad index is reported in the status word and emptied.  (2) One thread per
 // (candidate, group) reports a group_info entry that clear_kernel had to empty.
-// (3) One thread per segment finds the segment's first leaf.
+// (3) One thread per segment finds the segment's first leaf.  (4) The latency tables are looked
+// through for entries that are not >= 0 (kIrregularLatency).
 __global__ void build_tables_kernel(const KernelArgs a, const ClearArgs c)
 {
     const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -136,6 +135,11 @@ __global__ void build_tables_kernel(const KernelArgs a, const ClearArgs c)
     for (int64_t q = tid; q <= a.NS; q += nth)
         a.seg_first_leaf[q] = q == 0 ? 0 : q == a.NS ? a.num_leaves
             : leaf_lower_bound(a.leaf_start, a.num_leaves, q * a.seg_len);
+    const int64_t entries = (int64_t)a.M * a.C * a.S;
+    bool odd = false;
+    for (int64_t i = tid; i < (a.latency_stride ? a.B * entries : entries); i += nth)
+        odd |= !(a.latency[i / entries * a.latency_stride + i % entries] >= 0.0f);
+    if (odd) atomicOr(c.irregular, kIrregularLatency);
     for (int64_t i = tid; i < (int64_t)a.B * a.G; i += nth)
         if (!group_info_valid(a, c.group_info_in[i]))
             atomicOr(&a.status[i / a.G], MMS_STATUS_BAD_INDEX);
@@ -161,12 +165,13 @@ __global__ void build_tables_kernel(const KernelArgs a, const ClearArgs c)
                     const uint32_t was = atomicCAS(&c.column_stages[ent >> 24], 0u, ns);
                     if ((was != 0 && was != ns) ||
                         ((c.group_info_in[(size_t)b * a.G + (ent & 0xFFu)] & 0xFFFFu) != (first | (ns << 8))))
-                        *c.irregular = 1;
+                        atomicOr(c.irregular, kIrregularLayout);
                     const size_t gg = (size_t)b * a.G + (ent & 0xFFu);
                     const uint32_t col = atomicCAS(&c.group_column[gg], 0xFFFFFFFFu, ent >> 24);
-                    if (col != 0xFFFFFFFFu && col != ent >> 24) *c.irregular = 1;
+                    if (col != 0xFFFFFFFFu && col != ent >> 24) atomicOr(c.irregular, kIrregularLayout);
                     // ... and take the first of the smallest clocks for the lowest group number
-                    if (r > lo && (a.model_rep[(size_t)b * a.P + r - 1] & 0xFFu) >= (ent & 0xFFu)) *c.irregular = 1;
+                    if (r > lo && (a.model_rep[(size_t)b * a.P + r - 1] & 0xFFu) >= (ent & 0xFFu))
+                        atomicOr(c.irregular, kIrregularLayout);
                     if (a.K > 1 && c.group_words)
                         atomicOr((unsigned long long *)&c.group_models[gg * c.group_words + (m >> 6)], 1ull << (m & 63));
                     if (r - lo < 8)

@@ -69,7 +69,8 @@ struct BatchArgs {
     int32_t K;                    // chunks
     int32_t chunk_len;            // arrivals per chunk (the last one takes the rest)
     int32_t warmup;               // run-in arrivals of a speculative chunk
-    const int32_t *unsorted;      // != 0: arrival times not sorted / not finite -> one chunk
+    const int32_t *unsorted;      // != 0: arrival times not sorted / not finite, or a latency not
+                                  //   >= 0 -> one chunk
     unsigned char *snap_start;    // [K][B][state_bytes]: state a speculative chunk started from
     unsigned char *snap_end;      // [K][B][state_bytes]: state after the chunk's last arrival
     uint32_t *chunk_counters;     // [K][B][2M + 2G]
@@ -1042,15 +1043,21 @@ __global__ void batch_sum_kernel(const BatchArgs a)
     else a.group_num_good[(size_t)b * a.G + (c - 2 * a.M - a.G)] = (int32_t)v;
 }
 
-// Number of positions where the arrival times are not finite or go backwards.
-__global__ void unsorted_kernel(const double *arrivals, int64_t N, int32_t *count)
+// Number of positions where the arrival times are not finite or go backwards, and of latencies
+// that are not >= 0 (batch_equivalent needs clocks that an accepted request leaves at or behind
+// its arrival, see kIrregularLatency).
+__global__ void uncuttable_kernel(const BatchArgs a, int32_t *count)
 {
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+    const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     int32_t bad = 0;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < N; i += stride) {
-        const double t = arrivals[i];
-        if (!(t - t == 0.0) || (i > 0 && !(arrivals[i - 1] <= t))) ++bad;
+    for (int64_t i = tid; i < a.N; i += stride) {
+        const double t = a.arrivals[i];
+        if (!(t - t == 0.0) || (i > 0 && !(a.arrivals[i - 1] <= t))) ++bad;
     }
+    const int64_t entries = (int64_t)a.M * a.C * a.S * a.NB;
+    for (int64_t i = tid; i < (a.latency_stride ? a.B * entries : entries); i += stride)
+        bad += !(a.latency[i / entries * a.latency_stride + i % entries] >= 0.0f);
     if (bad) atomicAdd(count, bad);
 }
 

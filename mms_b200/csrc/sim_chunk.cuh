@@ -12,6 +12,16 @@
 
 namespace mms {
 
+// What build_tables_kernel finds in a call's tables (KernelArgs::irregular).
+// The layout the window kernels make of them would not do: a column is used with different
+// numbers of stages, a replica's slots are not its group's, a group has several columns, or a
+// replica list is not in ascending group order.
+constexpr uint32_t kIrregularLayout = 1;
+// A latency is negative or not a number.  An accepted request may then leave a clock BEFORE its
+// arrival time, and neither cutting in time (states_equivalent) nor comparing clocks by their bits
+// (window_groups) is sound: such a call is simulated in one piece, in the layout as given.
+constexpr uint32_t kIrregularLatency = 2;
+
 struct KernelArgs {
     // trace
     const double *arrivals;
@@ -77,7 +87,7 @@ struct KernelArgs {
     uint8_t *relabelled;          // [B]: some segment has one
     int32_t *seg_first_leaf;      // [NS + 1]: first leaf of each segment
     int32_t win_table_elems;      // entries of the window kernels' on-chip latency table; 0: off chip
-    const uint32_t *column_stages, *irregular, *group_column;    // see ClearArgs
+    const uint32_t *column_stages, *irregular, *group_column;    // see ClearArgs, kIrregularLayout
     bool window;                  // the speculative pass is window_stream_kernel's
     int32_t round;
     // outputs
@@ -120,10 +130,10 @@ __device__ inline size_t row_plane(const KernelArgs &a)
     return (size_t)((a.B + kLanes - 1) / kLanes) * (a.M + 1) * kLanes;
 }
 
-// True when the trace can be cut (sorted, finite arrival times).
+// True when the trace can be cut (sorted, finite arrival times; no negative latencies).
 __device__ inline bool can_chunk(const KernelArgs &a)
 {
-    return a.K > 1 && *a.unsorted == 0;
+    return a.K > 1 && *a.unsorted == 0 && !(*a.irregular & kIrregularLatency);
 }
 
 // Offset of request 0 of the trace candidate b simulates.
@@ -149,8 +159,8 @@ __device__ inline double arrival_at(const KernelArgs &a, int64_t b, int64_t i)
 //      so for the ones in the past the ORDER among them (ties included) must
 //      agree as well.  A clock in the past is below every clock that is not,
 //      in both vectors, so mixed comparisons agree by (1).
-// Each accepted request overwrites clocks with values >= tau that are equal
-// in both runs, so the relation is preserved step by step, and it is
+// Each accepted request overwrites clocks with values >= tau (latencies are not
+// negative, see kIrregularLatency) that are equal in both runs, so the relation is preserved step by step, and it is
 // transitive.  LoadX / LoadY map a clock slot to its value.
 template <typename LoadX, typename LoadY, typename Stale>
 __device__ inline bool states_equivalent(const KernelArgs &a, int64_t b, LoadX X, LoadY Y,

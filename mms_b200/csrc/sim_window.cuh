@@ -318,8 +318,8 @@ __device__ __noinline__ WindowTies window_ties(uint32_t need, uint32_t clk, uint
 // The requests `todo` of the window (lanes), one after the other, with a GROUP per lane: lane g
 // keeps the clocks of group g in registers and works out, for every request, when group g would
 // finish it; the group whose last-stage clock is smallest among the model's replicas is found
-// by the warp (clocks are not negative, so doubles are compared as integers, high word
-// first), and its lane takes the request.  A request costs the same whatever the number of
+// by the warp (clocks are not negative — neither the first arrival nor a latency is, see by_group
+// and kIrregularLatency — so doubles are compared as integers, high word first), and its lane takes the request.  A request costs the same whatever the number of
 // replicas and whoever else is waiting, and nothing of it passes through shared memory: the
 // orders — arrival time, SLO, the model's groups as a mask, its latency row — are laid out there
 // beforehand.  For candidates of up to 32 groups, or 64 in pipelines of one or two stages (two

@@ -155,3 +155,48 @@ def test_replica_lists_in_any_order_and_negative_times():
         assert fin.tobytes() == efin.tobytes() and np.array_equal(good, egood)
         for x, y in zip(got, exp):
             assert np.array_equal(x, y)
+
+
+@pytest.mark.parametrize("gap", [1e-6, 1e-4, 0.05])
+@pytest.mark.parametrize("which", ["mixed", "legacy", "batching"])
+def test_negative_latencies_of_dense_tables(which, gap):
+    """The drop-ins take any table.  With a negative latency a clock may lie before the arrival
+    that set it: clocks of both signs are compared (a dense trace stays near time zero), and what
+    a cut rests on does not hold."""
+    from mms_b200 import simulator
+    from oracle import cpu
+    rng = np.random.RandomState(7)
+    n, M, G, S = 9000, 4, 5, 2
+    ts = np.cumsum(rng.gamma(0.2, gap, size=n))
+    ids = rng.randint(-1, M, size=n).astype(np.int32)
+    slo = np.full(n, 0.3, np.float32)
+    m2g = np.array([[0, 1, 2, -1, -1], [1, 3, -1, -1, -1], [2, 4, -1, -1, -1], [0, 1, 3, 4, -1]], np.int32)
+    ns = np.array([2, 1, 2, 1, 2], np.int32)
+    fin = np.empty(n); good = np.empty(n, bool)
+    efin = np.empty(n); egood = np.empty(n, bool)
+    if which == "mixed":
+        lat = rng.uniform(-0.15, 0.12, size=(M, G, S)).astype(np.float32)
+        got = simulator.simulate_requests_mixed(fin, good, ts, ids, slo, m2g, ns, lat, n)
+        exp = cpu.simulate_requests_mixed(efin, egood, ts, ids, slo, m2g, ns, lat, n)
+    elif which == "legacy":
+        pair = rng.uniform(-0.15, 0.12, size=(2, M, G)).astype(np.float32)
+        got = simulator.simulate_requests(fin, good, ts, ids, slo, m2g, pair[0], pair[1], n)
+        exp = cpu.simulate_requests(efin, egood, ts, ids, slo, m2g, pair[0], pair[1], n)
+    else:
+        g2m = np.full((G, M + 1), -1, np.int32)
+        for g in range(G):
+            ms = [m for m in range(M) if g in m2g[m]]
+            g2m[g, :len(ms)] = ms
+        sizes = [1, 2, 4, 8]
+        old = list(simulator.batchsize_config)
+        simulator.batchsize_config[:] = sizes
+        try:
+            lat = rng.uniform(-0.05, 0.12, size=(M, G, S, 4)).astype(np.float32)
+            got = simulator.simulate_requests_mixed_batching(fin, good, ts, ids, slo, m2g, g2m, ns, lat, n)
+            exp = cpu.simulate_requests_mixed_batching(efin, egood, ts, ids, slo, m2g, g2m, ns, lat, n,
+                                                       sizes)
+        finally:
+            simulator.batchsize_config[:] = old
+    assert fin.tobytes() == efin.tobytes() and np.array_equal(good, egood)
+    for x, y in zip(got, exp):
+        assert np.array_equal(x, y)
