@@ -246,7 +246,10 @@ int mms_trace_pad_rows(const int64_t *lengths, int64_t num_traces, int64_t num_r
 int mms_trace_rows_histogram(const double *arrivals, const int32_t *model_ids, int64_t num_traces,
                              int64_t num_requests, int32_t num_models, int32_t *hist, void *stream);
 
-/* Bytes of scratch mms_sim_mixed needs for this shape and these options. */
+/* Bytes of scratch mms_sim_mixed needs for this shape and these options: about a byte per request
+ * and candidate, 8 bytes per clock slot, candidate and 1024 requests (128 where that is at most
+ * 256 MB) and, unless MMS_FLAG_NO_TWINS is set, a byte or less per request and candidate for
+ * interchangeable groups.  4096 candidates, 180 000 requests, 64 slots: 1.5 GB. */
 size_t mms_sim_workspace_bytes(int64_t num_requests, const mms_placements *cands,
                                const mms_sim_options *opts, uint32_t flags);
 
@@ -272,9 +275,11 @@ int mms_sim_mixed(const mms_trace *trace, const mms_placements *cands,
  * cudaMalloc, cudaFree or other allocating routine.
  *
  *  - Inputs and outputs are passed as for mms_sim_mixed; only `ws` is gone.
- *  - A shape whose scratch need (mms_sim_workspace_bytes) exceeds
- *    MMS_STATIC_SCRATCH_BYTES is rejected with MMS_ERR_UNSUPPORTED and a
- *    message in mms_last_error(); nothing is launched.
+ *  - A shape whose usual scratch need (mms_sim_workspace_bytes) exceeds
+ *    MMS_STATIC_SCRATCH_BYTES is cut more coarsely and, if that is not enough,
+ *    simulated without looking for interchangeable groups: slower, the results
+ *    are the same.  One that does not fit even so is rejected with
+ *    MMS_ERR_UNSUPPORTED and a message in mms_last_error(); nothing is launched.
  *  - The first call on a device looks up the array's device address (once
  *    per device, with that device current; host threads that make it together
  *    are serialised).  Make that first call outside any stream capture.

@@ -45,8 +45,8 @@ struct Geometry {
     size_t smem_stream, smem_window;
     size_t off_leaf, off_seg_end, off_chunk_start, off_decisions, off_work_count, off_work_items,
         off_rows, off_seg_leaf, off_group_info, off_columns, off_stamp, off_link, off_flags, off_rel,
-        off_tie, off_swaps, off_perm, off_twin_class, off_group_column, off_group_models;
-    int32_t group_words;
+        off_tie, off_swap_mask, off_swap_at, off_swap_count, off_perm, off_twin_class, off_group_column, off_group_models;
+    int32_t group_words, swap_cap;
     size_t smem_count;        // shared memory of count_kernel
     size_t total;
 };
@@ -69,10 +69,14 @@ static bool window_pays(int64_t N, int64_t B, int64_t K_wide, int64_t K_win, int
     return t_win < n_wide * (0.5 + 0.4 * share);
 }
 
-// Chunking, shared-memory and scratch geometry of one call.
+// Chunking, shared-memory and scratch geometry of one call.  `thrift` > 0 asks for less scratch at
+// the price of speed (never of results): 1 = long segments and chunks, 2 = also no bookkeeping of
+// interchangeable groups, 3 = also few chunks.
+constexpr int kMaxThrift = 3;
 static int plan_call(int64_t N, const mms_placements *c, const mms_sim_options *opts,
-                     uint32_t flags, bool group_good, Geometry *g)
+                     uint32_t flags, bool group_good, int thrift, Geometry *g)
 {
+    *g = Geometry();
     if (!c || N < 0 || c->num_candidates < 0 || c->num_models < 0 || c->max_groups < 0 ||
         c->max_placed < 0 || c->max_slots < 0 || c->max_stages < 1 || c->num_columns < 0)
         return MMS_ERR_ARG;
@@ -179,9 +183,11 @@ static int plan_call(int64_t N, const mms_placements *c, const mms_sim_options *
     };
     // segments of 128 requests where the snapshots are few (they are 8 bytes per clock slot,
     // candidate and segment), of 1024 in the large batches
-    const int64_t seg = (double)N * (double)c->max_slots * (double)B * 8.0 / 128.0 <= 256e6 ? 128 : 1024;
-    const Cut wide = cut_trace(seg, resident_slots * kLanes, seg == 1024 ? 3 * seg : warm / 2);
-    const Cut win = cut_trace(seg, (int64_t)g->window_blocks * kWindowWarps, seg);
+    const int64_t seg = !thrift && (double)N * (double)c->max_slots * (double)B * 8.0 / 128.0 <= 256e6 ? 128 : 1024;
+    const int64_t thrifty = thrift == 0 ? 0 : thrift < 3 ? 3 * seg : 12 * seg;     // shortest chunk
+    const Cut wide = cut_trace(seg, resident_slots * kLanes,
+                               thrifty ? thrifty : seg == 1024 ? 3 * seg : warm / 2);
+    const Cut win = cut_trace(seg, (int64_t)g->window_blocks * kWindowWarps, thrifty ? thrifty : seg);
     // Which speculative pass: see window_pays.
     g->window = window_pays(N, B, wide.K, win.K, warm, sm_count);
     const Cut &x = g->window ? win : wide;
@@ -229,20 +235,29 @@ static int plan_call(int64_t N, const mms_placements *c, const mms_sim_options *
     g->off_columns = off;     off += align256(sizeof(uint32_t) * ((size_t)c->num_columns + 1));
     g->off_flags = off;       off += align256(3 * (size_t)B + 4);      // relabelled, open, twins
     g->group_words = 0;
+    // Entries of a segment's list of swaps.  Of placements with twins 0.05 to 4 % of the requests
+    // are one, in bursts: of the segments of 128 requests of an hour on 64 devices at most 12
+    // entries, of bursts on 16 devices 1 % have more than 18 and 0.1 % more than 34; of those of
+    // 1024 requests 43, and 1 % have more than 65.  A full list costs walks, never results.
+    g->swap_cap = seg == 128 ? 24 : 64;
     if (K > 1) {
         const size_t G = (size_t)c->max_groups;
         g->off_stamp = off;        off += align256((size_t)K * B);
         g->off_link = off;         off += align256((size_t)K * B);
         g->off_rel = off;          off += align256((size_t)NS * B);
-        g->off_tie = off;          off += align256(sizeof(uint64_t) * (size_t)NS * B);
-        g->off_perm = off;         off += align256((size_t)NS * B * G + 4);
-        g->off_twin_class = off;   off += align256(sizeof(uint16_t) * (size_t)B * G + 4);
-        if (c->num_models <= kTwinModels && !(flags & MMS_FLAG_NO_TWINS))
+        if (c->num_models <= kTwinModels && !(flags & MMS_FLAG_NO_TWINS) && thrift < 2)
             g->group_words = (c->num_models + 63) / 64;
-        g->off_swaps = off;
-        if (g->group_words) off += align256(sizeof(uint32_t) * (size_t)((N + 3) / 4 * 4 + 4) * (size_t)((B + 31) / 32 * 32));
-        g->off_group_models = off;
-        off += align256(sizeof(uint64_t) * (size_t)B * G * (size_t)g->group_words + 8);
+        if (g->group_words) {
+            const size_t cells = (size_t)NS * B;
+            g->off_twin_class = off;  off += align256(sizeof(uint16_t) * (size_t)B * G + 4);
+            g->off_tie = off;         off += align256(sizeof(uint64_t) * cells);
+            g->off_perm = off;        off += align256(cells * G + 4);
+            g->off_swap_count = off;  off += align256(cells);
+            g->off_swap_mask = off;   off += align256(sizeof(uint32_t) * cells * g->swap_cap);
+            g->off_swap_at = off;     off += align256(sizeof(uint16_t) * cells * g->swap_cap);
+            g->off_group_models = off;
+            off += align256(sizeof(uint64_t) * (size_t)B * G * (size_t)g->group_words);
+        }
         g->off_seg_end = off;     off += align256(sizeof(double) * (size_t)NS * c->max_slots * B);
         g->off_chunk_start = off; off += align256(sizeof(double) * (size_t)K * c->max_slots * B);
     }
@@ -334,11 +349,11 @@ static int launch_sim(KernelArgs &ka, const ClearArgs &ca, const Geometry &g, cu
         return (unsigned)(blocks < g.window_blocks ? blocks : g.window_blocks);
     };
     if (g.window) {
-        auto stream_k = ka.swaps ? window_stream_kernel<kLegacy, true> : window_stream_kernel<kLegacy, false>;
+        auto stream_k = ka.swap_mask ? window_stream_kernel<kLegacy, true> : window_stream_kernel<kLegacy, false>;
         MMS_TRY(allow_smem((const void *)stream_k, g.smem_window));
         stream_k<<<window_blocks(streams), kWindowWarps * kLanes, g.smem_window, st>>>(ka);
     } else {
-        auto stream_k = ka.swaps ? sim_stream_kernel<kFull, kLegacy, true> : sim_stream_kernel<kFull, kLegacy, false>;
+        auto stream_k = ka.swap_mask ? sim_stream_kernel<kFull, kLegacy, true> : sim_stream_kernel<kFull, kLegacy, false>;
         MMS_TRY(allow_smem((const void *)stream_k, g.smem_stream));
         const int64_t per_block = (int64_t)kLanes * g.block_warps;
         stream_k<<<(unsigned)((streams + per_block - 1) / per_block), (unsigned)per_block,
@@ -347,8 +362,8 @@ static int launch_sim(KernelArgs &ka, const ClearArgs &ca, const Geometry &g, cu
     MMS_CUDA(cudaGetLastError());
     stream_span.stop();
     if (ka.K > 1) {
-        auto walk_k = ka.swaps ? walk_kernel<kLegacy, true> : walk_kernel<kLegacy, false>;
-        auto finish_k = ka.swaps ? finish_kernel<kLegacy, true> : finish_kernel<kLegacy, false>;
+        auto walk_k = ka.swap_mask ? walk_kernel<kLegacy, true> : walk_kernel<kLegacy, false>;
+        auto finish_k = ka.swap_mask ? finish_kernel<kLegacy, true> : finish_kernel<kLegacy, false>;
         MMS_TRY(allow_smem((const void *)walk_k, g.smem_window));
         MMS_TRY(allow_smem((const void *)finish_k, g.smem_window));
         const int64_t bounds = (int64_t)ka.B * (ka.K - 1);
@@ -379,7 +394,7 @@ static int launch_sim(KernelArgs &ka, const ClearArgs &ca, const Geometry &g, cu
 
 extern "C" {
 
-int mms_abi_version(void) { return 9; }
+int mms_abi_version(void) { return 10; }
 
 const char *mms_last_error(void) { return mms::g_last_error; }
 
@@ -468,17 +483,20 @@ size_t mms_sim_workspace_bytes(int64_t num_requests, const mms_placements *cands
                                const mms_sim_options *opts, uint32_t flags)
 {
     mms::Geometry g;
-    if (mms::plan_call(num_requests, cands, opts, flags, !(flags & MMS_FLAG_NO_GROUP_GOOD), &g) !=
+    if (mms::plan_call(num_requests, cands, opts, flags, !(flags & MMS_FLAG_NO_GROUP_GOOD), 0, &g) !=
         MMS_OK)
         return 0;
     return g.total;
 }
 
-int mms_sim_mixed(const mms_trace *trace, const mms_placements *cands, const mms_sum_plan *plan,
-                  const int32_t *model_hist, const mms_sim_options *opts, const mms_workspace *ws,
-                  const mms_results *out, uint32_t flags, void *stream)
+}  // extern "C"
+
+namespace mms {
+
+static int sim_mixed(const mms_trace *trace, const mms_placements *cands, const mms_sum_plan *plan,
+                     const int32_t *model_hist, const mms_sim_options *opts, const mms_workspace *ws,
+                     const mms_results *out, uint32_t flags, int thrift, void *stream)
 {
-    using namespace mms;
     if (!trace || !cands || !plan || !ws || !out) return MMS_ERR_ARG;
     if (flags & ~(MMS_FLAG_PER_REQUEST | MMS_FLAG_LEGACY_CLOCK | MMS_FLAG_NO_GROUP_GOOD |
                   MMS_FLAG_CROWDED | MMS_FLAG_NO_TWINS | MMS_FLAG_TRACE_ROWS))
@@ -487,7 +505,7 @@ int mms_sim_mixed(const mms_trace *trace, const mms_placements *cands, const mms
     const bool gg = !(flags & MMS_FLAG_NO_GROUP_GOOD);
     if (gg && !out->group_num_good) return MMS_ERR_ARG;
     Geometry g;
-    int rc = plan_call(N, cands, opts, flags, gg, &g);
+    int rc = plan_call(N, cands, opts, flags, gg, thrift, &g);
     if (rc) return rc;
     const int32_t B = cands->num_scored ? cands->num_scored : cands->num_candidates;
     if (B == 0) return MMS_OK;
@@ -541,7 +559,9 @@ int mms_sim_mixed(const mms_trace *trace, const mms_placements *cands, const mms
     ka.stamp = scratch + g.off_stamp; ka.link = scratch + g.off_link;
     ka.relabelled = scratch + g.off_flags; ka.open = ka.relabelled + B;
     ka.rel = scratch + g.off_rel; ka.tie = (uint64_t *)(scratch + g.off_tie); ka.perm = scratch + g.off_perm;
-    ka.swaps = g.group_words ? (uint32_t *)(scratch + g.off_swaps) : nullptr;
+    ka.swap_mask = g.group_words ? (uint32_t *)(scratch + g.off_swap_mask) : nullptr;
+    ka.swap_at = (uint16_t *)(scratch + g.off_swap_at); ka.swap_count = scratch + g.off_swap_count;
+    ka.swap_cap = g.swap_cap;
     ka.seg_first_leaf = (int32_t *)(scratch + g.off_seg_leaf);
     ka.window = g.window;
     ka.seg_end = (double *)(scratch + g.off_seg_end);
@@ -597,9 +617,16 @@ int mms_sim_mixed(const mms_trace *trace, const mms_placements *cands, const mms
     return MMS_OK;
 }
 
-}  // extern "C"
+}  // namespace mms
 
 extern "C" {
+
+int mms_sim_mixed(const mms_trace *trace, const mms_placements *cands, const mms_sum_plan *plan,
+                  const int32_t *model_hist, const mms_sim_options *opts, const mms_workspace *ws,
+                  const mms_results *out, uint32_t flags, void *stream)
+{
+    return mms::sim_mixed(trace, cands, plan, model_hist, opts, ws, out, flags, 0, stream);
+}
 
 int mms_trace_pack(const double *arrivals, const int32_t *model_ids, const float *slos,
                    const int64_t *offsets, int64_t num_traces, int64_t padded_requests,
@@ -688,11 +715,16 @@ int mms_sim_mixed_static(const mms_trace *trace, const mms_placements *cands,
 {
     if (!trace || !cands) return MMS_ERR_ARG;
     // the same shape checks as mms_sim_mixed, with the same return codes; only a
-    // shape that is fine but needs more scratch than the array holds is new
+    // shape that is fine but needs more scratch than the array holds, however thrifty the plan, is new
     mms::Geometry geo;
-    const int rc = mms::plan_call(trace->num_requests, cands, opts, flags,
-                                  !(flags & MMS_FLAG_NO_GROUP_GOOD), &geo);
-    if (rc != MMS_OK) return rc;
+    int thrift = 0;
+    for (;; ++thrift) {
+        const int rc = mms::plan_call(trace->num_requests, cands, opts, flags,
+                                      !(flags & MMS_FLAG_NO_GROUP_GOOD), thrift, &geo);
+        if (rc != MMS_OK) return rc;
+        if (thrift == mms::kMaxThrift || geo.total <= (size_t)MMS_STATIC_SCRATCH_BYTES)
+            break;
+    }
     if (geo.total > (size_t)MMS_STATIC_SCRATCH_BYTES) {
         snprintf(mms::g_last_error, sizeof(mms::g_last_error),
                  "mms_sim_mixed_static: needs %zu bytes of scratch, the built-in array holds %u; "
@@ -716,7 +748,7 @@ int mms_sim_mixed_static(const mms_trace *trace, const mms_placements *cands,
     mms_workspace ws;
     ws.ptr = mms::g_static_scratch_ptr[dev];
     ws.bytes = (size_t)MMS_STATIC_SCRATCH_BYTES;
-    return mms_sim_mixed(trace, cands, plan, model_hist, opts, &ws, out, flags, stream);
+    return mms::sim_mixed(trace, cands, plan, model_hist, opts, &ws, out, flags, thrift, stream);
 }
 
 int mms_trace_next_same_model(const mms_trace *trace, int32_t num_models, int32_t *next_same,

@@ -95,11 +95,6 @@ __global__ void clear_kernel(const KernelArgs a, const ClearArgs c)
         }
         for (int64_t i = tid; i < a.B; i += nth) { c.twins[i] = 0; a.open[i] = 0; a.relabelled[i] = 0; }
     }
-    if (a.swaps && !a.window) {          // the windows write every word of a candidate with twins
-        const int64_t quads = (a.N + 3) / 4 * a.dec_pitch;
-        for (int64_t i = tid; i < quads; i += nth)
-            reinterpret_cast<uint4 *>(a.swaps)[i] = make_uint4(0, 0, 0, 0);
-    }
     for (int64_t i = tid; i < (int64_t)a.B * a.G; i += nth) {
         c.group_column[i] = 0xFFFFFFFFu;
         const uint32_t info = c.group_info_in[i];
@@ -220,8 +215,10 @@ __device__ inline Lane setup_lane(const KernelArgs &a, int64_t b, int lane, int 
     ln.M = a.M; ln.C = a.C; ln.S = a.S;
     ln.status = 0;
     ln.tie = 0;
-    ln.swaps = a.swaps ? a.swaps + 4 * b : nullptr;
-    ln.twin_class = a.swaps && a.twins[b] ? a.twin_class + (size_t)b * a.G : nullptr;
+    ln.args = &a;
+    ln.b = (int32_t)b;
+    ln.q = ln.swaps = 0;
+    ln.twin_class = a.swap_mask && a.twins[b] ? a.twin_class + (size_t)b * a.G : nullptr;
     for (int t = 0; t < a.T + kClockPad; ++t) SM_F64(ln.clk + t * kLanes) = 0.0;
     return ln;
 }
@@ -560,30 +557,53 @@ __device__ inline void name_segment(const KernelArgs &a, int64_t b, Labels &l, i
     const int32_t i1 = seg_leaf(a, q + 1) < a.num_leaves ? a.leaf_start[seg_leaf(a, q + 1)] : (int32_t)a.N;
     const uint32_t flag = a.dec_wide ? 0x8000u : 0x80u;
     auto place = [&](int32_t i) { return (((size_t)(i >> 2) * a.dec_pitch) + b) * 4 + (size_t)(i & 3); };
-    auto fetch = [&](int32_t base, uint32_t &rec, uint32_t &swap) {
+    auto fetch = [&](int32_t base, uint32_t &rec) {
         const int32_t i = base + lane;
-        rec = swap = 0;
-        if (i < i1) {
+        rec = 0;
+        if (i < i1)
             rec = a.dec_wide ? static_cast<uint16_t *>(a.decisions)[place(i)]
                              : static_cast<uint8_t *>(a.decisions)[place(i)];
-            swap = a.swaps[place(i)];
+    };
+    // the segment's list of swaps, an entry per lane at a time
+    const int32_t swaps = a.swap_count[(size_t)q * a.B + b];
+    uint32_t swap_mask = 0;
+    int32_t swap_i = 0, swap_base = 0, next_swap = 0;      // swap_i: the request; next_swap: entry
+    auto load_swaps = [&](int32_t from) {
+        const size_t cell = ((size_t)q * a.swap_cap + from + lane) * a.B + b;
+        swap_base = from;
+        swap_i = 0x7FFFFFFF;
+        if (from + lane < swaps) {
+            swap_mask = a.swap_mask[cell];
+            swap_i = i0 + a.swap_at[cell];
         }
     };
-    auto window = [&](int32_t base, uint32_t rec, uint32_t swap) {
+    load_swaps(0);
+    // the request and the mask of the next swap (behind the last one: request 0x7FFFFFFF)
+    auto peek_swap = [&](int32_t &i, uint32_t &mask) {
+        if (next_swap - swap_base == kLanes) load_swaps(next_swap);
+        i = __shfl_sync(0xFFFFFFFFu, swap_i, next_swap - swap_base);
+        mask = __shfl_sync(0xFFFFFFFFu, swap_mask, next_swap - swap_base);
+    };
+    auto window = [&](int32_t base, uint32_t rec) {
         const uint32_t label = rec ? (rec & (flag - 1)) - 1 : 0u;
         const bool moves = rec && (class_bit(l.cls[label]) & l.moved);
-        if (!__any_sync(0xFFFFFFFFu, moves)) return;
+        const uint32_t movers = __ballot_sync(0xFFFFFFFFu, moves);
         uint32_t group = label;
         int from = 0;
         bool changed = false;
-        for (uint32_t todo = __ballot_sync(0xFFFFFFFFu, moves && swap);; todo &= todo - 1) {
-            const int k = todo ? __ffs((int)todo) - 1 : kLanes;
+        for (;;) {
+            int32_t i;
+            uint32_t mask;
+            peek_swap(i, mask);
+            const int k = i - base < kLanes ? i - base : kLanes;
+            if (k < kLanes) ++next_swap;
+            if (k < kLanes && !((movers >> k) & 1u)) continue;
             if (lane >= from && lane < k && moves) group = smem[l.pi + label];
-            if (!todo) break;
+            if (k == kLanes) break;
             from = k;
             // the true choice is the smallest group number among the replicas in the picked one's
             // state; the label that has it changes places with the picked one
-            const uint32_t mask = __shfl_sync(0xFFFFFFFFu, swap, k), mine = __shfl_sync(0xFFFFFFFFu, label, k);
+            const uint32_t mine = __shfl_sync(0xFFFFFFFFu, label, k);
             uint32_t key = 0xFFFFFFFFu;              // group << 8 | label
             for (int g = lane; g < a.G; g += kLanes)
                 if ((l.cls[g] & 0xFFu) == (l.cls[mine] & 0xFFu) && (l.cls[g] >> 8) < 32 &&
@@ -614,15 +634,15 @@ __device__ inline void name_segment(const KernelArgs &a, int64_t b, Labels &l, i
             l.moved = moved_classes(l.cls, a.G, [&](int g) { return smem[l.pi + g]; });
         }
     };
-    uint32_t rec[kAhead], swap[kAhead];
+    uint32_t rec[kAhead];
 #pragma unroll
-    for (int u = 0; u < kAhead; ++u) fetch(i0 + u * kLanes, rec[u], swap[u]);
+    for (int u = 0; u < kAhead; ++u) fetch(i0 + u * kLanes, rec[u]);
     for (int32_t base = i0; base < i1 && l.moved; base += kAhead * kLanes) {
 #pragma unroll
         for (int u = 0; u < kAhead; ++u) {
-            const uint32_t r = rec[u], s = swap[u];
-            fetch(base + (u + kAhead) * kLanes, rec[u], swap[u]);
-            if (l.moved) window(base + u * kLanes, r, s);
+            const uint32_t r = rec[u];
+            fetch(base + (u + kAhead) * kLanes, rec[u]);
+            if (l.moved) window(base + u * kLanes, r);
         }
     }
 }

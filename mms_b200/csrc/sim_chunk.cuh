@@ -81,9 +81,12 @@ struct KernelArgs {
     uint8_t *perm;                // [NS][B][G]: label in segment q -> label in segment q-1
     uint64_t *tie;                // [NS][B]: classes of twins (class_bit) for which a group number
                                   //   decided a choice in segment q between different states
-    uint32_t *swaps;              // laid out as byte decisions: twins between which a group number
-                                  //   decided, all in the same state (bit k: rank k of the class);
-                                  //   0: none.  Null: no candidate has twins
+    // choices that a group number decided between twins in the same state: per segment and
+    // candidate a list, in order, of at most swap_cap.  Null: no candidate has twins
+    uint32_t *swap_mask;          // [NS][swap_cap][B]: those twins (bit k: rank k of the class)
+    uint16_t *swap_at;            // [NS][swap_cap][B]: the request, counted from the segment's first
+    uint8_t *swap_count;          // [NS][B]
+    int32_t swap_cap;
     uint8_t *relabelled;          // [B]: some segment has one
     int32_t *seg_first_leaf;      // [NS + 1]: first leaf of each segment
     int32_t win_table_elems;      // entries of the window kernels' on-chip latency table; 0: off chip
@@ -250,9 +253,10 @@ __device__ inline bool warp_equivalent(int G, Info info, LoadX X, LoadZ Z, doubl
 // decides (bursts of requests with one arrival time do that all the time).  Mostly those are
 // twins in the same state, all clocks alike: then any of them can stand for any other, and p
 // is replaced, from that request on, by the permutation with two of them exchanged that
-// translates the run's choice into the true one.  The simulation notes these requests (`swaps`).
-// Where the replicas are not in the same state it notes their classes for the segment
-// (`tie`), and a segment is only taken over under labels that leave those classes alone.
+// translates the run's choice into the true one.  The simulation notes these requests in a list
+// per segment (`swap_mask`, `swap_at`; a word per request instead was five sixths of a call's
+// scratch, nearly all of it zero).  Where the replicas are not in the same state, or the list is
+// full, it notes their classes for the segment (`tie`), and a segment is only taken over under labels that leave those classes alone.
 // finish_kernel translates the decision records into group numbers; nothing else has labels.
 //
 // p has to keep the order of the last-stage clocks within a class (every group of a class serves
@@ -325,6 +329,44 @@ __device__ inline uint64_t moved_classes(const uint16_t *twin_class, int G, Perm
     return ((uint64_t)hi << 32) | lo;
 }
 
+template <int kStride>
+__device__ Tie note_tie(const KernelArgs *args, int32_t b, int32_t q, int32_t swaps, int32_t i,
+                        const uint16_t *twin_class, const uint32_t *list, int n, uint32_t clk,
+                        double best, uint32_t pick, double ts)
+{
+    const KernelArgs &a = *args;
+    Tie t;
+    t.classes = 0;
+    t.noted = 0;
+    const uint32_t pns = rep_stages(pick), p0 = clk + (rep_last(pick) + 1 - pns) * kStride;
+    const uint16_t own = twin_class[rep_group(pick)];
+    uint32_t swap = 0;
+    for (int r = 0; r < n; ++r) {
+        const uint32_t e = rep_to_last(__ldg(list + r));
+        if (!(SM_F64(clk + rep_last(e) * kStride) == best)) continue;
+        const uint16_t other = twin_class[rep_group(e)];
+        bool same = (other & 0xFFu) == (own & 0xFFu) && (other >> 8) < 32;
+        const uint32_t e0 = clk + (rep_last(e) + 1 - pns) * kStride;
+        for (uint32_t k = 0; k + 1 < pns && same; ++k) {
+            const double x = SM_F64(p0 + k * kStride), y = SM_F64(e0 + k * kStride);
+            same = x == y || (x < ts && y < ts);
+        }
+        if (same) swap |= 1u << (other >> 8);
+        else t.classes |= (1ull << (own & 63u)) | (1ull << (other & 63u));
+    }
+    if (swap & (swap - 1)) {                 // more than the picked one
+        if (swaps < a.swap_cap) {
+            const size_t cell = ((size_t)q * a.swap_cap + swaps) * a.B + b;
+            a.swap_mask[cell] = swap;
+            a.swap_at[cell] = (uint16_t)(i - a.leaf_start[seg_leaf(a, q)]);
+            t.noted = 1;
+        } else {
+            t.classes |= 1ull << (own & 63u);
+        }
+    }
+    return t;
+}
+
 // Runs chunk j of candidate b on this lane, speculatively: requests [begin, first)
 // as run-in (nothing recorded; `first` is the chunk's first request), then the
 // chunk's segments, recording decisions, per-request outputs (kFull) and one latency
@@ -345,6 +387,7 @@ __device__ inline void run_chunk(const KernelArgs &a, Lane &ln, Pipe &p, int64_t
     leaf -= 1;                      // the run-in counts as a leaf that is not recorded
     int32_t i = begin, span_end = first;
     bool record = false;
+    ln.q = q;
     pipe_prime(ln, p, begin);
     for (;;) {
         // Within a leaf the latency of request k goes to partial sum k mod 8
@@ -389,7 +432,10 @@ __device__ inline void run_chunk(const KernelArgs &a, Lane &ln, Pipe &p, int64_t
                 if (snapshots) {
                     if constexpr (kTwins) {
                         a.tie[(size_t)q * a.B + b] = ln.tie;
+                        a.swap_count[(size_t)q * a.B + b] = (uint8_t)ln.swaps;
                         ln.tie = 0;
+                        ln.swaps = 0;
+                        ln.q = q + 1;
                     }
                     for (int t = 0; t < a.T; ++t)
                         a.seg_end[((size_t)q * a.T + t) * a.B + b] = SM_F64(ln.clk + t * kLanes);

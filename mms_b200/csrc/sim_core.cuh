@@ -107,7 +107,8 @@ struct Lane {
     const uint16_t *twin_class;   // [G], or null: no group has an interchangeable one
     uint64_t tie;             // classes among whose groups the group number decided a choice
                               //   between different states (see warp_relabel)
-    uint32_t *swaps;          // element (request 0, this candidate) of KernelArgs::swaps
+    const struct KernelArgs *args;    // the candidate, the segment at hand and the entries of its
+    int32_t b, q, swaps;      //   list of swaps so far, for note_tie
 };
 
 // Row words that are not replicas.  Both address clock slot 0 / one stage /
@@ -185,38 +186,19 @@ __device__ __forceinline__ uint32_t rep_to_last(uint32_t e)
     return (e & 0xFFFF00FFu) | (((first + ns - 1) & 0xFFu) << 8);
 }
 
-// A choice that the group number decided: `pick` among the `n` replicas at `list` whose
-// last-stage clock is `best`.  The picked one's twins in its state (every clock equal, or past
-// in both: before `ts`) are given as a mask of their ranks in the class, if there are any besides
-// itself; the classes of all others, and its own with them, as `classes`.
-// Clock entries are kStride apart.
-struct Tie { uint64_t classes; uint32_t swap; };
+// A choice for request i that the group number decided: `pick` among the `n` replicas at `list`
+// whose last-stage clock is `best`.  The picked one's twins in its state (every clock equal, or
+// past in both: before `ts`) go to the segment's list of swaps (KernelArgs::swap_mask), which has
+// `swaps` entries, if there are any besides itself; the classes of all others, and its own with
+// them, are returned, and its own where the list is full.  Clock entries are kStride apart.  Not
+// inlined: the step is at the size of the instruction cache.
+struct Tie { uint64_t classes; int32_t noted; };
 
 template <int kStride>
-__device__ __noinline__ Tie look_at_tie(const uint16_t *twin_class, const uint32_t *list, int n,
-                                        uint32_t clk, double best, uint32_t pick, double ts)
-{
-    Tie t;
-    t.classes = 0;
-    t.swap = 0;
-    const uint32_t pns = rep_stages(pick), p0 = clk + (rep_last(pick) + 1 - pns) * kStride;
-    const uint16_t own = twin_class[rep_group(pick)];
-    for (int r = 0; r < n; ++r) {
-        const uint32_t e = rep_to_last(__ldg(list + r));
-        if (!(SM_F64(clk + rep_last(e) * kStride) == best)) continue;
-        const uint16_t other = twin_class[rep_group(e)];
-        bool same = (other & 0xFFu) == (own & 0xFFu) && (other >> 8) < 32;
-        const uint32_t e0 = clk + (rep_last(e) + 1 - pns) * kStride;
-        for (uint32_t k = 0; k + 1 < pns && same; ++k) {
-            const double x = SM_F64(p0 + k * kStride), y = SM_F64(e0 + k * kStride);
-            same = x == y || (x < ts && y < ts);
-        }
-        if (same) t.swap |= 1u << (other >> 8);
-        else t.classes |= (1ull << (own & 63u)) | (1ull << (other & 63u));
-    }
-    if ((t.swap & (t.swap - 1)) == 0) t.swap = 0;      // the picked one alone
-    return t;
-}
+__device__ __noinline__ Tie note_tie(const struct KernelArgs *args, int32_t b, int32_t q,
+                                     int32_t swaps, int32_t i, const uint16_t *twin_class,
+                                     const uint32_t *list, int n, uint32_t clk, double best,
+                                     uint32_t pick, double ts);
 
 // Executes request `i` (controller.py:579-622, or :519-555 with kLegacy) and
 // advances the pipe.  Returns finish - arrival, which is 0.0 for a dropped
@@ -291,10 +273,11 @@ __device__ __forceinline__ double sim_step(Lane &ln, Pipe &p, int32_t i, bool re
                 (e2 < kMoreReplicas && c2 == best && pick != e2) ||
                 (e3 < kMoreReplicas && c3 == best && pick != e3);
         if (tied && record && ln.twin_class) {
-            const Tie tie = look_at_tie<kLanes>(ln.twin_class, ln.rep_raw + ln.rep_off[m],
-                                                ln.rep_off[m + 1] - ln.rep_off[m], ln.clk, best, pick, ts);
+            const Tie tie = note_tie<kLanes>(ln.args, ln.b, ln.q, ln.swaps, i, ln.twin_class,
+                                             ln.rep_raw + ln.rep_off[m], ln.rep_off[m + 1] - ln.rep_off[m],
+                                             ln.clk, best, pick, ts);
             ln.tie |= tie.classes;
-            if (tie.swap) ln.swaps[(size_t)(i >> 2) * ln.dec_pitch * 4 + (size_t)(i & 3)] = tie.swap;
+            ln.swaps += tie.noted;
         }
     }
     const bool found = best < kInf;

@@ -659,7 +659,7 @@ constexpr int32_t kMaxPause = 1024;    // requests between two comparisons, at m
 
 //
 // kTwins: stored runs may be compared under other labels.  kLog: choices that the group number
-// decides are noted (tie, swaps) for those who compare later.
+// decides are noted (tie, swap_mask) for those who compare later.
 template <bool kLegacy, int kDepth, bool kTwins, bool kLog>
 __device__ inline int32_t window_run_depth(const KernelArgs &a, Window &w, WalkMode walk, int32_t j,
                                            int32_t begin, bool snapshots, int32_t q_begin)
@@ -693,6 +693,7 @@ __device__ inline int32_t window_run_depth(const KernelArgs &a, Window &w, WalkM
     bool serves = false;
     double fin = 0.0;
     uint32_t rec = 0, swap = 0;
+    int32_t swap_n = 0;                            // entries of segment q's list of swaps
     int32_t decoded = -1;
     // a stretch that is empty (no run-in, or an empty segment) falls straight through
     for (;;) {
@@ -770,8 +771,21 @@ __device__ inline int32_t window_run_depth(const KernelArgs &a, Window &w, WalkM
                     if (in && (lane & 3) == 0)
                         static_cast<uint32_t *>(a.decisions)[(size_t)(at >> 2) * a.dec_pitch + b] = word;
                 }
-                if (kLog && in)              // which choices the group number decided
-                    a.swaps[((size_t)(at >> 2) * a.dec_pitch + b) * 4 + (at & 3)] = swap;
+                if constexpr (kLog) {        // which choices the group number decided
+                    const bool some = in && swap && rec;
+                    const uint32_t who = __ballot_sync(0xFFFFFFFFu, some);
+                    if (who) {
+                        const int32_t k = swap_n + __popc(who & ((1u << lane) - 1u));
+                        if (some && k < a.swap_cap) {
+                            const size_t cell = ((size_t)q * a.swap_cap + k) * B + b;
+                            a.swap_mask[cell] = swap;
+                            a.swap_at[cell] = (uint16_t)(at - a.leaf_start[seg_leaf(a, q)]);
+                        } else if (some) {
+                            tie |= class_bit(SM_U16(w.cls + (rec & (a.dec_wide ? 0x7FFFu : 0x7Fu)) - 1u));
+                        }
+                        swap_n += __popc(who);
+                    }
+                }
                 if (a.finish && in) {
                     a.finish[(size_t)b * a.N + at] = fin;
                     a.good[(size_t)b * a.N + at] = rec & (a.dec_wide ? 0x8000u : 0x80u) ? 1 : 0;
@@ -824,7 +838,11 @@ __device__ inline int32_t window_run_depth(const KernelArgs &a, Window &w, WalkM
                 const uint32_t lo = __reduce_or_sync(0xFFFFFFFFu, (uint32_t)tie);
                 const uint32_t hi = __reduce_or_sync(0xFFFFFFFFu, (uint32_t)(tie >> 32));
                 tie = 0;
-                if (lane == 0) a.tie[(size_t)q * B + b] = ((uint64_t)hi << 32) | lo;
+                if (lane == 0) {
+                    a.tie[(size_t)q * B + b] = ((uint64_t)hi << 32) | lo;
+                    a.swap_count[(size_t)q * B + b] = (uint8_t)(swap_n < a.swap_cap ? swap_n : a.swap_cap);
+                }
+                swap_n = 0;
             }
             const bool inside = q + 1 < q1;
             int same = 0;

@@ -200,3 +200,31 @@ def test_negative_latencies_of_dense_tables(which, gap):
     assert fin.tobytes() == efin.tobytes() and np.array_equal(good, egood)
     for x, y in zip(got, exp):
         assert np.array_equal(x, y)
+
+
+@pytest.mark.parametrize("copies", [1, 40, 3000])
+@pytest.mark.parametrize("twins", [3, 30, 40])
+def test_more_swaps_than_a_segment_has_room_for(copies, twins):
+    """Bursts of 32 requests with one arrival time on idle twins: the group number decides nearly
+    every choice, and the list of a segment (of 128 requests; of 1024 with 3000 placements) is full
+    before its end.  Exact all the same, under any cut."""
+    from mms_b200 import engine
+    from oracle import tables
+    M, n = 3, 40000
+    profs = _profiles(M, (1, 2), 13)
+    rng = np.random.RandomState(14)
+    ts = np.repeat(np.arange(n // 32) * 0.3, 32) + np.where(np.arange(n) % 320 < 32, 0.1, 0.0)
+    ts.sort()
+    ids = (rng.rand(n) < 0.3).astype(np.int32)
+    slos = np.full(n, 0.4, np.float32)
+    p = _placement([1] * twins + [2, 2], [[0, 1]] * twins + [[1, 2], [0, 2]])
+    fin, good, mreq, mgood, greq, ggood = tables.one_placement(p, profs, ids, slos, ts)
+    trace, table = engine.DeviceTrace(ts, ids, slos, M), engine.LatencyTable(profs)
+    enc = engine.encode_placements([p], table, M).repeat(copies)
+    for chunk, run_in in ((0, 0), (1024, 16), (3072, 100)):
+        res, _, _ = engine.run_batch(trace, enc, table, group_good=True,
+                                     options=engine.sim_options(chunk, run_in))
+        assert np.all(res.latency_sum == float(np.add.reduce(fin - ts)))
+        assert np.all(res.model_num_good == mgood)
+        assert np.all(res.group_num_requests[:, :len(greq)] == greq)
+        assert np.all(res.group_num_good[:, :len(ggood)] == ggood)

@@ -393,3 +393,49 @@ def test_mirror_words_in_batches_equal_one_by_one():
     assert np.array_equal(rep[enc.B:], enc.model_rep[owners])
     firsts = partner[[b for (b, _), c in zip(enc.twins, counts.tolist()) if c]]
     assert np.array_equal(firsts, enc.B + (np.cumsum(counts) - counts)[counts > 0])
+
+
+@pytest.mark.parametrize("candidates,requests,groups,slots", [
+    (8, 180000, 32, 64), (100, 60000, 16, 16),
+    # the longest traces that fitted while scratch held no more than decisions and snapshots of
+    # 1024 requests
+    (1, 838000, 8, 16), (64, 137847, 128, 162), (33, 152575, 255, 256), (400, 23600, 128, 128)])
+def test_static_entry_point_takes_the_shapes_it_took(candidates, requests, groups, slots):
+    """mms_sim_mixed_static refuses a shape (MMS_ERR_UNSUPPORTED) before it looks for a device;
+    without one, a shape that is taken gets as far as MMS_ERR_CUDA."""
+    import ctypes
+
+    import torch
+
+    from mms_b200 import _native as nat
+    if torch.cuda.is_available():
+        pytest.skip("would launch on made-up addresses")
+    some = ctypes.c_void_p(256)
+    cands = nat.Placements(candidates, 8, groups, 1000, slots, 2, 4, 0, some, some, some, some, 0,
+                           None, None)
+    trace = nat.Trace(requests, some, some, some)
+    plan, opts = nat.SumPlan(0, 0, some, some), nat.SimOptions(0, 0, 0, 0)
+    out = nat.Results(*([some] * 10))
+    rc = nat.lib().mms_sim_mixed_static(ctypes.byref(trace), ctypes.byref(cands),
+                                        ctypes.byref(plan), some, ctypes.byref(opts),
+                                        ctypes.byref(out), 0, None)
+    assert rc == -3, nat.lib().mms_last_error()
+
+
+def test_scratch_per_request():
+    """What a call needs beyond the decision records (a byte per request and candidate) stays
+    small: snapshots and, with interchangeable groups, lists of swaps."""
+    import ctypes
+
+    from mms_b200 import _native as nat
+    for candidates, requests, slots in ((4096, 180000, 64), (2343, 144000, 64), (100, 60000, 16)):
+        cands = nat.Placements(candidates, 32, 32, 200, slots, 8, 5, 0, None, None, None, None, 0,
+                               None, None)
+        opts = nat.SimOptions(0, 0, 0, 0)
+        need = nat.lib().mms_sim_workspace_bytes(requests, ctypes.byref(cands), ctypes.byref(opts), 0)
+        # per segment of 1024 requests (of 128 while that is at most 256 MB): a snapshot, at most
+        # another one if chunks are that short, a permutation and a list of 64 or 24 swaps; a tenth
+        # for leaf sums, tables and marks
+        seg, swaps = (128, 24) if requests * slots * candidates / 16 <= 256e6 else (1024, 64)
+        per = (16 * slots + slots + 6 * swaps) / seg * candidates + -(-candidates // 32) * 32
+        assert need < 1.1 * per * requests

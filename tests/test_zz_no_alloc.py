@@ -94,3 +94,27 @@ def test_static_scratch_entry_point_matches_workspace_entry_point():
     assert rc == -2                                                     # MMS_ERR_UNSUPPORTED
     msg = nat.lib().mms_last_error().decode()
     assert "scratch" in msg and str(nat.STATIC_SCRATCH_BYTES) in msg
+
+
+@pytest.mark.parametrize("count,requests", [(8, 180000), (100, 60000), (100, 110000), (128, 125000),
+                                            (128, 145000)])
+def test_shapes_that_fit_only_with_a_thriftier_plan(count, requests):
+    """The built-in array takes a shape whose usual plan does not fit it, cut more coarsely or
+    without the bookkeeping of interchangeable groups; the results are those of mms_sim_mixed."""
+    from mms_b200 import _native as nat
+    from mms_b200 import cases, engine
+    from mms_b200.simulator import workload_arrays
+    case = cases.candidate_batch_case(num_candidates=16, duration=600.0, placement_seed=22)
+    names = [d.name for d in case.model_datas]
+    mids, slos = workload_arrays(case.workload, names)
+    times = -(-requests // len(mids))
+    arrivals = np.concatenate([case.workload.arrivals + 620.0 * k for k in range(times)])[:requests]
+    trace = engine.DeviceTrace(arrivals, np.tile(mids, times)[:requests],
+                               np.tile(slos, times)[:requests], len(names))
+    table = engine.LatencyTable([d.profiling_result for d in case.model_datas])
+    enc = engine.encode_placements((case.placements * 8)[:count], table, len(names))
+    rc_s, got = _call("static", trace, enc, table, engine.sim_options(), False)
+    rc_w, want = _call("workspace", trace, enc, table, engine.sim_options(), False)
+    assert rc_s == 0 and rc_w == 0
+    for key in ("mreq", "mgood", "greq", "ggood", "total", "lsum"):
+        assert got[key].tobytes() == want[key].tobytes(), key
