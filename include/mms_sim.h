@@ -248,8 +248,8 @@ int mms_trace_rows_histogram(const double *arrivals, const int32_t *model_ids, i
 
 /* Bytes of scratch mms_sim_mixed needs for this shape and these options: about a byte per request
  * and candidate, 8 bytes per clock slot, candidate and 1024 requests (128 where that is at most
- * 256 MB) and, unless MMS_FLAG_NO_TWINS is set, a byte or less per request and candidate for
- * interchangeable groups.  4096 candidates, 180 000 requests, 64 slots: 1.5 GB. */
+ * 256 MB) and, unless MMS_FLAG_NO_TWINS is set, one to three bytes per request and candidate for
+ * interchangeable groups.  4096 candidates, 180 000 requests, 64 slots: 1.9 GB (1.2 without). */
 size_t mms_sim_workspace_bytes(int64_t num_requests, const mms_placements *cands,
                                const mms_sim_options *opts, uint32_t flags);
 

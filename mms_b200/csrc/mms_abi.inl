@@ -236,10 +236,12 @@ static int plan_call(int64_t N, const mms_placements *c, const mms_sim_options *
     g->off_flags = off;       off += align256(3 * (size_t)B + 4);      // relabelled, open, twins
     g->group_words = 0;
     // Entries of a segment's list of swaps.  Of placements with twins 0.05 to 4 % of the requests
-    // are one, in bursts: of the segments of 128 requests of an hour on 64 devices at most 12
-    // entries, of bursts on 16 devices 1 % have more than 18 and 0.1 % more than 34; of those of
-    // 1024 requests 43, and 1 % have more than 65.  A full list costs walks, never results.
-    g->swap_cap = seg == 128 ? 24 : 64;
+    // are one, in bursts: of the segments of 128 requests of an hour on 64 devices at most 12, of
+    // bursts on 16 devices 0.1 % have more than 34; of those of 1024 requests 43, and 0.1 % have
+    // more than 123.  Arrival times on a grid make it 20 to 45 % (of 117 chunks of such a trace 77
+    // are simulated again with room for 24 of 128, 10 with 48, 8 with 64, 1 with 96).  A full list
+    // costs walks, never results.
+    g->swap_cap = seg == 128 ? 64 : 160;
     if (K > 1) {
         const size_t G = (size_t)c->max_groups;
         g->off_stamp = off;        off += align256((size_t)K * B);

@@ -434,8 +434,8 @@ def test_scratch_per_request():
         opts = nat.SimOptions(0, 0, 0, 0)
         need = nat.lib().mms_sim_workspace_bytes(requests, ctypes.byref(cands), ctypes.byref(opts), 0)
         # per segment of 1024 requests (of 128 while that is at most 256 MB): a snapshot, at most
-        # another one if chunks are that short, a permutation and a list of 64 or 24 swaps; a tenth
+        # another one if chunks are that short, a permutation and a list of 160 or 64 swaps; a tenth
         # for leaf sums, tables and marks
-        seg, swaps = (128, 24) if requests * slots * candidates / 16 <= 256e6 else (1024, 64)
+        seg, swaps = (128, 64) if requests * slots * candidates / 16 <= 256e6 else (1024, 160)
         per = (16 * slots + slots + 6 * swaps) / seg * candidates + -(-candidates // 32) * 32
         assert need < 1.1 * per * requests
