@@ -251,7 +251,7 @@ static int plan_call(int64_t N, const mms_placements *c, const mms_sim_options *
             g->group_words = (c->num_models + 63) / 64;
         if (g->group_words) {
             const size_t cells = (size_t)NS * B;
-            g->off_twin_class = off;  off += align256(sizeof(uint16_t) * (size_t)B * G + 4);
+            g->off_twin_class = off;  off += align256(sizeof(uint32_t) * (size_t)B * G + 4);
             g->off_tie = off;         off += align256(sizeof(uint64_t) * cells);
             g->off_perm = off;        off += align256(cells * G + 4);
             g->off_swap_count = off;  off += align256(cells);
@@ -584,7 +584,7 @@ static int sim_mixed(const mms_trace *trace, const mms_placements *cands, const 
     ca.group_words = g.group_words;
     ca.group_models = (uint64_t *)(scratch + g.off_group_models);
     ca.group_column = (uint32_t *)(scratch + g.off_group_column);
-    ca.twin_class = (uint16_t *)(scratch + g.off_twin_class); ca.twins = ka.open + B;
+    ca.twin_class = (uint32_t *)(scratch + g.off_twin_class); ca.twins = ka.open + B;
     ka.group_column = ca.group_column;
     ka.twin_class = ca.twin_class; ka.twins = ca.twins;
     ka.column_stages = ca.column_stages; ka.irregular = ca.irregular;

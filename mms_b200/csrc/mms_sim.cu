@@ -71,7 +71,7 @@ struct ClearArgs {
     int32_t group_words;              // 64-bit words of a group's model set; 0: too many models
     uint64_t *group_models;           // [B][G][group_words]
     uint32_t *group_column;           // [B][G] latency column of the group; 0xFFFFFFFF: no model
-    uint16_t *twin_class;             // see KernelArgs
+    uint32_t *twin_class;             // see KernelArgs
     uint8_t *twins;
     uint32_t *column_stages;          // [C] stages of the groups that use the column
     uint32_t *irregular;              // kIrregularLayout | kIrregularLatency
@@ -296,18 +296,21 @@ __global__ void twins_kernel(const KernelArgs a, const ClearArgs c)
     uint64_t some = 0;
     for (int k = 0; k < W; ++k) some |= mine[k];
     const uint32_t ns = (a.group_info[t] >> 8) & 0xFFu, column = c.group_column[t];
-    int cls = g, rank = 0;
+    int cls = g, rank = 0, last = g;
     if (some && ns && column < (uint32_t)a.C) {
-        for (int h = 0; h < g; ++h) {
+        for (int h = 0; h < a.G; ++h) {
+            if (h == g) continue;
             const size_t u = (size_t)b * a.G + h;
             if (((a.group_info[u] >> 8) & 0xFFu) != ns || c.group_column[u] != column) continue;
             const uint64_t *other = c.group_models + u * W;
             bool same = true;
             for (int k = 0; k < W && same; ++k) same = mine[k] == other[k];
-            if (same) { if (cls == g) cls = h; ++rank; }
+            if (!same) continue;
+            if (h > g) last = h;
+            else { if (cls == g) cls = h; ++rank; }
         }
     }
-    c.twin_class[t] = (uint16_t)(cls | (rank << 8));
+    c.twin_class[t] = (uint32_t)(cls | (rank << 8) | (last << 16));
     if (cls != g) c.twins[b] = 1;
 }
 
@@ -498,7 +501,7 @@ walk_kernel(const __grid_constant__ KernelArgs a)
 // shared memory) translates the labels of the segment at hand into group numbers.
 struct Labels {
     uint32_t pi, tmp;                        // u8 indices; tmp: scratch of the same size
-    const uint16_t *cls;                     // the candidate's classes of twins
+    const uint32_t *cls;                     // the candidate's classes of twins
     uint64_t moved;                          // classes in which pi is not the identity
 };
 
@@ -606,8 +609,8 @@ __device__ inline void name_segment(const KernelArgs &a, int64_t b, Labels &l, i
             const uint32_t mine = __shfl_sync(0xFFFFFFFFu, label, k);
             uint32_t key = 0xFFFFFFFFu;              // group << 8 | label
             for (int g = lane; g < a.G; g += kLanes)
-                if ((l.cls[g] & 0xFFu) == (l.cls[mine] & 0xFFu) && (l.cls[g] >> 8) < 32 &&
-                    ((mask >> (l.cls[g] >> 8)) & 1u)) {
+                if (class_first(l.cls[g]) == class_first(l.cls[mine]) && class_rank(l.cls[g]) < 32 &&
+                    ((mask >> class_rank(l.cls[g])) & 1u)) {
                     const uint32_t mapped = ((uint32_t)smem[l.pi + g] << 8) | (uint32_t)g;
                     key = mapped < key ? mapped : key;
                 }

@@ -74,8 +74,8 @@ struct KernelArgs {
     uint8_t *link;                // [K][B]: the run of chunk j continues the run of chunk j-1
     uint8_t *open;                // [B]: some boundary of the candidate does not
     // relabelling, see warp_relabel
-    const uint16_t *twin_class;   // [B][G]: smallest group interchangeable with the group | the
-                                  //   group's rank among those << 8
+    const uint32_t *twin_class;   // [B][G]: smallest group interchangeable with the group | the
+                                  //   group's rank among those << 8 | the largest one << 16
     const uint8_t *twins;         // [B]: some group has an interchangeable one
     uint8_t *rel;                 // [NS][B]: segment q is written in other labels than segment q-1
     uint8_t *perm;                // [NS][B][G]: label in segment q -> label in segment q-1
@@ -255,8 +255,9 @@ __device__ inline bool warp_equivalent(int G, Info info, LoadX X, LoadZ Z, doubl
 // is replaced, from that request on, by the permutation with two of them exchanged that
 // translates the run's choice into the true one.  The simulation notes these requests in a list
 // per segment (`swap_mask`, `swap_at`; a word per request instead was five sixths of a call's
-// scratch, nearly all of it zero).  Where the replicas are not in the same state, or the list is
-// full, it notes their classes for the segment (`tie`), and a segment is only taken over under labels that leave those classes alone.
+// scratch, nearly all of it zero).  Where the replicas are not in the same state and that matters
+// (tie_matters), or the list is full, it notes their classes for the segment (`tie`), and a segment
+// is only taken over under labels that leave those classes alone.
 // finish_kernel translates the decision records into group numbers; nothing else has labels.
 //
 // p has to keep the order of the last-stage clocks within a class (every group of a class serves
@@ -268,7 +269,7 @@ __device__ inline bool warp_equivalent(int G, Info info, LoadX X, LoadZ Z, doubl
 struct RelabelScratch { uint32_t z, last, perm, rank; };       // f64, f64, u8, u8 indices
 
 template <typename Info, typename LoadX>
-__device__ inline bool warp_relabel(int G, int T, const uint16_t *cls, Info info, LoadX X,
+__device__ inline bool warp_relabel(int G, int T, const uint32_t *cls, Info info, LoadX X,
                                     const double *Y, size_t pitch, const RelabelScratch &s)
 {
     const int lane = threadIdx.x & (kLanes - 1);
@@ -282,11 +283,11 @@ __device__ inline bool warp_relabel(int G, int T, const uint16_t *cls, Info info
     for (int g = lane; g < G; g += kLanes) {
         const uint32_t in = info(g);
         const uint32_t ns = (in >> 8) & 0xFFu;
-        const uint32_t c = cls[g] & 0xFFu;
+        const uint32_t c = class_first(cls[g]);
         const double x = ns ? X((in & 0xFFu) + ns - 1) : 0.0, y = SM_F64(s.last + g);
         uint32_t rx = 0, ry = 0;
         for (int h = (int)c; h < G; ++h) {                // members of the class: c is its smallest
-            if ((cls[h] & 0xFFu) != c || h == g) continue;
+            if (class_first(cls[h]) != c || h == g) continue;
             const uint32_t ih = info(h);
             const double xh = X((ih & 0xFFu) + ((ih >> 8) & 0xFFu) - 1), yh = SM_F64(s.last + h);
             rx += xh < x || (xh == x && h < g);
@@ -298,10 +299,10 @@ __device__ inline bool warp_relabel(int G, int T, const uint16_t *cls, Info info
     __syncwarp();
     bool moved = false;
     for (int g = lane; g < G; g += kLanes) {
-        const uint32_t c = cls[g] & 0xFFu, r = smem[s.rank + G + g];
+        const uint32_t c = class_first(cls[g]), r = smem[s.rank + G + g];
         int to = g;
         for (int h = (int)c; h < G; ++h)
-            if ((cls[h] & 0xFFu) == c && smem[s.rank + h] == r) { to = h; break; }
+            if (class_first(cls[h]) == c && smem[s.rank + h] == r) { to = h; break; }
         smem[s.perm + g] = (uint8_t)to;
         moved |= to != g;
         const uint32_t ig = info(g), it = info(to);
@@ -313,13 +314,25 @@ __device__ inline bool warp_relabel(int G, int T, const uint16_t *cls, Info info
     return __any_sync(0xFFFFFFFFu, moved);
 }
 
+// Does it matter, under labels that move the class `picked` or the class `other`, that a group number
+// decided between a picked group of the former and one of the latter?  Not if all of the
+// former's numbers are smaller than all of the latter's: then the true choice is among the picked one's
+// twins as well, whatever the labels.  (Placements that a search has normalized have their twins
+// side by side, where this is always so; of random ones on 64 devices 0.001 % of the requests are
+// such a choice, 0.03 % on 16.  Without the test 0.01 to 1.6 % were, and the last pass walked most
+// candidates with twins from end to end because of them.)
+__device__ __forceinline__ bool tie_matters(uint32_t picked, uint32_t other)
+{
+    return class_first(picked) == class_first(other) || class_last(picked) > class_first(other);
+}
+
 // Bit of a class of twins in a tie mask (more than 64 classes share bits, which only costs
 // re-simulations).
-__device__ __forceinline__ uint64_t class_bit(uint16_t twin_class) { return 1ull << (twin_class & 63u); }
+__device__ __forceinline__ uint64_t class_bit(uint32_t twin_class) { return 1ull << (twin_class & 63u); }
 
 // Classes that a permutation moves, by a warp: perm(g) is the image of group g.
 template <typename Perm>
-__device__ inline uint64_t moved_classes(const uint16_t *twin_class, int G, Perm perm)
+__device__ inline uint64_t moved_classes(const uint32_t *twin_class, int G, Perm perm)
 {
     uint64_t moved = 0;
     for (int g = threadIdx.x & (kLanes - 1); g < G; g += kLanes)
@@ -331,7 +344,7 @@ __device__ inline uint64_t moved_classes(const uint16_t *twin_class, int G, Perm
 
 template <int kStride>
 __device__ Tie note_tie(const KernelArgs *args, int32_t b, int32_t q, int32_t swaps, int32_t i,
-                        const uint16_t *twin_class, const uint32_t *list, int n, uint32_t clk,
+                        const uint32_t *twin_class, const uint32_t *list, int n, uint32_t clk,
                         double best, uint32_t pick, double ts)
 {
     const KernelArgs &a = *args;
@@ -339,20 +352,20 @@ __device__ Tie note_tie(const KernelArgs *args, int32_t b, int32_t q, int32_t sw
     t.classes = 0;
     t.noted = 0;
     const uint32_t pns = rep_stages(pick), p0 = clk + (rep_last(pick) + 1 - pns) * kStride;
-    const uint16_t own = twin_class[rep_group(pick)];
+    const uint32_t own = twin_class[rep_group(pick)];
     uint32_t swap = 0;
     for (int r = 0; r < n; ++r) {
         const uint32_t e = rep_to_last(__ldg(list + r));
         if (!(SM_F64(clk + rep_last(e) * kStride) == best)) continue;
-        const uint16_t other = twin_class[rep_group(e)];
-        bool same = (other & 0xFFu) == (own & 0xFFu) && (other >> 8) < 32;
+        const uint32_t other = twin_class[rep_group(e)];
+        bool same = class_first(other) == class_first(own) && class_rank(other) < 32;
         const uint32_t e0 = clk + (rep_last(e) + 1 - pns) * kStride;
         for (uint32_t k = 0; k + 1 < pns && same; ++k) {
             const double x = SM_F64(p0 + k * kStride), y = SM_F64(e0 + k * kStride);
             same = x == y || (x < ts && y < ts);
         }
-        if (same) swap |= 1u << (other >> 8);
-        else t.classes |= (1ull << (own & 63u)) | (1ull << (other & 63u));
+        if (same) swap |= 1u << class_rank(other);
+        else if (tie_matters(own, other)) t.classes |= class_bit(own) | class_bit(other);
     }
     if (swap & (swap - 1)) {                 // more than the picked one
         if (swaps < a.swap_cap) {
@@ -361,7 +374,7 @@ __device__ Tie note_tie(const KernelArgs *args, int32_t b, int32_t q, int32_t sw
             a.swap_at[cell] = (uint16_t)(i - a.leaf_start[seg_leaf(a, q)]);
             t.noted = 1;
         } else {
-            t.classes |= 1ull << (own & 63u);
+            t.classes |= class_bit(own);
         }
     }
     return t;

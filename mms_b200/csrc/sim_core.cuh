@@ -104,7 +104,7 @@ struct Lane {
     bool lat_f64;             // on chip as doubles
     int32_t M, C, S;
     uint32_t status;
-    const uint16_t *twin_class;   // [G], or null: no group has an interchangeable one
+    const uint32_t *twin_class;   // [G], or null: no group has an interchangeable one
     uint64_t tie;             // classes among whose groups the group number decided a choice
                               //   between different states (see warp_relabel)
     const struct KernelArgs *args;    // the candidate, the segment at hand and the entries of its
@@ -115,6 +115,11 @@ struct Lane {
 // latency column 0, so that the branch-free step can load through them.
 constexpr uint32_t kNoReplica = 0xFF010000u;
 constexpr uint32_t kMoreReplicas = 0xFE010000u;
+
+// Entries of KernelArgs::twin_class.
+__device__ __forceinline__ uint32_t class_first(uint32_t c) { return c & 0xFFu; }
+__device__ __forceinline__ uint32_t class_rank(uint32_t c) { return (c >> 8) & 0xFFu; }
+__device__ __forceinline__ uint32_t class_last(uint32_t c) { return (c >> 16) & 0xFFu; }
 
 // Requests in flight.  Request i is ready to execute: its replica row is in
 // registers, and so is the row of request i+1.  While i executes, the row of
@@ -189,14 +194,14 @@ __device__ __forceinline__ uint32_t rep_to_last(uint32_t e)
 // A choice for request i that the group number decided: `pick` among the `n` replicas at `list`
 // whose last-stage clock is `best`.  The picked one's twins in its state (every clock equal, or
 // past in both: before `ts`) go to the segment's list of swaps (KernelArgs::swap_mask), which has
-// `swaps` entries, if there are any besides itself; the classes of all others, and its own with
-// them, are returned, and its own where the list is full.  Clock entries are kStride apart.  Not
+// `swaps` entries, if there are any besides itself; the classes of all others that matter
+// (tie_matters), and its own with them, are returned, and its own where the list is full.  Clock entries are kStride apart.  Not
 // inlined: the step is at the size of the instruction cache.
 struct Tie { uint64_t classes; int32_t noted; };
 
 template <int kStride>
 __device__ __noinline__ Tie note_tie(const struct KernelArgs *args, int32_t b, int32_t q,
-                                     int32_t swaps, int32_t i, const uint16_t *twin_class,
+                                     int32_t swaps, int32_t i, const uint32_t *twin_class,
                                      const uint32_t *list, int n, uint32_t clk, double best,
                                      uint32_t pick, double ts);
 

@@ -74,8 +74,8 @@ __host__ __device__ inline WindowLayout window_layout(int T, int G, int S, int P
     L.orders = off;    off += kOrderBytes * kLanes;
     L.info = off;      off += sizeof(uint32_t) * (size_t)G;
     L.slot_at = off;   off += sizeof(uint16_t) * (size_t)T;
-    L.cls = off;       off += sizeof(uint16_t) * (size_t)G;
     off = (off + 3) & ~(size_t)3;
+    L.cls = off;       off += sizeof(uint32_t) * (size_t)G;
     L.list = off;      off += P <= kWindowList ? sizeof(uint32_t) * (size_t)P : 0;
     L.perm = off;      off += (size_t)G;
     L.labels = off;    off += (size_t)G;
@@ -97,7 +97,7 @@ struct Window {
     const uint4 *rows;
     const uint16_t *off;                     // the candidate's model_off
     uint32_t list;                           // u32 index of its replica list, if it is on chip
-    uint32_t cls;                            // u16 index of its classes of twins
+    uint32_t cls;                            // u32 index of its classes of twins
     uint32_t orders;                         // byte offset, see window_groups
     bool by_group;                           // window_groups can be used
     uint32_t column;                         // per lane: latency columns of groups lane and lane + 32
@@ -157,7 +157,7 @@ __device__ inline void window_setup(const KernelArgs &a, Window &w, int64_t b)
     w.rows = reinterpret_cast<const uint4 *>(a.rep_rows) + row_index(a, b, 0);
     w.off = a.model_off + (size_t)b * (a.M + 1);
     w.list = (uint32_t)((base + L.list) / sizeof(uint32_t));
-    w.cls = (uint32_t)((base + L.cls) / sizeof(uint16_t));
+    w.cls = (uint32_t)((base + L.cls) / sizeof(uint32_t));
     w.orders = (uint32_t)(base + L.orders);
     const size_t tb = trace_base(a, b);
     w.arrivals = a.arrivals + tb; w.model_ids = a.model_ids + tb; w.slos = a.slos + tb;
@@ -169,7 +169,7 @@ __device__ inline void window_setup(const KernelArgs &a, Window &w, int64_t b)
     for (int g = lane; g < a.G; g += kLanes) {
         const uint32_t info = a.group_info[(size_t)b * a.G + g];
         SM_U32(w.info + g) = info;
-        if (kTwins) SM_U16(w.cls + g) = a.twin_class[(size_t)b * a.G + g];
+        if (kTwins) SM_U32(w.cls + g) = a.twin_class[(size_t)b * a.G + g];
         const uint32_t ns = (info >> 8) & 0xFFu;
         depth = ns > depth ? ns : depth;
     }
@@ -264,7 +264,7 @@ __device__ __forceinline__ uint32_t window_replica(const KernelArgs &a, const Wi
 // The choices of `need` (lanes of the window) that the group number decided, between replicas
 // whose last-stage clock is the lane's `best`: see warp_relabel.  `swap`: the twins of
 // the picked one in its state, as a mask of their ranks in the class; `classes`: those of the
-// others.  Lanes of one model saw the same clocks: the warp looks at each model once, replica r in
+// others that matter (tie_matters), and its own with them.  Lanes of one model saw the same clocks: the warp looks at each model once, replica r in
 // lane r.
 struct WindowTies { uint64_t classes; uint32_t swap; };
 
@@ -288,20 +288,20 @@ __device__ __noinline__ WindowTies window_ties(uint32_t need, uint32_t clk, uint
         auto last_at = [&](uint32_t e) {
             return clk + (kDepth > 0 ? rep_group(e) * (uint32_t)kDepth + (kDepth - 1) : rep_last(e));
         };
-        const uint16_t own = SM_U16(cls + rep_group(pk));
+        const uint32_t own = SM_U32(cls + rep_group(pk));
         uint32_t swap = 0;
         uint64_t classes = 0;
         for (uint32_t r = lane; r < nk; r += kLanes) {
             const uint32_t e = list_gl ? rep_to_last(__ldg(list_gl + lok + r)) : SM_U32(list + lok + r);
             if (!(SM_F64(last_at(e)) == bk)) continue;
-            const uint16_t other = SM_U16(cls + rep_group(e));
-            bool same = (other & 0xFFu) == (own & 0xFFu) && (other >> 8) < 32;
+            const uint32_t other = SM_U32(cls + rep_group(e));
+            bool same = class_first(other) == class_first(own) && class_rank(other) < 32;
             for (uint32_t s = 1; s < rep_stages(pk) && same; ++s) {
                 const double x = SM_F64(last_at(pk) - s), y = SM_F64(last_at(e) - s);
                 same = x == y || (x < tk && y < tk);
             }
-            if (same) swap |= 1u << (other >> 8);
-            else classes |= class_bit(own) | class_bit(other);
+            if (same) swap |= 1u << class_rank(other);
+            else if (tie_matters(own, other)) classes |= class_bit(own) | class_bit(other);
         }
         swap = __reduce_or_sync(0xFFFFFFFFu, swap);
         const uint32_t c0 = __reduce_or_sync(0xFFFFFFFFu, (uint32_t)classes);
@@ -420,21 +420,21 @@ __device__ __forceinline__ void window_groups(const KernelArgs &a, const Window 
                     win[h] &= __ballot_sync(0xFFFFFFFFu, low[h] == low_least);
                 if (kTwins && several()) {      // the group number decides, see warp_relabel
                     const int ph = win[0] ? 0 : kPer - 1, p = __ffs((int)win[ph]) - 1;
-                    const uint32_t other = SM_U16(w.cls + p + ph * kLanes);
+                    const uint32_t picked = SM_U32(w.cls + p + ph * kLanes);
                     uint32_t alike = 0;
 #pragma unroll
                     for (int h = 0; h < kPer; ++h) {
                         const int g = lane + h * kLanes;
-                        const uint32_t own = g < a.G ? SM_U16(w.cls + g) : 0u;
-                        bool same = (own & 0xFFu) == (other & 0xFFu) && (own >> 8) < 32;
+                        const uint32_t own = g < a.G ? SM_U32(w.cls + g) : 0u;
+                        bool same = class_first(own) == class_first(picked) && class_rank(own) < 32;
 #pragma unroll
                         for (int s = 0; s + 1 < kDepth; ++s) {
                             const double x = __shfl_sync(0xFFFFFFFFu, kPer == 2 && ph ? c[kPer - 1][s] : c[0][s], p);
                             same = same && (x == c[h][s] || (x < ts && c[h][s] < ts));
                         }
                         const bool in = (win[h] >> lane) & 1u;
-                        if (in && same) alike |= 1u << (own >> 8);
-                        if (in && !same) tie |= class_bit((uint16_t)own) | class_bit((uint16_t)other);
+                        if (in && same) alike |= 1u << class_rank(own);
+                        if (in && !same && tie_matters(picked, own)) tie |= class_bit(own) | class_bit(picked);
                     }
                     alike = __reduce_or_sync(0xFFFFFFFFu, alike);
                     if (lane == k) swap = (alike & (alike - 1)) ? alike : 0u;
@@ -781,7 +781,7 @@ __device__ inline int32_t window_run_depth(const KernelArgs &a, Window &w, WalkM
                             a.swap_mask[cell] = swap;
                             a.swap_at[cell] = (uint16_t)(at - a.leaf_start[seg_leaf(a, q)]);
                         } else if (some) {
-                            tie |= class_bit(SM_U16(w.cls + (rec & (a.dec_wide ? 0x7FFFu : 0x7Fu)) - 1u));
+                            tie |= class_bit(SM_U32(w.cls + (rec & (a.dec_wide ? 0x7FFFu : 0x7Fu)) - 1u));
                         }
                         swap_n += __popc(who);
                     }
@@ -850,7 +850,7 @@ __device__ inline int32_t window_run_depth(const KernelArgs &a, Window &w, WalkM
             // the chunk was decided by a group number between different states
             auto usable = [&](int how, int32_t from, int32_t to_seg) {
                 if (how != 2) return how;
-                const uint16_t *cls = a.twin_class + (size_t)b * a.G;
+                const uint32_t *cls = a.twin_class + (size_t)b * a.G;
                 const uint64_t moved = moved_classes(cls, a.G, [&](int g) { return smem[w.re.perm + g]; });
                 bool some = false;
                 for (int32_t s = from + lane; s < to_seg; s += kLanes)

@@ -133,6 +133,24 @@ def test_relabelling_spares_repairs():
     assert with_ * 4 < without
 
 
+@pytest.mark.parametrize("depth", [1, 2])
+def test_ties_with_groups_behind_all_twins_spare_repairs(depth):
+    """Twins side by side, as a search's normalized placements have them: a choice that the group
+    number decides between one of them and a group behind them all is the same under any labels, and
+    is no reason to simulate a chunk again.  The same groups in an order in which it is one: exact."""
+    M = 4
+    profs = _profiles(M, (depth,), 9)
+    rng = np.random.RandomState(10)
+    ts = np.floor(np.cumsum(rng.exponential(1 / 60.0, size=30000)) / 0.02) * 0.02
+    ids = rng.randint(0, M, size=30000).astype(np.int32)
+    slos = np.full(30000, 0.5, np.float32)
+    side = [[0, 1]] * 4 + [[0, 1, 2]] * 4 + [[2, 3]] * 4
+    mixed = [side[k % 3 * 4 + k // 3] for k in range(12)]
+    redone = [_check([_placement([depth] * 12, models)] * 3, profs, ts, ids, slos, 256, 256,
+                     per_request=False).resimulated.max() for models in (side, mixed)]
+    assert redone[0] <= 12, redone          # of 117 chunks
+
+
 def test_replica_lists_in_any_order_and_negative_times():
     """The drop-in takes rows of m_id2g_id as they are: ties go to the first of the row, not to
     the lowest group; arrival times may be negative."""
