@@ -45,7 +45,7 @@ struct Geometry {
     size_t smem_stream, smem_window;
     size_t off_leaf, off_seg_end, off_chunk_start, off_decisions, off_work_count, off_work_items,
         off_rows, off_seg_leaf, off_group_info, off_columns, off_stamp, off_link, off_flags, off_rel,
-        off_tie, off_swap_mask, off_swap_at, off_swap_count, off_perm, off_twin_class, off_group_column, off_group_models;
+        off_tie, off_swap_mask, off_swap_at, off_swap_count, off_name_from, off_perm, off_twin_class, off_group_column, off_group_models;
     int32_t group_words, swap_cap;
     size_t smem_count;        // shared memory of count_kernel
     size_t total;
@@ -255,6 +255,7 @@ static int plan_call(int64_t N, const mms_placements *c, const mms_sim_options *
             g->off_tie = off;         off += align256(sizeof(uint64_t) * cells);
             g->off_perm = off;        off += align256(cells * G + 4);
             g->off_swap_count = off;  off += align256(cells);
+            g->off_name_from = off;   off += align256(sizeof(int32_t) * cells);
             g->off_swap_mask = off;   off += align256(sizeof(uint32_t) * cells * g->swap_cap);
             g->off_swap_at = off;     off += align256(sizeof(uint16_t) * cells * g->swap_cap);
             g->off_group_models = off;
@@ -387,6 +388,12 @@ static int launch_sim(KernelArgs &ka, const ClearArgs &ca, const Geometry &g, cu
         finish_k<<<(unsigned)((ka.B + kWindowWarps - 1) / kWindowWarps), kWindowWarps * kLanes,
                    g.smem_window, st>>>(ka);
         MMS_CUDA(cudaGetLastError());
+        if (ka.swap_mask) {
+            const int64_t warps = (int64_t)ka.B * ((ka.NS + kNameSegments - 1) / kNameSegments);
+            name_kernel<<<(unsigned)((warps + kNameWarps - 1) / kNameWarps), kNameWarps * kLanes,
+                          (size_t)kNameWarps * ka.G, st>>>(ka);
+            MMS_CUDA(cudaGetLastError());
+        }
         chain_span.stop();
     }
     return MMS_OK;
@@ -564,6 +571,7 @@ static int sim_mixed(const mms_trace *trace, const mms_placements *cands, const 
     ka.swap_mask = g.group_words ? (uint32_t *)(scratch + g.off_swap_mask) : nullptr;
     ka.swap_at = (uint16_t *)(scratch + g.off_swap_at); ka.swap_count = scratch + g.off_swap_count;
     ka.swap_cap = g.swap_cap;
+    ka.name_from = (int32_t *)(scratch + g.off_name_from);
     ka.seg_first_leaf = (int32_t *)(scratch + g.off_seg_leaf);
     ka.window = g.window;
     ka.seg_end = (double *)(scratch + g.off_seg_end);

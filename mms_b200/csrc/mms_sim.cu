@@ -27,8 +27,9 @@
 //                   wrong state has to be done again).
 //   finish kernel   one warp per candidate that is still open, or has relabelled segments,
 //                   goes through them in order, re-simulates whatever the rounds
-//                   left and translates labels into group numbers — it makes the result exact
+//                   left and follows the labels — it makes the result exact
 //                   whatever the chunking and the rounds.
+//   name kernel     translates labels into group numbers, a warp per few segments.
 //   count kernel    tallies the recorded decisions into the counters and combines the
 //                   per-leaf latency sums in numpy's pairwise order.
 #include <cuda_runtime.h>
@@ -394,7 +395,7 @@ link_kernel(const __grid_constant__ KernelArgs a)
         const size_t cell = (size_t)q0 * B + bb;
         for (int g = lane; g < a.G; g += kLanes) a.perm[cell * a.G + g] = smem[s.perm + g];
         if (lane == 0) {
-            a.rel[cell] = 1;
+            a.rel[cell] = kRelOther;
             a.relabelled[bb] = 1;
             a.link[(size_t)jj * B + bb] = 1;
         }
@@ -531,21 +532,97 @@ __device__ inline void labels_take(Labels &l, int G, uint64_t moved)
     __syncwarp();
 }
 
-// The first segment from q on that changes labels or starts a chunk behind a failed boundary
-// (NS: none).
-__device__ inline int32_t next_event(const KernelArgs &a, int64_t b, int32_t q)
+// The list of swaps of a segment (KernelArgs::swap_mask), an entry per lane at a time.
+struct Swaps {
+    size_t cell;                             // entry 0
+    int32_t count, base, next;               // base: entry in lane 0; next: the one peeked at
+    int32_t first, at;                       // the segment's first request; this lane's entry
+    uint32_t mask;
+};
+
+__device__ inline void swaps_load(const KernelArgs &a, Swaps &s, int32_t from)
 {
-    const int lane = threadIdx.x & (kLanes - 1);
-    const size_t B = (size_t)a.B;
-    for (; q < a.NS; q += kLanes) {
-        const int32_t s = q + lane;
-        const bool event = s < a.NS &&
-                           (a.rel[(size_t)s * B + b] ||
-                            (s % a.seg_per_chunk == 0 && !a.link[(size_t)(s / a.seg_per_chunk) * B + b]));
-        const uint32_t todo = __ballot_sync(0xFFFFFFFFu, event);
-        if (todo) return q + __ffs((int)todo) - 1;
+    const int32_t k = from + (int32_t)(threadIdx.x & (kLanes - 1));
+    s.base = from;
+    s.at = 0x7FFFFFFF;
+    s.mask = 0;
+    if (k < s.count) {
+        s.mask = a.swap_mask[s.cell + (size_t)k * a.B];
+        s.at = s.first + a.swap_at[s.cell + (size_t)k * a.B];
     }
-    return a.NS;
+}
+
+__device__ inline Swaps swaps_of(const KernelArgs &a, int64_t b, int32_t q, int32_t first)
+{
+    Swaps s;
+    s.cell = (size_t)q * a.swap_cap * a.B + b;
+    s.count = a.swap_count[(size_t)q * a.B + b];
+    s.first = first;
+    s.next = 0;
+    swaps_load(a, s, 0);
+    return s;
+}
+
+// The request of the next swap (behind the last one: 0x7FFFFFFF) and its mask.
+__device__ inline int32_t swaps_peek(const KernelArgs &a, Swaps &s, uint32_t &mask)
+{
+    if (s.next - s.base == kLanes) swaps_load(a, s, s.next);
+    mask = __shfl_sync(0xFFFFFFFFu, s.mask, s.next - s.base);
+    return __shfl_sync(0xFFFFFFFFu, s.at, s.next - s.base);
+}
+
+// A choice between twins in the same state: the true one is the smallest group number among the
+// labels of `mask` (ranks in the class of `mine`, the picked one); the label that has it changes
+// places with the picked one.  Returns whether they did.
+__device__ inline bool labels_swap(const KernelArgs &a, Labels &l, uint32_t mine, uint32_t mask)
+{
+    uint32_t key = 0xFFFFFFFFu;              // group << 8 | label
+    for (int g = threadIdx.x & (kLanes - 1); g < a.G; g += kLanes)
+        if (class_first(l.cls[g]) == class_first(l.cls[mine]) && class_rank(l.cls[g]) < 32 &&
+            ((mask >> class_rank(l.cls[g])) & 1u)) {
+            const uint32_t mapped = ((uint32_t)smem[l.pi + g] << 8) | (uint32_t)g;
+            key = mapped < key ? mapped : key;
+        }
+    key = __reduce_min_sync(0xFFFFFFFFu, key);
+    const uint32_t other = key & 0xFFu;
+    if (other == mine) return false;
+    __syncwarp();
+    if ((threadIdx.x & (kLanes - 1)) == 0) {
+        const uint8_t g = smem[l.pi + mine];
+        smem[l.pi + mine] = (uint8_t)(key >> 8);
+        smem[l.pi + other] = g;
+    }
+    __syncwarp();
+    return true;
+}
+
+// First request of segment q.
+__device__ inline int32_t segment_first(const KernelArgs &a, int32_t q)
+{
+    return seg_leaf(a, q) < a.num_leaves ? a.leaf_start[seg_leaf(a, q)] : (int32_t)a.N;
+}
+
+// Where the decision record of request i is.
+__device__ inline size_t record_at(const KernelArgs &a, int64_t b, int32_t i)
+{
+    return ((size_t)(i >> 2) * a.dec_pitch + b) * 4 + (size_t)(i & 3);
+}
+
+// Follows the labels through segment q.  Returns whether they changed.
+__device__ inline bool labels_follow(const KernelArgs &a, int64_t b, Labels &l, int32_t q)
+{
+    Swaps s = swaps_of(a, b, q, segment_first(a, q));
+    bool changed = false;
+    for (;; ++s.next) {
+        uint32_t mask;
+        const int32_t i = swaps_peek(a, s, mask);
+        if (i == 0x7FFFFFFF) break;
+        const uint32_t rec = a.dec_wide ? static_cast<uint16_t *>(a.decisions)[record_at(a, b, i)] & 0x7FFFu
+                                        : static_cast<uint8_t *>(a.decisions)[record_at(a, b, i)] & 0x7Fu;
+        if (rec && (class_bit(l.cls[rec - 1]) & l.moved)) changed |= labels_swap(a, l, rec - 1, mask);
+    }
+    if (changed) l.moved = moved_classes(l.cls, a.G, [&](int g) { return smem[l.pi + g]; });
+    return changed;
 }
 
 // Translates the decision records of segment q into group numbers, 32 requests at a time, and
@@ -556,37 +633,16 @@ __device__ inline void name_segment(const KernelArgs &a, int64_t b, Labels &l, i
 {
     constexpr int kAhead = 4;
     const int lane = threadIdx.x & (kLanes - 1);
-    const int32_t i0 = a.leaf_start[seg_leaf(a, q)];
-    const int32_t i1 = seg_leaf(a, q + 1) < a.num_leaves ? a.leaf_start[seg_leaf(a, q + 1)] : (int32_t)a.N;
+    const int32_t i0 = segment_first(a, q), i1 = segment_first(a, q + 1);
     const uint32_t flag = a.dec_wide ? 0x8000u : 0x80u;
-    auto place = [&](int32_t i) { return (((size_t)(i >> 2) * a.dec_pitch) + b) * 4 + (size_t)(i & 3); };
     auto fetch = [&](int32_t base, uint32_t &rec) {
         const int32_t i = base + lane;
         rec = 0;
         if (i < i1)
-            rec = a.dec_wide ? static_cast<uint16_t *>(a.decisions)[place(i)]
-                             : static_cast<uint8_t *>(a.decisions)[place(i)];
+            rec = a.dec_wide ? static_cast<uint16_t *>(a.decisions)[record_at(a, b, i)]
+                             : static_cast<uint8_t *>(a.decisions)[record_at(a, b, i)];
     };
-    // the segment's list of swaps, an entry per lane at a time
-    const int32_t swaps = a.swap_count[(size_t)q * a.B + b];
-    uint32_t swap_mask = 0;
-    int32_t swap_i = 0, swap_base = 0, next_swap = 0;      // swap_i: the request; next_swap: entry
-    auto load_swaps = [&](int32_t from) {
-        const size_t cell = ((size_t)q * a.swap_cap + from + lane) * a.B + b;
-        swap_base = from;
-        swap_i = 0x7FFFFFFF;
-        if (from + lane < swaps) {
-            swap_mask = a.swap_mask[cell];
-            swap_i = i0 + a.swap_at[cell];
-        }
-    };
-    load_swaps(0);
-    // the request and the mask of the next swap (behind the last one: request 0x7FFFFFFF)
-    auto peek_swap = [&](int32_t &i, uint32_t &mask) {
-        if (next_swap - swap_base == kLanes) load_swaps(next_swap);
-        i = __shfl_sync(0xFFFFFFFFu, swap_i, next_swap - swap_base);
-        mask = __shfl_sync(0xFFFFFFFFu, swap_mask, next_swap - swap_base);
-    };
+    Swaps swaps = swaps_of(a, b, q, i0);
     auto window = [&](int32_t base, uint32_t rec) {
         const uint32_t label = rec ? (rec & (flag - 1)) - 1 : 0u;
         const bool moves = rec && (class_bit(l.cls[label]) & l.moved);
@@ -595,42 +651,21 @@ __device__ inline void name_segment(const KernelArgs &a, int64_t b, Labels &l, i
         int from = 0;
         bool changed = false;
         for (;;) {
-            int32_t i;
             uint32_t mask;
-            peek_swap(i, mask);
+            const int32_t i = swaps_peek(a, swaps, mask);
             const int k = i - base < kLanes ? i - base : kLanes;
-            if (k < kLanes) ++next_swap;
+            if (k < kLanes) ++swaps.next;
             if (k < kLanes && !((movers >> k) & 1u)) continue;
             if (lane >= from && lane < k && moves) group = smem[l.pi + label];
             if (k == kLanes) break;
             from = k;
-            // the true choice is the smallest group number among the replicas in the picked one's
-            // state; the label that has it changes places with the picked one
-            const uint32_t mine = __shfl_sync(0xFFFFFFFFu, label, k);
-            uint32_t key = 0xFFFFFFFFu;              // group << 8 | label
-            for (int g = lane; g < a.G; g += kLanes)
-                if (class_first(l.cls[g]) == class_first(l.cls[mine]) && class_rank(l.cls[g]) < 32 &&
-                    ((mask >> class_rank(l.cls[g])) & 1u)) {
-                    const uint32_t mapped = ((uint32_t)smem[l.pi + g] << 8) | (uint32_t)g;
-                    key = mapped < key ? mapped : key;
-                }
-            key = __reduce_min_sync(0xFFFFFFFFu, key);
-            const uint32_t other = key & 0xFFu;
-            if (other != mine) {
-                __syncwarp();
-                if (lane == 0) {
-                    const uint8_t g = smem[l.pi + mine];
-                    smem[l.pi + mine] = (uint8_t)(key >> 8);
-                    smem[l.pi + other] = g;
-                }
-                changed = true;
-                __syncwarp();
-            }
+            changed |= labels_swap(a, l, __shfl_sync(0xFFFFFFFFu, label, k), mask);
         }
         if (moves && group != label) {
             rec = (rec & flag) | (group + 1);
-            if (a.dec_wide) static_cast<uint16_t *>(a.decisions)[place(base + lane)] = (uint16_t)rec;
-            else static_cast<uint8_t *>(a.decisions)[place(base + lane)] = (uint8_t)rec;
+            const size_t at = record_at(a, b, base + lane);
+            if (a.dec_wide) static_cast<uint16_t *>(a.decisions)[at] = (uint16_t)rec;
+            else static_cast<uint8_t *>(a.decisions)[at] = (uint8_t)rec;
         }
         if (changed) {
             __syncwarp();
@@ -650,9 +685,42 @@ __device__ inline void name_segment(const KernelArgs &a, int64_t b, Labels &l, i
     }
 }
 
+constexpr int kNameWarps = 4;
+constexpr int kNameSegments = 8;             // segments to a warp
+
+// The segments that finish_kernel left to be named: a warp per stretch of kNameSegments, each
+// with the labels noted for its start.  (finish_kernel did this itself, in order: 27 ns a request
+// and candidate, 4 ms for one placement over 150 000 requests; it now follows the labels through
+// the lists of swaps alone.)
+__global__ void __launch_bounds__(kNameWarps * kLanes)
+name_kernel(const __grid_constant__ KernelArgs a)
+{
+    const int lane = threadIdx.x & (kLanes - 1);
+    const int64_t w = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / kLanes;
+    const int32_t parts = (a.NS + kNameSegments - 1) / kNameSegments;
+    const int64_t b = w / parts;
+    if (!can_chunk(a) || b >= a.B || !a.relabelled[b]) return;
+    const size_t B = (size_t)a.B;
+    const int32_t q0 = (int32_t)(w % parts) * kNameSegments, s = q0 + lane;
+    const bool mine = lane < kNameSegments && s < a.NS && a.rel[(size_t)s * B + b] == kRelNamed;
+    Labels l;
+    l.pi = (threadIdx.x / kLanes) * (uint32_t)a.G;
+    l.tmp = l.pi;
+    l.cls = a.twin_class + (size_t)b * a.G;
+    for (uint32_t todo = __ballot_sync(0xFFFFFFFFu, mine); todo; todo &= todo - 1) {
+        const int32_t q = q0 + __ffs((int)todo) - 1;
+        const uint8_t *pi = a.perm + ((size_t)a.name_from[(size_t)q * B + b] * B + b) * a.G;
+        __syncwarp();
+        for (int g = lane; g < a.G; g += kLanes) smem[l.pi + g] = pi[g];
+        __syncwarp();
+        l.moved = moved_classes(l.cls, a.G, [&](int g) { return smem[l.pi + g]; });
+        name_segment(a, b, l, q);
+    }
+}
+
 // One warp per candidate that has an open boundary or relabelled segments: goes through the
-// segments in order with the translation of their labels into group numbers, and translates
-// their records.  At a failed boundary, and at a segment in other labels in which a group number
+// segments in order with the translation of their labels into group numbers, and notes it where
+// name_kernel is to translate their records.  At a failed boundary, and at a segment in other labels in which a group number
 // decided between different states, it walks from the true state (under the true labels)
 // until what is stored can take over.  After it, every segment was simulated from a state
 // equivalent to the true one under a translation that is exact for it: the result does
@@ -677,9 +745,37 @@ finish_kernel(const __grid_constant__ KernelArgs a)
     l.cls = a.twin_class + (size_t)b * a.G;
     labels_reset(l, a.G);
     int32_t q = a.seg_per_chunk;             // chunk 0 is the true run
-    for (;;) {
-        if (!l.moved) q = next_event(a, b, q);
-        if (q >= a.NS) break;
+    int32_t noted = -1;                      // segment in whose `perm` l.pi is noted
+    // segments [q, q + n) are to be named with l.pi at their start
+    auto note = [&](int32_t n) {
+        if (!kTwins || !l.moved) return;
+        __syncwarp();
+        if (noted < 0) {
+            noted = q;
+            for (int g = lane; g < a.G; g += kLanes) a.perm[((size_t)q * B + b) * a.G + g] = smem[l.pi + g];
+        }
+        if (lane < n) {
+            a.rel[(size_t)(q + lane) * B + b] = kRelNamed;
+            a.name_from[(size_t)(q + lane) * B + b] = noted;
+        }
+        __syncwarp();
+    };
+    while (q < a.NS) {
+        // the first of 32 segments in which something happens; those before it keep the labels
+        const int32_t s = q + lane;
+        bool event = false;
+        if (s < a.NS) {
+            const size_t at = (size_t)s * B + b;
+            event = s % a.seg_per_chunk == 0 && !a.link[(size_t)(s / a.seg_per_chunk) * B + b];
+            if constexpr (kTwins)
+                event |= a.rel[at] || (l.moved && (a.swap_count[at] || (a.tie[at] & l.moved)));
+        }
+        const uint32_t todo = __ballot_sync(0xFFFFFFFFu, event);
+        int32_t quiet = todo ? __ffs((int)todo) - 1 : kLanes;
+        if (quiet > a.NS - q) quiet = a.NS - q;
+        if (quiet) note(quiet);              // (the labels in front of an event are still to be read)
+        q += quiet;
+        if (!todo) continue;
         const size_t cell = (size_t)q * B + b;
         const int32_t j = q / a.seg_per_chunk;
         const bool first = q % a.seg_per_chunk == 0;
@@ -688,8 +784,12 @@ finish_kernel(const __grid_constant__ KernelArgs a)
             const bool other = a.rel[cell] != 0;
             if (other) moved = labels_through(l, a.G, a.perm + cell * a.G);
             if (!(moved && (a.tie[cell] & moved))) {
-                if (other) labels_take(l, a.G, moved);
-                if (l.moved) name_segment(a, b, l, q);
+                if (other) {
+                    labels_take(l, a.G, moved);
+                    noted = -1;
+                }
+                note(1);
+                if (l.moved && labels_follow(a, b, l, q)) noted = -1;
                 ++q;
                 continue;
             }
@@ -713,6 +813,7 @@ finish_kernel(const __grid_constant__ KernelArgs a)
         // (nothing is noted about choices between twins: nobody compares with these segments again)
         const int32_t e = window_run<kLegacy, kTwins, false>(a, w, kWalkChain, j, a.leaf_start[seg_leaf(a, q)], true, q);
         labels_reset(l, a.G);
+        noted = -1;
         q = e;
     }
     if (w.status) atomicOr(&a.status[b], w.status);

@@ -22,6 +22,8 @@ constexpr uint32_t kIrregularLayout = 1;
 // (window_groups) is sound: such a call is simulated in one piece, in the layout as given.
 constexpr uint32_t kIrregularLatency = 2;
 
+constexpr uint8_t kRelOther = 1, kRelNamed = 2;       // KernelArgs::rel
+
 struct KernelArgs {
     // trace
     const double *arrivals;
@@ -78,7 +80,10 @@ struct KernelArgs {
                                   //   group's rank among those << 8 | the largest one << 16
     const uint8_t *twins;         // [B]: some group has an interchangeable one
     uint8_t *rel;                 // [NS][B]: segment q is written in other labels than segment q-1
-    uint8_t *perm;                // [NS][B][G]: label in segment q -> label in segment q-1
+                                  //   (kRelOther); its records are to be named (kRelNamed)
+    uint8_t *perm;                // [NS][B][G]: label in segment q -> label in segment q-1; behind
+                                  //   finish_kernel, where name_from says so: -> group number
+    int32_t *name_from;           // [NS][B], where rel is kRelNamed: segment with the labels to use
     uint64_t *tie;                // [NS][B]: classes of twins (class_bit) for which a group number
                                   //   decided a choice in segment q between different states
     // choices that a group number decided between twins in the same state: per segment and
@@ -258,7 +263,7 @@ __device__ inline bool warp_equivalent(int G, Info info, LoadX X, LoadZ Z, doubl
 // scratch, nearly all of it zero).  Where the replicas are not in the same state and that matters
 // (tie_matters), or the list is full, it notes their classes for the segment (`tie`), and a segment
 // is only taken over under labels that leave those classes alone.
-// finish_kernel translates the decision records into group numbers; nothing else has labels.
+// name_kernel translates the decision records into group numbers; nothing else has labels.
 //
 // p has to keep the order of the last-stage clocks within a class (every group of a class serves
 // a replicated model), so it is the one that sorts them, equal ones by group number.

@@ -901,7 +901,7 @@ __device__ inline int32_t window_run_depth(const KernelArgs &a, Window &w, WalkM
                     for (int g = lane; g < a.G; g += kLanes)
                         perm[g] = smem[w.re.perm + (had && inside ? perm[g] : (uint8_t)g)];
                     if (lane == 0) {
-                        a.rel[cell] = 1;
+                        a.rel[cell] = kRelOther;
                         a.relabelled[b] = 1;
                     }
                 }

@@ -246,3 +246,19 @@ def test_more_swaps_than_a_segment_has_room_for(copies, twins):
         assert np.all(res.model_num_good == mgood)
         assert np.all(res.group_num_requests[:, :len(greq)] == greq)
         assert np.all(res.group_num_good[:, :len(ggood)] == ggood)
+
+
+@pytest.mark.parametrize("groups", [12, 130])
+@pytest.mark.parametrize("n", [513, 1024, 1025, 1151, 3072, 3329])
+def test_naming_at_the_ends_of_its_stretches(n, groups):
+    """Records of taken-over runs are translated eight segments to a warp: numbers of segments
+    around multiples of eight, records of one and (more than 126 groups) of two bytes."""
+    M = 6
+    profs = _profiles(M, (1, 2), 15)
+    ts, ids, slos = _trace(n, M, 7.0 * groups, 16, 0.01)
+    quarter = groups // 4
+    sols = [_placement([1] * groups, [[0, 1]] * quarter + [[0, 2]] * quarter + [[1, 3]] * quarter
+                       + [[4, 5]] * (groups - 3 * quarter)),
+            _placement([1] * groups, [[[0, 1], [0, 2], [3, 4, 5]][g % 3] for g in range(groups)])]
+    _check(sols * 2, profs, ts, ids, slos, 128, 128)
+    _check(sols * 20, profs, ts, ids, slos, 256, 64, per_request=False)
