@@ -41,7 +41,7 @@ static int32_t plan_leaves(int64_t n)
 struct Geometry {
     int32_t K, NS, seg_len, seg_per_chunk, warmup, lat_smem_elems, rounds,
         block_warps, lat_f64, window_blocks, win_table_elems;
-    bool window;
+    bool window, restart;
     size_t smem_stream, smem_window;
     size_t off_leaf, off_seg_end, off_chunk_start, off_decisions, off_work_count, off_work_items,
         off_rows, off_seg_leaf, off_group_info, off_columns, off_stamp, off_link, off_flags, off_rel,
@@ -147,9 +147,15 @@ static int plan_call(int64_t N, const mms_placements *c, const mms_sim_options *
     const int64_t chunk = opts ? opts->chunk_requests : 0;
     int64_t warm = opts ? opts->warmup_requests : 0;
     // Run-in: enough requests for every group to have had an idle moment and every replicated
-    // model a request.  Both grow with the cluster: of the boundaries of random placements at
-    // 0.8 to 2 requests a second and device, with 16 clock slots none fails behind 256
-    // requests, with 64 slots 5 % fail behind 1024 and 1.7 % behind 2048.
+    // model a request, most of the time.  Both grow with the cluster.  Chunks simulated again, of
+    // those of lists of 500 to 2000 placements at 0.6 to 2 requests a second and device, and the
+    // call, with 32 requests per clock slot and with 64:
+    //     8 slots    random  1.6 and 0.4 %   5.0 and 4.3 ms    grown   3 and 0.3 %   5.7 and 5.6 ms
+    //    16 slots    random  1.2 and 0.3 %   6.1 and 6.0 ms    grown   9 and 1 %     7.7 and 7.0 ms
+    //    32 slots    random  1.8 and 0.2 %   6.5 and 7.7 ms    grown  22 and 9 %    13.3 and 15.2 ms
+    //    64 slots    random  1.1 and 0.1 %   9.8 and 12.1 ms   grown  22 and 8 %    36.6 and 42 ms
+    // What fails is repaired in parallel (restart_kernel), at less than a longer run-in costs all
+    // chunks: 4096 placements on 64 devices 24 and 27 ms, a layer of 2343 on 64 47 and 48.
     if (warm <= 0) {
         warm = 32 * (int64_t)c->max_slots;
         if (warm < 128) warm = 128;
@@ -181,8 +187,12 @@ static int plan_call(int64_t N, const mms_placements *c, const mms_sim_options *
         x.K = (x.NS + x.spc - 1) / x.spc;
         return x;
     };
-    // segments of 128 requests where the snapshots are few (they are 8 bytes per clock slot,
-    // candidate and segment), of 1024 in the large batches
+    // Segments of 128 requests where the snapshots are few (they are 8 bytes per clock slot,
+    // candidate and segment), of 1024 in the large batches, whose chunks then have at least three.
+    // Calls with the line at 64, 256 and 1024 MB of snapshots at 128: 600 random placements on 16
+    // devices (90 MB) 5.0, 3.9 and 3.9 ms, 1500 on 32 (180) 8.1, 7.3, 7.4; 500 on 64 (360) 9.8, 9.8,
+    // 8.0, 1536 (670) 11.4, 11.4, 12.8; grown ones: 1000 on 32 devices (300) 14.6, 14.6, 16.7, 1000 on
+    // 64 (400) 29, 29, 36.
     const int64_t seg = !thrift && (double)N * (double)c->max_slots * (double)B * 8.0 / 128.0 <= 256e6 ? 128 : 1024;
     const int64_t thrifty = thrift == 0 ? 0 : thrift < 3 ? 3 * seg : 12 * seg;     // shortest chunk
     const Cut wide = cut_trace(seg, resident_slots * kLanes,
@@ -208,6 +218,11 @@ static int plan_call(int64_t N, const mms_placements *c, const mms_sim_options *
     if (rounds <= 0) rounds = kDefaultRepairRounds;
     if (rounds > kMaxRepairRounds) rounds = kMaxRepairRounds;
     g->rounds = rounds;
+    // Where a chunk is shorter than the run-in, one more chunk of history changes little and walks
+    // are better done in order.  With the line at half the run-in: 1500 placements on 32 devices, of
+    // which 61 with interchangeable groups have chunks of 512 behind 1024, 7.3 -> 8.3 ms, 1025 on 16
+    // (256 behind 512) 3.8 -> 4.25, but 200 grown ones on 32 (512 behind 1024) 5.6 -> 4.9.
+    g->restart = spc * x.seg >= warm;
     g->K = (int32_t)K; g->NS = (int32_t)NS; g->seg_len = (int32_t)x.seg;
     g->seg_per_chunk = (int32_t)spc; g->warmup = (int32_t)warm;
 
@@ -378,7 +393,10 @@ static int launch_sim(KernelArgs &ka, const ClearArgs &ca, const Geometry &g, cu
                           kLinkWarps * kLanes, link_smem, st>>>(ka);
             MMS_CUDA(cudaGetLastError());
             if (r == g.rounds) break;
-            resolve_kernel<<<(unsigned)((ka.B + 3) / 4), 4 * kLanes, 0, st>>>(ka);
+            if (r == 0 && g.restart)
+                restart_kernel<<<(unsigned)((bounds + 127) / 128), 128, 0, st>>>(ka);
+            else
+                resolve_kernel<<<(unsigned)((ka.B + 3) / 4), 4 * kLanes, 0, st>>>(ka);
             MMS_CUDA(cudaGetLastError());
             // sized for the worst case; blocks past the work list return at once
             walk_k<<<window_blocks(bounds), kWindowWarps * kLanes, g.smem_window, st>>>(ka);

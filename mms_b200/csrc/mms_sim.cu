@@ -20,11 +20,11 @@
 //                   EQUIVALENT to the one the run before it ended in (states_equivalent:
 //                   equal futures, provably), as it is or under other labels of
 //                   interchangeable groups (warp_relabel)?
-//   resolve kernel  one warp per candidate lists the chunks behind failed boundaries.
+//   restart or      lists the chunks behind failed boundaries, all of them or the first of each
+//   resolve kernel  failed stretch.
 //   walk kernel     one warp per listed chunk re-simulates it, and what follows, from the state
 //                   the chunk before it ended in until the stored run can take over.
-//                   link + resolve + walk run a few rounds (a walk that started from a
-//                   wrong state has to be done again).
+//                   (A walk that started from a wrong state has to be done again.)
 //   finish kernel   one warp per candidate that is still open, or has relabelled segments,
 //                   goes through them in order, re-simulates whatever the rounds
 //                   left and follows the labels — it makes the result exact
@@ -50,9 +50,10 @@ constexpr int kMaxSumDepth = 48;        // pair-sum stack of the numpy order
 constexpr int kLatSmemBytes = 32 * 1024;
 constexpr int kMaxRepairRounds = 16;
 constexpr int kTwinModels = 256;        // models a launch with interchangeable groups may have
-// One round of parallel walks: what it leaves open is walked once more by finish_kernel in any
-// case, and each further round is three launches (4 rounds and 1: one placement 405 and 386 us,
-// a layer of 2343 86.7 and 79.1 ms, a search 197 and 193 ms, 4096 placements the same).
+// One round of parallel walks: what it leaves open finish_kernel walks in any case, all candidates
+// beside each other, and each further round is three launches and waits for its longest walk
+// (a second one: 1000 placements on 64 devices 18.6 -> 15.7 ms, but 500 9.7 -> 10.5, grown ones on
+// 64 devices 73 -> 86 and 37.4 -> 36.6, a layer of 2343 47 -> 50, 4096 placements the same).
 constexpr int kDefaultRepairRounds = 1;
 
 // What a call clears before its kernels run, in one launch (grid-stride): the
@@ -402,12 +403,42 @@ link_kernel(const __grid_constant__ KernelArgs a)
     }
 }
 
-// One warp per candidate: lists the chunks to be walked in this round — those behind a failed
-// boundary that itself has a good one before it — and copies the state they start from.
-// The walk from there goes through the failed boundaries behind it.  Where a third of the
-// boundaries fail (a placement under sustained overload: states hardly ever settle) most walks
-// would start from states that are not the true ones either and have to be done again; such a
-// candidate is left to finish_kernel, which walks once.
+// One thread per boundary, the first round where chunks are at least as long as the run-in: lists
+// EVERY chunk behind a failed boundary, to be simulated again from the state that the run before
+// it ended in, as stored.  That state has a run-in and a whole chunk of history and is usually the
+// true one, although the one that the listed chunk's speculative run started from was not.  (While
+// only the first chunk of each failed stretch was walked, and none of a candidate a third of
+// whose boundaries fail, the rest was left to finish_kernel, one chunk after the other: 1500
+// placements with 1 in 60 boundaries failing 9.1 ms, all at once 7.3; 700 grown ones on 32 devices,
+// 1 in 4 failing, 17.8 and 13.3; a layer of 2343 59 and 47; 4096 on 64 devices 25.7 and 24.)
+__global__ void restart_kernel(const __grid_constant__ KernelArgs a)
+{
+    if (!can_chunk(a)) return;
+    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const size_t B = (size_t)a.B;
+    const size_t cell = (size_t)t + B;                   // chunk 0 is the true run
+    const bool failed = t < (int64_t)a.B * (a.K - 1) && !a.link[cell];
+    const uint32_t all = __ballot_sync(0xFFFFFFFFu, failed);
+    if (!all) return;
+    const int lane = threadIdx.x & (kLanes - 1);
+    uint32_t at = 0;
+    if (lane == 0) at = atomicAdd(&a.work_count[a.round], (uint32_t)__popc(all));
+    at = __shfl_sync(0xFFFFFFFFu, at, 0) + __popc(all & ((1u << lane) - 1u));
+    if (!failed) return;
+    const int64_t b = t % a.B;
+    const int32_t j = (int32_t)(t / a.B) + 1;
+    a.work_items[at] = (uint32_t)cell;
+    a.stamp[cell] = (uint8_t)(a.round + 1);
+    a.open[b] = 1;
+    if (a.resimulated) atomicAdd(&a.resimulated[b], 1);
+    const double *X = a.seg_end + (size_t)(j * a.seg_per_chunk - 1) * a.T * B + b;
+    double *Y = a.chunk_start + (size_t)j * a.T * B + b;
+    for (int s = 0; s < a.T; ++s) Y[s * B] = X[s * B];
+}
+
+// One warp per candidate, the other rounds: lists the chunks behind a failed boundary that itself
+// has a good one before it, and copies the state they start from.  The walk from there goes
+// through the failed boundaries behind it.
 __global__ void resolve_kernel(const __grid_constant__ KernelArgs a)
 {
     const int lane = threadIdx.x & (kLanes - 1);
@@ -418,7 +449,7 @@ __global__ void resolve_kernel(const __grid_constant__ KernelArgs a)
     for (int32_t j = 1 + lane; j < a.K; j += kLanes) fails += !a.link[(size_t)j * B + b];
     fails = __reduce_add_sync(0xFFFFFFFFu, fails);
     if (lane == 0) a.open[b] = fails != 0;
-    if (fails == 0 || (a.K > 8 && (int64_t)fails * 3 >= (int64_t)(a.K - 1))) return;
+    if (fails == 0) return;
     int32_t listed = 0;
     for (int32_t j0 = 1; j0 < a.K; j0 += kLanes) {
         const int32_t j = j0 + lane;
