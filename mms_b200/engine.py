@@ -1142,8 +1142,10 @@ def _launch(*args, rows_on_device=False, **kwargs):
     return _collect(_submit(*args, **kwargs), rows_on_device)
 
 
-# A batch is split when it has at least so many placements without interchangeable groups
-SPLIT_MIN_EASY = 512
+# A batch is split when it has at least so many placements without interchangeable groups (with 512:
+# 500 random placements on 64 devices 9.8 instead of 8.5 ms; with 128: 700 grown ones on 32 devices
+# 16.2 instead of 13.3 ms, their two launches short of candidates)
+SPLIT_MIN_EASY = 256
 SPLIT_MIN_HARD = 32       # ... and so many with such groups
 _SIDE_STREAMS = {}
 
