@@ -127,18 +127,20 @@ class PlacementEvaluator:
                                         len(self.model_names), device=device)
         self.table = engine.LatencyTable(self.prof_ress)
         self.options = options          # engine.sim_options(...) or None
-        # A list of some length is encoded and launched in parts.  The first part only has
-        # to cover the host's work on the second, so it is the smaller one; more
-        # and smaller parts cost more on the GPU (shorter chunks, more run-in)
-        # than the encoding they hide.  A long list (pipeline_max_list) goes out as one: what
-        # parts cost grows with it (4096 placements: 29.8 ms as one, 32.8 ms in two parts).
+        # A list of some length is encoded and launched in parts, the host encoding one while the
+        # GPU simulates those before it.  The first only has to cover the host's work on the
+        # second, so it is the smaller one; parts cost shorter chunks and walks of their own.
+        # Random lists on 8, 16, 32 and 64 devices, as one and in two parts, ms: 1536 placements 4.6
+        # and 5.1, 5.9 and 5.7, 7.0 and 7.0, 10.9 and 12.0; 1792 4.7 and 5.2, 6.2 and 7.6, 7.1 and 6.9,
+        # 11.4 and 12.2; 2560 5.5 and 6.0, 10.6 and 11.4, 8.5 and 8.8, 13.3 and 14.9; 4096 7.9 and 8.2,
+        # 14.6 and 14.0, 12.1 and 11.1, 17.2 and 17.9: from 1792 on it goes out as one.
         self.pipeline_parts = 2
         self.pipeline_min_part = 768    # placements per part, at least
-        self.pipeline_max_list = 2048
+        self.pipeline_max_list = 1792
         self.pipeline_shares = (3, 5)   # relative sizes of the parts (None: equal)
         # placements with interchangeable groups as a launch of their own inside a
         # part: one flag, or one per part.  Only the last part needs it: the
-        # serial repairs of an earlier part run beside the parts behind it anyway.
+        # walks of an earlier part run beside the parts behind it anyway.
         self.pipeline_split = (False, True)
         # engine.sim_options per part (None: self.options for every part)
         self.pipeline_options = None
