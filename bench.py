@@ -100,18 +100,16 @@ def parse_args():
     ap.add_argument("--chunk", type=int, default=0, help="requests per chunk (0 auto, <0 one)")
     ap.add_argument("--run-in", type=int, default=0, help="run-in requests per chunk (0 auto)")
     ap.add_argument("--rounds", type=int, default=0, help="validate+repair rounds (0 auto)")
-    ap.add_argument("--repair-segments", type=int, default=0,
-                    help="segments a repair runs per round (0 auto, <0 no cap)")
     ap.add_argument("--hard", default="",
-                    help="candidates: chunk,run-in,rounds,repair-segments of the launch that holds "
-                         "the placements with mirror candidates (default: as the others)")
+                    help="candidates: chunk,run-in,rounds of the launch that holds the placements "
+                         "with interchangeable groups (default: as the others)")
     ap.add_argument("--traces", type=int, default=0, help="sweep: traces per GPU (default 1024)")
     ap.add_argument("--placement-seed", type=int, default=-1,
                     help="seed of the candidate list (default: the rank; strong scaling: 0)")
     ap.add_argument("--no-split", action="store_true",
-                    help="one launch per step even when some placements have mirror candidates")
+                    help="one launch per step even when some placements have interchangeable groups")
     ap.add_argument("--no-mirrors", action="store_true",
-                    help="no mirror candidates for placements with interchangeable groups")
+                    help="interchangeable groups are not looked for")
     return ap.parse_args()
 
 
@@ -443,7 +441,7 @@ def run_candidates(args, D):
     lo, hi = shard_bounds(args.candidates, rank, world) if strong else (0, args.candidates)
     mine = case.placements[lo:hi]
     first_index = lo if strong else rank * args.candidates
-    opts = engine.sim_options(args.chunk, args.run_in, args.rounds, args.repair_segments)
+    opts = engine.sim_options(args.chunk, args.run_in, args.rounds)
     ev = PlacementEvaluator(case.model_datas, case.cluster_env, case.workload, device=dev,
                             options=opts)
     N, B = ev.trace.num_requests, len(mine)
@@ -970,7 +968,7 @@ def run_sweep(args, D, traces=1024, duration=3600.0, steps=None, cpu=True):
     t_gen = time.perf_counter()
     workloads = [case.trace(rank * T + t) for t in range(T)]
     t_gen = time.perf_counter() - t_gen
-    opts = engine.sim_options(args.chunk, args.run_in, args.rounds, args.repair_segments)
+    opts = engine.sim_options(args.chunk, args.run_in, args.rounds)
     sweep = TraceSweep(case.model_datas, case.cluster_env, case.placement, device=dev,
                        options=opts, cells=16, first_trace=rank * T)
     names = sweep.model_names

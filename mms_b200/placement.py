@@ -194,8 +194,7 @@ class PlacementEvaluator:
                 opts_k = self.pipeline_options[k]
             with torch.cuda.stream(self._streams[k]):
                 jobs.append(engine.submit_batch(self.trace, enc, self.table, pinned=pinned,
-                                                options=opts_k, split=split[k],
-                                                crowded=k + 1 < parts))
+                                                options=opts_k, split=split[k]))
             encs.append(enc)
         done = [engine.collect_batch(job) for job in jobs]
         for k in range(parts):

@@ -138,13 +138,12 @@ def test_short_and_ragged_traces(loaded, n):
     (-1, 0, 0, 0, False), (1024, 2048, 0, 0, False), (4096, 1, 0, 0, False),
     (2048, 64, 2, 1, False), (8192, 2048, 6, 2, False), (8192, 16, 1, 1, False),
     (0, 0, 0, 0, False), (0, 0, 16, 3, False),
-    # with the hint, more than 48 failing chunks are repaired 32 to a warp
+    # with MMS_FLAG_CROWDED, which is accepted and changes nothing
     (4096, 1, 0, 0, True), (2048, 64, 2, 1, True), (3072, 8, 16, 0, True)])
 def test_results_do_not_depend_on_chunking(loaded, chunk, run_in, rounds, cap, crowded):
     """Speculative chunks are kept only when provably equivalent, so any cut of
     the trace — even a run-in of one request, which makes nearly every chunk
-    wrong and re-simulated — gives the sequential results bit for bit, whether
-    the repairs run one chunk to a warp or 32."""
+    wrong and re-simulated — gives the sequential results bit for bit."""
     from mms_b200 import cases, engine
     from mms_b200.placement import PlacementEvaluator
     from mms_b200.simulator import workload_arrays
