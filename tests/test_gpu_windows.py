@@ -264,6 +264,26 @@ def test_naming_at_the_ends_of_its_stretches(n, groups):
     _check(sols * 20, profs, ts, ids, slos, 256, 64, per_request=False)
 
 
+@pytest.mark.parametrize("chunk,run_in", [(256, 512), (512, 1024)])
+def test_chunks_that_mostly_fail_are_walked_once(chunk, run_in):
+    """Many groups that share their models without being interchangeable: most boundaries of a cut
+    shorter than its run-in fail, also for a walk that starts behind one of them.  No candidate is
+    walked in the parallel round and then in the last pass again."""
+    M, n = 6, 30000
+    profs = _profiles(M, (1,), 9)
+    rng = np.random.RandomState(10)
+    ts = np.cumsum(rng.exponential(1 / 30.0, size=n))
+    ids = rng.randint(0, M, size=n).astype(np.int32)
+    slos = np.full(n, 0.5, np.float32)
+    sols = []
+    for s in range(6):
+        pick = np.random.RandomState(s)
+        sols.append(_placement([1] * 16, [sorted({0} | set(pick.choice(M, 3, replace=False).tolist()))
+                                          for _ in range(16)]))
+    redone = _check(sols, profs, ts, ids, slos, chunk, run_in, per_request=False).resimulated
+    assert n // chunk // 2 < redone.max() < n // chunk
+
+
 def test_failed_chunks_are_not_left_to_the_last_pass():
     """A list of which 1 to 2 % of the boundaries fail, some candidates' mostly: the last pass, which
     walks a candidate's chunks one after the other, is a small part of the call.  (Its share of the
