@@ -407,9 +407,10 @@ static int launch_sim(KernelArgs &ka, const ClearArgs &ca, const Geometry &g, cu
                    g.smem_window, st>>>(ka);
         MMS_CUDA(cudaGetLastError());
         if (ka.swap_mask) {
-            const int64_t warps = (int64_t)ka.B * ((ka.NS + kNameSegments - 1) / kNameSegments);
+            const int32_t segments = (int64_t)ka.B * ka.NS <= kNameAlone ? 1 : kNameSegments;
+            const int64_t warps = (int64_t)ka.B * ((ka.NS + segments - 1) / segments);
             name_kernel<<<(unsigned)((warps + kNameWarps - 1) / kNameWarps), kNameWarps * kLanes,
-                          (size_t)kNameWarps * ka.G, st>>>(ka);
+                          (size_t)kNameWarps * ka.G, st>>>(ka, segments);
             MMS_CUDA(cudaGetLastError());
         }
         chain_span.stop();

@@ -721,23 +721,25 @@ __device__ inline void name_segment(const KernelArgs &a, int64_t b, Labels &l, i
 }
 
 constexpr int kNameWarps = 4;
-constexpr int kNameSegments = 8;             // segments to a warp
+constexpr int kNameSegments = 8;             // segments to a warp, at most 32
+// Segments of a call up to which each has a warp of its own: they all run at once then.
+constexpr int64_t kNameAlone = 148 * 64;
 
-// The segments that finish_kernel left to be named: a warp per stretch of kNameSegments, each
+// The segments that finish_kernel left to be named: a warp per stretch of `segments`, each
 // with the labels noted for its start.  (finish_kernel did this itself, in order: 27 ns a request
 // and candidate, 4 ms for one placement over 150 000 requests; it now follows the labels through
 // the lists of swaps alone.)
 __global__ void __launch_bounds__(kNameWarps * kLanes)
-name_kernel(const __grid_constant__ KernelArgs a)
+name_kernel(const __grid_constant__ KernelArgs a, const int32_t segments)
 {
     const int lane = threadIdx.x & (kLanes - 1);
     const int64_t w = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / kLanes;
-    const int32_t parts = (a.NS + kNameSegments - 1) / kNameSegments;
+    const int32_t parts = (a.NS + segments - 1) / segments;
     const int64_t b = w / parts;
     if (!can_chunk(a) || b >= a.B || !a.relabelled[b]) return;
     const size_t B = (size_t)a.B;
-    const int32_t q0 = (int32_t)(w % parts) * kNameSegments, s = q0 + lane;
-    const bool mine = lane < kNameSegments && s < a.NS && a.rel[(size_t)s * B + b] == kRelNamed;
+    const int32_t q0 = (int32_t)(w % parts) * segments, s = q0 + lane;
+    const bool mine = lane < segments && s < a.NS && a.rel[(size_t)s * B + b] == kRelNamed;
     Labels l;
     l.pi = (threadIdx.x / kLanes) * (uint32_t)a.G;
     l.tmp = l.pi;

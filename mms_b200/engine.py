@@ -1142,10 +1142,16 @@ def _launch(*args, rows_on_device=False, **kwargs):
     return _collect(_submit(*args, **kwargs), rows_on_device)
 
 
-# A batch is split when it has at least so many placements without interchangeable groups (with 512:
-# 500 random placements on 64 devices 9.8 instead of 8.5 ms; with 128: 700 grown ones on 32 devices
-# 16.2 instead of 13.3 ms, their two launches short of candidates)
-SPLIT_MIN_EASY = 256
+# A batch is split when it has at least so many placements without interchangeable groups ...
+SPLIT_MIN_EASY = 512
+# ... or so many, when all its placements together simulate so many requests: a second launch costs
+# 0.15 to 0.2 ms, and one whose launches are short of candidates cuts both finer.  As one call and as
+# two, ms: 442 on 8 devices over 3 300 requests 1.24 and 1.41, 420 random ones over 100 000 on 16 devices
+# 5.48 and 4.54, on 64 6.20 and 6.84, 500 over 180 000 on 64 9.8 and 8.5; 1000 grown ones over 100 000,
+# 650 of them with interchangeable groups, on 16 devices 9.32 and 8.53, on 64 29.4 and 26.2.  With fewer
+# than 256: 700 grown ones over 100 000, on 32 devices 10.4 and 12.2, on 64 23.2 and 32.7.
+SPLIT_MIN_EASY_LONG = 256
+SPLIT_LONG = 64e6
 SPLIT_MIN_HARD = 32       # ... and so many with such groups
 _SIDE_STREAMS = {}
 
@@ -1188,7 +1194,10 @@ class ResidentBatch:
         parts = [(None, enc)]
         if split and mirrors and enc.has_twins is not None:
             hard = np.flatnonzero(enc.has_twins)
-            if len(hard) >= SPLIT_MIN_HARD and enc.B - len(hard) >= SPLIT_MIN_EASY:
+            least = SPLIT_MIN_EASY
+            if trace.num_requests * enc.B >= SPLIT_LONG:
+                least = min(least, SPLIT_MIN_EASY_LONG)
+            if len(hard) >= SPLIT_MIN_HARD and enc.B - len(hard) >= least:
                 easy = np.flatnonzero(~enc.has_twins)
                 parts = [(hard, enc.take(hard)), (easy, enc.take(easy))]
         self.index = [p[0] for p in parts]

@@ -471,10 +471,9 @@ def test_twin_groups_keep_exact_counters(loaded, chunk, run_in):
 @pytest.mark.parametrize("chunk,run_in,rounds,cap", [
     (0, 0, 0, 0), (4096, 512, 0, 0), (2048, 16, 2, 1), (4096, 2048, 1, 0), (8192, 1, 16, 2)])
 def test_mirror_candidates_change_nothing_but_speed(loaded, chunk, run_in, rounds, cap):
-    """Placements with interchangeable groups get a mirror candidate whose
-    speculative chunks start with those groups exchanged; a chunk is taken
-    from whichever run continues the chain.  Every reduced output must equal
-    the run without mirrors and the checker, for any cut of the trace."""
+    """Of placements with interchangeable groups, speculative runs in which
+    those have changed places are taken over.  Every reduced output must equal
+    the run in which none is and the checker, for any cut of the trace."""
     from mms_b200 import cases, engine
     from mms_b200.placement import ModelPlacement, PlacementEvaluator
     from mms_b200.profiling import ParallelConfig
@@ -495,7 +494,7 @@ def test_mirror_candidates_change_nothing_but_speed(loaded, chunk, run_in, round
                             options=engine.sim_options(chunk, run_in, rounds, cap))
     enc = engine.encode_placements(sols, ev.table, len(ev.model_names))
     ext = enc.with_mirrors()
-    assert ext is not None and len(ext[3]) >= enc.B + 4      # most hand-made ones get mirrors
+    assert ext is not None and len(ext[3]) >= enc.B + 4      # most hand-made ones have some
     with_m, _, _ = engine.run_batch(ev.trace, enc, ev.table, group_good=True, options=ev.options)
     without, _, _ = engine.run_batch(ev.trace, enc, ev.table, group_good=True, options=ev.options,
                                      mirrors=False)
@@ -550,7 +549,7 @@ def test_pipelined_evaluation_equals_one_launch(loaded):
     assert np.array_equal(res4.group_num_requests[:, :G], res1.group_num_requests)
     assert np.array_equal(enc4.num_groups, enc1.num_groups)
     assert ev.get_scores(case.placements[:5]) == scores4[:5]
-    # the defaults: two unequal parts, placements with mirrors launched apart inside each
+    # the defaults: two unequal parts, in the second placements with interchangeable groups apart
     ev2 = PlacementEvaluator(case.model_datas, case.cluster_env, case.workload)
     enc2, res2 = ev2.evaluate(case.placements)
     assert [e.B for e in enc2.parts] == [638, 1062]
@@ -604,7 +603,7 @@ def test_trace_sweep_one_placement_many_traces(loaded):
 
 
 def test_split_launch_equals_one_launch(loaded, monkeypatch):
-    """Placements with mirror candidates go into a launch of their own beside
+    """Placements with interchangeable groups go into a launch of their own beside
     the rest (two streams); every output equals the single launch's, in the
     order of the batch."""
     from mms_b200 import cases, engine
@@ -625,6 +624,29 @@ def test_split_launch_equals_one_launch(loaded, monkeypatch):
                  "good_total", "latency_sum", "status"):
         assert getattr(first, name).tobytes() == getattr(one, name).tobytes(), name
         assert getattr(again, name).tobytes() == getattr(one, name).tobytes(), name
+
+
+def test_short_lists_are_split_when_they_simulate_much(loaded, monkeypatch):
+    """Fewer than SPLIT_MIN_EASY placements without interchangeable groups go out as a launch of
+    their own from SPLIT_LONG requests on, over all placements; the outputs are the same."""
+    from mms_b200 import cases, engine
+    from mms_b200.placement import PlacementEvaluator
+    monkeypatch.setattr(engine, "SPLIT_MIN_HARD", 4)
+    case = cases.candidate_batch_case(num_candidates=300, duration=100.0, placement_seed=11)
+    ev = PlacementEvaluator(case.model_datas, case.cluster_env, case.workload)
+    enc = engine.encode_placements(case.placements, ev.table, len(ev.model_names))
+    easy = enc.B - int(enc.has_twins.sum())
+    assert engine.SPLIT_MIN_EASY_LONG <= easy < engine.SPLIT_MIN_EASY
+    requests = ev.trace.num_requests * enc.B
+    res = []
+    for line, jobs in ((requests, 2), (requests + 1, 1)):
+        monkeypatch.setattr(engine, "SPLIT_LONG", line)
+        batch = engine.ResidentBatch(ev.trace, enc, ev.table, group_good=True)
+        assert len(batch.jobs) == jobs
+        res.append(batch.launch().results()[0])
+        batch.release()
+    for name in ("model_num_good", "group_num_requests", "group_num_good", "good_total", "latency_sum"):
+        assert getattr(res[0], name).tobytes() == getattr(res[1], name).tobytes(), name
 
 
 def test_plain_placement_through_approximate_one_case(loaded, golden):

@@ -251,7 +251,7 @@ def test_more_swaps_than_a_segment_has_room_for(copies, twins):
 @pytest.mark.parametrize("groups", [12, 130])
 @pytest.mark.parametrize("n", [513, 1024, 1025, 1151, 3072, 3329])
 def test_naming_at_the_ends_of_its_stretches(n, groups):
-    """Records of taken-over runs are translated eight segments to a warp: numbers of segments
+    """Records of taken-over runs are translated one or eight segments to a warp: numbers of segments
     around multiples of eight, records of one and (more than 126 groups) of two bytes."""
     M = 6
     profs = _profiles(M, (1, 2), 15)
@@ -262,6 +262,28 @@ def test_naming_at_the_ends_of_its_stretches(n, groups):
             _placement([1] * groups, [[[0, 1], [0, 2], [3, 4, 5]][g % 3] for g in range(groups)])]
     _check(sols * 2, profs, ts, ids, slos, 128, 128)
     _check(sols * 20, profs, ts, ids, slos, 256, 64, per_request=False)
+
+
+@pytest.mark.parametrize("n,copies", [(1025, 1184), (1025, 1185), (513, 2369), (3329, 365)])
+def test_naming_of_long_lists(n, copies):
+    """Up to 9 472 segments in a call each is translated by a warp of its own, beyond that eight by
+    one: both sides of the line, and stretches that end short of eight segments."""
+    from mms_b200 import engine
+    from oracle import tables
+    M, groups = 6, 12
+    profs = _profiles(M, (1, 2), 15)
+    ts, ids, slos = _trace(n, M, 7.0 * groups, 16, 0.01)
+    p = _placement([1] * groups, [[0, 1]] * 3 + [[0, 2]] * 3 + [[1, 3]] * 3 + [[4, 5]] * 3)
+    table = engine.LatencyTable(profs)
+    enc = engine.encode_placements([p] * copies, table, M)
+    res, _, _ = engine.run_batch(engine.DeviceTrace(ts, ids, slos, M), enc, table, group_good=True,
+                                 options=engine.sim_options(128, 128, 0), split=False)
+    fin, good, _, mgood, greq, ggood = tables.one_placement(p, profs, ids, slos, ts)
+    assert np.all(res.good_total == np.count_nonzero(good))
+    assert np.all(res.latency_sum == float(np.add.reduce(fin - ts)))
+    assert np.all(res.model_num_good == mgood)
+    assert np.all(res.group_num_requests[:, :len(greq)] == greq)
+    assert np.all(res.group_num_good[:, :len(ggood)] == ggood)
 
 
 @pytest.mark.parametrize("chunk,run_in", [(256, 512), (512, 1024)])
