@@ -352,6 +352,7 @@ static int launch_sim(KernelArgs &ka, const ClearArgs &ca, const Geometry &g, cu
         if (blocks < 1) blocks = 1;
         clear_kernel<<<(unsigned)blocks, 256, 0, st>>>(ka, ca);
         MMS_CUDA(cudaGetLastError());
+        if (blocks < kTableBlocks) blocks = kTableBlocks;
         build_tables_kernel<<<(unsigned)blocks, 256, 0, st>>>(ka, ca);
         MMS_CUDA(cudaGetLastError());
     }

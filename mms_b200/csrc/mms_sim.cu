@@ -124,22 +124,28 @@ __global__ void clear_kernel(const KernelArgs a, const ClearArgs c)
 // bad index is reported in the status word and emptied.  (2) One thread per
 // (candidate, group) reports a group_info entry that clear_kernel had to empty.
 // (3) One thread per segment finds the segment's first leaf.  (4) The latency tables are looked
-// through for entries that are not >= 0 (kIrregularLatency).
+// through for entries that are not >= 0 (kIrregularLatency).  Each is a chain of loads: each part
+// begins at another quarter of the grid, so that the four run beside each other in a small call.
+constexpr int kTableBlocks = 4;              // blocks of build_tables_kernel, at least
 __global__ void build_tables_kernel(const KernelArgs a, const ClearArgs c)
 {
-    const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const int64_t nth = (int64_t)gridDim.x * blockDim.x;
+    int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const auto next_quarter = [&] { tid = tid >= nth / 4 ? tid - nth / 4 : tid + nth - nth / 4; };
     for (int64_t q = tid; q <= a.NS; q += nth)
         a.seg_first_leaf[q] = q == 0 ? 0 : q == a.NS ? a.num_leaves
             : leaf_lower_bound(a.leaf_start, a.num_leaves, q * a.seg_len);
     const int64_t entries = (int64_t)a.M * a.C * a.S;
     bool odd = false;
+    next_quarter();
     for (int64_t i = tid; i < (a.latency_stride ? a.B * entries : entries); i += nth)
         odd |= !(a.latency[i / entries * a.latency_stride + i % entries] >= 0.0f);
     if (odd) atomicOr(c.irregular, kIrregularLatency);
+    next_quarter();
     for (int64_t i = tid; i < (int64_t)a.B * a.G; i += nth)
         if (!group_info_valid(a, c.group_info_in[i]))
             atomicOr(&a.status[i / a.G], MMS_STATUS_BAD_INDEX);
+    next_quarter();
     for (int64_t t = tid; t < (int64_t)a.B * (a.M + 1); t += nth) {
         const int64_t b = t / (a.M + 1);
         const int m = (int)(t % (a.M + 1));
