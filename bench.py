@@ -49,8 +49,8 @@ FALLBACK_HBM_GBS = 6650.0
 # dram__bytes_read.sum + dram__bytes_write.sum of ONE sim_stream_kernel launch (ncu) on the
 # default workload: only valid for the library version and the launch shape it was taken
 # with, and reported as null for any other.
-STREAM_KERNEL_TRAFFIC = {"abi_version": 9, "candidates": 3695, "requests": 180715,
-                         "bytes": 41885184 + 1057393152}
+STREAM_KERNEL_TRAFFIC = {"abi_version": 10, "candidates": 3695, "requests": 180715,
+                         "bytes": 41764352 + 1057750272}
 
 _REAL_STDOUT = None
 
@@ -111,6 +111,13 @@ def parse_args():
     ap.add_argument("--no-mirrors", action="store_true",
                     help="interchangeable groups are not looked for")
     return ap.parse_args()
+
+
+def sim_launches(args):
+    """Kernels of a mms_sim_mixed call without interchangeable groups (with: two more): clear,
+    tables, stream, (link, restart or resolve, walk) per round, link, finish, count, requests per
+    model."""
+    return 7 + 3 * (args.rounds if args.rounds > 0 else 1)
 
 
 def hbm_peak():
@@ -626,10 +633,9 @@ def run_candidates(args, D):
                          "algorithmic_bytes_per_launch": kernel_units * BYTES_PER_UNIT},
             "e2e": {"value": e2e_value, "unit": UNIT, "h2d_bytes_per_step": int(h2d),
                     "d2h_bytes_per_step": int(d2h)},
-            # clear, tables, stream, (link, resolve, walk) per round, link, finish, count,
-            # requests per model — per launch — and the argmax
-            "gpu_launches": ((7 + 3 * (args.rounds if args.rounds > 0 else 1) + 1) * args.steps
-                             * len(resident.jobs)),
+            # of every call, and the argmax; at most one call has interchangeable groups
+            "gpu_launches": ((sim_launches(args) + 1) * len(resident.jobs)
+                             + (2 if not args.no_mirrors and enc.may_have_twins() else 0)) * args.steps,
             "launches_per_step": len(resident.jobs),
             # each rank's simulation per step, before the selection and its exchange
             "kernel_ms_per_step_by_rank": by_rank,
@@ -745,7 +751,7 @@ def run_batching(args, D, candidates=1024, duration=3600.0, steps=None, cpu=True
         return None
     peak, which = hbm_peak()
     k_ms = float(np.mean(stream_ms)) if len(stream_ms) else float("nan")
-    dominant, dom_ms = "batch_stream_kernel", k_ms
+    dominant, dom_ms = "batch_simd_kernel" if B >= 24 else "batch_stream_kernel", k_ms
     if len(chain_ms) and float(np.mean(chain_ms)) > k_ms:
         dominant, dom_ms = "batch_chain_kernel", float(np.mean(chain_ms))
     achieved = B * N * BYTES_PER_UNIT_FULL / (dom_ms * 1e-3) / 1e9
@@ -766,7 +772,9 @@ def run_batching(args, D, candidates=1024, duration=3600.0, steps=None, cpu=True
                      "algorithmic_bytes_per_launch": B * N * BYTES_PER_UNIT_FULL},
         "e2e": {"value": e2e_value, "unit": UNIT, "h2d_bytes_per_step": int(h2d),
                 "d2h_bytes_per_step": int(d2h)},
-        "gpu_launches": 6 * steps,
+        # cut-or-not, tables, stream, three rounds of validate and repair, validate, chain, counters,
+        # leaf sums, totals; the tables only where 32 candidates go to a warp
+        "gpu_launches": (14 if B >= 24 else 13) * steps,
         "chunks_resimulated_per_candidate": float(np.mean(res.resimulated)),
         "clocks": clk.summary(),
     }
@@ -1075,7 +1083,7 @@ def run_sweep(args, D, traces=1024, duration=3600.0, steps=None, cpu=True):
                      "algorithmic_bytes_per_launch": dom_units * BYTES_PER_UNIT},
         "e2e": {"value": e2e_value, "unit": UNIT, "h2d_bytes_per_step": int(sweep.last_h2d_bytes),
                 "d2h_bytes_per_step": int(sweep.last_d2h_bytes)},
-        "gpu_launches": (7 + 3 * (args.rounds if args.rounds > 0 else 1)) * n_groups * steps,
+        "gpu_launches": (sim_launches(args) + (2 if sweep.enc.may_have_twins() else 0)) * n_groups * steps,
         "chunks_resimulated_per_trace": float(np.mean(res.resimulated)),
         "clocks": clk.summary(),
         "goodput_mean_per_cell": [float(x) for x in (tally_host[:, 0] / np.maximum(tally_host[:, 1], 1))],
