@@ -41,7 +41,7 @@ static int32_t plan_leaves(int64_t n)
 struct Geometry {
     int32_t K, NS, seg_len, seg_per_chunk, warmup, lat_smem_elems, rounds,
         block_warps, lat_f64, window_blocks, win_table_elems;
-    bool window, restart;
+    bool window, restart, finish_at_once;     // finish_at_once: see kFinishBlocksPerSm
     size_t smem_stream, smem_window;
     size_t off_leaf, off_seg_end, off_chunk_start, off_decisions, off_work_count, off_work_items,
         off_rows, off_seg_leaf, off_group_info, off_columns, off_stamp, off_link, off_flags, off_rel,
@@ -279,6 +279,8 @@ static int plan_call(int64_t N, const mms_placements *c, const mms_sim_options *
         g->off_seg_end = off;     off += align256(sizeof(double) * (size_t)NS * c->max_slots * B);
         g->off_chunk_start = off; off += align256(sizeof(double) * (size_t)K * c->max_slots * B);
     }
+    g->finish_at_once = (B + kWindowWarps - 1) / kWindowWarps <= (int64_t)kFinishBlocksPerSm * sm_count &&
+                        (g->group_words || c->max_stages <= kGroupDepth);
     g->total = off;
     return MMS_OK;
 }
@@ -382,7 +384,11 @@ static int launch_sim(KernelArgs &ka, const ClearArgs &ca, const Geometry &g, cu
     stream_span.stop();
     if (ka.K > 1) {
         auto walk_k = ka.swap_mask ? walk_kernel<kLegacy, true> : walk_kernel<kLegacy, false>;
-        auto finish_k = ka.swap_mask ? finish_kernel<kLegacy, true> : finish_kernel<kLegacy, false>;
+        auto finish_k = g.finish_at_once
+                            ? (ka.swap_mask ? finish_kernel<kLegacy, true, kFinishBlocksPerSm>
+                                            : finish_kernel<kLegacy, false, kFinishBlocksPerSm>)
+                            : (ka.swap_mask ? finish_kernel<kLegacy, true, kWindowBlocksPerSm>
+                                            : finish_kernel<kLegacy, false, kWindowBlocksPerSm>);
         MMS_TRY(allow_smem((const void *)walk_k, g.smem_window));
         MMS_TRY(allow_smem((const void *)finish_k, g.smem_window));
         const int64_t bounds = (int64_t)ka.B * (ka.K - 1);

@@ -267,7 +267,8 @@ def test_naming_at_the_ends_of_its_stretches(n, groups):
 @pytest.mark.parametrize("n,copies", [(1025, 1184), (1025, 1185), (513, 2369), (3329, 365)])
 def test_naming_of_long_lists(n, copies):
     """Up to 9 472 segments in a call each is translated by a warp of its own, beyond that eight by
-    one: both sides of the line, and stretches that end short of eight segments."""
+    one: both sides of the line, and stretches that end short of eight segments.  (1 184 candidates
+    are also the last that the last pass takes with two blocks per SM.)"""
     from mms_b200 import engine
     from oracle import tables
     M, groups = 6, 12
