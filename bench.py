@@ -751,7 +751,7 @@ def run_batching(args, D, candidates=1024, duration=3600.0, steps=None, cpu=True
         return None
     peak, which = hbm_peak()
     k_ms = float(np.mean(stream_ms)) if len(stream_ms) else float("nan")
-    dominant, dom_ms = "batch_simd_kernel" if B >= 24 else "batch_stream_kernel", k_ms
+    dominant, dom_ms = "batch_stream_kernel", k_ms
     if len(chain_ms) and float(np.mean(chain_ms)) > k_ms:
         dominant, dom_ms = "batch_chain_kernel", float(np.mean(chain_ms))
     achieved = B * N * BYTES_PER_UNIT_FULL / (dom_ms * 1e-3) / 1e9
@@ -774,7 +774,8 @@ def run_batching(args, D, candidates=1024, duration=3600.0, steps=None, cpu=True
                 "d2h_bytes_per_step": int(d2h)},
         # cut-or-not, tables, stream, three rounds of validate and repair, validate, chain, counters,
         # leaf sums, totals; the tables only where 32 candidates go to a warp
-        "gpu_launches": (14 if B >= 24 else 13) * steps,
+        # (short chunks, of few placements, get a round of walks)
+        "gpu_launches": (8 if B > 26 else 10) * steps,
         "chunks_resimulated_per_candidate": float(np.mean(res.resimulated)),
         "clocks": clk.summary(),
     }

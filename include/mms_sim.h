@@ -338,7 +338,8 @@ typedef struct {
 
 /* next_same[i] = index of the next request with request i's model, or -1:
  * the per-model FIFO queues of controller.py:648 are runs of this list.
- * next_same: i32[N], filled once per trace. */
+ * next_same: i32[N].  mms_sim_batching accepts it (or NULL) and does not need it: it sorts
+ * the trace by model itself. */
 int mms_trace_next_same_model(const mms_trace *trace, int32_t num_models, int32_t *next_same,
                               void *stream);
 
@@ -348,7 +349,7 @@ size_t mms_sim_batching_workspace_bytes(int64_t num_requests, const mms_placemen
 
 /* The trace is cut in time like in mms_sim_mixed (speculative chunks, then an
  * exact chain pass), so results do not depend on the cut; out->resimulated,
- * when not NULL, gets the number of chunks the chain pass re-simulated. */
+ * when not NULL, gets the number of stretches that were simulated again. */
 
 int mms_sim_batching(const mms_trace *trace, const mms_placements *cands,
                      const mms_batching *batching, const int32_t *next_same,

@@ -16,6 +16,8 @@ HEADERS = [os.path.join(REPO_DIR, "include", "mms_sim.h"),
            os.path.join(PKG_DIR, "csrc", "sim_chunk.cuh"),
            os.path.join(PKG_DIR, "csrc", "sim_window.cuh"),
            os.path.join(PKG_DIR, "csrc", "sim_batching.cuh"),
+           os.path.join(PKG_DIR, "csrc", "batch_lists.cuh"),
+           os.path.join(PKG_DIR, "csrc", "batch_groups.cuh"),
            os.path.join(PKG_DIR, "csrc", "mms_abi.inl")]
 
 NVCC_FLAGS = [
@@ -24,6 +26,7 @@ NVCC_FLAGS = [
     # time arithmetic must keep the reference's operation order
     "-fmad=false", "-prec-div=true", "-prec-sqrt=true",
     "-Xcompiler", "-fPIC", "-shared",
+    "--split-compile=0",          # the kernels side by side on the host's cores
 ]
 
 

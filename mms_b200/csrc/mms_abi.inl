@@ -808,75 +808,142 @@ int mms_trace_next_same_model(const mms_trace *trace, int32_t num_models, int32_
 namespace mms {
 
 struct BatchGeometry {
-    int32_t simd, H, K, chunk_len, warmup, Bp;
-    size_t smem_single, smem_simd;
-    size_t off_leaf, off_start, off_end, off_counters, off_carry, off_flag, off_tables, off_work,
+    int32_t per_lane;         // groups per lane of the kernels with a group per lane; 0: lists
+    int32_t H, event_rows, K, NS, seg_len, seg_per_chunk, warmup, table_elems, warps, blocks;
+    bool lean;
+    int32_t list_elems, list_warps, list_blocks;      // the list kernels beside the others
+    size_t list_smem;
+    size_t smem, smem_judge, state_bytes;
+    size_t off_leaf, off_start, off_end, off_carry, off_carry_n, off_carry_seg, off_walk_carry,
+        off_run_status, off_perm, off_tie, off_swaps, off_swap_n, off_walk_swaps, off_counts, off_flag, off_work, off_items, off_marks, off_first, off_pos, off_req, off_ts, off_dl,
         total;
     int32_t rounds;
 };
 
-constexpr int kBatchRepairRounds = 3;
+constexpr size_t kBatchSnapshotBytes = 256u << 20;
 
 // Chunking and scratch layout of one mms_sim_batching call.
 static int plan_batching(int64_t N, const mms_placements *c, const mms_batching *bt,
                          BatchGeometry *g)
 {
+    *g = BatchGeometry();
     if (!c || !bt || N < 0 || N > 0x7FFFFFFF || c->num_candidates < 0) return MMS_ERR_ARG;
     const int64_t B = c->num_candidates;
     g->H = bt->heap_capacity > 0 ? bt->heap_capacity : c->max_groups + 16;
-    // 32 candidates per warp (batch_simd_kernel) once there are enough of them to fill
-    // warps; else one candidate per warp
-    g->simd = B >= 24 ? 1 : 0;
-    g->Bp = (int32_t)((B + kLanes - 1) / kLanes * kLanes);
-    g->smem_single = batch_smem(c->num_models, c->max_groups, c->max_placed, c->max_slots,
-                                g->H, 1).total;
-    g->smem_simd = batch_smem(c->num_models, c->max_groups, c->max_placed, c->max_slots,
-                              g->H, kLanes).total;
-    if (g->smem_simd > 227 * 1024) g->simd = 0;
+    g->event_rows = (g->H + kLanes - 1) / kLanes;
+    g->state_bytes = batch_state_bytes(c->num_models, c->max_slots, g->event_rows);
     int sm_count = 148, dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess ||
         cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
         (void)cudaGetLastError();
         sm_count = 148;
     }
-    // Run-in as in plan_call; chunks: as many as fill ONE wave of the blocks that can be
-    // resident (shared memory decides), none shorter than half the run-in, and no cut at all
-    // when that leaves fewer than two.
+    // Shared memory: the latency table on chip where it takes little of it; the candidate's tables
+    // too, unless they would not fit; as many warps to a block as fit.
+    const size_t table = (size_t)c->num_models * c->num_columns * c->max_stages * bt->num_batch_sizes;
+    const auto layout = [&](int32_t elems, int warps) {
+        if (g->per_lane)
+            return ((sizeof(double) * (size_t)elems + 15) & ~(size_t)15) +
+                   warps * group_smem(c->num_models, c->max_slots, g->H).bytes;
+        return batch_smem(c->num_models, c->max_groups, c->max_placed, c->max_slots, g->event_rows, elems,
+                          g->lean, warps).total;
+    };
+    // A group per lane where groups and models fit masks, the table as doubles fits beside the
+    // warps, and more events than groups may be pending; else lists, with the candidate's tables
+    // on chip unless they would not fit.
+    const auto list_plan = [&]() {
+        g->per_lane = 0;
+        g->table_elems = c->latency_stride == 0 && table * sizeof(float) <= 2 * (size_t)kLatSmemBytes ? (int32_t)table : 0;
+        g->lean = false;
+        g->lean = layout(0, 1) > 227 * 1024;
+        if (g->lean && layout(0, 1) > 227 * 1024) return false;
+        if (layout(g->table_elems, 1) > 227 * 1024) g->table_elems = 0;
+        g->warps = kBatchWarps;
+        while (g->warps > 1 && layout(g->table_elems, g->warps) > 227 * 1024) --g->warps;
+        g->smem = layout(g->table_elems, g->warps);
+        return true;
+    };
+    if (!list_plan()) return MMS_ERR_UNSUPPORTED;
+    g->list_elems = g->table_elems; g->list_warps = g->warps; g->list_smem = g->smem;
+    int64_t per_sm = 1;
+    const auto resident = [&]() {
+        per_sm = (int64_t)(233472 / (g->smem + 1024));
+        const int64_t most = (kBatchWarps * kBatchBlocksPerSm) / g->warps;     // registers
+        if (per_sm > most) per_sm = most;
+        if (per_sm < 1) per_sm = 1;
+        g->blocks = (int32_t)(per_sm * sm_count);
+    };
+    resident();
+    g->list_blocks = g->blocks;
+    if (c->max_groups <= kGroupLimit && c->num_models <= kGroupLimit && g->H >= c->max_groups &&
+        c->latency_stride == 0 && table > 0 && table * sizeof(double) <= 3 * (size_t)kLatSmemBytes) {
+        g->per_lane = c->max_groups <= kLanes ? 1 : 2;
+        g->table_elems = (int32_t)table + kBatchDepth * bt->num_batch_sizes;
+        g->warps = kBatchWarps;
+        g->event_rows = g->per_lane + (g->H + kLanes - 1) / kLanes;
+        g->smem = layout(g->table_elems, g->warps);
+        if (g->smem <= 227 * 1024) resident();
+        else if (list_plan()) { g->event_rows = (g->H + kLanes - 1) / kLanes; resident(); }
+    }
+    g->state_bytes = batch_state_bytes(c->num_models, c->max_slots, g->event_rows);
+    g->smem_judge = layout(0, g->warps);
+    // Run-in as in plan_call; as many chunks as there are resident warps, none shorter than half
+    // the run-in (one placement on 16 devices, 27 000 requests, two traces, speculative pass and repairs:
+    // chunks of 128 0.80 + 2.5 and 0.61 + 0.1 ms, 256 0.93 + 1.1 and 0.71 + 0.1, 512 1.31 + 0.9 and 1.04 +
+    // 0.04), and no cut at all when that leaves fewer than two.
     int64_t warm = 32 * (int64_t)c->max_slots;
     if (warm < 128) warm = 128;
     if (warm > 2048) warm = 2048;
     g->warmup = (int32_t)warm;
-    const int64_t min_chunk = warm / 2 > 256 ? warm / 2 : 256;
-    int64_t K = 1;
-    if (B > 0 && N >= 4 * min_chunk) {
-        const size_t smem = g->simd ? g->smem_simd : g->smem_single;
-        int64_t per_sm = (int64_t)(233472 / (smem + 1024));
-        if (per_sm > kBatchBlocksPerSm) per_sm = kBatchBlocksPerSm;
-        if (per_sm < 1) per_sm = 1;
-        const int64_t blocks_per_chunk = g->simd ? g->Bp / kLanes : B;
-        K = per_sm * sm_count / blocks_per_chunk;
-        if (K > N / min_chunk) K = N / min_chunk;
-        if (K < 2) K = 1;
+    int64_t seg = 128;
+    while (seg < N && (size_t)(N / seg) * (size_t)B * g->state_bytes > kBatchSnapshotBytes) seg *= 2;
+    int64_t NS = N / seg > 0 ? N / seg : 1, spc = NS;
+    if (B > 0 && N >= 1024) {
+        const int64_t K = (int64_t)g->blocks * g->warps / B, least = (warm / 2 + seg - 1) / seg;
+        if (K >= 2) spc = (NS + K - 1) / K;
+        if (spc < least) spc = least;
+        if (spc > NS) spc = NS;
     }
-    const int64_t len = (N + K - 1) / (K > 0 ? K : 1);
-    g->chunk_len = (int32_t)(len > 0 ? len : 1);
-    g->K = (int32_t)(N > 0 ? (N + g->chunk_len - 1) / g->chunk_len : 1);
-    const size_t cells = (size_t)g->K * (size_t)(B > 0 ? B : 1);
-    const size_t sb = batch_state_bytes(c->num_models, c->max_groups, c->max_slots, g->H);
+    g->K = (int32_t)((NS + spc - 1) / spc);
+    g->seg_len = (int32_t)seg;
+    g->NS = (int32_t)NS;
+    g->seg_per_chunk = (int32_t)spc;
+    const size_t b = (size_t)(B > 0 ? B : 1), cells = (size_t)g->K * b, segs = (size_t)NS * b;
+    if (cells >= 0x7FFFFFFF) return MMS_ERR_UNSUPPORTED;
     size_t off = 0;
-    g->off_leaf = off;     off += align256(sizeof(double) * (size_t)plan_leaves(N) * (size_t)B + 8);
-    g->off_flag = off;     off += 256;
-    g->off_counters = off; off += align256(sizeof(uint32_t) * cells * (2 * c->num_models + 2 * c->max_groups));
-    g->off_carry = off;    off += align256(cells * batch_carry_bytes());
-    g->off_tables = off;
-    if (g->simd)           // t_mrep, t_gcfg, t_status (u32), then t_moff, t_goff, t_gmod (u16)
-        off += align256((size_t)g->Bp * (4 * ((size_t)c->max_placed + c->max_groups + 1) +
-                                          2 * ((size_t)c->num_models + c->max_groups + 2 +
-                                               c->max_placed)) + 64);
-    g->rounds = kBatchRepairRounds;
-    g->off_work = off;     off += g->K > 1 ? align256(sizeof(uint32_t) * (cells + 64) + cells) : 0;
-    g->off_start = off;    off += g->K > 1 ? align256(cells * sb) : 0;
-    g->off_end = off;      off += g->K > 1 ? align256(cells * sb) : 0;
+    const auto take = [&](size_t bytes) { const size_t at = off; off += align256(bytes + 8); return at; };
+    g->off_leaf = take(sizeof(double) * (size_t)plan_leaves(N) * b);
+    g->off_flag = take(256);
+    g->off_first = take(sizeof(int32_t) * ((size_t)c->num_models + 1));
+    g->off_pos = take(sizeof(int32_t) * (size_t)N);
+    g->off_req = take(sizeof(int32_t) * (size_t)N);
+    g->off_ts = take(sizeof(double) * (size_t)N);
+    g->off_dl = take(sizeof(double) * (size_t)N);
+    g->off_counts = take(2 * sizeof(uint32_t) * segs * c->max_groups);
+    // A round of walks beside each other takes as long as a chunk: it pays where chunks are short
+    // (the trace of above, chunks of 128: 0.34 + 1.5 instead of 2.1 ms), not where the chain has
+    // little to do (256 placements on 64 devices, 45 000 requests, chunks of 5 000: 4.6 + 1.8
+    // instead of 1.8 ms; with twice as many chunks 12.3 -> 16).
+    g->rounds = g->seg_per_chunk * g->seg_len <= g->warmup ? 1 : 0;
+    if (g->K > 1) {
+        g->off_start = take(cells * g->state_bytes);
+        g->off_end = take(segs * g->state_bytes);
+        g->off_carry = take(cells * sizeof(Carried) * kMaxCarry);
+        g->off_carry_n = take(cells * sizeof(uint32_t));
+        g->off_carry_seg = take(segs);
+        g->off_walk_carry = take((size_t)g->blocks * g->warps * sizeof(Carried) * kMaxCarry);
+        g->off_run_status = take(cells * sizeof(uint32_t));
+        if (g->per_lane) {
+            g->off_perm = take(cells * kGroupLimit);
+            g->off_tie = take(segs * sizeof(uint64_t));
+            g->off_swaps = take(cells * sizeof(Swap) * kSwapCap);
+            g->off_swap_n = take(cells * sizeof(uint32_t));
+            g->off_walk_swaps = take((size_t)g->blocks * g->warps * sizeof(Swap) * kSwapCap);
+        }
+        g->off_work = take(2 * sizeof(uint32_t) * (size_t)(g->rounds + 1));
+        g->off_items = take(cells * sizeof(uint32_t));
+        g->off_marks = take(2 * cells);
+    }
     g->total = off;
     return MMS_OK;
 }
@@ -917,8 +984,8 @@ int mms_sim_batching(const mms_trace *trace, const mms_placements *cands,
     if (!out->model_num_requests || !out->model_num_good || !out->group_num_requests ||
         !out->group_num_good || !out->good_total || !out->latency_sum || !out->status)
         return MMS_ERR_ARG;
-    if (N > 0 && (!trace->arrivals || !trace->model_ids || !trace->slos || !next_same ||
-                  !out->finish || !out->good))
+    (void)next_same;                       // accepted and not needed any more
+    if (N > 0 && (!trace->arrivals || !trace->model_ids || !trace->slos || !out->finish || !out->good))
         return MMS_ERR_ARG;
     if (!cands->model_off || !cands->model_rep || !cands->latency || !batching->group_off ||
         !batching->group_mod || !batching->group_cfg)
@@ -926,16 +993,19 @@ int mms_sim_batching(const mms_trace *trace, const mms_placements *cands,
     if (plan->num_leaves != plan_leaves(N)) return MMS_ERR_ARG;
     if (plan->num_leaves > 0 && (!plan->leaf_start || !plan->leaf_merges)) return MMS_ERR_ARG;
     BatchGeometry geo;
-    if (plan_batching(N, cands, batching, &geo) != MMS_OK) return MMS_ERR_ARG;
+    {
+        const int rc = plan_batching(N, cands, batching, &geo);
+        if (rc != MMS_OK) return rc;
+    }
     if (!ws->ptr || ws->bytes < geo.total) return MMS_ERR_ARG;
 
     BatchArgs a;
     memset(&a, 0, sizeof(a));
     a.arrivals = trace->arrivals; a.model_ids = trace->model_ids; a.slos = trace->slos;
-    a.next_same = next_same; a.N = N;
+    a.N = N;
     a.B = B; a.M = cands->num_models; a.G = cands->max_groups; a.P = cands->max_placed;
     a.T = cands->max_slots; a.S = cands->max_stages; a.C = cands->num_columns; a.NB = NB;
-    a.H = geo.H;
+    a.H = geo.H; a.event_rows = geo.event_rows;
     for (int j = 0; j < NB; ++j) {
         const int32_t bs = batching->batch_sizes[j];
         if (bs < 1 || (bs & (bs - 1)) || (j > 0 && bs <= batching->batch_sizes[j - 1]))
@@ -950,102 +1020,137 @@ int mms_sim_batching(const mms_trace *trace, const mms_placements *cands,
     a.group_off = batching->group_off; a.group_mod = batching->group_mod;
     a.group_cfg = batching->group_cfg;
     a.latency = cands->latency; a.latency_stride = cands->latency_stride;
+    a.table_elems = geo.table_elems;
+    a.at = group_smem(a.M, a.T, a.H);
+    a.warp0 = (uint32_t)((sizeof(double) * (size_t)a.table_elems + 15) & ~(size_t)15);
+    a.warp_bytes = (uint32_t)a.at.bytes;
     a.finish = out->finish; a.good = out->good;
-    a.model_num_requests = out->model_num_requests; a.model_num_good = out->model_num_good;
-    a.group_num_requests = out->group_num_requests; a.group_num_good = out->group_num_good;
     a.status = out->status;
-    a.lanes = geo.simd ? kLanes : 1;
-    if (geo.smem_single > 227 * 1024) return MMS_ERR_UNSUPPORTED;
-    unsigned char *scratch = (unsigned char *)ws->ptr;
-    a.K = geo.K; a.chunk_len = geo.chunk_len; a.warmup = geo.warmup;
-    a.unsorted = (const int32_t *)(scratch + geo.off_flag);
-    a.chunk_counters = (uint32_t *)(scratch + geo.off_counters);
-    a.carry = scratch + geo.off_carry;
-    a.snap_start = scratch + geo.off_start;
-    a.snap_end = scratch + geo.off_end;
     a.resimulated = out->resimulated;
-    a.Bp = geo.Bp;
-    if (geo.simd) {
-        const size_t Bp = (size_t)geo.Bp;
-        unsigned char *t = scratch + geo.off_tables;
-        a.t_mrep = (uint32_t *)t;   t += 4 * Bp * (size_t)a.P;
-        a.t_gcfg = (uint32_t *)t;   t += 4 * Bp * (size_t)a.G;
-        a.t_status = (uint32_t *)t; t += 4 * Bp;
-        a.t_moff = (uint16_t *)t;   t += 2 * Bp * (size_t)(a.M + 1);
-        a.t_goff = (uint16_t *)t;   t += 2 * Bp * (size_t)(a.G + 1);
-        a.t_gmod = (uint16_t *)t;
+    unsigned char *scratch = (unsigned char *)ws->ptr;
+    a.K = geo.K; a.NS = geo.NS; a.seg_len = geo.seg_len; a.seg_per_chunk = geo.seg_per_chunk;
+    a.warmup = geo.warmup; a.state_bytes = geo.state_bytes; a.rounds = geo.rounds;
+    a.odd = (const int32_t *)(scratch + geo.off_flag);
+    a.first_of = (int32_t *)(scratch + geo.off_first);
+    a.pos = (int32_t *)(scratch + geo.off_pos);
+    a.req = (int32_t *)(scratch + geo.off_req);
+    a.pos_ts = (double *)(scratch + geo.off_ts);
+    a.pos_dl = (double *)(scratch + geo.off_dl);
+    a.seg_counts = (uint32_t *)(scratch + geo.off_counts);
+    if (a.K > 1) {
+        a.chunk_start = scratch + geo.off_start;
+        a.seg_end = scratch + geo.off_end;
+        a.carry = (Carried *)(scratch + geo.off_carry);
+        a.carry_n = (uint32_t *)(scratch + geo.off_carry_n);
+        a.carry_seg = scratch + geo.off_carry_seg;
+        a.walk_carry = (Carried *)(scratch + geo.off_walk_carry);
+        a.run_status = (uint32_t *)(scratch + geo.off_run_status);
+        a.perm = scratch + geo.off_perm;
+        a.tie = (uint64_t *)(scratch + geo.off_tie);
+        if (geo.per_lane) {
+            a.swaps = (Swap *)(scratch + geo.off_swaps);
+            a.swap_n = (uint32_t *)(scratch + geo.off_swap_n);
+            a.walk_swaps = (Swap *)(scratch + geo.off_walk_swaps);
+        }
+        a.work_count = (uint32_t *)(scratch + geo.off_work);
+        a.work_next = a.work_count + a.rounds + 1;
+        a.work_items = (uint32_t *)(scratch + geo.off_items);
+        a.link = scratch + geo.off_marks;
+        a.stamp = a.link + (size_t)a.K * B;
     }
 
     cudaStream_t st = (cudaStream_t)stream;
+    const unsigned threads = (unsigned)(geo.warps * kLanes);
+    const auto blocks_for = [&](int64_t warps, bool resident) {
+        const int64_t blocks = (warps + geo.warps - 1) / geo.warps;
+        return (unsigned)(resident && blocks > geo.blocks ? geo.blocks : blocks);
+    };
     MMS_CUDA(cudaMemsetAsync(scratch + geo.off_flag, 0, 256, st));
-    MMS_CUDA(cudaMemsetAsync(out->status, 0, sizeof(uint32_t) * (size_t)B, st));
-    if (out->resimulated)
-        MMS_CUDA(cudaMemsetAsync(out->resimulated, 0, sizeof(int32_t) * (size_t)B, st));
+    {
+        BatchClear c;
+        c.odd = (int32_t *)(scratch + geo.off_flag);
+        c.model_num_good = out->model_num_good;
+        int64_t cells = N > (int64_t)a.K * B ? N : (int64_t)a.K * B;
+        if ((int64_t)B * a.M > cells) cells = (int64_t)B * a.M;
+        int64_t blocks = (cells + kOrderWarps * kLanes - 1) / (kOrderWarps * kLanes);
+        if (blocks > 148) blocks = 148;
+        batch_order_kernel<<<(unsigned)(a.M + blocks), kOrderWarps * kLanes, 0, st>>>(a, c);
+        MMS_CUDA(cudaGetLastError());
+    }
+    struct Kernels { void (*stream)(BatchArgs), (*judge)(BatchArgs), (*walk)(BatchArgs), (*chain)(BatchArgs); };
+#define MMS_BATCH_KERNELS(W) \
+    Kernels{batch_stream_kernel<W>, batch_validate_kernel<W>, batch_walk_kernel<W>, batch_chain_kernel<W>}
+    const Kernels lists = geo.lean ? MMS_BATCH_KERNELS(ListWarp<true>) : MMS_BATCH_KERNELS(ListWarp<false>);
+    const Kernels kern = geo.per_lane == 1 ? MMS_BATCH_KERNELS(GroupWarp<1>)
+                         : geo.per_lane == 2 ? MMS_BATCH_KERNELS(GroupWarp<2>) : lists;
+#undef MMS_BATCH_KERNELS
+    if (N > 0) {
+        ProfileSpan stream_span(MMS_PROFILE_BATCH_STREAM, st);
+        MMS_TRY(allow_smem((const void *)kern.stream, geo.smem));
+        kern.stream<<<blocks_for((int64_t)B * a.K, true), threads, geo.smem, st>>>(a);
+        MMS_CUDA(cudaGetLastError());
+        if (geo.per_lane) {                // ... and where the trace is odd
+            BatchArgs odd = a;
+            odd.table_elems = geo.list_elems;
+            odd.event_rows = (geo.H + kLanes - 1) / kLanes;
+            odd.only_odd = true;
+            MMS_TRY(allow_smem((const void *)lists.stream, geo.list_smem));
+            const int64_t blocks = (B + geo.list_warps - 1) / geo.list_warps;
+            lists.stream<<<(unsigned)(blocks < geo.list_blocks ? blocks : geo.list_blocks),
+                           (unsigned)(geo.list_warps * kLanes), geo.list_smem, st>>>(odd);
+            MMS_CUDA(cudaGetLastError());
+        }
+        stream_span.stop();
+    }
     if (N > 0 && a.K > 1) {
-        uncuttable_kernel<<<296, 256, 0, st>>>(a, (int32_t *)(scratch + geo.off_flag));
-        MMS_CUDA(cudaGetLastError());
-    }
-    MMS_TRY(allow_smem((const void *)batch_chain_kernel, geo.smem_single));
-    if (geo.simd) {
-        // the lanes add to the chunks' counters in global memory
-        MMS_CUDA(cudaMemsetAsync(a.chunk_counters, 0,
-                                 sizeof(uint32_t) * (size_t)a.K * B * (2 * a.M + 2 * a.G), st));
-        batch_tables_kernel<<<(unsigned)((geo.Bp + 127) / 128), 128, 0, st>>>(a);
-        MMS_CUDA(cudaGetLastError());
-        MMS_TRY(allow_smem((const void *)batch_simd_kernel, geo.smem_simd));
-        ProfileSpan stream_span(MMS_PROFILE_BATCH_STREAM, st);
-        batch_simd_kernel<<<(unsigned)((int64_t)a.K * (geo.Bp / kLanes)), kLanes, geo.smem_simd,
-                            st>>>(a);
-        MMS_CUDA(cudaGetLastError());
-        stream_span.stop();
-    } else {
-        MMS_TRY(allow_smem((const void *)batch_stream_kernel, geo.smem_single));
-        ProfileSpan stream_span(MMS_PROFILE_BATCH_STREAM, st);
-        batch_stream_kernel<<<(unsigned)((int64_t)B * a.K), kLanes, geo.smem_single, st>>>(a);
-        MMS_CUDA(cudaGetLastError());
-        stream_span.stop();
-    }
-    if (a.K > 1) {
-        // a few rounds of parallel repairs, one re-simulated chunk per warp, then the chain
-        a.work_count = (uint32_t *)(scratch + geo.off_work);
-        a.work_items = a.work_count + 64;
-        a.link = (uint8_t *)(a.work_items + (size_t)a.K * B);
-        MMS_CUDA(cudaMemsetAsync(a.work_count, 0, sizeof(uint32_t) * 64, st));
-        MMS_TRY(allow_smem((const void *)batch_repair_kernel, geo.smem_single));
+        MMS_TRY(allow_smem((const void *)kern.judge, geo.smem_judge));
+        MMS_TRY(allow_smem((const void *)kern.walk, geo.smem));
+        MMS_TRY(allow_smem((const void *)kern.chain, geo.smem));
         const int64_t bounds = (int64_t)B * (a.K - 1);
         ProfileSpan repair_span(MMS_PROFILE_BATCH_REPAIR, st);
-        a.rounds = geo.rounds;
-        for (int r = 0; r <= geo.rounds; ++r) {
+        // round a.rounds only judges the boundaries, for batch_chain_kernel
+        for (int r = 0; r <= a.rounds; ++r) {
             a.round = r;
-            batch_validate_kernel<<<(unsigned)((bounds + 127) / 128), 128, 0, st>>>(a);
+            BatchArgs judge = a;
+            judge.table_elems = 0;
+            judge.warp0 = 0;
+            kern.judge<<<blocks_for(bounds, false), threads, geo.smem_judge, st>>>(judge);
             MMS_CUDA(cudaGetLastError());
-            if (r == geo.rounds) break;
-            batch_repair_kernel<<<(unsigned)bounds, kLanes, geo.smem_single, st>>>(a);
+            if (r == a.rounds) break;
+            kern.walk<<<blocks_for(bounds, true), threads, geo.smem, st>>>(a);
             MMS_CUDA(cudaGetLastError());
         }
         repair_span.stop();
         ProfileSpan chain_span(MMS_PROFILE_BATCH_CHAIN, st);
-        batch_chain_kernel<<<(unsigned)B, kLanes, geo.smem_single, st>>>(a);
+        kern.chain<<<blocks_for(B, false), threads, geo.smem, st>>>(a);
         MMS_CUDA(cudaGetLastError());
         chain_span.stop();
     }
-    const int64_t sum_cells = (int64_t)B * (2 * a.M + 2 * a.G);
-    batch_sum_kernel<<<(unsigned)((sum_cells + 127) / 128), 128, 0, st>>>(a);
-    MMS_CUDA(cudaGetLastError());
     double *leaf_sums = (double *)(scratch + geo.off_leaf);
     if (plan->num_leaves > 0) {
-        const int64_t cells = (int64_t)B * plan->num_leaves;
-        leaf_sums_from_finish_kernel<<<(unsigned)((cells + 127) / 128), 128, 0, st>>>(
-            out->finish, trace->arrivals, N, B, plan->num_leaves, plan->leaf_start, leaf_sums);
+        const int64_t slices = (plan->num_leaves + kTallyLeaves - 1) / kTallyLeaves;
+        const size_t bytes = sizeof(uint32_t) * (size_t)a.M;
+        if (bytes > 227 * 1024 || slices * B > 0x7FFFFFFF) return MMS_ERR_UNSUPPORTED;
+        MMS_TRY(allow_smem((const void *)batch_tally_kernel, bytes));
+        batch_tally_kernel<<<(unsigned)(slices * B), kTallyThreads, bytes, st>>>(
+            a, plan->num_leaves, plan->leaf_start, out->model_num_good, leaf_sums);
+        MMS_CUDA(cudaGetLastError());
+    }
+    if (a.G > 0) {
+        if (N == 0) a.NS = 0;              // nothing was simulated
+        const int64_t warps = (int64_t)B * ((2 * a.G + kLanes - 1) / kLanes);
+        batch_count_kernel<<<(unsigned)((warps + 3) / 4), 4 * kLanes, 0, st>>>(
+            a, out->group_num_requests, out->group_num_good);
         MMS_CUDA(cudaGetLastError());
     }
     KernelArgs fa;                         // what finalize_kernel reads; one run per candidate
     memset(&fa, 0, sizeof(fa));
     fa.B = B; fa.M = a.M; fa.num_leaves = plan->num_leaves; fa.N = N;
-    fa.leaf_start = plan->leaf_start;
+    fa.leaf_start = plan->leaf_start; fa.model_off = a.model_off;
     fa.leaf_sums = leaf_sums; fa.status = out->status;
     finalize_kernel<<<(B + 3) / 4, 4 * kLanes, 0, st>>>(
-        fa, plan->leaf_merges, out->model_num_good, out->good_total, out->latency_sum);
+        fa, plan->leaf_merges, a.first_of, out->model_num_good, out->model_num_requests,
+        out->good_total, out->latency_sum);
     MMS_CUDA(cudaGetLastError());
     return MMS_OK;
 }

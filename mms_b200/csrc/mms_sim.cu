@@ -933,17 +933,22 @@ __device__ inline void sum_leaves(const KernelArgs &a, int64_t b, const uint8_t 
     if (lane == 0) latency_sum[b] = v;
 }
 
-// One warp per candidate: the latency sum, and the total of the good
-// requests (controller.py:401) from the per-model counts.
-__global__ void finalize_kernel(const KernelArgs a, const uint8_t *leaf_merges,
-                                const int32_t *model_num_good, int64_t *good_total,
-                                double *latency_sum)
+// The batching simulator's reductions, one warp per candidate: the latency sum, the total
+// of the good requests (controller.py:401) from the per-model counts, and the requests of each
+// model that has a replica.
+__global__ void finalize_kernel(const KernelArgs a, const uint8_t *leaf_merges, const int32_t *first_of,
+                                const int32_t *model_num_good, int32_t *model_num_requests,
+                                int64_t *good_total, double *latency_sum)
 {
     const int64_t b = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / kLanes;
     if (b >= a.B) return;
     sum_leaves(a, b, leaf_merges, latency_sum);
     int32_t total = 0;
-    for (int m = threadIdx.x & (kLanes - 1); m < a.M; m += kLanes) total += model_num_good[(size_t)b * a.M + m];
+    const uint16_t *off = a.model_off + (size_t)b * (a.M + 1);
+    for (int m = threadIdx.x & (kLanes - 1); m < a.M; m += kLanes) {
+        total += model_num_good[(size_t)b * a.M + m];
+        model_num_requests[(size_t)b * a.M + m] = a.N > 0 && off[m + 1] > off[m] ? first_of[m + 1] - first_of[m] : 0;
+    }
     total = __reduce_add_sync(0xFFFFFFFFu, total);
     if ((threadIdx.x & (kLanes - 1)) == 0) good_total[b] = total;
 }

@@ -1430,7 +1430,6 @@ class ResidentBatching:
                                    at["group_num_requests"], at["group_num_good"],
                                    at["good_total"], at["latency_sum"], at["status"], _ptr(o_fin),
                                    _ptr(o_good), at["resimulated"])
-            self.next_same = trace.next_same_model()
         self.keep = (d_off, d_rep, d_goff, d_gmod, d_gcfg, d_lat, ws_t)
         self.rows = (o_fin, o_good)
 
@@ -1439,7 +1438,7 @@ class ResidentBatching:
         with _on(trace.device):
             tr, plan = trace.c_trace(), trace.c_plan()
             rc = nat.lib().mms_sim_batching(ctypes.byref(tr), ctypes.byref(self.cands),
-                                            ctypes.byref(self.bat), _ptr(self.next_same),
+                                            ctypes.byref(self.bat), None,
                                             ctypes.byref(plan), ctypes.byref(self.ws),
                                             ctypes.byref(self.res), _stream_ptr())
             nat.check(rc, "mms_sim_batching")
