@@ -26,7 +26,6 @@ NVCC_FLAGS = [
     # time arithmetic must keep the reference's operation order
     "-fmad=false", "-prec-div=true", "-prec-sqrt=true",
     "-Xcompiler", "-fPIC", "-shared",
-    "--split-compile=0",          # the kernels side by side on the host's cores
 ]
 
 
