@@ -46,7 +46,7 @@ struct Geometry {
     size_t off_leaf, off_seg_end, off_chunk_start, off_decisions, off_work_count, off_work_items,
         off_rows, off_seg_leaf, off_group_info, off_columns, off_stamp, off_link, off_flags, off_rel,
         off_tie, off_swap_mask, off_swap_at, off_swap_count, off_name_from, off_perm, off_twin_class, off_group_column, off_group_models;
-    int32_t group_words, swap_cap;
+    int32_t group_words, swap_cap, row_planes;
     size_t smem_count;        // shared memory of count_kernel
     size_t total;
 };
@@ -73,6 +73,7 @@ static bool window_pays(int64_t N, int64_t B, int64_t K_wide, int64_t K_win, int
 // the price of speed (never of results): 1 = long segments and chunks, 2 = also no bookkeeping of
 // interchangeable groups, 3 = also few chunks.
 constexpr int kMaxThrift = 3;
+constexpr int kMaxRowReplicas = 64;      // of a model in the replica rows
 static int plan_call(int64_t N, const mms_placements *c, const mms_sim_options *opts,
                      uint32_t flags, bool group_good, int thrift, Geometry *g)
 {
@@ -237,8 +238,16 @@ static int plan_call(int64_t N, const mms_placements *c, const mms_sim_options *
     g->smem_count = sizeof(uint32_t) * (size_t)(c->max_groups + (c->num_models + 1) / 2) * kLanes;
     if (g->smem_count > 227 * 1024) return MMS_ERR_UNSUPPORTED;
     size_t off = 0;
-    g->off_rows = off;        off += align256(2 * sizeof(uint32_t) * kRowWords * (size_t)((B + kLanes - 1) / kLanes * kLanes) *
-                                               (c->num_models + 1) + 256);
+    // Replica rows: two of four, and for a model of more than eight replicas as many more as
+    // there can be, up to kMaxRowReplicas, with one that is not full and one to spare for reading ahead.
+    g->row_planes = 2;
+    if (!thrift && c->max_groups > 8 && c->max_placed > 8) {
+        const int32_t most = c->max_groups < c->max_placed ? c->max_groups : c->max_placed;
+        g->row_planes = 3 + (most < kMaxRowReplicas ? most : kMaxRowReplicas) / 4;
+    }
+    g->off_rows = off;
+    off += align256((g->row_planes + (g->row_planes > 2)) * sizeof(uint32_t) * kRowWords *
+                        (size_t)((B + kLanes - 1) / kLanes * kLanes) * (c->num_models + 1) + 256);
     g->off_leaf = off;        off += align256(sizeof(double) * (size_t)plan_leaves(N) * B);
     g->off_decisions = off;   off += align256((c->max_groups > 126 ? 2 : 1) * (size_t)((N + 3) / 4 * 4 + 4) *
                                                (size_t)((B + 31) / 32 * 32));
@@ -584,6 +593,7 @@ static int sim_mixed(const mms_trace *trace, const mms_placements *cands, const 
     ka.warmup = g.warmup;
     ka.num_leaves = plan->num_leaves; ka.leaf_start = plan->leaf_start;
     ka.rep_rows = (uint32_t *)(scratch + g.off_rows);
+    ka.row_planes = g.row_planes;
     ka.leaf_sums = (double *)(scratch + g.off_leaf);
     ka.decisions = scratch + g.off_decisions;
     ka.dec_wide = cands->max_groups > 126;

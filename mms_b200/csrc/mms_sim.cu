@@ -180,7 +180,19 @@ __global__ void build_tables_kernel(const KernelArgs a, const ClearArgs c)
                     if (r - lo < 8)
                         e[r - lo] = rep_to_last(ent);
                 }
-                if (hi - lo > 8) e[7] = kMoreReplicas;
+                if (hi - lo > 8) {
+                    // the eighth and those behind, four to a row, up to a row that is not full
+                    e[7] = kMoreReplicas;
+                    uint4 *more = reinterpret_cast<uint4 *>(a.rep_rows) + row_index(a, b, m);
+                    uint32_t r = lo + 7;
+                    for (int p = 2; p < a.row_planes && r <= hi && !bad; ++p, r += 4) {
+                        uint32_t x[4];
+                        for (uint32_t k = 0; k < 4; ++k)
+                            x[k] = r + k < hi ? rep_to_last(a.model_rep[(size_t)b * a.P + r + k]) : kNoReplica;
+                        if (p + 1 == a.row_planes && r + 4 <= hi) x[3] = kMoreReplicas;
+                        more[(size_t)p * row_plane(a)] = make_uint4(x[0], x[1], x[2], x[3]);
+                    }
+                }
             }
             if (bad) {
                 atomicOr(&a.status[b], MMS_STATUS_BAD_INDEX);
@@ -214,7 +226,9 @@ __device__ inline Lane setup_lane(const KernelArgs &a, int64_t b, int lane, int 
     ln.dec_pitch = (uint32_t)a.dec_pitch;
     ln.dec_word = 0;
     ln.rows = reinterpret_cast<const uint4 *>(a.rep_rows) + row_index(a, b, 0);
-    ln.rows_b = ln.rows + row_plane(a);
+    ln.plane = (uint32_t)row_plane(a);
+    ln.rows_b = ln.rows + ln.plane;
+    ln.rows_c = a.row_planes > 2 ? ln.rows_b + ln.plane : nullptr;
     ln.rep_raw = a.model_rep + (size_t)b * a.P;
     ln.rep_off = a.model_off + (size_t)b * (a.M + 1);
     ln.lat_gl = a.latency + (size_t)b * a.latency_stride;

@@ -95,8 +95,10 @@ struct Lane {
                               //   model's first four replicas, kNoReplica where it has fewer;
                               //   row M is empty (unknown models)
     const uint4 *rows_b;      // the same for replicas five to eight; a model with more than
-                              //   eight has kMoreReplicas in word 3 of this row (the full list
-                              //   is then read from the caller's tables)
+                              //   eight has kMoreReplicas in word 3 of this row, and its eighth and
+                              //   later ones in further rows, `plane` apart, the first of which is
+    const uint4 *rows_c;      //   here; the last one has kNoReplica at its end (kMoreReplicas, and
+    uint32_t plane;           //   rows_c null: not all are, the full list is in the caller's tables)
     const uint32_t *rep_raw;  // the caller's model_rep row of this candidate
     const uint16_t *rep_off;  // the caller's model_off row of this candidate
     const float *lat_gl;      // this candidate's table in global memory
@@ -205,6 +207,51 @@ __device__ __noinline__ Tie note_tie(const struct KernelArgs *args, int32_t b, i
                                      const uint32_t *list, int n, uint32_t clk, double best,
                                      uint32_t pick, double ts);
 
+// The choice of a model with more than eight replicas, behind the first seven (`best`, `pick`): the
+// further rows from `row` on, four replicas each, two rows in flight.  The model a cluster has most
+// replicas of gets most of the requests (in a layer of a search up to 30 in 64 groups), and while
+// the caller's list was read, a dependent load per replica, warps with such a lane stood still for
+// it.  With candidates of one depth side by side as well (EncodedBatch.by_depth) the speculative passes
+// of grown lists went from 3.4 to 2.3 ms (500 on 16 devices), 8.0 to 5.3 (1000 on 32), 14.6 to 9.3 (1000
+// on 64), 26.8 to 17.3 (a layer of 2343, the call 46.7 to 38.0); random lists the same.  Not
+// inlined, like note_tie.
+struct Choice { double best; uint32_t pick; bool tied; };
+
+__device__ __noinline__ Choice long_list(const uint4 *row, uint32_t plane, uint32_t clk, double best,
+                                         uint32_t pick, const uint32_t *list, int32_t n)
+{
+    Choice r = {best, pick, false};
+    bool whole = !row;
+    if (row) {
+        uint4 x = __ldg(row), y = __ldg(row + plane);     // (there is a plane to spare)
+        const auto consider = [&](uint32_t e) {
+            const double c = SM_F64(clk + rep_last(e) * kLanes);
+            if (e < kMoreReplicas && c == r.best) r.tied = true;
+            if (e < kMoreReplicas && c < r.best) { r.best = c; r.pick = e; r.tied = false; }
+        };
+        for (;;) {
+            const uint4 now = x;
+            x = y;
+            row += plane;
+            const bool last = now.w >= kMoreReplicas;
+            if (!last && x.w < kMoreReplicas) y = __ldg(row + plane);
+            consider(now.x); consider(now.y); consider(now.z); consider(now.w);
+            if (last) { whole = now.w == kMoreReplicas; break; }
+        }
+    }
+    if (whole) {                          // from the caller's tables
+        r.best = kInf;
+        r.pick = 0x00010000u;
+        for (int32_t k = 0; k < n; ++k) {
+            const uint32_t e = rep_to_last(__ldg(list + k));
+            const double c = SM_F64(clk + rep_last(e) * kLanes);
+            if (c == r.best) r.tied = true;
+            if (c < r.best) { r.best = c; r.pick = e; r.tied = false; }
+        }
+    }
+    return r;
+}
+
 // Executes request `i` (controller.py:579-622, or :519-555 with kLegacy) and
 // advances the pipe.  Returns finish - arrival, which is 0.0 for a dropped
 // request (the reference stores finish = arrival for those).
@@ -256,20 +303,46 @@ __device__ __forceinline__ double sim_step(Lane &ln, Pipe &p, int32_t i, bool re
         if (e5 < kMoreReplicas && c5 < best) { best = c5; pick = e5; }
         if (e6 < kMoreReplicas && c6 < best) { best = c6; pick = e6; }
         if (e7 < kMoreReplicas && c7 < best) { best = c7; pick = e7; }
-        tied = (c4 == best && pick != e4) || (e5 < kMoreReplicas && c5 == best && pick != e5) ||
-               (e6 < kMoreReplicas && c6 == best && pick != e6) ||
-               (e7 < kMoreReplicas && c7 == best && pick != e7);
-        if (e7 == kMoreReplicas) {        // rare: the whole list, from the caller's tables
-            const uint32_t lo = ln.rep_off[m], hi = ln.rep_off[m + 1];
-            best = kInf;
-            pick = 0x00010000u;
-            for (uint32_t r = lo; r < hi; ++r) {
-                const uint32_t e = rep_to_last(__ldg(ln.rep_raw + r));
-                const double c = SM_F64(ln.clk + rep_last(e) * kLanes);
-                if (c == best) tied = true;
-                if (c < best) { best = c; pick = e; tied = false; }
+        if (e7 == kMoreReplicas) {
+            if constexpr (kTwins) {
+                const Choice c = long_list(ln.rows_c ? ln.rows_c + m * kLanes : nullptr, ln.plane, ln.clk,
+                                           best, pick, ln.rep_raw + ln.rep_off[m],
+                                           ln.rep_off[m + 1] - ln.rep_off[m]);
+                best = c.best;
+                pick = c.pick;
+                tied = c.tied;
+            } else {                      // (a call of its own slows this form's other lanes by 4 %)
+                const uint4 *row = ln.rows_c + m * kLanes;
+                bool more = ln.rows_c != nullptr, whole = !more;
+                while (more) {
+                    const uint4 x = __ldg(row);
+                    row += ln.plane;
+                    const double d0 = SM_F64(ln.clk + rep_last(x.x) * kLanes);
+                    const double d1 = SM_F64(ln.clk + rep_last(x.y) * kLanes);
+                    const double d2 = SM_F64(ln.clk + rep_last(x.z) * kLanes);
+                    const double d3 = SM_F64(ln.clk + rep_last(x.w) * kLanes);
+                    if (x.x < kMoreReplicas && d0 < best) { best = d0; pick = x.x; }
+                    if (x.y < kMoreReplicas && d1 < best) { best = d1; pick = x.y; }
+                    if (x.z < kMoreReplicas && d2 < best) { best = d2; pick = x.z; }
+                    if (x.w < kMoreReplicas && d3 < best) { best = d3; pick = x.w; }
+                    more = x.w < kMoreReplicas;
+                    whole = x.w == kMoreReplicas;
+                }
+                if (whole) {
+                    best = kInf;
+                    pick = 0x00010000u;
+                    for (uint32_t r = ln.rep_off[m], hi = ln.rep_off[m + 1]; r < hi; ++r) {
+                        const uint32_t e = rep_to_last(__ldg(ln.rep_raw + r));
+                        const double c = SM_F64(ln.clk + rep_last(e) * kLanes);
+                        if (c < best) { best = c; pick = e; }
+                    }
+                }
             }
         }
+        if constexpr (kTwins)
+            tied |= (c4 == best && pick != e4) || (e5 < kMoreReplicas && c5 == best && pick != e5) ||
+                    (e6 < kMoreReplicas && c6 == best && pick != e6) ||
+                    (e7 < kMoreReplicas && c7 == best && pick != e7);
     }
     if constexpr (kTwins) {
         // several replicas with the smallest clock: the group number decided (see warp_relabel)

@@ -455,6 +455,7 @@ class EncodedBatch:
         # bool[B]: the placement has interchangeable groups at all (None: not known)
         self.has_twins = has_twins
         self._mirror_table = None         # see mirror_table()
+        self._depth = None                # u8[B], or 0: see by_depth()
 
     @property
     def twins(self):
@@ -476,8 +477,33 @@ class EncodedBatch:
             self._mirror_table = mirror_swaps_batch([classes for _, classes in (self.twins or [])])
         return self._mirror_table
 
+    def by_depth(self, index=None):
+        """`index` (None: all placements) ordered by the depth of their pipelines, in lists that mix
+        partitions of a cluster.  32 neighbours share a warp in large batches and wait for one
+        another: partitions into single devices have up to 30 replicas of a model to choose from,
+        those into eight none of that but long pipelines."""
+        count = self.B if index is None else len(index)
+        if count < MIN_BY_DEPTH or self.G == 0:
+            return index
+        if self._depth is None:
+            def stages(rows):             # the second byte of group_info; 0: no group
+                return rows.view(np.uint8).reshape(len(rows), -1, 4)[:, :, 1]
+
+            # worth it where most placements have pipelines of one depth, as those of a search
+            info = np.ascontiguousarray(self.group_info)
+            sample = stages(np.ascontiguousarray(info[::max(self.B // 64, 1)]))
+            alike = np.where(sample == 0, 255, sample).min(axis=1) == sample.max(axis=1)
+            self._depth = stages(info).max(axis=1) if 2 * np.count_nonzero(alike) > len(alike) else 0
+        if isinstance(self._depth, int):
+            return index
+        depth = self._depth if index is None else self._depth[index]
+        if depth.min() == depth.max():
+            return index
+        order = np.argsort(depth, kind="stable")
+        return order if index is None else index[order]
+
     def take(self, index):
-        """The sub-batch of the placements `index` (ascending)."""
+        """The sub-batch of the placements `index`."""
         index = np.asarray(index, np.int64)
 
         def kept():
@@ -1142,6 +1168,10 @@ def _launch(*args, rows_on_device=False, **kwargs):
     return _collect(_submit(*args, **kwargs), rows_on_device)
 
 
+# Placements from which a list is ordered by depth (by_depth): below, making the copies costs more
+# than neighbours that wait less for one another give.
+MIN_BY_DEPTH = 128
+
 # A batch is split when it has at least so many placements without interchangeable groups ...
 SPLIT_MIN_EASY = 512
 # ... or so many, when all its placements together simulate so many requests: a second launch costs
@@ -1191,15 +1221,16 @@ class ResidentBatch:
         while the host prepares the second."""
         self.trace, self.enc = trace, enc
         dev = trace.device
-        parts = [(None, enc)]
+        parts = [None]
         if split and mirrors and enc.has_twins is not None:
             hard = np.flatnonzero(enc.has_twins)
             least = SPLIT_MIN_EASY
             if trace.num_requests * enc.B >= SPLIT_LONG:
                 least = min(least, SPLIT_MIN_EASY_LONG)
             if len(hard) >= SPLIT_MIN_HARD and enc.B - len(hard) >= least:
-                easy = np.flatnonzero(~enc.has_twins)
-                parts = [(hard, enc.take(hard)), (easy, enc.take(easy))]
+                parts = [hard, np.flatnonzero(~enc.has_twins)]
+        parts = [enc.by_depth(index) for index in parts]
+        parts = [(index, enc if index is None else enc.take(index)) for index in parts]
         self.index = [p[0] for p in parts]
         self.jobs = []
         self.h2d_bytes = 0
@@ -1261,7 +1292,7 @@ class ResidentBatch:
         """Waits and downloads: (BatchResult in the order of the batch, d2h bytes)."""
         done = [_download(job) for job in self.jobs]
         d2h = sum(d[1] for d in done)
-        if len(done) == 1:
+        if self.index[0] is None:
             return done[0][0], d2h
         res = BatchResult()
         B = self.enc.B

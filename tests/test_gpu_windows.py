@@ -333,3 +333,31 @@ def test_failed_chunks_are_not_left_to_the_last_pass():
         spent = {t: sum(ms[i] for i in range(n.value) if tags[i] == t) for t in (1, 4)}
         best = min(best, spent[1] / spent[4])
     assert best < 0.45
+
+
+@pytest.mark.parametrize("replicas", [7, 8, 9, 11, 12, 15, 16, 63, 64, 67, 68, 100])
+@pytest.mark.parametrize("copies", [1, 300])
+def test_models_with_many_replicas(replicas, copies):
+    """Replica rows hold seven or eight replicas, then four at a time, 64 at most; in large batches
+    (300 copies of each, 32 to a warp) longer lists are read from the caller's tables.  With and
+    without interchangeable groups, in lists that mix depths, and depths of one kind (ordered by them)."""
+    M, n = 5, 3000
+    profs = _profiles(M, (1, 2, 4), 21)
+    ts, ids, slos = _trace(n, M, 120.0, replicas, 0.01)
+    rng = np.random.RandomState(replicas)
+    alone = [[0] + sorted(set(rng.choice([1, 2, 3, 4], size=rng.randint(0, 4)).tolist()))
+             for _ in range(replicas)]
+    sols = [_placement([1] * replicas, [[0]] * replicas),
+            _placement([1] * replicas, alone),
+            _placement([2 if replicas < 90 else 1] * replicas + [1], alone + [[1, 2, 3, 4]]),
+            _placement([4] * min(replicas, 50), alone[:50])]
+    res = _check(sols * copies, profs, ts, ids, slos, 0, 0, per_request=False) if copies == 1 else None
+    if res is None:
+        from mms_b200 import engine
+        trace = engine.DeviceTrace(ts, ids, slos, M)
+        table = engine.LatencyTable(profs)
+        both = [engine.run_batch(trace, engine.encode_placements(s, table, M), table, group_good=True)[0]
+                for s in (sols, [p for p in sols for _ in range(copies)])]
+        for name in ("good_total", "latency_sum", "model_num_good", "group_num_requests", "group_num_good"):
+            few, many = (getattr(r, name) for r in both)
+            assert np.repeat(few, copies, axis=0).tobytes() == many.tobytes(), name
