@@ -115,9 +115,8 @@ def parse_args():
 
 def sim_launches(args):
     """Kernels of a mms_sim_mixed call without interchangeable groups (with: two more): clear,
-    tables, stream, (link, restart or resolve, walk) per round, link, finish, count, requests per
-    model."""
-    return 7 + 3 * (args.rounds if args.rounds > 0 else 1)
+    tables, stream, (link, restart or resolve, walk) per round, link, finish, count."""
+    return 6 + 3 * (args.rounds if args.rounds > 0 else 1)
 
 
 def hbm_peak():

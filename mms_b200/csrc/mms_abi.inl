@@ -405,8 +405,11 @@ static int launch_sim(KernelArgs &ka, const ClearArgs &ca, const Geometry &g, cu
         // round g.rounds only judges the boundaries, for finish_kernel
         for (int r = 0; r <= g.rounds; ++r) {
             ka.round = r;
-            link_kernel<<<(unsigned)((bounds + kLinkWarps * kLanes - 1) / (kLinkWarps * kLanes)),
-                          kLinkWarps * kLanes, link_smem, st>>>(ka);
+            if (ka.swap_mask || bounds <= kLinkAlone)
+                link_warp_kernel<<<(unsigned)((bounds + kLinkWarps - 1) / kLinkWarps), kLinkWarps * kLanes,
+                                   link_smem, st>>>(ka);
+            else
+                link_kernel<<<(unsigned)((bounds + 127) / 128), 128, 0, st>>>(ka);
             MMS_CUDA(cudaGetLastError());
             if (r == g.rounds) break;
             if (r == 0 && g.restart)
@@ -620,6 +623,7 @@ static int sim_mixed(const mms_trace *trace, const mms_placements *cands, const 
     ca.group_info_in = cands->group_info;
     ca.group_info = (uint32_t *)(scratch + g.off_group_info);
     ca.model_num_good = out->model_num_good;
+    ca.model_num_requests = out->model_num_requests;
     ca.group_num_requests = out->group_num_requests;
     ca.group_num_good = gg ? out->group_num_good : nullptr;
     ca.good_total = out->good_total;
@@ -641,6 +645,17 @@ static int sim_mixed(const mms_trace *trace, const mms_placements *cands, const 
     if (rc) return rc;
 
     // tally the recorded decisions (outputs were cleared up front)
+    const size_t few_bytes = sizeof(uint32_t) * (size_t)(2 * ka.G + ka.M + 1);
+    if (ka.B <= kCountFew && few_bytes <= 48 * 1024) {
+        auto count_k = ka.dec_wide ? count_few_kernel<uint16_t> : count_few_kernel<uint8_t>;
+        const int64_t slices = (N + 4 * kCountThreads - 1) / (4 * kCountThreads);
+        count_k<<<(unsigned)(ka.B * (1 + slices)), kCountThreads, few_bytes, st>>>(
+            ka, gg, out->model_num_good, out->group_num_requests, out->group_num_good, out->good_total,
+            plan->leaf_merges, out->latency_sum);
+        MMS_CUDA(cudaGetLastError());
+        call_span.stop();
+        return MMS_OK;
+    }
     const size_t hist_bytes = g.smem_count;
     auto count_k = ka.dec_wide ? count_kernel<uint16_t> : count_kernel<uint8_t>;
     MMS_TRY(allow_smem((const void *)count_k, hist_bytes));
@@ -654,11 +669,6 @@ static int sim_mixed(const mms_trace *trace, const mms_placements *cands, const 
                                                     out->good_total, plan->leaf_merges,
                                                     out->latency_sum);
     MMS_CUDA(cudaGetLastError());
-    if (ka.M > 0) {
-        const int64_t cells = (int64_t)ka.B * ka.M;
-        model_requests_kernel<<<(unsigned)((cells + 127) / 128), 128, 0, st>>>(ka, out->model_num_requests);
-        MMS_CUDA(cudaGetLastError());
-    }
     call_span.stop();
     return MMS_OK;
 }

@@ -66,6 +66,7 @@ struct ClearArgs {
     const uint32_t *group_info_in;    // the caller's [B][G]
     uint32_t *group_info;             // scratch copy the kernels read
     int32_t *model_num_good;          // [B][M]
+    int32_t *model_num_requests;      // [B][M]
     int32_t *group_num_requests;      // [B][G]
     int32_t *group_num_good;          // [B][G] or null
     int64_t *good_total;              // [B]
@@ -102,7 +103,11 @@ __global__ void clear_kernel(const KernelArgs a, const ClearArgs c)
         const uint32_t info = c.group_info_in[i];
         c.group_info[i] = group_info_valid(a, info) ? (info & ~0x10000u) : 0u;
     }
-    for (int64_t i = tid; i < (int64_t)a.B * a.M; i += nth) c.model_num_good[i] = 0;
+    // model_num_requests (controller.py:587) does not depend on the placement: the trace's histogram
+    for (int64_t i = tid; i < (int64_t)a.B * a.M; i += nth) {
+        c.model_num_good[i] = 0;
+        c.model_num_requests[i] = a.model_hist[(a.many_traces ? i / a.M * (a.M + 1) : 0) + i % a.M];
+    }
     for (int64_t i = tid; i < (int64_t)a.B * a.G; i += nth) {
         c.group_num_requests[i] = 0;
         if (c.group_num_good) c.group_num_good[i] = 0;
@@ -365,31 +370,41 @@ __host__ __device__ inline size_t link_warp_bytes(int T, int G)
     return (sizeof(double) * (2 * (size_t)T + (size_t)G) + 3 * (size_t)G + 15) & ~(size_t)15;
 }
 
-// Judges the chunk boundaries whose sides the round before changed (all of them in round 0): one
-// thread per boundary compares the states as they are; those that differ and belong to a
-// candidate with interchangeable groups are then compared under other labels, by the whole
-// warp.
-__global__ void __launch_bounds__(kLinkWarps * kLanes)
+// Judges the chunk boundaries whose sides the round before changed (all of them in round 0), of
+// candidates without interchangeable groups: one thread per boundary.
+constexpr int64_t kLinkAlone = 148 * 64;     // boundaries that all have a warp at once
+
+__global__ void __launch_bounds__(128)
 link_kernel(const __grid_constant__ KernelArgs a)
 {
     if (!can_chunk(a) || nothing_changed(a)) return;
-    const int lane = threadIdx.x & (kLanes - 1), warp = threadIdx.x / kLanes;
     const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= (int64_t)a.B * (a.K - 1)) return;
+    const int64_t b = t % a.B;
+    const int32_t j = (int32_t)(t / a.B) + 1;
+    const size_t cell = (size_t)j * a.B + b;
+    if (a.round != 0 && a.stamp[cell - a.B] != (uint8_t)a.round && a.stamp[cell] != (uint8_t)a.round) return;
+    a.link[cell] = continues(a, j, b);
+    a.rel[(size_t)(j * a.seg_per_chunk) * a.B + b] = 0;
+}
+
+// The same with a warp per boundary, its lanes over the groups, and under other labels: for calls with few boundaries, where a
+// thread's way through two states is what takes the time (70 boundaries of one placement on 16 devices
+// 27 to 46 us, by warps 9; 3 700 of 37 placements 32 and 10), and for candidates with interchangeable
+// groups, whose failed boundaries are compared under other labels by a warp in any case (46 000 of a layer on 64
+// devices 498 and 190, the second time 305 and 74).
+__global__ void __launch_bounds__(kLinkWarps * kLanes)
+link_warp_kernel(const __grid_constant__ KernelArgs a)
+{
+    if (!can_chunk(a) || nothing_changed(a)) return;
+    const int lane = threadIdx.x & (kLanes - 1), warp = threadIdx.x / kLanes;
+    const int64_t t = (int64_t)blockIdx.x * kLinkWarps + warp;
+    if (t >= (int64_t)a.B * (a.K - 1)) return;
     const size_t B = (size_t)a.B;
     const int64_t b = t % a.B;
     const int32_t j = (int32_t)(t / a.B) + 1;
-    bool again = false;
-    if (t < (int64_t)a.B * (a.K - 1)) {
-        const size_t cell = (size_t)j * B + b;
-        if (a.round == 0 || a.stamp[cell - B] == (uint8_t)a.round || a.stamp[cell] == (uint8_t)a.round) {
-            const bool ok = continues(a, j, b);
-            a.link[cell] = ok;
-            a.rel[(size_t)(j * a.seg_per_chunk) * B + b] = 0;
-            again = !ok && a.twins[b];
-        }
-    }
-    uint32_t todo = __ballot_sync(0xFFFFFFFFu, again);
-    if (!todo) return;
+    const size_t cell = (size_t)j * B + b;
+    if (a.round != 0 && a.stamp[cell - B] != (uint8_t)a.round && a.stamp[cell] != (uint8_t)a.round) return;
     const size_t base = (size_t)warp * link_warp_bytes(a.T, a.G);
     const uint32_t x = (uint32_t)(base / sizeof(double));
     RelabelScratch s;
@@ -397,29 +412,28 @@ link_kernel(const __grid_constant__ KernelArgs a)
     s.last = s.z + a.T;
     s.perm = (uint32_t)(base + sizeof(double) * (2 * (size_t)a.T + (size_t)a.G));
     s.rank = s.perm + a.G;
-    for (; todo; todo &= todo - 1) {
-        const int k = __ffs((int)todo) - 1;
-        const int64_t bb = __shfl_sync(0xFFFFFFFFu, b, k);
-        const int32_t jj = __shfl_sync(0xFFFFFFFFu, j, k);
-        const int32_t q0 = jj * a.seg_per_chunk;
-        const double tau = arrival_at(a, bb, a.leaf_start[seg_leaf(a, q0)]);
-        __syncwarp();
-        for (int t = lane; t < a.T; t += kLanes)
-            SM_F64(x + t) = a.seg_end[((size_t)(q0 - 1) * a.T + t) * B + bb];
-        __syncwarp();
-        const auto info = [&](int g) { return a.group_info[(size_t)bb * a.G + g]; };
-        const auto X = [&](uint32_t t) { return SM_F64(x + t); };
-        if (!warp_relabel(a.G, a.T, a.twin_class + (size_t)bb * a.G, info, X,
-                          a.chunk_start + (size_t)jj * a.T * B + bb, B, s) ||
-            !warp_equivalent(a.G, info, X, [&](uint32_t t) { return SM_F64(s.z + t); }, tau))
-            continue;
-        const size_t cell = (size_t)q0 * B + bb;
-        for (int g = lane; g < a.G; g += kLanes) a.perm[cell * a.G + g] = smem[s.perm + g];
-        if (lane == 0) {
-            a.rel[cell] = kRelOther;
-            a.relabelled[bb] = 1;
-            a.link[(size_t)jj * B + bb] = 1;
-        }
+    const int32_t q0 = j * a.seg_per_chunk;
+    const double *Y = a.chunk_start + (size_t)j * a.T * B + b;
+    const double tau = arrival_at(a, b, a.leaf_start[seg_leaf(a, q0)]);
+    for (int k = lane; k < a.T; k += kLanes) {
+        SM_F64(x + k) = a.seg_end[((size_t)(q0 - 1) * a.T + k) * B + b];
+        SM_F64(s.z + k) = Y[(size_t)k * B];
+    }
+    __syncwarp();
+    const auto info = [&](int g) { return a.group_info[(size_t)b * a.G + g]; };
+    const auto X = [&](uint32_t k) { return SM_F64(x + k); };
+    const auto Z = [&](uint32_t k) { return SM_F64(s.z + k); };
+    bool ok = warp_equivalent(a.G, info, X, Z, tau), other = false;
+    if (!ok && a.twins[b] &&
+        warp_relabel(a.G, a.T, a.twin_class + (size_t)b * a.G, info, X, Y, B, s))
+        ok = other = warp_equivalent(a.G, info, X, Z, tau);
+    const size_t at = (size_t)q0 * B + b;
+    if (other)
+        for (int g = lane; g < a.G; g += kLanes) a.perm[at * a.G + g] = smem[s.perm + g];
+    if (lane == 0) {
+        a.link[cell] = ok;
+        a.rel[at] = other ? kRelOther : 0;
+        if (other) a.relabelled[b] = 1;
     }
 }
 
@@ -663,7 +677,7 @@ __device__ inline size_t record_at(const KernelArgs &a, int64_t b, int32_t i)
     return ((size_t)(i >> 2) * a.dec_pitch + b) * 4 + (size_t)(i & 3);
 }
 
-// Follows the labels through segment q.  Returns whether they changed.
+// Follows the labels through segment q, which has swaps.  Returns whether they changed.
 __device__ inline bool labels_follow(const KernelArgs &a, int64_t b, Labels &l, int32_t q)
 {
     Swaps s = swaps_of(a, b, q, segment_first(a, q));
@@ -806,7 +820,7 @@ finish_kernel(const __grid_constant__ KernelArgs a)
     Labels l;
     l.pi = w.labels;
     l.tmp = w.re.perm;
-    l.cls = a.twin_class + (size_t)b * a.G;
+    l.cls = &SM_U32(w.cls);                  // (window_setup's copy; not looked at without twins)
     labels_reset(l, a.G);
     int32_t q = a.seg_per_chunk;             // chunk 0 is the true run
     int32_t noted = -1;                      // segment in whose `perm` l.pi is noted
@@ -826,13 +840,21 @@ finish_kernel(const __grid_constant__ KernelArgs a)
     };
     while (q < a.NS) {
         // the first of 32 segments in which something happens; those before it keep the labels
+        // (each lane keeps what it loads: an event is a chain of loads as it is)
         const int32_t s = q + lane;
-        bool event = false;
+        bool event = false, linked = true;
+        uint8_t rel = 0, swap_count = 0;
+        uint64_t tie = 0;
         if (s < a.NS) {
             const size_t at = (size_t)s * B + b;
-            event = s % a.seg_per_chunk == 0 && !a.link[(size_t)(s / a.seg_per_chunk) * B + b];
-            if constexpr (kTwins)
-                event |= a.rel[at] || (l.moved && (a.swap_count[at] || (a.tie[at] & l.moved)));
+            linked = s % a.seg_per_chunk != 0 || a.link[(size_t)(s / a.seg_per_chunk) * B + b];
+            event = !linked;
+            if constexpr (kTwins) {
+                rel = a.rel[at];
+                swap_count = a.swap_count[at];
+                tie = a.tie[at];
+                event |= rel || (l.moved && (swap_count || (tie & l.moved)));
+            }
         }
         const uint32_t todo = __ballot_sync(0xFFFFFFFFu, event);
         int32_t quiet = todo ? __ffs((int)todo) - 1 : kLanes;
@@ -843,17 +865,17 @@ finish_kernel(const __grid_constant__ KernelArgs a)
         const size_t cell = (size_t)q * B + b;
         const int32_t j = q / a.seg_per_chunk;
         const bool first = q % a.seg_per_chunk == 0;
-        if (!first || a.link[(size_t)j * B + b]) {
+        if (__shfl_sync(0xFFFFFFFFu, linked, quiet)) {
             uint64_t moved = l.moved;
-            const bool other = a.rel[cell] != 0;
+            const bool other = __shfl_sync(0xFFFFFFFFu, rel, quiet) != 0;
             if (other) moved = labels_through(l, a.G, a.perm + cell * a.G);
-            if (!(moved && (a.tie[cell] & moved))) {
+            if (!(moved & __shfl_sync(0xFFFFFFFFu, tie, quiet))) {
                 if (other) {
                     labels_take(l, a.G, moved);
                     noted = -1;
                 }
                 note(1);
-                if (l.moved && labels_follow(a, b, l, q)) noted = -1;
+                if (l.moved && __shfl_sync(0xFFFFFFFFu, swap_count, quiet) && labels_follow(a, b, l, q)) noted = -1;
                 ++q;
                 continue;
             }
@@ -1060,15 +1082,57 @@ count_kernel(const KernelArgs a, int32_t seg_per_block, bool group_good, int32_t
     }
 }
 
-// model_num_requests (controller.py:587) does not depend on the placement:
-// one thread per (candidate, model) copies the trace's histogram.
-__global__ void model_requests_kernel(const KernelArgs a, int32_t *model_num_requests)
+// The same for few candidates, whose lanes count_kernel would leave idle: a block takes 1024
+// consecutive requests of one, four to a thread.  The first B blocks form the latency sums.  A thread
+// reads 4 bytes of a sector, which is why this is for few: 57 600 requests of one candidate 55 -> 10 us,
+// 30 000 of 37 46 -> 8 us.
+constexpr int kCountThreads = 256;
+constexpr int kCountFew = 64;
+template <typename Dec>
+__global__ void __launch_bounds__(kCountThreads)
+count_few_kernel(const KernelArgs a, bool group_good, int32_t *model_num_good, int32_t *group_num_requests,
+                 int32_t *group_num_good, int64_t *good_total, const uint8_t *leaf_merges, double *latency_sum)
 {
-    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= (int64_t)a.B * a.M) return;
-    const int64_t b = t / a.M;
-    const int m = (int)(t % a.M);
-    model_num_requests[t] = a.model_hist[(a.many_traces ? (size_t)b * (a.M + 1) : 0) + m];
+    if ((int)blockIdx.x < a.B) {
+        if (threadIdx.x < kLanes) sum_leaves(a, blockIdx.x, leaf_merges, latency_sum);
+        return;
+    }
+    constexpr int kAcceptedBit = 8 * sizeof(Dec) - 1;
+    extern __shared__ uint32_t hist[];               // [G] requests, [G] good, [M] good, good in all
+    const int cells = 2 * a.G + a.M + 1;
+    for (int c = threadIdx.x; c < cells; c += blockDim.x) hist[c] = 0;
+    __syncthreads();
+    const int64_t block = blockIdx.x - a.B;
+    const int64_t b = block % a.B;
+    const int64_t i0 = (block / a.B * kCountThreads + threadIdx.x) * 4;
+    if (i0 < a.N) {
+        struct alignas(4 * sizeof(Dec)) Quad { Dec r[4]; };
+        const Quad d = static_cast<const Quad *>(a.decisions)[(size_t)(i0 >> 2) * a.dec_pitch + b];
+        const size_t tb = trace_base(a, b);
+        uint32_t good = 0;
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const uint32_t rec = i0 + u < a.N ? d.r[u] : 0u;
+            if (!rec) continue;
+            const uint32_t g = (rec & ((1u << kAcceptedBit) - 1)) - 1;
+            atomicAdd(&hist[g], 1u);
+            if (rec >> kAcceptedBit) {
+                atomicAdd(&hist[a.G + g], 1u);
+                atomicAdd(&hist[2 * a.G + a.model_ids[(size_t)(i0 + u) * a.trace_pitch + tb]], 1u);
+                ++good;
+            }
+        }
+        if (good) atomicAdd(&hist[cells - 1], good);
+    }
+    __syncthreads();
+    for (int c = threadIdx.x; c < cells; c += blockDim.x) {
+        const uint32_t n = hist[c];
+        if (!n) continue;
+        if (c < a.G) atomicAdd(&group_num_requests[(size_t)b * a.G + c], (int32_t)n);
+        else if (c < 2 * a.G) { if (group_good) atomicAdd(&group_num_good[(size_t)b * a.G + (c - a.G)], (int32_t)n); }
+        else if (c < 2 * a.G + a.M) atomicAdd(&model_num_good[(size_t)b * a.M + (c - 2 * a.G)], (int32_t)n);
+        else atomicAdd(reinterpret_cast<unsigned long long *>(good_total + b), (unsigned long long)n);
+    }
 }
 
 // Per-model request counts, plus the number of positions where the arrival

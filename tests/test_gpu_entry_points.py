@@ -280,3 +280,32 @@ def test_pinned_stager_uploads_arrays_and_lazy_arrays():
         assert d_slo.cpu().numpy().tobytes() == slo64.astype(np.float32).tobytes()
     with pytest.raises(ValueError):
         stager.upload([(torch.empty(3, dtype=torch.float64, device=dev), np.zeros(4))])
+
+
+@pytest.mark.parametrize("count", [1, 31, 64, 65, 97])
+@pytest.mark.parametrize("n", [1, 3, 1023, 1024, 1025, 5000])
+def test_tallies_of_few_and_many_candidates(count, n):
+    """Up to 64 candidates are tallied by blocks of 1024 requests, more of them 32 to a warp."""
+    from mms_b200 import cases, engine
+    from mms_b200.simulator import workload_arrays
+    from oracle import tables
+    case = cases.candidate_batch_case(num_candidates=count, duration=120.0, num_models=7,
+                                      num_devices=8, total_rate=50.0)
+    names = [d.name for d in case.model_datas]
+    profs = [d.profiling_result for d in case.model_datas]
+    mids, slos = workload_arrays(case.workload, names)
+    arr, mids, slos = (np.ascontiguousarray(x[:n]) for x in (case.workload.arrivals, mids, slos))
+    trace = engine.DeviceTrace(arr, mids, slos, len(names))
+    table = engine.LatencyTable(profs)
+    enc = engine.encode_placements(case.placements, table, len(names))
+    for per_request in (False, True):
+        res, _, _ = engine.run_batch(trace, enc, table, per_request=per_request, group_good=True)
+        for b in {0, count // 2, count - 1}:
+            fin, good, mreq, mgood, greq, ggood = tables.one_placement(case.placements[b], profs, mids,
+                                                                       slos, arr)
+            assert np.array_equal(res.model_num_requests[b], mreq)
+            assert np.array_equal(res.model_num_good[b], mgood)
+            assert np.array_equal(res.group_num_requests[b, :len(greq)], greq)
+            assert np.array_equal(res.group_num_good[b, :len(ggood)], ggood)
+            assert res.good_total[b] == np.count_nonzero(good)
+            assert res.latency_sum[b] == float(np.add.reduce(fin - arr))
