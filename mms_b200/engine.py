@@ -12,7 +12,7 @@ import functools
 import operator
 from contextlib import nullcontext
 from itertools import chain, permutations, product
-from math import factorial
+from math import factorial, prod
 from typing import List, Sequence
 
 import numpy as np
@@ -26,6 +26,8 @@ _PP = operator.itemgetter(2)     # pipeline degree of a ParallelConfig(dp, op, p
 
 
 def _require_cuda():
+    if torch.cuda.is_initialized():       # (there was a device, and it is cheaper to ask)
+        return
     if not torch.cuda.is_available():
         raise RuntimeError("mms_b200 needs a CUDA device: the simulator has no CPU path")
 
@@ -34,8 +36,29 @@ def _ptr(t):
     return ctypes.c_void_p(t.data_ptr()) if t is not None and t.numel() > 0 else ctypes.c_void_p(0)
 
 
+def _raw_stream():
+    """The current stream of the current device as CUDA's handle, 0 for the default one
+    (torch.cuda.current_stream() makes an object of it, which takes longer than a launch)."""
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
+
+
 def _stream_ptr():
-    return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    return ctypes.c_void_p(_raw_stream())
+
+
+def _layout(fields):
+    """{name: (offset, bytes, dtype, shape)} of arrays one behind the other, each 16-byte aligned, and
+    the bytes of all; a field without a shape is left out."""
+    at, total = {}, 0
+    for name, dtype, shape in fields:
+        if shape is not None:
+            size = prod(shape) * _ITEM_BYTES[dtype]
+            at[name] = (total, size, dtype, shape)
+            total += (size + 15) & ~15
+    return at, max(total, 16)
+
+
+_ITEM_BYTES = {t: np.dtype(t).itemsize for t in (np.int32, np.uint32, np.int64, np.float64)}
 
 
 _NO_CONTEXT = nullcontext()
@@ -71,15 +94,35 @@ def _to_device_many(arrays, device):
     memory from torch's host allocator (which keeps a block until the copies
     from it are done).  Returns device tensors that are views of one buffer, each
     16-byte aligned."""
-    device = torch.device(device)
     arrays = [np.ascontiguousarray(a) for a in arrays]
+    buf, offsets = _pack(arrays, device)
+    if buf is None:
+        return [_to_device(a, device) for a in arrays]
+    return [buf[o:o + a.nbytes].view(_TORCH_TYPE[a.dtype]).reshape(a.shape)
+            for a, o in zip(arrays, offsets)]
+
+
+def _upload(arrays, device):
+    """_to_device_many for callers that only need addresses: (what to keep, [pointer, ...])."""
+    arrays = [np.ascontiguousarray(a) for a in arrays]
+    buf, offsets = _pack(arrays, device)
+    if buf is None:
+        keep = [_to_device(a, device) for a in arrays]
+        return keep, [_ptr(t) for t in keep]
+    base = buf.data_ptr()
+    return buf, [ctypes.c_void_p(base + o if a.size else 0) for a, o in zip(arrays, offsets)]
+
+
+def _pack(arrays, device):
+    """The transfer of _to_device_many: (buffer, offsets), or (None, None) where the arrays are so large
+    that they go one by one."""
     offsets, total = [], 0
     for a in arrays:
         offsets.append(total)
         total += (a.nbytes + 15) & ~15
     total = max(total, 16)
     if total > _STAGED_UPLOAD:
-        return [_to_device(a, device) for a in arrays]
+        return None, None
     small = total <= _SMALL_UPLOAD
     stage = torch.empty(total, dtype=torch.uint8, pin_memory=not small)
     host = stage.numpy()
@@ -88,8 +131,7 @@ def _to_device_many(arrays, device):
             host[o:o + a.nbytes] = a.reshape(-1).view(np.uint8)
     buf = torch.empty(total, dtype=torch.uint8, device=device)
     buf.copy_(stage, non_blocking=True)
-    return [buf[o:o + a.nbytes].view(_TORCH_TYPE[a.dtype]).reshape(a.shape)
-            for a, o in zip(arrays, offsets)]
+    return buf, offsets
 
 
 @functools.lru_cache(maxsize=64)
@@ -405,22 +447,26 @@ class LatencyTable:
         old = self._host
         tab = np.zeros((M, C, S) + old.shape[3:], np.float32)
         tab[:, :old.shape[1], :old.shape[2]] = old
+        # the new columns as one list of numbers: 1 + the penalty times each latency in f64, rounded
+        # to f32 once, as controller.py:467-476 does it array by array
+        sizes = (1,) if self.batch_sizes is None else self.batch_sizes
+        rows = []
+        for prof in self.prof_ress:
+            for c in new:
+                value, pp = prof.para_dict.get(c, None), int(c.pp)
+                if value:
+                    factor = 1 + 0.009 * len(value.latency[1])
+                    lats = [list(value.latency[b][:pp]) for b in sizes]
+                    lats = [lat * pp if len(lat) == 1 else lat for lat in lats]   # one for all stages
+                    if any(len(lat) != pp for lat in lats):
+                        raise ValueError(f"fewer latencies than stages of {c}")
+                    rows += [float(lat[k]) * factor for k in range(pp) for lat in lats]
+                    rows += [0.0] * ((S - pp) * len(sizes))
+                else:
+                    rows += [inf] * (S * len(sizes))
         with np.errstate(over="ignore"):
-            for m, prof in enumerate(self.prof_ress):
-                for c in new:
-                    col = self.column[c]
-                    value = prof.para_dict.get(c, None)
-                    if value:
-                        penalty = 0.009 * len(value.latency[1])
-                        pp = int(c.pp)
-                        if self.batch_sizes is None:
-                            tab[m, col, :pp] = np.asarray(value.latency[1][:pp], np.float64) * (1 + penalty)
-                        else:
-                            for j, bs in enumerate(self.batch_sizes):
-                                tab[m, col, :pp, j] = \
-                                    np.asarray(value.latency[bs][:pp], np.float64) * (1 + penalty)
-                    else:
-                        tab[m, col] = np.float32(inf)
+            tab[:, len(self.configs) - len(new):] = np.array(rows, np.float64).reshape(
+                (M, len(new), S) + old.shape[3:])
         self._host = tab
         self.max_stages = S
         self._device = None
@@ -432,11 +478,15 @@ class LatencyTable:
     def device(self, dev):
         """The table on `dev`; uploaded on the current stream when it changed,
         and any stream that asks for it waits for that upload."""
-        if self._device is None or self._device.device != dev:
-            self._device = _to_device(self._host, dev)
-            self._ready = torch.cuda.Event()
-            self._ready.record(torch.cuda.current_stream(dev))
-        torch.cuda.current_stream(dev).wait_event(self._ready)
+        with _on(torch.device(dev)):
+            here = _raw_stream()
+            if self._device is None or self._device.device != dev:
+                self._device = _to_device(self._host, dev)
+                self._ready = torch.cuda.Event()
+                self._ready.record()
+                self._uploaded_on = here
+            elif here or self._uploaded_on:           # (the default stream is in order with itself)
+                torch.cuda.current_stream().wait_event(self._ready)
         return self._device
 
 
@@ -972,8 +1022,7 @@ class _Pending:
 
     def field(self, name):
         """One output as a device tensor (a view of the launch's output buffer)."""
-        at, dtype, shape = self.fields[name]
-        size = int(np.prod(shape)) * np.dtype(dtype).itemsize
+        at, size, dtype, shape = self.fields[name]
         return self.buf[at:at + size].view(_TORCH_TYPE[np.dtype(dtype)]).reshape(shape)
 
 
@@ -1022,7 +1071,8 @@ def _enqueue(job: _Pending):
                                      _ptr(trace.model_hist), ctypes.byref(opts), ctypes.byref(ws),
                                      ctypes.byref(out), flags, _stream_ptr())
         nat.check(rc, "mms_sim_mixed")
-        job.stream = torch.cuda.current_stream()
+        # None: the default stream
+        job.stream = torch.cuda.current_stream() if _raw_stream() else None
 
 
 def _prepare(trace: DeviceTrace, B, M, G, P, T, S, C, model_off, model_rep, group_info,
@@ -1040,15 +1090,18 @@ def _prepare(trace: DeviceTrace, B, M, G, P, T, S, C, model_off, model_rep, grou
     job = _Pending()
     with _on(dev):
         h2d = model_off.nbytes + model_rep.nbytes + group_info.nbytes
+        tables = (model_off, model_rep, group_info)
+        host_latency = not isinstance(latency, torch.Tensor)
+        if host_latency:
+            tables += (latency,)
         if pinned:
-            d_off = _to_device(model_off, dev, pinned)
-            d_rep = _to_device(model_rep, dev, pinned)
-            d_info = _to_device(group_info, dev, pinned)
+            d_tables = [_to_device(t, dev, pinned) for t in tables]
+            at_tables = [_ptr(t) for t in d_tables]
         else:
-            d_off, d_rep, d_info = _to_device_many((model_off, model_rep, group_info), dev)
-        d_lat = latency if isinstance(latency, torch.Tensor) else _to_device(latency, dev, pinned)
-        cands = nat.Placements(B, M, G, P, T, S, C, 0, _ptr(d_off), _ptr(d_rep), _ptr(d_info),
-                               _ptr(d_lat), int(latency_stride), None, None)
+            d_tables, at_tables = _upload(tables, dev)
+        cands = nat.Placements(B, M, G, P, T, S, C, 0, *at_tables[:3],
+                               at_tables[3] if host_latency else _ptr(latency), int(latency_stride),
+                               None, None)
         need = L.mms_sim_workspace_bytes(N, ctypes.byref(cands), ctypes.byref(opts), flags)
         if need == 0 and B > 0:
             raise NotImplementedError("placement batch outside the kernel limits "
@@ -1057,18 +1110,14 @@ def _prepare(trace: DeviceTrace, B, M, G, P, T, S, C, model_off, model_rep, grou
         ws = nat.Workspace(_ptr(ws_t), need)
         # the outputs in one buffer: one allocation here, one transfer when they are read
         rows = max(B, 1)
-        fields, total = {}, 0
-        for name, dtype, shape in (
-                ("good_total", np.int64, (rows,)), ("latency_sum", np.float64, (rows,)),
-                ("model_num_requests", np.int32, (rows, max(M, 1))),
-                ("model_num_good", np.int32, (rows, max(M, 1))),
-                ("group_num_requests", np.int32, (rows, G)),
-                ("group_num_good", np.int32, (rows, G) if want_group_good else None),
-                ("status", np.uint32, (rows,)), ("resimulated", np.int32, (rows,))):
-            if shape is not None:
-                fields[name] = (total, dtype, shape)
-                total += (int(np.prod(shape)) * np.dtype(dtype).itemsize + 15) & ~15
-        buf = torch.empty(max(total, 16), dtype=torch.uint8, device=dev)
+        fields, total = _layout((
+            ("good_total", np.int64, (rows,)), ("latency_sum", np.float64, (rows,)),
+            ("model_num_requests", np.int32, (rows, max(M, 1))),
+            ("model_num_good", np.int32, (rows, max(M, 1))),
+            ("group_num_requests", np.int32, (rows, G)),
+            ("group_num_good", np.int32, (rows, G) if want_group_good else None),
+            ("status", np.uint32, (rows,)), ("resimulated", np.int32, (rows,))))
+        buf = torch.empty(total, dtype=torch.uint8, device=dev)
         full = bool(flags & nat.FLAG_PER_REQUEST)
         o_fin = torch.empty((rows, max(N, 1)), dtype=torch.float64, device=dev) if full else None
         o_good = torch.empty((rows, max(N, 1)), dtype=torch.uint8, device=dev) if full else None
@@ -1079,10 +1128,10 @@ def _prepare(trace: DeviceTrace, B, M, G, P, T, S, C, model_off, model_rep, grou
         out = nat.Results(at("model_num_requests"), at("model_num_good"), at("group_num_requests"),
                           at("group_num_good"), at("good_total"), at("latency_sum"), at("status"),
                           _ptr(o_fin), _ptr(o_good), at("resimulated"))
-        job.stream = torch.cuda.current_stream()
+    job.stream = None
     job.call = (cands, opts, ws, out, flags)
     job.trace = trace
-    job.keep = (d_off, d_rep, d_info, d_lat)
+    job.keep = (d_tables, latency)
     job.scratch = ws_t
     job.buf, job.fields, job.rows = buf, fields, (o_fin, o_good)
     job.B, job.M, job.N, job.full = B, M, N, full
@@ -1102,6 +1151,14 @@ def _to_host(t):
     return stage.numpy().copy()
 
 
+def _on_stream(stream, dev):
+    """`stream` (None: the default one) of `dev` as the current stream, where it is not."""
+    with _on(dev):
+        if _raw_stream() == (stream.cuda_stream if stream is not None else 0):
+            return _on(dev)
+    return torch.cuda.stream(stream if stream is not None else torch.cuda.default_stream(dev))
+
+
 def _download(job: _Pending, rows_on_device=False):
     """Waits for the launch and copies its results to the host.  Returns
     (BatchResult, d2h_bytes).  rows_on_device: the per-request outputs are not
@@ -1110,10 +1167,9 @@ def _download(job: _Pending, rows_on_device=False):
     o_fin, o_good = job.rows
     res = BatchResult()
     host_rows = full and not rows_on_device
-    with torch.cuda.stream(job.stream):
+    with _on_stream(job.stream, job.buf.device):
         host = _to_host(job.buf)
-        for name, (at, dtype, shape) in job.fields.items():
-            size = int(np.prod(shape)) * np.dtype(dtype).itemsize
+        for name, (at, size, dtype, shape) in job.fields.items():
             setattr(res, name, host[at:at + size].view(dtype).reshape(shape)[:B])
         res.model_num_requests = res.model_num_requests[:, :M]
         res.model_num_good = res.model_num_good[:, :M]
@@ -1432,27 +1488,25 @@ class ResidentBatching:
         goff, gmod, gcfg = group_lists(model_off, model_rep, group_info, G)
         self.h2d_bytes = sum(x.nbytes for x in (model_off, model_rep, goff, gmod, gcfg))
         with _on(dev):
-            d_off, d_rep, d_goff, d_gmod, d_gcfg = _to_device_many(
-                (model_off, model_rep, goff, gmod, gcfg), dev)
-            d_lat = latency if isinstance(latency, torch.Tensor) else _to_device(latency, dev)
-            self.cands = nat.Placements(B, M, G, P, T, S, C, 0, _ptr(d_off), _ptr(d_rep), None,
-                                        _ptr(d_lat), int(latency_stride))
-            self.bat = nat.Batching(_ptr(d_goff), _ptr(d_gmod), _ptr(d_gcfg), len(batch_sizes),
-                                    int(heap_capacity), (ctypes.c_int32 * 8)(*list(batch_sizes)))
+            tables = (model_off, model_rep, goff, gmod, gcfg)
+            host_latency = not isinstance(latency, torch.Tensor)
+            d_tables, at_tables = _upload(tables + ((latency,) if host_latency else ()), dev)
+            self.cands = nat.Placements(B, M, G, P, T, S, C, 0, *at_tables[:2], None,
+                                        at_tables[5] if host_latency else _ptr(latency),
+                                        int(latency_stride))
+            self.bat = nat.Batching(*at_tables[2:5], len(batch_sizes), int(heap_capacity),
+                                    (ctypes.c_int32 * 8)(*list(batch_sizes)))
             need = L.mms_sim_batching_workspace_bytes(N, ctypes.byref(self.cands),
                                                       ctypes.byref(self.bat))
             ws_t = torch.empty(max(need, 256), dtype=torch.uint8, device=dev)
             self.ws = nat.Workspace(_ptr(ws_t), need)
-            self.fields, total = {}, 0
-            for name, dtype, shape in (
-                    ("good_total", np.int64, (B,)), ("latency_sum", np.float64, (B,)),
-                    ("model_num_requests", np.int32, (B, max(M, 1))),
-                    ("model_num_good", np.int32, (B, max(M, 1))),
-                    ("group_num_requests", np.int32, (B, G)), ("group_num_good", np.int32, (B, G)),
-                    ("status", np.uint32, (B,)), ("resimulated", np.int32, (B,))):
-                self.fields[name] = (total, dtype, shape)
-                total += (int(np.prod(shape)) * np.dtype(dtype).itemsize + 15) & ~15
-            self.buf = torch.zeros(max(total, 16), dtype=torch.uint8, device=dev)
+            self.fields, total = _layout((
+                ("good_total", np.int64, (B,)), ("latency_sum", np.float64, (B,)),
+                ("model_num_requests", np.int32, (B, max(M, 1))),
+                ("model_num_good", np.int32, (B, max(M, 1))),
+                ("group_num_requests", np.int32, (B, G)), ("group_num_good", np.int32, (B, G)),
+                ("status", np.uint32, (B,)), ("resimulated", np.int32, (B,))))
+            self.buf = torch.zeros(total, dtype=torch.uint8, device=dev)
             o_fin = torch.empty((B, max(N, 1)), dtype=torch.float64, device=dev)
             o_good = torch.empty((B, max(N, 1)), dtype=torch.uint8, device=dev)
             base = self.buf.data_ptr()
@@ -1461,7 +1515,7 @@ class ResidentBatching:
                                    at["group_num_requests"], at["group_num_good"],
                                    at["good_total"], at["latency_sum"], at["status"], _ptr(o_fin),
                                    _ptr(o_good), at["resimulated"])
-        self.keep = (d_off, d_rep, d_goff, d_gmod, d_gcfg, d_lat, ws_t)
+        self.keep = (d_tables, latency, ws_t)
         self.rows = (o_fin, o_good)
 
     def launch(self):
@@ -1482,8 +1536,7 @@ class ResidentBatching:
         M, N = self.M, self.N
         res = BatchResult()
         host = _to_host(self.buf)
-        for name, (at, dtype, shape) in self.fields.items():
-            size = int(np.prod(shape)) * np.dtype(dtype).itemsize
+        for name, (at, size, dtype, shape) in self.fields.items():
             setattr(res, name, host[at:at + size].view(dtype).reshape(shape))
         res.model_num_requests = res.model_num_requests[:, :M]
         res.model_num_good = res.model_num_good[:, :M]
@@ -1598,13 +1651,10 @@ def device_compute_stats(arrivals, model_ids, num_models: int, finish, good, fir
             raise NotImplementedError("statistics outside the kernel limits")
         ws_t = _take_scratch(dev, max(need, 256))
         ws = nat.Workspace(_ptr(ws_t), need)
-        fields, total = {}, 0
-        for name, dtype, shape in (
-                [("good_total", np.int64, (B,)), ("latency_sum", np.float64, (B,))]
-                + [(k, np.float64, (B, max(M, 1))) for k in STATS_FIELDS[1:]]
-                + [("num_good", np.int32, (B, max(M, 1))), ("num_requests", np.int32, (max(M, 1),))]):
-            fields[name] = (total, dtype, shape)
-            total += (int(np.prod(shape)) * np.dtype(dtype).itemsize + 15) & ~15
+        fields, total = _layout(
+            [("good_total", np.int64, (B,)), ("latency_sum", np.float64, (B,))]
+            + [(k, np.float64, (B, max(M, 1))) for k in STATS_FIELDS[1:]]
+            + [("num_good", np.int32, (B, max(M, 1))), ("num_requests", np.int32, (max(M, 1),))])
         buf = torch.zeros(total, dtype=torch.uint8, device=dev)
         out = nat.StatsOut(*[ctypes.c_void_p(buf.data_ptr() + fields[k][0])
                              for k in ("num_requests",) + STATS_FIELDS + ("good_total", "latency_sum")])
@@ -1614,8 +1664,8 @@ def device_compute_stats(arrivals, model_ids, num_models: int, finish, good, fir
         nat.check(rc, "mms_compute_stats")
         host = _to_host(buf)                                  # waits for the kernels
         _return_scratch(dev, ws_t)
-    res = {k: host[at:at + int(np.prod(shape)) * np.dtype(dtype).itemsize].view(dtype).reshape(shape)
-           for k, (at, dtype, shape) in fields.items()}
+    res = {k: host[at:at + size].view(dtype).reshape(shape)
+           for k, (at, size, dtype, shape) in fields.items()}
     res["d2h_bytes"] = sum(v.nbytes for v in res.values())
     res["num_requests"] = res["num_requests"][:M]
     for name in STATS_FIELDS:

@@ -301,10 +301,13 @@ def device_stats(workload, start, finish_dev, good_dev, warmup) -> StatsResult:
                                      good_dev.reshape(1, -1), lo, window)
     start_w, which_w = np.asarray(start)[lo:hi], which[lo:hi]
     # names in order of first appearance, then a stable sort by request count (:321-326)
-    first = np.full(K, len(which_w), np.int64)
-    first[which_w[::-1]] = np.arange(len(which_w) - 1, -1, -1)      # the last write is the first one
-    seen = [int(k) for k in np.argsort(first, kind="stable") if first[k] < len(which_w)]
-    ordered = sorted(seen, key=lambda k: int(st["num_requests"][k]))
+    counts = st["num_requests"].tolist()
+    present, seen = sum(c > 0 for c in counts), []
+    for size in (256, 4096, window):      # (most have appeared long before the end)
+        if len(seen) < present:
+            names, at = np.unique(which_w[:size], return_index=True)
+            seen = names[np.argsort(at)].tolist()
+    ordered = sorted(seen, key=counts.__getitem__)
     host = {}
 
     def rows():
