@@ -201,6 +201,18 @@ static int plan_call(int64_t N, const mms_placements *c, const mms_sim_options *
     const Cut win = cut_trace(seg, (int64_t)g->window_blocks * kWindowWarps, thrifty ? thrifty : seg);
     // Which speculative pass: see window_pays.
     g->window = window_pays(N, B, wide.K, win.K, warm, sm_count);
+    // Few candidates cut into many chunks wait for the walks behind failed boundaries, one after the
+    // other for each candidate, and those of many groups of few stages fail most (9 % of grown
+    // ones on 16 devices with 32 requests a slot, 1 % with 64: the order in which idle replicas were
+    // used).  A search on 16 devices over 30 000 requests, four traces, with 32 a slot and with 64 a
+    // group: 77, 84, 81, 108 and 64, 64, 65, 69 ms; a search over 5 600 35 and 36, three placements over
+    // 11 900 0.78 and 0.86: there the longer pass costs more than the walks.  Random placements have a
+    // third as many groups as slots.
+    if (g->window && !(opts && opts->warmup_requests > 0) && 2 * c->max_groups > c->max_slots &&
+        N >= 128 * 128) {
+        warm = 64 * (int64_t)c->max_groups;
+        if (warm > 2048) warm = 2048;
+    }
     const Cut &x = g->window ? win : wide;
     const int64_t NS = x.NS, spc = x.spc, K = x.K;
     if (K * (B > 0 ? B : 1) >= 0x7FFFFFFFLL) return MMS_ERR_UNSUPPORTED;   // work-list encoding

@@ -361,3 +361,17 @@ def test_models_with_many_replicas(replicas, copies):
         for name in ("good_total", "latency_sum", "model_num_good", "group_num_requests", "group_num_good"):
             few, many = (getattr(r, name) for r in both)
             assert np.repeat(few, copies, axis=0).tobytes() == many.tobytes(), name
+
+
+@pytest.mark.parametrize("n", [128 * 128 - 1, 128 * 128, 128 * 128 + 200])
+@pytest.mark.parametrize("groups", [7, 8, 9, 40])
+def test_longer_run_in_of_many_groups(n, groups):
+    """From 16 384 requests on few candidates of many groups get a run-in by groups instead of by
+    slots: below, at and above that, and with just half as many groups as slots."""
+    M = 6
+    profs = _profiles(M, (1, 2, 4), 31)
+    ts, ids, slos = _trace(n, M, 60.0, groups)
+    rng = np.random.RandomState(groups)
+    kinds = [sorted(set(rng.choice(M, size=rng.randint(1, 4)).tolist())) for _ in range(groups)]
+    degrees = [1] * groups if groups != 8 else [2] * groups          # 8: 16 slots
+    _check([_placement(degrees, kinds), _placement(degrees, sorted(kinds))], profs, ts, ids, slos, 0, 0)
