@@ -51,7 +51,8 @@ extern "C" {
 #define MMS_FLAG_LEGACY_CLOCK 2u  /* one clock per group: controller.py:506-558  */
 #define MMS_FLAG_NO_GROUP_GOOD 4u /* group_num_good is not wanted (not written);
                                      pass the same flags to the workspace query  */
-#define MMS_FLAG_CROWDED 8u       /* accepted, without effect                        */
+#define MMS_FLAG_CROWDED 8u       /* a hint, results do not depend on it: another call is
+                                     to run beside this one                          */
 #define MMS_FLAG_NO_TWINS 16u     /* a hint, results do not depend on it: do not look for
                                      interchangeable groups.  For lists whose placements
                                      have none (saves the bookkeeping); pass the same

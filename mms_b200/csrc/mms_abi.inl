@@ -53,12 +53,26 @@ struct Geometry {
 
 static size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 
-// Is the speculative pass of this batch faster with one candidate per warp than with 32?  A
-// warp of the former takes 0.15 to 0.2 us a request when it is alone on its scheduler and 0.4
+// Is the call faster with one candidate per warp in the speculative pass than with 32?  A warp of
+// the former takes 0.15 to 0.2 us a request when it is alone on its scheduler and up to 0.4
 // us beside two others; a warp of the latter 0.5 us alone and 0.9 us beside eleven on its SM, but
 // for 32 candidates: one candidate per warp pays while the GPU is short of candidates.
-// Estimated microseconds of both.
-static bool window_pays(int64_t N, int64_t B, int64_t K_wide, int64_t K_win, int64_t warm, int sm_count)
+// Estimated microseconds of both passes.
+//
+// What follows the pass counts too (`worth`).  One candidate per warp goes with longer chunks, so
+// fewer boundaries fail, and with a longer run-in where there are many groups (plan_call): the
+// pass may take four times as long with pipelines of up to four stages (whose windows go by groups), and twice as
+// long with deeper ones and more than two groups to three slots.  Measured over 209 lists of 4 to 330
+// placements (4 to 64 devices, 2 500 to 150 000 requests), both ways for each, by the ratio of the
+// estimates, 32 to a warp / one: up to four stages 1 to 2 0.73 / 0.59 ms (160 placements, 2 500
+// requests), 2 to 4 1.86 / 1.12 (75 on 8 devices, 30 000), 4 to 6 3.83 / 3.28 and 1.34 / 1.65, 7 to 9
+// 1.83 / 3.86; deeper ones of many groups 1 to 2 12.0 / 4.5 (75 on 32 devices, 80 000), 2.03 and 2.25
+// 1.97 / 2.26 and 2.18 / 2.04, 3 to 4 3.06 / 3.32; of few groups 1.34 2.47 / 3.95, 2.67 2.79 / 9.13.
+// Not on more than 32 slots (280 grown placements on 64 devices, 30 000 requests 14.1 / 18.5) and not
+// beside another call, whose warps want the issue slots (1025 placements on 16 devices in two
+// calls 3.7 / 4.7).
+static bool window_pays(int64_t N, int64_t B, int64_t K_wide, int64_t K_win, int64_t warm, int sm_count,
+                        double worth)
 {
     const double n_win = (double)N / K_win + (K_win > 1 ? warm : 0);
     const double n_wide = (double)N / K_wide + (K_wide > 1 ? warm : 0);
@@ -66,7 +80,7 @@ static bool window_pays(int64_t N, int64_t B, int64_t K_wide, int64_t K_win, int
     const double t_win = n_win * (warps_win <= 1.0 ? 0.18 : 0.18 + 0.11 * (warps_win - 1.0));
     double share = (double)((B + 31) / 32) * K_wide / (12.0 * sm_count);
     if (share > 1.0) share = 1.0;
-    return t_win < n_wide * (0.5 + 0.4 * share);
+    return t_win < worth * n_wide * (0.5 + 0.4 * share);
 }
 
 // Chunking, shared-memory and scratch geometry of one call.  `thrift` > 0 asks for less scratch at
@@ -200,7 +214,11 @@ static int plan_call(int64_t N, const mms_placements *c, const mms_sim_options *
                                thrifty ? thrifty : seg == 1024 ? 3 * seg : warm / 2);
     const Cut win = cut_trace(seg, (int64_t)g->window_blocks * kWindowWarps, thrifty ? thrifty : seg);
     // Which speculative pass: see window_pays.
-    g->window = window_pays(N, B, wide.K, win.K, warm, sm_count);
+    const double worth = flags & MMS_FLAG_CROWDED || c->max_slots > 32 ? 1.0
+                         : c->max_stages <= kGroupDepth                ? 4.0
+                         : 3 * c->max_groups > 2 * c->max_slots        ? 2.0
+                                                                       : 1.0;
+    g->window = window_pays(N, B, wide.K, win.K, warm, sm_count, worth);
     // Few candidates cut into many chunks wait for the walks behind failed boundaries, one after the
     // other for each candidate, and those of many groups of few stages fail most (9 % of grown
     // ones on 16 devices with 32 requests a slot, 1 % with 64: the order in which idle replicas were
@@ -541,11 +559,16 @@ int mms_trace_model_histogram(const mms_trace *trace, int32_t num_models, int32_
 size_t mms_sim_workspace_bytes(int64_t num_requests, const mms_placements *cands,
                                const mms_sim_options *opts, uint32_t flags)
 {
+    // enough with and without MMS_FLAG_CROWDED, which callers need not pass here
     mms::Geometry g;
-    if (mms::plan_call(num_requests, cands, opts, flags, !(flags & MMS_FLAG_NO_GROUP_GOOD), 0, &g) !=
-        MMS_OK)
-        return 0;
-    return g.total;
+    size_t most = 0;
+    for (const uint32_t crowded : {0u, (uint32_t)MMS_FLAG_CROWDED}) {
+        if (mms::plan_call(num_requests, cands, opts, (flags & ~MMS_FLAG_CROWDED) | crowded,
+                           !(flags & MMS_FLAG_NO_GROUP_GOOD), 0, &g) != MMS_OK)
+            return 0;
+        if (g.total > most) most = g.total;
+    }
+    return most;
 }
 
 }  // extern "C"

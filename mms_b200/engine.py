@@ -1269,7 +1269,8 @@ class ResidentBatch:
                  hard_options=None, launch_now=False):
         """mirrors: False = the library does not look for interchangeable groups
         (slower on placements that have them).
-        crowded: passes MMS_FLAG_CROWDED, which has no effect.
+        crowded: another batch is to run beside this one (MMS_FLAG_CROWDED, a hint; passed
+        for a split batch in any case).
         hard_options: sim_options for the launch that holds the placements with
         interchangeable groups, when the batch is split (default: `options`).
         launch_now: every call is enqueued as soon as its tables are uploaded
@@ -1297,7 +1298,7 @@ class ResidentBatch:
             main = torch.cuda.current_stream(dev)
             sides = _side_streams(main)
         for k, (_, e) in enumerate(parts):
-            flags = nat.FLAG_CROWDED if crowded else 0
+            flags = nat.FLAG_CROWDED if crowded or len(parts) > 1 else 0
             if not mirrors or not e.may_have_twins():
                 flags |= nat.FLAG_NO_TWINS
             opts_k = hard_options if len(parts) > 1 and k == 0 and hard_options is not None else options
@@ -1387,7 +1388,7 @@ def run_batch(trace: DeviceTrace, enc: EncodedBatch, table: LatencyTable,
     may take over speculative runs in which interchangeable groups have changed
     places (a speed-up of the time-parallel execution; results are the same
     with and without).
-    `crowded`: passes MMS_FLAG_CROWDED, which has no effect.
+    `crowded`: passes MMS_FLAG_CROWDED, a hint that another batch is to run beside this one.
     `rows_on_device` (with per_request): finish and good stay on the GPU, as
     BatchResult.finish_device / .good_device."""
     if not per_request:

@@ -375,3 +375,31 @@ def test_longer_run_in_of_many_groups(n, groups):
     kinds = [sorted(set(rng.choice(M, size=rng.randint(1, 4)).tolist())) for _ in range(groups)]
     degrees = [1] * groups if groups != 8 else [2] * groups          # 8: 16 slots
     _check([_placement(degrees, kinds), _placement(degrees, sorted(kinds))], profs, ts, ids, slos, 0, 0)
+
+
+@pytest.mark.parametrize("devices,degrees", [(16, (1,)), (16, (2, 4)), (16, (8, 1)), (32, (1, 8)), (33, (1,))])
+@pytest.mark.parametrize("copies", [3, 30])
+def test_either_speculative_pass(devices, degrees, copies):
+    """Lists in between, which are simulated one candidate to a warp when they are alone and 32 to a warp
+    beside another call, at the limits of that choice (stages, groups for slots, slots)."""
+    from mms_b200 import engine
+    M, n = 6, 20000
+    profs = _profiles(M, (1, 2, 4, 8), 41)
+    ts, ids, slos = _trace(n, M, 4.0 * devices, devices + copies, 0.01)
+    rng = np.random.RandomState(devices + len(degrees))
+    sols = []
+    for k in range(4):
+        dims = [degrees[0]] * (devices // degrees[0]) if k % 2 == 0 or len(degrees) == 1 else \
+            [degrees[1]] + [degrees[0]] * ((devices - degrees[1]) // degrees[0])
+        kinds = [sorted(set(rng.choice(M, size=rng.randint(1, 4)).tolist())) for _ in dims]
+        sols.append(_placement(dims, kinds if k < 2 else sorted(kinds)))
+    _check(sols, profs, ts, ids, slos, 0, 0)
+    trace = engine.DeviceTrace(ts, ids, slos, M)
+    table = engine.LatencyTable(profs)
+    enc = engine.encode_placements(sols * copies, table, M)
+    alone, beside = (engine.run_batch(trace, enc, table, group_good=True, crowded=c)[0] for c in (False, True))
+    few = engine.run_batch(trace, engine.encode_placements(sols, table, M), table, group_good=True)[0]
+    for name in ("good_total", "latency_sum", "model_num_good", "group_num_requests", "group_num_good"):
+        want = np.concatenate([getattr(few, name)] * copies)
+        assert getattr(alone, name).tobytes() == want.tobytes(), name
+        assert getattr(beside, name).tobytes() == want.tobytes(), name
