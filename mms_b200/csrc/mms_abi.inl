@@ -68,6 +68,10 @@ static size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 // requests), 2 to 4 1.86 / 1.12 (75 on 8 devices, 30 000), 4 to 6 3.83 / 3.28 and 1.34 / 1.65, 7 to 9
 // 1.83 / 3.86; deeper ones of many groups 1 to 2 12.0 / 4.5 (75 on 32 devices, 80 000), 2.03 and 2.25
 // 1.97 / 2.26 and 2.18 / 2.04, 3 to 4 3.06 / 3.32; of few groups 1.34 2.47 / 3.95, 2.67 2.79 / 9.13.
+// With few deep groups half as long again, for lists that do not fill the 32 lanes on up to 16
+// slots and any on up to 8 (15 random placements over 110 000 requests on 16 devices 1.43 / 1.13 ms, 6 on 8
+// over 150 000 0.61 / 0.46; 16 lists 0.85 to 1.44 times as fast, 1.17 in the mean), but not for more
+// on 16 (37 over 30 000 1.49 / 1.78, 230 over 8 000 1.75 / 2.71).
 // Not on more than 32 slots (280 grown placements on 64 devices, 30 000 requests 14.1 / 18.5) and not
 // beside another call, whose warps want the issue slots (1025 placements on 16 devices in two
 // calls 3.7 / 4.7).
@@ -217,6 +221,7 @@ static int plan_call(int64_t N, const mms_placements *c, const mms_sim_options *
     const double worth = flags & MMS_FLAG_CROWDED || c->max_slots > 32 ? 1.0
                          : c->max_stages <= kGroupDepth                ? 4.0
                          : 3 * c->max_groups > 2 * c->max_slots        ? 2.0
+                         : c->max_slots <= (B < kLanes ? 16 : 8)       ? 1.5
                                                                        : 1.0;
     g->window = window_pays(N, B, wide.K, win.K, warm, sm_count, worth);
     // Few candidates cut into many chunks wait for the walks behind failed boundaries, one after the

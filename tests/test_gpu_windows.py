@@ -377,8 +377,9 @@ def test_longer_run_in_of_many_groups(n, groups):
     _check([_placement(degrees, kinds), _placement(degrees, sorted(kinds))], profs, ts, ids, slos, 0, 0)
 
 
-@pytest.mark.parametrize("devices,degrees", [(16, (1,)), (16, (2, 4)), (16, (8, 1)), (32, (1, 8)), (33, (1,))])
-@pytest.mark.parametrize("copies", [3, 30])
+@pytest.mark.parametrize("devices,degrees", [(8, (8, 2)), (16, (1,)), (16, (2, 4)), (16, (8, 1)), (32, (1, 8)),
+                                             (33, (1,))])
+@pytest.mark.parametrize("copies", [3, 7, 8, 30])
 def test_either_speculative_pass(devices, degrees, copies):
     """Lists in between, which are simulated one candidate to a warp when they are alone and 32 to a warp
     beside another call, at the limits of that choice (stages, groups for slots, slots)."""
