@@ -1252,6 +1252,23 @@ def _side_streams(main):
     return _SIDE_STREAMS[key]
 
 
+def _calls_of(trace, enc, split, mirrors):
+    """The calls a batch is simulated in: [placement indices in the order of simulation, or None for all
+    as they are].  Where every placement has a trace of its own, placement k is simulated on trace k,
+    so such a batch is one call and stays in order."""
+    if getattr(trace, "num_traces", 1) > 1:
+        return [None]
+    parts = [None]
+    if split and mirrors and enc.has_twins is not None:
+        hard = np.flatnonzero(enc.has_twins)
+        least = SPLIT_MIN_EASY
+        if trace.num_requests * enc.B >= SPLIT_LONG:
+            least = min(least, SPLIT_MIN_EASY_LONG)
+        if len(hard) >= SPLIT_MIN_HARD and enc.B - len(hard) >= least:
+            parts = [hard, np.flatnonzero(~enc.has_twins)]
+    return [enc.by_depth(index) for index in parts]
+
+
 class ResidentBatch:
     """An encoded batch with its tables, scratch and outputs on the GPU, ready
     to be launched (any number of times).
@@ -1278,16 +1295,8 @@ class ResidentBatch:
         while the host prepares the second."""
         self.trace, self.enc = trace, enc
         dev = trace.device
-        parts = [None]
-        if split and mirrors and enc.has_twins is not None:
-            hard = np.flatnonzero(enc.has_twins)
-            least = SPLIT_MIN_EASY
-            if trace.num_requests * enc.B >= SPLIT_LONG:
-                least = min(least, SPLIT_MIN_EASY_LONG)
-            if len(hard) >= SPLIT_MIN_HARD and enc.B - len(hard) >= least:
-                parts = [hard, np.flatnonzero(~enc.has_twins)]
-        parts = [enc.by_depth(index) for index in parts]
-        parts = [(index, enc if index is None else enc.take(index)) for index in parts]
+        parts = [(index, enc if index is None else enc.take(index))
+                 for index in _calls_of(trace, enc, split, mirrors)]
         self.index = [p[0] for p in parts]
         self.jobs = []
         self.h2d_bytes = 0

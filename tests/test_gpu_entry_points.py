@@ -98,6 +98,45 @@ def test_trace_pack_matches_a_host_built_batch():
         assert per[t, 7] == 0
 
 
+@pytest.mark.parametrize("split", [True, False])
+@pytest.mark.parametrize("rows", [True, False])
+def test_placements_of_mixed_depth_keep_their_own_traces(rows, split):
+    """160 different placements, pipelines of eight and of one in turn, each on a trace of its own."""
+    from mms_b200 import cases, engine
+    from mms_b200.placement import ModelPlacement
+    from mms_b200.profiling import ParallelConfig
+    from oracle import tables
+    M, T = 8, 160
+    datas = cases.mixed_models(M, 20.0, 3.0)
+    profs = [d.profiling_result for d in datas]
+    rng = np.random.default_rng(21)
+    placements, arrivals, mids, slos = [], [], [], []
+    for t in range(T):
+        degree = 8 if t % 2 == 0 else 1
+        groups = 16 // degree
+        placements.append(ModelPlacement(
+            [ParallelConfig(1, 1, degree)] * groups,
+            [sorted(rng.choice(M, size=int(rng.integers(1, 4)), replace=False).tolist())
+             for _ in range(groups)]))
+        n = 300 + t
+        arrivals.append(np.cumsum(rng.exponential(1 / 30.0, n)))
+        mids.append(rng.integers(0, M, n).astype(np.int32))
+        slos.append(np.full(n, 0.6, np.float32))
+    layout = engine.DeviceTraceRows if rows else engine.DeviceTraceBatch
+    table = engine.LatencyTable(profs)
+    enc = engine.encode_placements(placements, table, M)
+    res, _, _ = engine.run_batch(layout(arrivals, mids, slos, M), enc, table, group_good=True,
+                                 split=split)
+    for t, p in enumerate(placements):
+        fin, good, mreq, mgood, greq, ggood = tables.one_placement(p, profs, mids[t], slos[t],
+                                                                   arrivals[t])
+        assert res.good_total[t] == np.count_nonzero(good), t
+        assert np.array_equal(res.model_num_requests[t], mreq), t
+        assert np.array_equal(res.model_num_good[t], mgood), t
+        assert np.array_equal(res.group_num_requests[t, :len(greq)], greq), t
+        assert np.array_equal(res.group_num_good[t, :len(ggood)], ggood), t
+
+
 def _device_stats(arrivals, which, K, finish, good, lo, window):
     import torch
     from mms_b200 import engine

@@ -439,3 +439,32 @@ def test_scratch_per_request():
         seg, swaps = (128, 64) if requests * slots * candidates / 16 <= 256e6 else (1024, 160)
         per = (16 * slots + slots + 6 * swaps) / seg * candidates + -(-candidates // 32) * 32
         assert need < 1.1 * per * requests
+
+
+def _one_depth_each(devices, count, twins_every):
+    """`count` placements that use every device, pipelines of eight and of one in turn, each group
+    with a model of its own; every `twins_every`-th one has two interchangeable groups."""
+    out = []
+    for k in range(count):
+        degree = (8, 1)[k % 2]
+        models = [[g] for g in range(devices // degree)]
+        if k % twins_every == 1:
+            models[1] = [0]
+        out.append(ModelPlacement([ParallelConfig(1, 1, degree)] * len(models), models))
+    return out
+
+
+@pytest.mark.parametrize("split", [True, False])
+def test_placements_with_traces_of_their_own_stay_in_order(split):
+    """Placement k is simulated on trace k: neither the order by depth nor the cut into two calls
+    may move it.  With one trace for all, the same list is both cut and ordered."""
+    from types import SimpleNamespace
+    datas = cases.mixed_models(32, 50.0, 3.0)
+    table = engine.LatencyTable([d.profiling_result for d in datas])
+    enc = engine.encode_placements(_one_depth_each(16, 700, 14), table, 32)
+    own = SimpleNamespace(num_requests=1000, num_traces=700)
+    assert engine._calls_of(own, enc, split, True) == [None]
+    shared = engine._calls_of(SimpleNamespace(num_requests=1000), enc, split, True)
+    assert len(shared) == (2 if split else 1)
+    assert sorted(np.concatenate(shared).tolist()) == list(range(700))
+    assert not np.array_equal(shared[-1], np.sort(shared[-1]))
