@@ -10,6 +10,7 @@ only; all compute goes through the C ABI in libmms_sim.so.
 import ctypes
 import functools
 import operator
+import threading
 from contextlib import nullcontext
 from itertools import chain, permutations, product
 from math import factorial, prod
@@ -245,7 +246,10 @@ class PinnedStager:
         from concurrent.futures import ThreadPoolExecutor
         self.device, self.threads, self.piece = torch.device(dev), int(threads), int(piece_bytes)
         self.pool = ThreadPoolExecutor(self.threads)
-        self.streams = [torch.cuda.Stream(device=self.device) for _ in range(self.threads)]
+        # of high priority, which torch takes from a pool of their own: a stream that kernels are
+        # queued on (torch has 32 per priority and hands them out in turn) would hold the copies up
+        self.streams = [torch.cuda.Stream(device=self.device, priority=-1)
+                        for _ in range(self.threads)]
         self.buffers = [[torch.empty(self.piece, dtype=torch.uint8).pin_memory() for _ in range(2)]
                         for _ in range(self.threads)]
 
@@ -276,7 +280,7 @@ class PinnedStager:
         def work(k):
             stream, bufs = self.streams[k], self.buffers[k]
             events = [None, None]
-            stream.wait_stream(main)            # the destinations were allocated there
+            stream.wait_stream(main)            # the destinations are free to write there
             with torch.cuda.device(self.device), torch.cuda.stream(stream):
                 for j, (d8, src, lo, hi) in enumerate(pieces[k]):
                     if events[j & 1] is not None:
@@ -314,9 +318,12 @@ class DeviceTraceBatch:
     flags = 0
 
     def __init__(self, arrivals: Sequence, model_ids: Sequence, slos: Sequence, num_models: int,
-                 device=None, staged=False):
-        """staged: upload through PinnedStager (worth it from about a gigabyte)."""
+                 device=None, staged=False, owner=None):
+        """staged: upload through PinnedStager (worth it from about a gigabyte).
+        owner: the stream from whose memory the traces are taken (None: the current one, on which
+        they are uploaded and counted in any case)."""
         _require_cuda()
+        self.owner = owner
         self.device = torch.device("cuda", torch.cuda.current_device()) if device is None \
             else torch.device(device)
         T = len(arrivals)
@@ -362,8 +369,16 @@ class DeviceTraceBatch:
                 dst.copy_(torch.from_numpy(src), non_blocking=True)
 
     def _empty(self, shape):
-        return tuple(torch.empty(shape, dtype=t, device=self.device)
-                     for t in (torch.float64, torch.int32, torch.float32))
+        here = torch.cuda.current_stream(self.device)
+        owner = here if self.owner is None else self.owner
+        with torch.cuda.stream(owner):
+            new = tuple(torch.empty(shape, dtype=t, device=self.device)
+                        for t in (torch.float64, torch.int32, torch.float32))
+        if owner != here:
+            here.wait_stream(owner)         # what used the memory before is in order there
+            for t in new:
+                t.record_stream(here)       # and it is not handed out again before `here` is done
+        return new
 
     def _store(self, sources, staged):
         N, T = self.num_requests, self.num_traces
@@ -1267,6 +1282,44 @@ def _calls_of(trace, enc, split, mirrors):
         if len(hard) >= SPLIT_MIN_HARD and enc.B - len(hard) >= least:
             parts = [hard, np.flatnonzero(~enc.has_twins)]
     return [enc.by_depth(index) for index in parts]
+
+
+class StreamLease:
+    """`count` streams of a device that nobody else has, until give_back() (or the end of this
+    object).  torch.cuda.Stream() hands out 32 streams in turn: of streams made for each call two
+    soon are one, and what was to run beside a kernel of 40 ms waits behind it; and torch keeps
+    freed memory by stream, so each new one begins with none."""
+
+    _lock = threading.RLock()       # (give_back may be called by the garbage collector)
+    _known, _free = {}, {}          # per device: handles that were ever lent, streams at hand
+
+    def __init__(self, count, main):
+        """main: the calling stream, which is not among them."""
+        dev = main.device
+        self.device, self.streams = dev, []
+        with self._lock:
+            known, free = self._known.setdefault(dev, set()), self._free.setdefault(dev, [])
+            while len(self.streams) < count:
+                spare = [s for s in free if s.cuda_stream != main.cuda_stream]
+                if spare:
+                    stream = spare[-1]
+                    free.remove(stream)
+                else:
+                    for _ in range(32):         # beyond that many there are no others: shared
+                        stream = torch.cuda.Stream(device=dev)
+                        if stream.cuda_stream not in known and stream != main:
+                            break
+                    known.add(stream.cuda_stream)
+                self.streams.append(stream)
+
+    def give_back(self):
+        with self._lock:
+            free = self._free[self.device]
+            # (in the order in which they go out again)
+            free.extend(s for s in reversed(self.streams) if s not in free)
+            self.streams = []
+
+    __del__ = give_back
 
 
 class ResidentBatch:

@@ -286,23 +286,24 @@ class ResidentSweep:
         if eager:                                   # the longest walk starts first
             self.groups.sort(key=lambda idx: -int(lengths[idx].max()))
         self.h2d_bytes = 0
-        self.jobs, self.streams, self.meta = [], [], []
+        self.jobs, self.meta = [], []
         main = torch.cuda.current_stream(self.device)
-        for idx in self.groups:
-            side = torch.cuda.Stream(device=self.device)
+        self.lease = engine.StreamLease(len(self.groups), main)
+        self.streams = list(self.lease.streams)
+        for idx, side in zip(self.groups, self.streams):
             side.wait_stream(main)
             with torch.cuda.stream(side if eager else main):
+                # (memory from the calling stream's: whatever runs there next can have it)
                 traces = engine.DeviceTraceRows([workloads[t].arrivals for t in idx],
                                                 [arrays[t][0] for t in idx],
                                                 [arrays[t][1] for t in idx], M,
-                                                device=self.device, staged=eager)
+                                                device=self.device, staged=eager, owner=main)
                 job = engine.ResidentBatch(traces, sweep.enc.repeat(len(idx)), sweep.table,
                                            options=sweep.options, split=False)
                 if eager:
                     job.launch()
             self.h2d_bytes += traces.h2d_bytes + job.h2d_bytes
             self.jobs.append(job)
-            self.streams.append(side)
             cell = torch.from_numpy(((sweep.first_trace + idx) % cells).astype(np.int64)).to(
                 self.device)
             n = torch.from_numpy(lengths[idx]).to(self.device)
@@ -357,9 +358,11 @@ class ResidentSweep:
         return res
 
     def release(self):
+        """Gives scratch and streams back; every launch has finished (results() waits)."""
         for job in self.jobs:
             job.release()
         self.jobs = []
+        self.lease.give_back()
 
 
 class TraceSweep:

@@ -98,6 +98,64 @@ def test_trace_pack_matches_a_host_built_batch():
         assert per[t, 7] == 0
 
 
+def _small_sweep():
+    """Eighty traces in two groups of lengths, 10 to 25 MB each on the device."""
+    from mms_b200 import cases
+    from mms_b200.placement import TraceSweep
+    case = cases.sweep_case(duration=40.0, total_rate=400.0)
+    sweep = TraceSweep(case.model_datas, case.cluster_env, case.placement, cells=16)
+    picked = [t for t in range(160) if t % 4 in (1, 2)]        # rate scales 1 and 2
+    return sweep, [case.trace(t) for t in picked]
+
+
+def test_sweeps_keep_their_streams_and_give_memory_back():
+    """A sweep's groups, the uploads and the caller are on streams of their own in every call, and
+    what a call takes is there for the next one."""
+    import torch
+    from mms_b200 import engine, placement
+    sweep, workloads = _small_sweep()
+    want, _ = sweep.evaluate_tally(workloads)
+    sweep.evaluate_tally(workloads)
+    reserved, seen = torch.cuda.memory_reserved(), set()
+    copies = {s.cuda_stream for s in engine.PinnedStager.get(torch.device("cuda", 0)).streams}
+    for _ in range(20):
+        run = placement.ResidentSweep(sweep, workloads, 16, eager=True)
+        mine = [s.cuda_stream for s in run.streams]
+        assert len(run.groups) >= 2 and len(set(mine)) == len(mine)
+        assert not copies & set(mine) and torch.cuda.current_stream().cuda_stream not in mine
+        seen |= set(mine)
+        run.tally_launched()
+        run.results()
+        run.release()
+        del run
+    assert len(seen) == len(mine)
+    got, _ = sweep.evaluate_tally(workloads)
+    assert torch.cuda.memory_reserved() == reserved
+    for a, b in zip(want, got):
+        assert a[0] == b[0] and a[2] == b[2] and np.array_equal(a[1], b[1])
+
+
+def test_two_sweeps_at_once_share_no_stream_and_no_memory():
+    import torch
+    from mms_b200 import placement
+    sweep, workloads = _small_sweep()
+    want, _ = sweep.evaluate_tally(workloads)
+    runs = [placement.ResidentSweep(sweep, ws, 16, eager=True)
+            for ws in (workloads, workloads[::-1])]
+    streams = [s.cuda_stream for run in runs for s in run.streams]
+    assert len(set(streams)) == len(streams)
+    other = torch.cuda.Stream()
+    with torch.cuda.stream(other):              # a caller that is not on the default stream
+        third, _ = sweep.evaluate_tally(workloads)
+    for run, order in zip(runs, (1, -1)):
+        run.tally_launched()
+        good = run.results().good_total[::order]
+        run.release()
+        assert np.array_equal(good / np.array([len(w.arrivals) for w in workloads]),
+                              [r[0] for r in want])
+    assert [r[0] for r in third] == [r[0] for r in want]
+
+
 @pytest.mark.parametrize("split", [True, False])
 @pytest.mark.parametrize("rows", [True, False])
 def test_placements_of_mixed_depth_keep_their_own_traces(rows, split):

@@ -468,3 +468,39 @@ def test_placements_with_traces_of_their_own_stay_in_order(split):
     assert len(shared) == (2 if split else 1)
     assert sorted(np.concatenate(shared).tolist()) == list(range(700))
     assert not np.array_equal(shared[-1], np.sort(shared[-1]))
+
+
+def test_lent_streams_are_nobody_elses(monkeypatch):
+    """torch hands out 32 streams in turn; those lent at one time differ from one another and from the
+    calling stream, come back in the order they went out, and are shared only when there are no more."""
+    from types import SimpleNamespace
+
+    import torch
+    made = []
+
+    def stream(device):
+        made.append(device)
+        return SimpleNamespace(cuda_stream=1 + (len(made) - 1) % 32, device=device)
+    monkeypatch.setattr(torch.cuda, "Stream", stream)
+    monkeypatch.setattr(engine.StreamLease, "_known", {})
+    monkeypatch.setattr(engine.StreamLease, "_free", {})
+
+    def handles(lease):
+        return [s.cuda_stream for s in lease.streams]
+    main = stream("gpu")                       # a stream of the user's from the same 32
+    one = engine.StreamLease(3, main)
+    two = engine.StreamLease(2, main)
+    first = handles(one)
+    assert len({1, *first, *handles(two)}) == 6
+    one.give_back()
+    for _ in range(40):                        # call after call: the same ones
+        again = engine.StreamLease(3, main)
+        assert handles(again) == first
+        del again
+    assert len(made) == 6
+    lent = [engine.StreamLease(1, main) for _ in range(29)]
+    everyone = {h for lease in lent for h in handles(lease)} | set(handles(two))
+    assert len(everyone) == 31 and 1 not in everyone
+    assert len(handles(engine.StreamLease(4, main))) == 4
+    other = engine.StreamLease(2, SimpleNamespace(cuda_stream=0, device="other"))
+    assert len(set(handles(other))) == 2
