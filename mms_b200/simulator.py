@@ -279,6 +279,19 @@ class DeviceColumn:
         return iter(self._get())
 
 
+def _by_appearance(which, counts):
+    """The numbers in `which`, each once, in order of first appearance; counts[k]: how often k is there.
+    Most have appeared long before the end, and one that has not costs a pass in linear time."""
+    present, seen = sum(c > 0 for c in counts), []
+    for size in (256, 4096, len(which)):
+        if len(seen) < present:
+            head = which[:size]
+            first = np.full(len(counts), len(head), np.int64)
+            first[head[::-1]] = np.arange(len(head) - 1, -1, -1)    # the last write is the first one
+            seen = np.argsort(first, kind="stable")[:np.count_nonzero(first < len(head))].tolist()
+    return seen
+
+
 def device_stats(workload, start, finish_dev, good_dev, warmup) -> StatsResult:
     """Workload.compute_stats (workload.py:308-354) from per-request outputs
     that are still on the GPU (finish f64[N], good u8[N] torch tensors): the
@@ -302,12 +315,7 @@ def device_stats(workload, start, finish_dev, good_dev, warmup) -> StatsResult:
     start_w, which_w = np.asarray(start)[lo:hi], which[lo:hi]
     # names in order of first appearance, then a stable sort by request count (:321-326)
     counts = st["num_requests"].tolist()
-    present, seen = sum(c > 0 for c in counts), []
-    for size in (256, 4096, window):      # (most have appeared long before the end)
-        if len(seen) < present:
-            names, at = np.unique(which_w[:size], return_index=True)
-            seen = names[np.argsort(at)].tolist()
-    ordered = sorted(seen, key=counts.__getitem__)
+    ordered = sorted(_by_appearance(which_w, counts), key=counts.__getitem__)
     host = {}
 
     def rows():

@@ -8,7 +8,7 @@ import pytest
 
 from mms_b200 import _native as nat
 from mms_b200 import build as mms_build
-from mms_b200 import cases, engine
+from mms_b200 import cases, engine, simulator
 from mms_b200.placement import ModelPlacement
 from mms_b200.profiling import ParallelConfig
 from oracle import tables
@@ -504,3 +504,39 @@ def test_lent_streams_are_nobody_elses(monkeypatch):
     assert len(handles(engine.StreamLease(4, main))) == 4
     other = engine.StreamLease(2, SimpleNamespace(cuda_stream=0, device="other"))
     assert len(set(handles(other))) == 2
+
+
+@pytest.mark.parametrize("n, rare_at", [(2, 1), (255, 254), (256, 200), (257, 256), (4097, 4096),
+                                        (5000, 4000), (150_000, 149_999), (150_000, 300)])
+def test_models_in_order_of_first_appearance(monkeypatch, n, rare_at):
+    """Statistics list models by request count, equal ones in order of first appearance.  A model that first
+    appears late costs a pass over the requests, not a sort of them (ten times as long)."""
+    from types import SimpleNamespace
+    K, rare = 7, 5                                 # model 6 is registered and never asked for
+    which = np.random.default_rng(n).integers(0, 5, n).astype(np.int32)
+    which[rare_at] = rare
+    counts = np.bincount(which, minlength=K)
+    sorted_at_once = [0]
+
+    def watched(name):
+        original = getattr(np, name)
+
+        def call(a, *args, **kwargs):
+            sorted_at_once[0] = max(sorted_at_once[0], np.size(a))
+            return original(a, *args, **kwargs)
+        monkeypatch.setattr(np, name, call)
+    fields = ("last_start", "first_start", "latency_mean", "latency_std", "latency_p90", "latency_p99")
+    stats = {f: np.ones((1, K)) for f in fields}
+    stats.update(num_requests=counts, num_good=np.zeros((1, K), np.int64), good_total=np.zeros(1),
+                 latency_sum=np.zeros(1))
+    monkeypatch.setattr(engine, "_to_device_many", lambda arrays, device: arrays)
+    monkeypatch.setattr(engine, "device_compute_stats", lambda *args: stats)
+    arrivals = np.arange(n, dtype=np.float64)
+    workload = SimpleNamespace(arrivals=arrivals, name_index=which, names=[f"m{k}" for k in range(K)])
+    rows = SimpleNamespace(device="none", reshape=lambda *shape: None)
+    for name in ("unique", "argsort", "sort"):
+        watched(name)
+    result = simulator.device_stats(workload, arrivals, rows, rows, 0)
+    want = sorted(dict.fromkeys(which.tolist()), key=lambda k: counts[k])
+    assert [m.name for m in result.per_model_stats] == [f"m{k}" for k in want]
+    assert sorted_at_once[0] <= 4096
