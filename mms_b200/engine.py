@@ -37,10 +37,10 @@ def _ptr(t):
     return ctypes.c_void_p(t.data_ptr()) if t is not None and t.numel() > 0 else ctypes.c_void_p(0)
 
 
-def _raw_stream():
-    """The current stream of the current device as CUDA's handle, 0 for the default one
+def _raw_stream(index=None):
+    """The current stream of a device (None: the current one) as CUDA's handle, 0 for the default one
     (torch.cuda.current_stream() makes an object of it, which takes longer than a launch)."""
-    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if index is None else index)
 
 
 def _stream_ptr():
@@ -1167,10 +1167,10 @@ def _to_host(t):
 
 
 def _on_stream(stream, dev):
-    """`stream` (None: the default one) of `dev` as the current stream, where it is not."""
-    with _on(dev):
-        if _raw_stream() == (stream.cuda_stream if stream is not None else 0):
-            return _on(dev)
+    """`dev` as the current device and `stream` (None: the default one) as its current stream, where they
+    are not."""
+    if _raw_stream(dev.index) == (stream.cuda_stream if stream is not None else 0):
+        return _on(dev)
     return torch.cuda.stream(stream if stream is not None else torch.cuda.default_stream(dev))
 
 

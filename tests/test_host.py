@@ -540,3 +540,31 @@ def test_models_in_order_of_first_appearance(monkeypatch, n, rare_at):
     want = sorted(dict.fromkeys(which.tolist()), key=lambda k: counts[k])
     assert [m.name for m in result.per_model_stats] == [f"m{k}" for k in want]
     assert sorted_at_once[0] <= 4096
+
+
+def _fake_devices(monkeypatch, raw):
+    """Two devices whose current streams have the handles `raw`; returns the number of the current one."""
+    from contextlib import contextmanager
+
+    import torch
+    current = [0]
+
+    @contextmanager
+    def device(d):
+        before, current[0] = current[0], torch.device(d).index
+        yield
+        current[0] = before
+    monkeypatch.setattr(torch.cuda, "current_device", lambda: current[0])
+    monkeypatch.setattr(torch.cuda, "device", device)
+    monkeypatch.setattr(torch._C, "_cuda_getCurrentRawStream", lambda index: raw[index], raising=False)
+    return current
+
+
+def test_results_are_read_on_the_device_they_are_on(monkeypatch):
+    """Another device is the current one when results are read: theirs is while they are, also where their
+    stream is its current one already."""
+    import torch
+    current = _fake_devices(monkeypatch, [7, 0])
+    with engine._on_stream(None, torch.device("cuda", 1)):
+        assert current[0] == 1
+    assert current[0] == 0
