@@ -39,8 +39,15 @@ def _ptr(t):
 
 def _raw_stream(index=None):
     """The current stream of a device (None: the current one) as CUDA's handle, 0 for the default one
-    (torch.cuda.current_stream() makes an object of it, which takes longer than a launch)."""
-    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if index is None else index)
+    (torch.cuda.current_stream() makes an object of it, which takes longer than a launch; the name in
+    torch._C is private, and a torch without it goes that way)."""
+    if index is None:
+        index = torch.cuda.current_device()
+    try:
+        ask = torch._C._cuda_getCurrentRawStream
+    except AttributeError:
+        return torch.cuda.current_stream(index).cuda_stream
+    return ask(index)
 
 
 def _stream_ptr():

@@ -568,3 +568,16 @@ def test_results_are_read_on_the_device_they_are_on(monkeypatch):
     with engine._on_stream(None, torch.device("cuda", 1)):
         assert current[0] == 1
     assert current[0] == 0
+
+
+def test_stream_handles_without_the_private_name(monkeypatch):
+    """A torch whose C module has no raw stream query: the public object's handle."""
+    from types import SimpleNamespace
+
+    import torch
+    _fake_devices(monkeypatch, [0, 0])
+    monkeypatch.delattr(torch._C, "_cuda_getCurrentRawStream")
+    monkeypatch.setattr(torch.cuda, "current_stream",
+                        lambda device=None: SimpleNamespace(cuda_stream={0: 40, 1: 41}[device]))
+    assert engine._raw_stream() == 40 and engine._raw_stream(1) == 41
+    assert engine._stream_ptr().value == 40
