@@ -59,22 +59,7 @@ static size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 // for 32 candidates: one candidate per warp pays while the GPU is short of candidates.
 // Estimated microseconds of both passes.
 //
-// What follows the pass counts too (`worth`).  One candidate per warp goes with longer chunks, so
-// fewer boundaries fail, and with a longer run-in where there are many groups (plan_call): the
-// pass may take four times as long with pipelines of up to four stages (whose windows go by groups), and twice as
-// long with deeper ones and more than two groups to three slots.  Measured over 209 lists of 4 to 330
-// placements (4 to 64 devices, 2 500 to 150 000 requests), both ways for each, by the ratio of the
-// estimates, 32 to a warp / one: up to four stages 1 to 2 0.73 / 0.59 ms (160 placements, 2 500
-// requests), 2 to 4 1.86 / 1.12 (75 on 8 devices, 30 000), 4 to 6 3.83 / 3.28 and 1.34 / 1.65, 7 to 9
-// 1.83 / 3.86; deeper ones of many groups 1 to 2 12.0 / 4.5 (75 on 32 devices, 80 000), 2.03 and 2.25
-// 1.97 / 2.26 and 2.18 / 2.04, 3 to 4 3.06 / 3.32; of few groups 1.34 2.47 / 3.95, 2.67 2.79 / 9.13.
-// With few deep groups half as long again, for lists that do not fill the 32 lanes on up to 16
-// slots and any on up to 8 (15 random placements over 110 000 requests on 16 devices 1.43 / 1.13 ms, 6 on 8
-// over 150 000 0.61 / 0.46; 16 lists 0.85 to 1.44 times as fast, 1.17 in the mean), but not for more
-// on 16 (37 over 30 000 1.49 / 1.78, 230 over 8 000 1.75 / 2.71).
-// Not on more than 32 slots (280 grown placements on 64 devices, 30 000 requests 14.1 / 18.5) and not
-// beside another call, whose warps want the issue slots (1025 placements on 16 devices in two
-// calls 3.7 / 4.7).
+// What follows the pass counts too: `worth`, below.
 static bool window_pays(int64_t N, int64_t B, int64_t K_wide, int64_t K_win, int64_t warm, int sm_count,
                         double worth)
 {
@@ -85,6 +70,41 @@ static bool window_pays(int64_t N, int64_t B, int64_t K_wide, int64_t K_win, int
     double share = (double)((B + 31) / 32) * K_wide / (12.0 * sm_count);
     if (share > 1.0) share = 1.0;
     return t_win < worth * n_wide * (0.5 + 0.4 * share);
+}
+
+// How many times as long the pass with one candidate per warp may take, by that estimate.  It goes with
+// longer chunks, so fewer boundaries fail, and with a longer run-in where there are many groups (plan_call),
+// and the walks behind failed boundaries are often most of the call; by how much depends on how
+// many groups there are to get out of order, and the more candidates, the less a failed one stands alone.
+// Where single devices are among the groups ("whole": as many groups as slots, the lists a search makes over all
+// partitions) that is most, in a few deep pipelines least.
+//
+// Measured: 3 664 lists of 1 to 800 placements (random, grown over all partitions and over one; 4 to 32
+// devices, 2 000 to 150 000 requests), both passes for each, 32 to a warp / one.  In geometric
+// mean, lists slower than 0.95 times: up to four stages, whole, fewer than 128 placements 1.87 and 1 %, more of them
+// 1.56 and 1 %; more than a group to three slots 1.48 and 1 %, fewer 1.29 and 2 %; deeper ones, whole
+// 1.51 and 2 %; on up to 8 slots 1.34 and 4 %.  Just behind these lines, up to half as much again, 25 to 50 % of
+// the lists are slower: 445 placements of two pipelines of four over 10 000 requests 0.47 / 1.17 ms, 262 random ones
+// on 16 devices over 12 000 3.4 / 7.1 (deep, 12 groups: no line at all, as in general on 16 slots and more).
+// (Of 2 267 further lists 1 211 are inside these lines: 1.57 times as fast in the mean, 0.8 % of them slower than
+// 0.95 times, the slowest 0.81.)
+// Not on more than 32 slots (280 grown placements on 64 devices, 30 000 requests 14.1 / 18.5) and not
+// in the two calls of a list that is split (1025 placements on 16 devices 3.7 / 4.7), which pass
+// MMS_FLAG_CROWDED.  The two parts of a list that goes out pipelined, and the groups of a sweep, do
+// not pass it: 754 such lists on 4 to 32 devices are 0.74 to 1.04 times as fast with it, 0.99 in the mean, 143
+// sweeps 0.75 to 1.04.
+static double window_worth(const mms_placements *c, int64_t B, uint32_t flags)
+{
+    const int32_t T = c->max_slots, G = c->max_groups;
+    if (flags & MMS_FLAG_CROWDED || T > 32) return 1.0;
+    const bool whole = G >= T, few = B < 128;
+    if (c->max_stages <= kGroupDepth) {
+        if (whole) return few ? 4.0 : c->max_stages == 1 || T > 8 ? 3.0 : 2.0;
+        return 3 * G > T ? (few ? 2.5 : 2.0) : 1.5;
+    }
+    if (whole) return few || T > 8 ? 2.0 : 1.5;
+    if (T > 8) return 1.0;
+    return few && 2 * G > T ? 2.0 : 1.25;
 }
 
 // Chunking, shared-memory and scratch geometry of one call.  `thrift` > 0 asks for less scratch at
@@ -218,12 +238,7 @@ static int plan_call(int64_t N, const mms_placements *c, const mms_sim_options *
                                thrifty ? thrifty : seg == 1024 ? 3 * seg : warm / 2);
     const Cut win = cut_trace(seg, (int64_t)g->window_blocks * kWindowWarps, thrifty ? thrifty : seg);
     // Which speculative pass: see window_pays.
-    const double worth = flags & MMS_FLAG_CROWDED || c->max_slots > 32 ? 1.0
-                         : c->max_stages <= kGroupDepth                ? 4.0
-                         : 3 * c->max_groups > 2 * c->max_slots        ? 2.0
-                         : c->max_slots <= (B < kLanes ? 16 : 8)       ? 1.5
-                                                                       : 1.0;
-    g->window = window_pays(N, B, wide.K, win.K, warm, sm_count, worth);
+    g->window = window_pays(N, B, wide.K, win.K, warm, sm_count, window_worth(c, B, flags));
     // Few candidates cut into many chunks wait for the walks behind failed boundaries, one after the
     // other for each candidate, and those of many groups of few stages fail most (9 % of grown
     // ones on 16 devices with 32 requests a slot, 1 % with 64: the order in which idle replicas were
