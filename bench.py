@@ -724,6 +724,7 @@ def run_batching(args, D, candidates=1024, duration=3600.0, steps=None, cpu=True
     span_ms, span_tag = nat.profile_end()
     stream_ms = span_ms[span_tag == nat.PROFILE_BATCH_STREAM]
     chain_ms = span_ms[span_tag == nat.PROFILE_BATCH_CHAIN]
+    repairs = int(np.count_nonzero(span_tag == nat.PROFILE_BATCH_REPAIR))
     res, _ = job.results(per_request=False)
     assert not np.any(res.status), "kernel status words are not clean"
     total_ms = D.reduce(sum(times), "max")
@@ -771,10 +772,9 @@ def run_batching(args, D, candidates=1024, duration=3600.0, steps=None, cpu=True
                      "algorithmic_bytes_per_launch": B * N * BYTES_PER_UNIT_FULL},
         "e2e": {"value": e2e_value, "unit": UNIT, "h2d_bytes_per_step": int(h2d),
                 "d2h_bytes_per_step": int(d2h)},
-        # cut-or-not, tables, stream, three rounds of validate and repair, validate, chain, counters,
-        # leaf sums, totals; the tables only where 32 candidates go to a warp
-        # (short chunks, of few placements, get a round of walks)
-        "gpu_launches": (8 if B > 26 else 10) * steps,
+        # order, stream, the same for odd traces, judge, chain, tally, counters, totals; with short
+        # chunks also a walk and a judgement (a span each round); of a trace in one piece no boundaries
+        "gpu_launches": 6 * steps + (2 * repairs - steps if repairs else 0) + len(chain_ms),
         "chunks_resimulated_per_candidate": float(np.mean(res.resimulated)),
         "clocks": clk.summary(),
     }

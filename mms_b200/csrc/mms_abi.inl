@@ -1182,20 +1182,21 @@ int mms_sim_batching(const mms_trace *trace, const mms_placements *cands,
         MMS_TRY(allow_smem((const void *)kern.walk, geo.smem));
         MMS_TRY(allow_smem((const void *)kern.chain, geo.smem));
         const int64_t bounds = (int64_t)B * (a.K - 1);
-        ProfileSpan repair_span(MMS_PROFILE_BATCH_REPAIR, st);
         // round a.rounds only judges the boundaries, for batch_chain_kernel
         for (int r = 0; r <= a.rounds; ++r) {
+            ProfileSpan repair_span(MMS_PROFILE_BATCH_REPAIR, st);
             a.round = r;
             BatchArgs judge = a;
             judge.table_elems = 0;
             judge.warp0 = 0;
             kern.judge<<<blocks_for(bounds, false), threads, geo.smem_judge, st>>>(judge);
             MMS_CUDA(cudaGetLastError());
-            if (r == a.rounds) break;
-            kern.walk<<<blocks_for(bounds, true), threads, geo.smem, st>>>(a);
-            MMS_CUDA(cudaGetLastError());
+            if (r < a.rounds) {
+                kern.walk<<<blocks_for(bounds, true), threads, geo.smem, st>>>(a);
+                MMS_CUDA(cudaGetLastError());
+            }
+            repair_span.stop();
         }
-        repair_span.stop();
         ProfileSpan chain_span(MMS_PROFILE_BATCH_CHAIN, st);
         kern.chain<<<blocks_for(B, false), threads, geo.smem, st>>>(a);
         MMS_CUDA(cudaGetLastError());
