@@ -193,8 +193,8 @@ class DeviceTrace:
                       "mms_trace_model_histogram")
 
     def next_same_model(self):
-        """i32[N] on the device: index of the next request with the same model
-        (the per-model FIFO queues of the batching simulator run along it)."""
+        """i32[N] on the device: index of the next request with the same model, -1 if there is none
+        (a model's FIFO queue is a run of this list)."""
         if getattr(self, "_next_same", None) is None:
             with _on(self.device):
                 buf = torch.empty(max(self.num_requests, 1), dtype=torch.int32,

@@ -7,7 +7,9 @@ import pytest
 pytestmark = pytest.mark.gpu
 
 
-def _check(placements, profs, ts, ids, slos, sizes=(1, 2, 4, 8)):
+def _check(placements, profs, ts, ids, slos, sizes=(1, 2, 4, 8), full_heap=False):
+    """Every placement against the CPU checker.  full_heap: room for one pending event per group of the
+    largest placement and no more."""
     import torch
     assert torch.cuda.is_available(), "GPU tests need a CUDA device"
     from mms_b200 import engine
@@ -15,7 +17,7 @@ def _check(placements, profs, ts, ids, slos, sizes=(1, 2, 4, 8)):
     trace = engine.DeviceTrace(ts, ids, slos, len(profs))
     table = engine.LatencyTable(profs, list(sizes))
     enc = engine.encode_placements(placements, table, len(profs))
-    res = engine.run_batch_batching(trace, enc, table)
+    res = engine.run_batch_batching(trace, enc, table, heap_capacity=enc.G if full_heap else 0)
     for b, p in enumerate(placements):
         fin, good, mreq, mgood, greq, ggood = tables.one_placement(p, profs, ids, slos, ts,
                                                                    batchsize_config=sizes)
@@ -67,6 +69,38 @@ def test_interchangeable_groups_that_take_turns(rate, grid):
             _placement([(1, [0, 1, 2])] * 8 + pairs),
             _placement([(1, [3]), (1, [3, 4]), (1, [3]), (1, [4, 3]), (2, [3])])]
     _check(sols, profs, ts, ids, slo[ids])
+
+
+@pytest.mark.parametrize("rate", [3.0, 20.0])
+def test_labels_spare_walks(rate):
+    """Two placements that do the same: in the second the groups of a pair are not interchangeable, because
+    one of each also has a model that is never asked for.  There a run with the pair the wrong way round is
+    simulated again; the first takes it over."""
+    profs, slo = _profiles(7)
+    ts, ids = _trace(24000, 6, rate, 0.0, 9)
+    alike = _placement([(1, [4]), (1, [4]), (2, [5]), (2, [5]), (1, [0]), (1, [0]), (4, [1, 2, 3])])
+    told_apart = _placement([(1, [4]), (1, [4, 6]), (2, [5]), (2, [5, 6]), (1, [0]), (1, [0, 6]), (4, [1, 2, 3])])
+    res = _check([alike, told_apart], profs, ts, ids, slo[ids])
+    assert np.array_equal(res.finish[0], res.finish[1])
+    assert 4 * res.resimulated[0] < res.resimulated[1]
+
+
+@pytest.mark.parametrize("rate", [60.0, 400.0])
+def test_room_for_one_pending_event_per_group(rate):
+    """Bursts on a grid, in which groups have several events pending at a time: with room for one per group
+    a run is right or reports that it was not enough, as it does for some; by default there is enough."""
+    profs, slo = _profiles(6)
+    ts, ids = _trace(6000, 6, rate, 0.05, 4)
+    overflows = 0
+    for groups in (3, 31, 32, 40):
+        sols = [_placement([(1, [k % 6, (k + 1) % 6]) for k in range(groups)])]
+        try:
+            _check(sols, profs, ts, ids, slo[ids], full_heap=True)
+        except RuntimeError as e:
+            assert "heap overflow" in str(e)
+            overflows += 1
+        _check(sols, profs, ts, ids, slo[ids])
+    assert overflows
 
 
 @pytest.mark.parametrize("groups", [31, 32, 33, 64, 65, 130])

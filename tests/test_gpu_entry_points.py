@@ -406,3 +406,20 @@ def test_tallies_of_few_and_many_candidates(count, n):
             assert np.array_equal(res.group_num_good[b, :len(ggood)], ggood)
             assert res.good_total[b] == np.count_nonzero(good)
             assert res.latency_sum[b] == float(np.add.reduce(fin - arr))
+
+
+@pytest.mark.parametrize("n", [1, 31, 32, 33, 511, 4097, 20011])
+def test_next_request_of_the_same_model(n):
+    """The list of each model's requests that mms_trace_next_same_model makes: models that are never
+    asked for, one that appears once, and requests of none."""
+    from mms_b200 import engine
+    rng = np.random.default_rng(n)
+    M = 7
+    ids = rng.choice([-1, 0, 1, 2, 5], size=n).astype(np.int32)
+    ids[n // 2] = 6
+    trace = engine.DeviceTrace(np.sort(rng.random(n)), ids, np.ones(n, np.float32), M)
+    want, last = np.full(n, -1, np.int32), {}
+    for i in range(n - 1, -1, -1):
+        if ids[i] >= 0:
+            want[i], last[ids[i]] = last.get(ids[i], -1), i
+    assert np.array_equal(trace.next_same_model().cpu().numpy()[:n], want)

@@ -274,11 +274,11 @@ def test_batching_kernel_golden(loaded, golden):
 
 
 @pytest.mark.parametrize("copies", [32, 45])
-def test_batching_kernel_golden_32_to_a_warp(loaded, golden, copies):
+def test_batching_kernel_golden_copies(loaded, golden, copies):
     """The same fixture (unknown models, a model without replica, +inf
-    latencies, replicated models) as a batch of identical candidates, which
-    takes the kernel that runs 32 candidates per warp: every copy — also in a
-    warp that is only partly filled — equals the reference's output."""
+    latencies, replicated models) as a batch of identical candidates, a warp
+    each: every copy — also in a block that is only partly filled — equals the
+    reference's output."""
     from mms_b200 import engine
     g = golden("kernel_batching")
     N = len(g["tstamps"])
