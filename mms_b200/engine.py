@@ -238,7 +238,8 @@ class PinnedStager:
     a stream of its own.  Pageable memory goes to the device at about a third
     of the rate of page-locked memory, whatever the number of threads that
     ask; staging by hand is what lets the threads help.  One instance per
-    device is kept (page-locked allocations are slow)."""
+    device is kept (page-locked allocations are slow); uploads from several
+    threads take turns, since they share its buffers."""
 
     _instances = {}
 
@@ -253,6 +254,7 @@ class PinnedStager:
         from concurrent.futures import ThreadPoolExecutor
         self.device, self.threads, self.piece = torch.device(dev), int(threads), int(piece_bytes)
         self.pool = ThreadPoolExecutor(self.threads)
+        self.turn = threading.Lock()
         # of high priority, which torch takes from a pool of their own: a stream that kernels are
         # queued on (torch has 32 per priority and hands them out in turn) would hold the copies up
         self.streams = [torch.cuda.Stream(device=self.device, priority=-1)
@@ -306,7 +308,8 @@ class PinnedStager:
                 if ev is not None:
                     ev.synchronize()
 
-        list(self.pool.map(work, [k for k in range(self.threads) if pieces[k]]))
+        with self.turn:
+            list(self.pool.map(work, [k for k in range(self.threads) if pieces[k]]))
         for k in range(self.threads):
             if pieces[k]:
                 main.wait_stream(self.streams[k])

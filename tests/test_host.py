@@ -581,3 +581,42 @@ def test_stream_handles_without_the_private_name(monkeypatch):
                         lambda device=None: SimpleNamespace(cuda_stream={0: 40, 1: 41}[device]))
     assert engine._raw_stream() == 40 and engine._raw_stream(1) == 41
     assert engine._stream_ptr().value == 40
+
+
+def test_uploads_from_two_threads_take_turns(monkeypatch):
+    """Two sweeps in two threads share a device's staging buffers: one's pieces must not be filled into a
+    buffer the other is still sending."""
+    import threading
+    import time
+    from contextlib import nullcontext
+    from types import SimpleNamespace
+
+    import torch
+    stream = SimpleNamespace(wait_stream=lambda other: None)
+    monkeypatch.setattr(torch.cuda, "Stream", lambda **kwargs: stream)
+    monkeypatch.setattr(torch.cuda, "Event", lambda: SimpleNamespace(record=lambda s: None,
+                                                                     synchronize=lambda: None))
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda device=None: stream)
+    for name in ("device", "stream"):
+        monkeypatch.setattr(torch.cuda, name, lambda x: nullcontext())
+    monkeypatch.setattr(torch.Tensor, "pin_memory", lambda self: self)
+    stager = engine.PinnedStager("cpu", 2, 64)
+    wrong = []
+
+    def user(value):
+        def fill(out, lo, hi):
+            out[:] = value
+            time.sleep(0.02 if lo == 0 else 0.0)         # the first thread is still at it, the second is free
+        for _ in range(4):
+            dst = torch.zeros(16, dtype=torch.int32)
+            other = torch.zeros(1, dtype=torch.int32)
+            stager.upload([(dst, engine.LazyArray(16, np.int32, fill)),
+                           (other, engine.LazyArray(1, np.int32, lambda out, lo, hi: out.fill(value)))])
+            if not (bool((dst == value).all()) and int(other) == value):
+                wrong.append(value)
+    threads = [threading.Thread(target=user, args=(v,)) for v in (1, 2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not wrong
